@@ -102,7 +102,7 @@ def draw(rng):
         return _emulated(None, R, _log_int(rng, 32, 8192 // R), 128 * rng.randint(2, 56), rng.randint(1, 6), E,
                          128 * rng.randint(1, 2), routing=rng.choice(["softmax", "zipf"]))  # fmt: skip
     E = rng.randint(4, 16)
-    S, H, K, inter = _log_int(rng, 32, 4096), 256 * rng.randint(2, 16), rng.randint(1, 4), 128 * rng.randint(2, 8)
+    S, H, K, inter = _log_int(rng, 32, 4096), 256 * rng.randint(2, 16), rng.randint(1, 4), 256 * rng.randint(1, 4)
     if kind == "layer":
         return _layer(None, S, H, K, E, inter, rng.random() < 0.5)
     return _block(None, min(S, 2048), min(H, 2048), K, E, inter)
