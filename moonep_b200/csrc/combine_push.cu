@@ -23,7 +23,7 @@
 // CTA order in a launch with all roles: FOLD/SUM CTAs first, PUSH CTAs last, so that the PUSH role only waits
 // for lower-numbered CTAs (which the hardware dispatches first) and the SUM role only for PUSH CTAs of this or
 // other GPUs; the grid never exceeds the number of SMs.  Emulated ranks that share one GPU launch the roles one
-// after the other.  With a single rank the FOLD role alone writes the results.
+// after the other.  A single rank has nothing to push: single_rank.cu.
 //
 // Parity: reference moonep_td/combine_prologue.py:19-40 and moonep_td/combine.py:22-68.
 #include <cstdlib>
@@ -67,7 +67,6 @@ struct PushArgs {
   uint16_t* fold_buf;       // [fold_rows, H] local: folded row of every duplicate group
   int* fold_flag;           // [fold_rows] local: COMB epoch of the combine that last folded the group
   int fold_rows;
-  int direct;               // single rank: FOLD writes the results straight into out / out_w
   int local_home;           // rows of this rank's own tokens go from FOLD straight into the local staging chunk
   int sum_two;              // SUM: a warp holds two tokens and sums the one that completes first
 };
@@ -147,8 +146,8 @@ __device__ __forceinline__ int group_rows(const MoonepDevCtx& c, const PushArgs&
 // ---- FOLD role ---------------------------------------------------------------------------------------
 
 // Duplicate groups are handed out from an atomic counter; a warp adds the rows of a group in fp32 (primary first,
-// then the duplicates in ascending k), rounds to bf16 and stores the row into fold_buf[g] (or, with a single rank,
-// straight into the token's output row), then releases fold_flag[g] for the PUSH role.
+// then the duplicates in ascending k), rounds to bf16 and stores the row into fold_buf[g], then releases fold_flag[g]
+// for the PUSH role.
 __device__ void fold_role(const MoonepDevCtx& c, const PushArgs& a) {
   const int lane = threadIdx.x & 31;
   const int NvS = c.NvS, K = c.K, H = c.H, S = c.S;
@@ -160,9 +159,9 @@ __device__ void fold_role(const MoonepDevCtx& c, const PushArgs& a) {
     if (ngroups > a.fold_rows) record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_COMBINE_PUSH, 10, ngroups, a.fold_rows, 0);
     ngroups = 0;
   }
-  // with a single rank this role also copies the rows that have no duplicates to the output; with local_home it
-  // copies those of this rank's own tokens into the local staging chunk (the PUSH role leaves them out)
-  const int nbatches = (a.direct || a.local_home) ? (NvS + kFoldRowBatch - 1) / kFoldRowBatch : 0;
+  // with local_home this role also copies the rows of this rank's own tokens that have no duplicates into the local
+  // staging chunk (the PUSH role leaves them out)
+  const int nbatches = a.local_home ? (NvS + kFoldRowBatch - 1) / kFoldRowBatch : 0;
   unsigned char* stage_local = a.local_home ? c.stage_peer[c.rank] : nullptr;
   for (;;) {
     int item = 0;
@@ -170,7 +169,7 @@ __device__ void fold_role(const MoonepDevCtx& c, const PushArgs& a) {
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= ngroups + nbatches) break;
     if (item >= ngroups) {
-      // single rank: rows without duplicates go to the output as they are
+      // rows without duplicates go to the staging chunk as they are
       const int base = (item - ngroups) * kFoldRowBatch;
       int si = -1, l = 0;
       if (lane < kFoldRowBatch && base + lane < NvS) {
@@ -186,26 +185,14 @@ __device__ void fold_role(const MoonepDevCtx& c, const PushArgs& a) {
         const int slot = p_si % NvS;
         if (slot >= S * K) continue;
         const int prow = base + j;
-        uint16_t* o = nullptr;
-        int* sflag = nullptr;
-        if (a.direct) {
-          o = a.out + (long long)(slot / K) * H;
-        } else {
-          // local_home: only the rows of this rank's own tokens; slot (token, position among the token's primaries)
-          const int ord = (p_l >> MOONEP_LINK_ORD_SHIFT) & MOONEP_LINK_ORD_MASK;
-          if (p_si / NvS != c.rank || ord >= c.kp) continue;
-          const long long stage_row = (long long)(slot / K) * c.kp + ord;
-          o = reinterpret_cast<uint16_t*>(stage_local + stage_row * row_bytes);
-          sflag = reinterpret_cast<int*>(stage_local + c.stage_flag_off) + stage_row;
-        }
+        // only the rows of this rank's own tokens; slot (token, position among the token's primaries)
+        const int ord = (p_l >> MOONEP_LINK_ORD_SHIFT) & MOONEP_LINK_ORD_MASK;
+        if (p_si / NvS != c.rank || ord >= c.kp) continue;
+        const long long stage_row = (long long)(slot / K) * c.kp + ord;
+        uint16_t* o = reinterpret_cast<uint16_t*>(stage_local + stage_row * row_bytes);
+        int* sflag = reinterpret_cast<int*>(stage_local + c.stage_flag_off) + stage_row;
         if (!wait_block_ready(c, a, prow, lane)) return;
-        if (a.in_w != nullptr && lane == 0) {
-          if (a.direct) {
-            if (a.out_w != nullptr) a.out_w[slot] = a.in_w[prow];
-          } else {
-            reinterpret_cast<float*>(stage_local + c.stage_w_off)[slot] = a.in_w[prow];
-          }
-        }
+        if (a.in_w != nullptr && lane == 0) reinterpret_cast<float*>(stage_local + c.stage_w_off)[slot] = a.in_w[prow];
         const uint16_t* src = a.in_rows + (long long)prow * H;
         if (a.vec_ok) {
           // kFoldVec loads in flight per lane: a plain load-store loop would run one 16-byte round trip at a time
@@ -228,12 +215,10 @@ __device__ void fold_role(const MoonepDevCtx& c, const PushArgs& a) {
         } else {
           for (int i = lane; i < H; i += 32) o[i] = src[i];
         }
-        if (sflag != nullptr) {
-          __syncwarp();
-          if (lane == 0) {
-            fence_gpu();
-            st_relaxed_gpu(sflag, epoch);
-          }
+        __syncwarp();
+        if (lane == 0) {
+          fence_gpu();
+          st_relaxed_gpu(sflag, epoch);
         }
       }
       continue;
@@ -264,26 +249,13 @@ __device__ void fold_role(const MoonepDevCtx& c, const PushArgs& a) {
         sflag = reinterpret_cast<int*>(stage_local + c.stage_flag_off) + stage_row;
       }
     }
-    if (!a.direct && a.in_w != nullptr && lane < n_rows) {
+    if (a.in_w != nullptr && lane < n_rows) {
       // gate weights of all entries of this group travel to the home rank's weight staging
       const int s_q = a.src_info[my_row];
       const int home = a.src_info[prow] / NvS;
       const int slot_q = s_q - home * NvS;
       if (s_q >= 0 && home >= 0 && home < c.R && slot_q >= 0 && slot_q < S * K)
         reinterpret_cast<float*>(c.stage_peer[home] + c.stage_w_off)[slot_q] = a.in_w[my_row];
-    }
-    if (a.direct) {
-      const int p_si = a.src_info[prow];
-      const int slot = p_si % NvS;
-      if (p_si < 0 || slot >= S * K) {
-        record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_COMBINE_PUSH, 8, p_si, prow, 0);
-        continue;
-      }
-      o = a.out + (long long)(slot / K) * H;
-      if (a.in_w != nullptr && a.out_w != nullptr && lane < n_rows) {
-        const int s_q = a.src_info[my_row];
-        if (s_q >= 0 && s_q % NvS < S * K) a.out_w[s_q % NvS] = a.in_w[my_row];
-      }
     }
     if (a.vec_ok) {
       const int nvec = H / 8;
@@ -337,7 +309,7 @@ __device__ void fold_role(const MoonepDevCtx& c, const PushArgs& a) {
       }
     }
     __syncwarp();
-    if (lane == 0 && !a.direct) {
+    if (lane == 0) {
       if (sflag != nullptr) {
         fence_gpu();  // row and weights are in this GPU's memory
         st_relaxed_gpu(sflag, epoch);
@@ -951,8 +923,7 @@ extern "C" long long moonep_stage_layout(int S, int K, int H, int kp, long long*
   return rows + flags + w;
 }
 
-// roles: MOONEP_ROLE_FOLD | MOONEP_ROLE_PUSH | MOONEP_ROLE_SUM (a single rank launches FOLD alone, which then writes the
-// results itself).  src_info / link: the plan's copies ([NvS] each); dup_groups / dup_loffs / dup_counts: the plan's
+// roles: MOONEP_ROLE_FOLD | MOONEP_ROLE_PUSH | MOONEP_ROLE_SUM.  src_info / link: the plan's copies ([NvS] each); dup_groups / dup_loffs / dup_counts: the plan's
 // duplicate map.  in_rows: the local expert output rows [NvS, H] (the shard or any other local tensor), in_w: their gate
 // weights [NvS] or null.  fold_buf [fold_rows, H] bf16 and fold_flag [fold_rows] int32 (zero-initialised once) are
 // local scratch of the Buffer; fold_rows bounds the number of duplicate groups.  ready / ready_expect: optional
@@ -966,8 +937,7 @@ extern "C" int moonep_combine_push(void* ctx, int roles, const int* src_info, co
   const MoonepDevCtx& c = h->dev;
   const int local_home = ((roles & MOONEP_ROLE_LOCAL_HOME) && c.R > 1 && c.stage_peer != nullptr) ? 1 : 0;
   roles &= ~MOONEP_ROLE_LOCAL_HOME;
-  const int direct = (c.R == 1 && roles == MOONEP_ROLE_FOLD) ? 1 : 0;
-  if (c.stage_peer == nullptr && !direct) {
+  if (c.stage_peer == nullptr) {
     set_error("moonep_combine_push: this Buffer has no combine staging memory");
     return 1;
   }
@@ -991,7 +961,6 @@ extern "C" int moonep_combine_push(void* ctx, int roles, const int* src_info, co
   a.fold_buf = (uint16_t*)fold_buf;
   a.fold_flag = fold_flag;
   a.fold_rows = fold_rows;
-  a.direct = direct;
   a.local_home = local_home;
   {
     const char* st = getenv("MOONEP_SUM_SLOTS");  // 2: a SUM warp holds two tokens (default 1)

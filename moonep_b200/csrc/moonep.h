@@ -72,7 +72,7 @@
 #define MOONEP_CTR_PLAN_DONE 19      // PLAN epoch of the last finished token stage
 #define MOONEP_CTR_PLAN_ARRIVE 20    // CTAs that finished the token stage
 #define MOONEP_CTR_SEND_ARRIVE 21    // CTAs that finished the send role
-#define MOONEP_CTR_DISPATCH_ARRIVE 22  // CTAs of the dispatch kernel that reached its end
+#define MOONEP_CTR_DISPATCH_ARRIVE 22  // CTAs of the single-rank dispatch kernel that reached its end
 #define MOONEP_CTR_PUSH_WORK 23      // row hand-out of the combine push role
 #define MOONEP_CTR_SUM_WORK 24       // token hand-out of the combine sum role
 #define MOONEP_CTR_COMBINE_ARRIVE 25 // CTAs of the push-combine kernel that reached its end
@@ -214,6 +214,19 @@ int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk, const int*
                     int with_weights, int* dup_groups, int* dup_loffs, int* dup_counts, int* plan_src_info,
                     int* plan_link, int wait_family, int wait_epoch, int epoch_tpe, int epoch_plan, int epoch_sent,
                     int path, int n_send, int n_expand, int build_only, const int* tpe_row, void* stream);
+
+// Dispatch of a Buffer with one rank: one launch, fresh (planner arguments as above, tpe [E]) or replayed (dst and
+// zero_fill come from the plan).  n_ctas bounds the grid (<= 0: every SM of local_sms).  Fresh plans need
+// moonep_single_supported(E, S, K).  See single_rank.cu.
+int moonep_single_supported(int E, int S, int K);
+int moonep_dispatch_single(void* ctx, int fresh, const int* topk, const int* tpe, int* dst, int* cu_seqlens,
+                           int* experts_to_copy, int* zero_fill, int* remote_stats, int* dup_groups, int* dup_loffs,
+                           int* dup_counts, int* plan_src_info, int* plan_link, const void* hidden, const float* weights,
+                           int with_weights, int epoch_tpe, int epoch_plan, int epoch_sent, int n_ctas, void* stream);
+// Combine of a Buffer with one rank: out[token] = the sum of the token's rows in ascending k (fp32, rounded once),
+// out_w[token, k] = in_w of the entry's row.  ready / ready_expect as in moonep_combine_push.
+int moonep_combine_single(void* ctx, const int* dst, const void* in_rows, const float* in_w, void* out, float* out_w,
+                          const int* ready, int ready_expect, void* stream);
 
 // Combine.
 int moonep_combine_prologue(void* ctx, const int* dup_groups, const int* dup_loffs, const int* dup_counts,

@@ -106,6 +106,8 @@ class CudaBackend:
         # Emulated ranks share one GPU and one stream: a kernel of one rank must never wait for a kernel of another
         # rank that is launched later, so they run the dispatch and combine kernels one role per phase.
         self.phased = (bool(getattr(world, "emulated", False)) and world.size > 1) or config.force_phased()
+        # one rank: dispatch and combine are kernels of their own (csrc/single_rank.cu)
+        self.single = R == 1 and bool(self.lib.moonep_single_supported(E, S, K)) and not self.phased
         self.combine_mode = config.combine_mode()
         self.n_expand = 0  # CTAs of the dispatch kernel's destination-side role; 0 = every SM the senders leave free
 
@@ -368,6 +370,10 @@ class CudaBackend:
         with_w = route_weights_sk is not None
         self._sent_weights = with_w
         lr = ROLE_LOCAL_ROWS if config.local_rows_by_expand() else 0
+        if self.single and lr and (planning_args is None or config.planner_on_gpu()):
+            self._dispatch_single(hidden_sh, route_weights_sk, plan, planning_args)
+            self._quiesced = True
+            return
         if planning_args is not None:
             topk_flat, tpe, cu_seqlens = planning_args
             on_dev = config.planner_on_gpu()
@@ -418,6 +424,21 @@ class CudaBackend:
                 self._dispatch_launch(ROLE_EXPAND | lr, False, plan, tag="dispatch_expand", **kw)
         self.world.step()
 
+    def _dispatch_single(self, hidden, weights, plan, planning_args):
+        """Fresh or replayed dispatch of a single rank: one launch, no READY round (there are no peers to wait for)."""
+        topk, tpe, cu = planning_args if planning_args is not None else (None, None, None)
+        if topk is not None:
+            self._topk = topk
+            self._next(FLAG_TPE)
+            self._next(FLAG_PLAN)
+        self._call(
+            "moonep_dispatch_single", int(topk is not None), _ptr(topk), _ptr(tpe), _ptr(plan.dst), _ptr(cu),
+            _ptr(plan.experts_to_copy), _ptr(plan.zero_fill_ranges), _ptr(plan.remote_stats), _ptr(plan.dup_groups),
+            _ptr(plan.dup_loffs), _ptr(plan.dup_counts), _ptr(plan.src_info), _ptr(plan.link), _ptr(hidden), _ptr(weights),
+            int(weights is not None), self._cur(FLAG_TPE), self._cur(FLAG_PLAN), self._next(FLAG_SENT), self.n_expand,
+            _stream(), tag="dispatch_single",
+        )  # fmt: skip
+
     def copy_out(self, out_hidden, out_weights):
         out_hidden.copy_(self.ctx["hidden_buf_local"])
         if out_weights is not None:
@@ -464,7 +485,7 @@ class CudaBackend:
         wf, we = -1, 0
         # A round of READY flags keeps a rank from overwriting staging rows (or shard rows) a peer still reads from
         # the previous combine; a dispatch that waited for all peers since then already gives that guarantee.
-        if inter_rank_sync and not self._quiesced:
+        if inter_rank_sync and not self._quiesced and self.ctx["R"] > 1:
             self.signal(FLAG_READY)
             wf, we = FLAG_READY, self._cur(FLAG_READY)
         if not self.can_push(plan):
@@ -472,6 +493,10 @@ class CudaBackend:
             self.combine_pull(plan.dst, out_hidden, out_weights_sk)
             return
         self._quiesced = False
+        if self.ctx["R"] == 1:  # nothing to stage or fold: the rows of a token are summed where they are
+            self._call("moonep_combine_single", _ptr(plan.dst), _ptr(hidden_nvsh), _ptr(route_weights_nvs), _ptr(out_hidden),
+                       _ptr(out_weights_sk), _ptr(ready), int(ready_expect), _stream(), tag="combine_single")  # fmt: skip
+            return
         comb = self._next(FLAG_COMB)
         lh = ROLE_LOCAL_HOME if config.local_home_by_fold() else 0
         fold_buf, fold_flag = self._fold_scratch()
@@ -479,9 +504,7 @@ class CudaBackend:
                 _ptr(out_hidden), _ptr(out_weights_sk), wf, we, comb, _ptr(ready), int(ready_expect),
                 _ptr(plan.dup_groups), _ptr(plan.dup_loffs), _ptr(plan.dup_counts), _ptr(fold_buf), _ptr(fold_flag),
                 int(fold_flag.numel()), 0, 0, _stream())  # fmt: skip
-        if self.ctx["R"] == 1:  # nothing to stage: the fold role writes the results itself
-            self._call("moonep_combine_push", ROLE_FOLD, *args, tag="combine_fold")
-        elif not self.phased:
+        if not self.phased:
             self._call("moonep_combine_push", ROLE_FOLD | ROLE_PUSH | ROLE_SUM | lh, *args, tag="combine_fused")
         else:
             self._call("moonep_combine_push", ROLE_FOLD | lh, *args, tag="combine_fold")
@@ -492,13 +515,12 @@ class CudaBackend:
 
     def _fold_scratch(self):
         """Local scratch of the push combine: one folded row and one flag per duplicate group (a group has at least two
-        rows of the shard, so there are at most NvS/2 of them).  A single rank folds straight into the output."""
+        rows of the shard, so there are at most NvS/2 of them)."""
         if getattr(self, "_fold", None) is None:
             c = self.ctx
-            rows = 1 if c["R"] == 1 else c["NvS"] // 2 + 1
-            dev = c["device"]
+            rows, dev = c["NvS"] // 2 + 1, c["device"]
             self._fold = (torch.empty(rows, c["H"], dtype=torch.bfloat16, device=dev),
-                          torch.zeros(c["NvS"] // 2 + 1, dtype=torch.int32, device=dev))  # fmt: skip
+                          torch.zeros(rows, dtype=torch.int32, device=dev))  # fmt: skip
         return self._fold
 
     def combine_prologue(self, plan, hidden_nvsh, route_weights_nvs, zero_copy, wait=None):

@@ -1,0 +1,91 @@
+"""Dispatch and combine kernels of a single rank (csrc/single_rank.cu) at the edges of their tiling, against the host
+planner and the two-rounding model: pieces of rows, tokens per CTA, steps of 512 entries, lists of 1024 groups, rows and
+routing that are not 16-byte aligned, replayed plans, token counts that do not match the routing."""
+
+import pytest
+import torch
+
+from moonep_b200 import Buffer
+from moonep_b200.errors import MoonEPIndexError
+from tests.harness import Case, assert_within_ulp, check_dispatch_records, expected_combine, run_round_trip
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    Case("one_token_many_pads", S=1, K=1, epn=3, H=8, token_padding=128, routing="single_expert"),
+    Case("fewer_tokens_than_ctas", S=147, K=3, epn=5, H=264, token_padding=16, routing="biased"),
+    Case("one_cta_with_one_token", S=149, K=2, epn=8, H=4104, token_padding=1, routing="softmax"),
+    Case("three_pieces_per_row", S=40, K=4, epn=6, H=8200, token_padding=32, routing="zipf"),
+    Case("several_steps_per_cta", S=12000, K=8, epn=16, H=64, token_padding=64, routing="zipf"),
+    Case("step_of_16_tokens", S=300, K=32, epn=40, H=32, token_padding=8, routing="softmax"),
+    Case("two_lists_of_groups", S=700, K=2, epn=1100, H=16, token_padding=4, routing="softmax", B=1),
+    Case("rows_of_40_bytes", S=333, K=5, epn=7, H=20, token_padding=16, routing="biased"),
+    Case("odd_rows", S=50, K=2, epn=4, H=13, token_padding=4, routing="softmax"),
+]
+
+
+@pytest.mark.parametrize("zero_copy", [False, True])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: c.name)
+def test_single_rank_round_trip(case, zero_copy):
+    recs = run_round_trip(case, 1, "cuda", zero_copy=zero_copy,
+                          expert_scale=lambda rec, r, E: (torch.arange(rec["hidden_nvsh"].shape[0]) % 5 + 1).float())  # fmt: skip
+    _, dst_pos, _, _ = check_dispatch_records(case, 1, recs)
+    scale = [(torch.arange(recs[0]["layout"]["NvS"]) % 5 + 1).float()]
+    want = expected_combine(case, 1, recs, dst_pos, scale)
+    assert_within_ulp(recs[0]["out"], want[0], max_ulps=1, what="combine")
+    assert torch.equal(recs[0]["weights_back"], recs[0]["w"])
+
+
+def _inputs(S, H, K, E, shift):
+    """Routing and rows that start ``shift`` elements into their storage (contiguous, not 16-byte aligned)."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    topk = torch.rand(S, E, generator=g, device="cuda").topk(K, dim=1).indices.to(torch.int32)
+    topk = torch.empty(S * K + shift, dtype=torch.int32, device="cuda")[shift:].view(S, K).copy_(topk)
+    x = torch.empty(S * H + shift, dtype=torch.bfloat16, device="cuda")[shift:].view(S, H)
+    x.copy_(torch.randn(S, H, generator=g, device="cuda"))
+    return x, topk, torch.bincount(topk.flatten().long(), minlength=E).to(torch.int32)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 4])
+@pytest.mark.parametrize("S,H,K,E,pad", [(1, 64, 2, 4, 8), (500, 520, 3, 9, 16), (3000, 64, 6, 12, 1)])
+def test_replay_and_unaligned_inputs(S, H, K, E, pad, shift):
+    buf = Buffer(S, H, K, E, 1, token_padding=pad)
+    x, topk, tpe = _inputs(S, H, K, E, shift)
+    gates = torch.rand(S, K, device="cuda")
+    rows, _, cu, plan = buf.dispatch(x, gates, topk, tpe)
+    x2 = torch.empty_like(x).copy_(-x)
+    buf._require_ctx()["hidden_buf_local"].fill_(7.0)
+    rows2, w2, _, _ = buf.dispatch(x2, gates, plan=plan, zero_copy=True)
+    loff = torch.where(plan.dst < 0, -plan.dst - 1, plan.dst).long()
+    end = int(cu[-1])
+    assert torch.equal(rows[loff], x.repeat_interleave(K, 0)) and torch.equal(rows2[loff], x2.repeat_interleave(K, 0))
+    pads = torch.ones(end, dtype=torch.bool, device="cuda")
+    pads[loff] = False
+    assert not bool(rows2[:end][pads].any()) and torch.equal(w2[loff], gates.flatten())
+    y = torch.randn(buf._require_ctx()["NvS"], H, device="cuda").to(torch.bfloat16)
+    out, back, _ = buf.combine(plan, y, w2.clone())
+    want = torch.zeros(S, H, device="cuda")
+    for k in range(K):  # the kernel's order: fp32, ascending k, rounded once
+        want += y[loff.view(S, K)[:, k]].float()
+    assert torch.equal(out, want.to(torch.bfloat16)) and torch.equal(back, gates)
+    buf.synchronize()
+    buf.destroy()
+
+
+def test_counts_that_do_not_match_the_routing():
+    """More rows counted than routed: the rows nothing lands in are marked unused.  Fewer, or an expert that does not
+    exist: an index error, and the Buffer works again afterwards."""
+    S, H, K, E = 200, 64, 2, 6
+    buf = Buffer(S, H, K, E, 1, token_padding=8)
+    x, topk, tpe = _inputs(S, H, K, E, 0)
+    plan = buf.dispatch(x, None, topk, tpe + torch.tensor([0, 3, 0, 0, 0, 1], dtype=torch.int32, device="cuda"))[3]
+    buf.synchronize()
+    assert int((plan.src_info >= 0).sum()) == S * K
+    for bad_topk, bad_tpe in ((topk, tpe - (tpe > 0).int()), (torch.where(topk == 2, E, topk), tpe)):
+        buf.dispatch(x, None, bad_topk.contiguous(), bad_tpe)
+        with pytest.raises(MoonEPIndexError):
+            buf.synchronize()
+    rows, _, _, plan = buf.dispatch(x, None, topk, tpe)
+    buf.synchronize()
+    assert torch.equal(buf.combine(plan, rows)[0], (x.float() * K).to(torch.bfloat16))
+    buf.destroy()
