@@ -7,10 +7,12 @@
 // dispatch at S=4096, H=7168, K=8, E=256 before most rows were written, and 65 of 84 us at S=16.  Here
 //
 //   dispatch   one launch whose CTAs wait for nobody.  Every CTA derives the whole group layout itself (E counts, one
-//              prefix sum), starts clearing its share of the pad rows with asynchronous bulk stores, counts the
-//              routing entries before its own contiguous range of tokens, gives its entries their rows, and streams
-//              its tokens through shared memory: one bulk load and K bulk stores per piece of a row.  The pad rows'
-//              stores (a third of the bytes at the size above) drain while the CTA plans.
+//              prefix sum).  Four warps clear pad rows with bulk stores from a piece of zeros, handed out from one
+//              counter; the others count the routing entries before the CTA's own contiguous range of tokens, give its
+//              entries their rows and publish "planned"; then four of them stream tokens through shared memory, one
+//              bulk load and K bulk stores per row.  A CTA that is done with its tokens takes rows over from CTAs that
+//              have planned theirs: SMs reach HBM at rates that differ by a quarter, and with a fixed share per SM the
+//              kernel took 138 (426) us at S=4096 (16384) where its average CTA was done after 117 (363); now 131 (400).
 //   combine    a warp per 512-byte piece of an output row, straight from the token's K destinations: no work counter,
 //              no lists.
 //
@@ -28,15 +30,24 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kCopyWarps = 8;     // warps that stream tokens, each through a ring of its own
-constexpr int kRing = 3;          // pieces per ring: two loads run ahead of the stores
-constexpr int kMaxPiece = 8192;   // bytes: 8 warps x 3 x 7 KB in flight at H=7168
-constexpr int kEntries = 512;     // routing entries planned at a time (whole tokens)
-constexpr int kPadGroups = 1024;  // groups whose pad rows are listed in shared memory at a time
-constexpr int kMaxExperts = 4096; // three words of shared memory per expert
+constexpr int kRing = 3;           // stages per ring: two loads run ahead of the stores
+constexpr int kMaxStage = 16384;   // bytes
+constexpr int kZeroBytes = 8192;
+constexpr int kPlanWarps = 12;     // warps 0..11 plan, then up to kCopyWarps of them copy; warps 12..15 clear pad rows
+// 4 with 14 KB rows, whose rings fill shared memory.  With more than 6 warps the stores an SM has queued outweigh what
+// they hide: 12 warps took 28 us where 6 take 22 at S=1777, H=2056, K=5; 3 warps took 102 us where 6 take 97 at S=8192,
+// H=4096, K=6.
+constexpr int kCopyWarps = 6;
+constexpr int kEntries = kPlanWarps * 32;  // routing entries planned at a time (whole tokens)
+constexpr int kUnits = 64;         // units remembered per copy warp: those loaded and those not flagged yet
+constexpr int kGrabs = 64;         // grabs of pad rows remembered per warp
+constexpr int kMaxGroups = 4096;   // experts, and prefetch slots: up to four words of shared memory each
 // Every CTA reads the routing before its own tokens: at 32 K entries that is 3 us for the last CTA, at 256 K about
 // 25 us, where the general kernel's per-block histograms are the better way.
 constexpr int kMaxEntries = 1 << 18;
+// work[]: pad rows handed out, then per CTA the tokens handed out, then per CTA the epoch at which its tokens were planned
+constexpr int kMaxCtas = 256;
+constexpr int kWorkPads = 0, kWorkNext = 1, kWorkReady = kWorkNext + kMaxCtas;
 
 struct SingleArgs {
   // planner (fresh plans)
@@ -59,18 +70,32 @@ struct SingleArgs {
   int topk_vec;  // topk can be read 16 bytes at a time
   int vec_ok;    // rows can be moved 16 bytes at a time
   int bulk;      // rows go through shared memory with bulk copies
-  int piece_bytes, npieces;
+  int stage_bytes, npieces;  // a row is moved in npieces pieces of at most stage_bytes
+  int copy_warps;            // warps that stream rows, each through a ring of its own
+  int tokens_per_unit;       // whole rows that share a stage (npieces == 1)
+  int pads_per_grab;
   int tokens_per_cta;
+  int* work;
   int epoch_tpe, epoch_plan, epoch_sent;
+};
+
+// What a copy warp moves at a time: rows [tok, tok + ntok) of the input, or bytes [off, off + len) of one row.
+struct Unit {
+  int tok, ntok;
+  unsigned off, len;
 };
 
 struct SingleShared {
   unsigned long long bar[kCopyWarps * kRing];
+  Unit unit[kCopyWarps][kUnits];
   int warp_sum[kWarps];
-  int pad_start[kPadGroups], pad_cum[kPadGroups];
+  int grab[kWarps - kPlanWarps][kGrabs];
   int loff[kEntries];  // destination row of every entry in hand, -1: none
   int bad;             // entries in hand without a row
+  int last;
 };
+
+__device__ __forceinline__ void plan_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kPlanWarps * 32) : "memory"); }
 
 // Inclusive prefix sum over the threads of the CTA; all threads call it.
 __device__ __forceinline__ int block_scan(int v, int* warp_sum, int& total) {
@@ -96,64 +121,59 @@ __device__ __forceinline__ int block_scan(int v, int* warp_sum, int& total) {
 
 __device__ __forceinline__ int padded_rows(int cnt, int P) { return cnt > 0 ? ((cnt + P - 1) / P) * P : 0; }
 
-// Visits this CTA's pad rows.  flag == false: clears them (bulk stores from `zeros`, not waited for) with their weights
-// and, for a fresh plan, marks them unused in src_info and the plan's copies; flag == true: releases their row flags.
-__device__ void visit_pads(const MoonepDevCtx& c, const SingleArgs& a, SingleShared& s, const int* cnt, const int* off,
-                           const unsigned char* zeros, uint16_t* shard, int* meta, int epoch, bool flag) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int groups = a.fresh ? c.E : c.E + c.B;  // the prefetch slots of a single rank are empty
-  const long long row_bytes = (long long)c.H * 2;
-  if (!a.fresh && a.zero_fill == nullptr) return;
-  for (int g0 = 0; g0 < groups; g0 += kPadGroups) {
-    const int n = min(kPadGroups, groups - g0);
-    if (!flag || groups > kPadGroups) {  // one list only: the flag pass finds it as the first pass left it
-      int carry = 0;
-      for (int i0 = 0; i0 < n; i0 += kThreads) {
-        const int i = i0 + threadIdx.x;
-        int first = 0, rows = 0;
-        if (i < n) {
-          if (a.fresh) {
-            const int k = cnt[g0 + i];
-            first = off[g0 + i] + k;
-            rows = k > 0 ? padded_rows(k, c.token_padding) - k : 0;
-          } else {
-            first = a.zero_fill[2 * (g0 + i)];
-            rows = max(0, a.zero_fill[2 * (g0 + i) + 1]);
-          }
-        }
-        int total;
-        const int incl = block_scan(rows, s.warp_sum, total);
-        if (i < n) {
-          s.pad_start[i] = first;
-          s.pad_cum[i] = carry + incl;
-        }
-        carry += total;
-      }
-      __syncthreads();
+// Group layout in shared memory: cnt/off of every expert (fresh plans) and the running total of pad rows per group.
+struct Layout {
+  const int* first;  // replay: first pad row of a group
+  const int* cnt;    // fresh
+  const int* off;    // fresh
+  const int* cum;    // inclusive running total of pad rows
+  int groups;
+  __device__ int pad_row(int j) const {
+    int lo = 0, hi = groups - 1;  // first group whose running total exceeds j
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (cum[mid] > j) hi = mid; else lo = mid + 1;
     }
-    const int total = s.pad_cum[n - 1];
-    auto row_of = [&](int j) {  // pad row j of the list, -1 when out of range
-      int lo = 0, hi = n - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (s.pad_cum[mid] > j) hi = mid; else lo = mid + 1;
-      }
-      const int row = s.pad_start[lo] + (j - (lo > 0 ? s.pad_cum[lo - 1] : 0));
-      return row >= 0 && row < c.NvS ? row : -1;
-    };
-    // a thread per row; with bulk copies not a thread of the copy warps, whose rings would wait behind the clears
-    const int first = a.bulk ? kCopyWarps * 32 : 0, nthr = kThreads - first;
-    for (int j = blockIdx.x + gridDim.x * ((int)threadIdx.x - first); j >= 0 && j < total; j += gridDim.x * nthr) {
-      const int row = row_of(j);
-      if (row < 0) continue;
-      if (flag) {
-        st_relaxed_gpu(meta + c.rowflag_off + row, epoch);
-        continue;
-      }
+    const int start = cnt != nullptr ? off[lo] + cnt[lo] : first[lo];
+    return start + (j - (lo > 0 ? cum[lo - 1] : 0));
+  }
+};
+
+// Warps kPlanWarps.. : clear pad rows (and their weights), mark them unused in a fresh plan.  Rows are handed out from
+// one counter, pads_per_grab at a time, a lane per row.  Their row flags are released at the end, behind one wait and one
+// fence: a fence per grab held the clears of S=128, H=7168, E=256 (31 K pad rows) to 5.3 TB/s.
+__device__ void clear_pads(const MoonepDevCtx& c, const SingleArgs& a, const Layout& lay, int* grabs,
+                           const unsigned char* zeros, uint16_t* shard, int* meta, int epoch) {
+  const int lane = threadIdx.x & 31;
+  const long long row_bytes = (long long)c.H * 2;
+  const int total = lay.groups > 0 ? lay.cum[lay.groups - 1] : 0;
+  auto row_of = [&](int j) {
+    const int row = lane < a.pads_per_grab && j + lane < total ? lay.pad_row(j + lane) : -1;
+    return row < c.NvS ? row : -1;
+  };
+  int held = 0;
+  auto flag_all = [&]() {
+    bulk_wait<0>();
+    fence_gpu();
+    __syncwarp();
+    for (int q = 0; q < held; ++q) {
+      const int row = row_of(grabs[q]);
+      if (row >= 0) st_relaxed_gpu(meta + c.rowflag_off + row, epoch);
+    }
+    held = 0;
+    __syncwarp();
+  };
+  for (;;) {
+    int j = 0;
+    if (lane == 0) j = atomicAdd(a.work + kWorkPads, a.pads_per_grab);
+    j = __shfl_sync(0xffffffffu, j, 0);
+    if (j >= total) break;
+    const int row = row_of(j);
+    if (row >= 0) {
       if (a.bulk) {
         unsigned char* p = reinterpret_cast<unsigned char*>(shard) + row * row_bytes;
-        for (long long o = 0; o < row_bytes; o += a.piece_bytes)
-          bulk_s2g(p + o, zeros, (unsigned)min((long long)a.piece_bytes, row_bytes - o));
+        for (long long o = 0; o < row_bytes; o += kZeroBytes)
+          bulk_s2g(p + o, zeros, (unsigned)min((long long)kZeroBytes, row_bytes - o));
       }
       if (a.with_weights) reinterpret_cast<float*>(meta + c.weights_off)[row] = 0.f;
       if (a.fresh) {
@@ -162,123 +182,338 @@ __device__ void visit_pads(const MoonepDevCtx& c, const SingleArgs& a, SingleSha
         if (a.plan_link != nullptr) a.plan_link[row] = 0;
       }
     }
-    if (!flag) {
-      if (a.bulk) {
-        bulk_commit();
-      } else {
-        for (int j = blockIdx.x + gridDim.x * warp; j < total; j += gridDim.x * kWarps) {  // a warp per row
-          const int row = row_of(j);
-          if (row < 0) continue;
-          uint16_t* p = shard + (long long)row * c.H;
-          if (a.vec_ok) {
-            for (int i = lane; i < c.H / 8; i += 32) st16(reinterpret_cast<int4*>(p) + i, make_int4(0, 0, 0, 0));
-          } else {
-            for (int i = lane; i < c.H; i += 32) p[i] = 0;
-          }
+    bulk_commit();
+    bulk_wait_read<3>();  // what an SM has queued stays small, so that the rows go to the SMs that are fastest
+    if (!a.bulk) {
+      for (int q = 0; q < a.pads_per_grab; ++q) {  // a warp per row
+        const int r = __shfl_sync(0xffffffffu, row, q);
+        if (r < 0) continue;
+        uint16_t* p = shard + (long long)r * c.H;
+        if (a.vec_ok) {
+          for (int i = lane; i < c.H / 8; i += 32) st16(reinterpret_cast<int4*>(p) + i, make_int4(0, 0, 0, 0));
+        } else {
+          for (int i = lane; i < c.H; i += 32) p[i] = 0;
         }
       }
+      fence_gpu();  // other lanes' stores precede the flag that lane q releases
     }
-    __syncthreads();  // the lists are rewritten for the next groups
+    if (lane == 0) grabs[held] = j;
+    __syncwarp();
+    if (++held == kGrabs) flag_all();
   }
+  flag_all();
 }
 
-// What one warp's ring holds.
-struct Ring {
-  unsigned char* stage;
-  unsigned long long* bar;
-  int loaded, stored;
+// Hands out units to a copy warp: those of its own CTA, then, from CTAs whose tokens are planned, whatever is left.
+struct Units {
+  const MoonepDevCtx& c;
+  const SingleArgs& a;
+  const int epoch;
+  int tok, piece;  // a row moved in several pieces: the piece that comes next
+  int state;  // 0: the unit that is this warp's from the start, 1: more of the own CTA's, 2: other CTAs'
+
+  __device__ int count_of(int cta) const { return max(0, min(c.S - cta * a.tokens_per_cta, a.tokens_per_cta)); }
+  // tokens of a CTA that are dealt to its warps without the counter
+  __device__ int dealt() const { return a.copy_warps * a.tokens_per_unit; }
+
+  __device__ bool take(int cta, Unit& u) {
+    int g = 0;
+    if ((threadIdx.x & 31) == 0) g = dealt() + atomicAdd(a.work + kWorkNext + cta, a.tokens_per_unit);
+    return unit_at(cta, __shfl_sync(0xffffffffu, g, 0), u);
+  }
+
+  __device__ bool unit_at(int cta, int g, Unit& u) {
+    const int n = count_of(cta);
+    if (g >= n) return false;
+    const long long row_bytes = (long long)c.H * 2;
+    u.tok = cta * a.tokens_per_cta + g;
+    u.ntok = min(a.tokens_per_unit, n - g);
+    u.off = 0;
+    u.len = a.npieces > 1 ? a.stage_bytes : (unsigned)(u.ntok * row_bytes);
+    tok = u.tok;
+    piece = 1;
+    return true;
+  }
+
+  __device__ bool next(Unit& u) {
+    const int lane = threadIdx.x & 31;
+    if (piece < a.npieces) {
+      u.tok = tok;
+      u.ntok = 1;
+      u.off = (unsigned)(piece * a.stage_bytes);
+      u.len = min((unsigned)a.stage_bytes, (unsigned)(c.H * 2) - u.off);
+      ++piece;
+      return true;
+    }
+    if (state == 0) {
+      state = 1;
+      if (unit_at(blockIdx.x, (int)(threadIdx.x >> 5) * a.tokens_per_unit, u)) return true;
+    }
+    if (a.tokens_per_cta <= dealt()) return false;  // nothing beyond what was dealt, here or elsewhere
+    if (state == 1) {
+      if (take(blockIdx.x, u)) return true;
+      state = 2;
+    }
+    for (;;) {
+      int left[kMaxCtas / 32], ready[kMaxCtas / 32];
+#pragma unroll
+      for (int i = 0; i < kMaxCtas / 32; ++i) {  // independent loads, all in flight together
+        const int v = i * 32 + lane;
+        left[i] = 0;
+        ready[i] = epoch;
+        if (v < (int)gridDim.x) {
+          left[i] = count_of(v) - dealt() - ld_volatile(a.work + kWorkNext + v);
+          if (a.fresh) ready[i] = ld_volatile(a.work + kWorkReady + v);
+        }
+      }
+      int most = 0, victim = -1;  // the CTA with the most tokens left; among equals another one for every thief
+#pragma unroll
+      for (int i = 0; i < kMaxCtas / 32; ++i)
+        if (left[i] > most && ready[i] - epoch >= 0) {
+          most = left[i];
+          victim = i * 32 + lane;
+        }
+      const int best = __reduce_max_sync(0xffffffffu, most);
+      if (best <= 0) return false;
+      const unsigned cand = __ballot_sync(0xffffffffu, most == best);
+      const unsigned after = cand & ~((2u << (blockIdx.x & 31)) - 1u);
+      victim = __shfl_sync(0xffffffffu, victim, __ffs(after ? after : cand) - 1);
+      if (a.fresh) ld_acquire_gpu(a.work + kWorkReady + victim);  // what it planned is visible from here on
+      if (take(victim, u)) return true;
+    }
+  }
 };
 
-// Copies the rows of `ntok` tokens (first: t0) to the rows in s.loff.  Pieces of rows are dealt to the copy warps; a
-// lane per destination stores, so the K stores of a piece are issued together.  The last stores are left in flight.
-__device__ bool copy_bulk(const MoonepDevCtx& c, const SingleArgs& a, const SingleShared& s, int t0, int ntok, Ring& r,
-                          unsigned char* shard) {
+// A copy warp: units go global -> shared -> their K destination rows; a lane per (row, destination) issues the store.
+// Row flags are released at the end, or when the list of units is full, behind one wait and one fence.
+__device__ bool copy_bulk(const MoonepDevCtx& c, const SingleArgs& a, SingleShared& s, unsigned char* stages,
+                          unsigned char* shard, int* meta, int epoch) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long row_bytes = (long long)c.H * 2;
-  const int items = ntok * a.npieces;
-  const int mine = warp < items ? (items - warp + kCopyWarps - 1) / kCopyWarps : 0;
-  auto load = [&](int n) {
-    const int item = warp + n * kCopyWarps;
-    const int tok = item / a.npieces, p = item - tok * a.npieces;
-    const int q = r.loaded % kRing;
+  const int K = c.K, NvS = c.NvS;
+  unsigned char* ring = stages + (size_t)warp * kRing * a.stage_bytes;
+  unsigned long long* bar = s.bar + warp * kRing;
+  Unit* units = s.unit[warp];
+  Units from = {c, a, epoch, 0, a.npieces, 0};
+  int loaded = 0, stored = 0;
+  auto load = [&]() {
+    Unit u;
+    if (!from.next(u)) return false;
     if (lane == 0) {
-      const long long o = (long long)p * a.piece_bytes;
-      const unsigned len = (unsigned)min((long long)a.piece_bytes, row_bytes - o);
-      mbar_expect_tx(r.bar + q, len);
-      bulk_g2s(r.stage + (size_t)q * a.piece_bytes,
-               reinterpret_cast<const unsigned char*>(a.hidden) + (t0 + tok) * row_bytes + o, len, r.bar + q);
+      units[loaded % kUnits] = u;
+      const int q = loaded % kRing;
+      mbar_expect_tx(bar + q, u.len);
+      bulk_g2s(ring + (size_t)q * a.stage_bytes, reinterpret_cast<const unsigned char*>(a.hidden) + u.tok * row_bytes + u.off,
+               u.len, bar + q);
     }
-    ++r.loaded;
-  };
-  int ahead = 0;
-  if (mine > 0) {
-    bulk_wait_read<0>();  // every stage has been read by the stores of the tokens before
     __syncwarp();
-    for (; ahead < min(mine, kRing - 1); ++ahead) load(ahead);
-  }
-  for (int n = 0; n < mine; ++n) {
-    const int item = warp + n * kCopyWarps;
-    const int tok = item / a.npieces, p = item - tok * a.npieces;
-    const int loff = lane < c.K ? s.loff[tok * c.K + lane] : -1;
-    const int q = r.stored % kRing;
-    const bool got = mbar_wait(r.bar + q, (unsigned)((r.stored / kRing) & 1), c.timeout_ns);
+    ++loaded;
+    return true;
+  };
+  auto row_of = [&](const Unit& u, int e) {
+    const int d = a.dst[u.tok * K + e];
+    const int loff = d < 0 ? -d - 1 : d;
+    return loff >= 0 && loff < NvS ? loff : -1;
+  };
+  int flagged = 0;
+  auto flag_stored = [&]() {  // a lane flags the rows it has stored itself
+    bulk_wait<0>();
+    fence_gpu();
+    for (; flagged < stored; ++flagged) {
+      const Unit u = units[flagged % kUnits];
+      if (u.ntok == 1 && u.off + u.len < row_bytes) continue;  // more pieces of the row follow
+      for (int e = lane; e < u.ntok * K; e += 32) {
+        const int loff = row_of(u, e);
+        if (loff >= 0) st_relaxed_gpu(meta + c.rowflag_off + loff, epoch);
+      }
+    }
+    __syncwarp();
+  };
+  bool more = true;
+  for (int q = 0; q < kRing - 1 && more; ++q) more = load();
+  while (stored < loaded) {
+    const Unit u = units[stored % kUnits];
+    const int q = stored % kRing;
+    const int mine = lane < u.ntok * K ? row_of(u, lane) : -1;
+    const bool got = mbar_wait(bar + q, (unsigned)((stored / kRing) & 1), c.timeout_ns);
     if (!__all_sync(0xffffffffu, got)) {
-      if (lane == 0) record_status(c, MOONEP_STATUS_TIMEOUT, MOONEP_K_DISPATCH_EXPAND, 100, q, r.stored, t0 + tok);
+      if (lane == 0) record_status(c, MOONEP_STATUS_TIMEOUT, MOONEP_K_DISPATCH_EXPAND, 100, q, stored, u.tok);
+      for (int n = stored; n < loaded; ++n)  // nothing may land in shared memory after the CTA has left
+        mbar_wait(bar + n % kRing, (unsigned)((n / kRing) & 1), c.timeout_ns);
       return false;
     }
-    if (loff >= 0) {
-      const long long o = (long long)p * a.piece_bytes;
-      bulk_s2g(shard + loff * row_bytes + o, r.stage + (size_t)q * a.piece_bytes,
-               (unsigned)min((long long)a.piece_bytes, row_bytes - o));
+    const unsigned len = u.ntok > 1 ? (unsigned)row_bytes : u.len;
+    for (int e = lane; e < u.ntok * K; e += 32) {
+      const int loff = e < 32 ? mine : row_of(u, e);
+      if (loff >= 0) bulk_s2g(shard + loff * row_bytes + u.off, ring + (size_t)q * a.stage_bytes + (e / K) * row_bytes, len);
     }
     bulk_commit();
-    ++r.stored;
-    if (ahead < mine) {
-      bulk_wait_read<1>();  // the stage to refill was stored from one item ago
+    ++stored;
+    if (more) {
+      bulk_wait_read<1>();  // the stage to refill was stored from one unit ago
       __syncwarp();
-      load(ahead++);
+      more = load();
     }
+    if (loaded - flagged == kUnits) flag_stored();
   }
+  flag_stored();
   return true;
 }
 
-// The same without bulk copies: a warp per row, 16 bytes or one element at a time.
-__device__ void copy_plain(const MoonepDevCtx& c, const SingleArgs& a, const SingleShared& s, int t0, int ntok,
-                           uint16_t* shard) {
+// The same without bulk copies: a warp per row of this CTA's tokens, 16 bytes or one element at a time.
+__device__ void copy_plain(const MoonepDevCtx& c, const SingleArgs& a, int t_lo, int t_hi, uint16_t* shard, int* meta,
+                           int epoch) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int tok = warp; tok < ntok; tok += kWarps) {
-    const uint16_t* src = a.hidden + (long long)(t0 + tok) * c.H;
+  for (int tok = t_lo + warp; tok < t_hi; tok += kPlanWarps) {
+    const uint16_t* src = a.hidden + (long long)tok * c.H;
+    const int d = lane < c.K ? a.dst[tok * c.K + lane] : 0;
+    int loff = d < 0 ? -d - 1 : d;
+    if (lane >= c.K || loff < 0 || loff >= c.NvS) loff = -1;
     const int n = a.vec_ok ? c.H / 8 : c.H;
-    for (int i = lane; i < n; i += 32) {
-      if (a.vec_ok) {
-        const int4 v = ld16(reinterpret_cast<const int4*>(src) + i);
-        for (int k = 0; k < c.K; ++k) {
-          const int loff = s.loff[tok * c.K + k];
-          if (loff >= 0) st16(reinterpret_cast<int4*>(shard + (long long)loff * c.H) + i, v);
-        }
+    for (int i0 = 0; i0 < n; i0 += 32) {  // whole warps: the shuffles need every lane
+      const int i = i0 + lane;
+      int4 v = make_int4(0, 0, 0, 0);
+      uint16_t w = 0;
+      if (i < n) {
+        if (a.vec_ok) v = ld16(reinterpret_cast<const int4*>(src) + i); else w = src[i];
+      }
+      for (int k = 0; k < c.K; ++k) {
+        const int row = __shfl_sync(0xffffffffu, loff, k);
+        if (row < 0 || i >= n) continue;
+        if (a.vec_ok) st16(reinterpret_cast<int4*>(shard + (long long)row * c.H) + i, v); else shard[(long long)row * c.H + i] = w;
+      }
+    }
+    fence_gpu();
+    __syncwarp();
+    if (loff >= 0) st_relaxed_gpu(meta + c.rowflag_off + loff, epoch);
+  }
+}
+
+// Threads of the planning warps: rows for the entries of tokens [t_lo, t_hi), and everything the plan says about them.
+__device__ void plan_tokens(const MoonepDevCtx& c, const SingleArgs& a, SingleShared& s, const int* cnt, const int* off,
+                            int* cur, int* meta, int t_lo, int t_hi) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int E = c.E, K = c.K, NvS = c.NvS;
+  float* wbuf = reinterpret_cast<float*>(meta + c.weights_off);
+  // routing entries before this CTA's tokens
+  const int before = t_lo * K;
+  const int nv = a.topk_vec ? before / 4 : 0;
+  auto count = [&](int e) {
+    if ((unsigned)e < (unsigned)E) atomicAdd(cur + e, 1);
+  };
+  for (int i0 = tid; i0 < nv; i0 += 8 * kEntries) {
+    int4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      v[u] = i0 + u * kEntries < nv ? __ldg(reinterpret_cast<const int4*>(a.topk) + i0 + u * kEntries)
+                                    : make_int4(-1, -1, -1, -1);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      count(v[u].x);
+      count(v[u].y);
+      count(v[u].z);
+      count(v[u].w);
+    }
+  }
+  for (int i = nv * 4 + tid; i < before; i += kEntries) count(a.topk[i]);
+  const int tokens_per_step = kEntries / K;
+  for (int t0 = t_lo; t0 < t_hi; t0 += tokens_per_step) {
+    const int nent = min(tokens_per_step, t_hi - t0) * K, slot = t0 * K + tid;
+    const bool in = tid < nent;
+    int e = in ? a.topk[slot] : -1;
+    if (in && (unsigned)e >= (unsigned)E) {
+      record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TOKENS, 2, e, E, slot);
+      e = -1;
+    }
+    plan_sync();  // the entries before are counted; the step before is done with s.loff and s.bad
+    if (tid == 0) s.bad = 0;
+    // in-order index among the entries of the same expert: warp by warp, the warps before have moved the cursors on
+    int idx = 0;
+    for (int w = 0; w * 32 < nent; ++w) {
+      if (warp == w) {
+        const unsigned same = __match_any_sync(0xffffffffu, e >= 0 ? e : -1 - lane);
+        if (e >= 0) idx = cur[e] + __popc(same & ((1u << lane) - 1u));
+        __syncwarp();
+        if (e >= 0 && lane == __ffs(same) - 1) cur[e] += __popc(same);
+      }
+      plan_sync();
+    }
+    int loff = -1;
+    if (e >= 0) {
+      if (idx >= cnt[e]) {
+        record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TOKENS, 4, idx, e, slot);
       } else {
-        const uint16_t v = src[i];
-        for (int k = 0; k < c.K; ++k) {
-          const int loff = s.loff[tok * c.K + k];
-          if (loff >= 0) shard[(long long)loff * c.H + i] = v;
+        loff = off[e] + idx;
+        if (loff < 0 || loff >= NvS) {
+          record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TOKENS, 3, loff, NvS, slot);
+          loff = -1;
         }
       }
     }
+    if (in) {
+      s.loff[tid] = loff;
+      if (loff < 0) s.bad = 1;
+    }
+    plan_sync();
+    if (!in) continue;
+    // all entries of a token land on this rank: the first is its primary row, the others its duplicates in order
+    const int k = tid % K, base = tid - k, tok = slot / K;
+    int prev = k - 1, next = k + 1;
+    if (s.bad) {  // some entry has no row (recorded above): skip such entries
+      while (prev >= 0 && s.loff[base + prev] < 0) --prev;
+      while (next < K && s.loff[base + next] < 0) ++next;
+    }
+    if (K > 1 && k == 0) {
+      int first = loff, n = K - 1;
+      if (s.bad) {
+        first = -1, n = -1;
+        for (int q = 0; q < K; ++q) {
+          const int l = s.loff[base + q];
+          if (l < 0) continue;
+          if (n >= 0) a.dup_loffs[tok * (K - 1) + n] = l; else first = l;
+          ++n;
+        }
+        if (n <= 0) first = -1, n = 0;
+      }
+      a.dup_groups[3 * tok] = first;
+      a.dup_groups[3 * tok + 1] = tok * (K - 1);
+      a.dup_groups[3 * tok + 2] = n;
+    }
+    if (loff < 0) {
+      a.dst[slot] = 0;
+      continue;
+    }
+    if (k > 0 && !s.bad) a.dup_loffs[tok * (K - 1) + k - 1] = loff;
+    a.dst[slot] = prev >= 0 ? -loff - 1 : loff;
+    const int link = (prev >= 0 ? 0 : MOONEP_LINK_PRIMARY) | (next < K ? MOONEP_LINK_HAS_NEXT | s.loff[base + next] : 0);
+    meta[c.src_info_off + loff] = slot;
+    meta[c.link_off + loff] = link;
+    if (a.plan_src_info != nullptr) a.plan_src_info[loff] = slot;
+    if (a.plan_link != nullptr) a.plan_link[loff] = link;
+    if (a.weights != nullptr) wbuf[loff] = a.weights[slot];
+  }
+  if (t_hi == c.S) {
+    // token counts above what was routed leave rows that nothing landed in
+    plan_sync();
+    for (int e = tid; e < E; e += kEntries)
+      for (int g = cur[e]; g < cnt[e] && off[e] + g < NvS; ++g) {
+        meta[c.src_info_off + off[e] + g] = -1;
+        if (a.plan_src_info != nullptr) a.plan_src_info[off[e] + g] = -1;
+        if (a.plan_link != nullptr) a.plan_link[off[e] + g] = 0;
+      }
   }
 }
 
 __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const MoonepDevCtx c, const SingleArgs a) {
-  extern __shared__ __align__(128) unsigned char s_dyn[];  // rings, a piece of zeros, counts / offsets / cursors
+  extern __shared__ __align__(128) unsigned char s_dyn[];  // rings, zeros, the group layout
   __shared__ __align__(8) SingleShared s;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5;
   const int E = c.E, K = c.K, NvS = c.NvS;
-  unsigned char* zeros = s_dyn + (size_t)kCopyWarps * kRing * a.piece_bytes;
-  int* cnt = reinterpret_cast<int*>(zeros + (a.bulk ? a.piece_bytes : 0));
-  int* off = cnt + E;
-  int* cur = off + E;
+  unsigned char* zeros = s_dyn + (size_t)a.copy_warps * kRing * a.stage_bytes;
+  int* tables = reinterpret_cast<int*>(zeros + (a.bulk ? kZeroBytes : 0));
   if (tid < kCopyWarps * kRing) mbar_init(s.bar + tid, 1);
   if (a.bulk)
-    for (int i = tid; i < a.piece_bytes / 16; i += kThreads) reinterpret_cast<int4*>(zeros)[i] = make_int4(0, 0, 0, 0);
+    for (int i = tid; i < kZeroBytes / 16; i += kThreads) reinterpret_cast<int4*>(zeros)[i] = make_int4(0, 0, 0, 0);
   fence_barrier_init();
   fence_proxy_async();
   griddep_wait();
@@ -291,23 +526,31 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
     int* meta = c.meta_peer[0];
     uint16_t* shard = c.hidden_peer[0];
     const int epoch = abs_epoch(c, MOONEP_FLAG_SENT, a.epoch_sent);
+    const int t_lo = min(c.S, (int)blockIdx.x * a.tokens_per_cta), t_hi = min(c.S, t_lo + a.tokens_per_cta);
+    Layout lay = {nullptr, nullptr, nullptr, nullptr, 0};
+    int *cnt = tables, *off = tables + E, *cur = tables + 2 * E;
     int used = NvS;
     if (a.fresh) {
-      int carry = 0;
+      int* cum = tables + 3 * E;
+      int carry = 0, pads = 0;
       for (int e0 = 0; e0 < E; e0 += kThreads) {
         const int e = e0 + tid;
         const int n = e < E ? a.tpe[e] : 0;
         const int rows = padded_rows(n, c.token_padding);
-        int total;
+        int total, total_pads;
         const int end = carry + block_scan(rows, s.warp_sum, total);
+        const int pend = pads + block_scan(rows > 0 ? rows - n : 0, s.warp_sum, total_pads);
         if (e < E) {
           cnt[e] = n;
           off[e] = end - rows;
           cur[e] = 0;
+          cum[e] = pend;
         }
         carry += total;
+        pads += total_pads;
       }
       used = min(max(carry, 0), NvS);
+      lay = {nullptr, cnt, off, cum, E};
       __syncthreads();
       if (blockIdx.x == 0) {
         for (int e = tid; e < E; e += kThreads) {
@@ -321,7 +564,7 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
           c.alloc_cum[e] = n;
           if (n > 0) c.expert_off[e] = off[e];
         }
-        for (int b = tid; b < c.B; b += kThreads) {
+        for (int b = tid; b < c.B; b += kThreads) {  // a single rank has no use for its prefetch slots
           a.cu_seqlens[E + b] = carry;
           a.zero_fill[2 * (E + b)] = 0;
           a.zero_fill[2 * (E + b) + 1] = 0;
@@ -338,174 +581,81 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
           st_release_gpu(c.counters + MOONEP_CTR_TABLES_READY, abs_epoch(c, MOONEP_FLAG_PLAN, a.epoch_plan));
         }
       }
-    }
-    visit_pads(c, a, s, cnt, off, zeros, shard, meta, epoch, false);
-
-    const int t_lo = min(c.S, (int)blockIdx.x * a.tokens_per_cta), t_hi = min(c.S, t_lo + a.tokens_per_cta);
-    if (a.fresh) {
-      for (int row = used + blockIdx.x * kThreads + tid; row < NvS; row += gridDim.x * kThreads) {
-        meta[c.src_info_off + row] = -1;
-        if (a.plan_src_info != nullptr) a.plan_src_info[row] = -1;
-        if (a.plan_link != nullptr) a.plan_link[row] = 0;
+    } else if (a.zero_fill != nullptr) {
+      const int groups = E + c.B;
+      int *first = tables, *cum = tables + groups;
+      int pads = 0;
+      for (int g0 = 0; g0 < groups; g0 += kThreads) {
+        const int g = g0 + tid;
+        int total;
+        const int pend = pads + block_scan(g < groups ? max(0, a.zero_fill[2 * g + 1]) : 0, s.warp_sum, total);
+        if (g < groups) {
+          first[g] = a.zero_fill[2 * g];
+          cum[g] = pend;
+        }
+        pads += total;
       }
-      if (t_lo < t_hi) {  // routing entries before this CTA's tokens
-        const int n = t_lo * K;
-        const int nv = a.topk_vec ? n / 4 : 0;
-        auto count = [&](int e) {
-          if ((unsigned)e < (unsigned)E) atomicAdd(cur + e, 1);
-        };
-        for (int i0 = tid; i0 < nv; i0 += 4 * kThreads) {
-          int4 v[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            v[u] = i0 + u * kThreads < nv ? __ldg(reinterpret_cast<const int4*>(a.topk) + i0 + u * kThreads)
-                                          : make_int4(-1, -1, -1, -1);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            count(v[u].x);
-            count(v[u].y);
-            count(v[u].z);
-            count(v[u].w);
-          }
-        }
-        for (int i = nv * 4 + tid; i < n; i += kThreads) count(a.topk[i]);
-      }
-    }
-    __syncthreads();
-
-    Ring ring = {s_dyn + (size_t)warp * kRing * a.piece_bytes, s.bar + (warp < kCopyWarps ? warp : 0) * kRing, 0, 0};
-    const int tokens_per_step = max(1, kEntries / K);
-    float* wbuf = reinterpret_cast<float*>(meta + c.weights_off);
-    for (int t0 = t_lo; t0 < t_hi; t0 += tokens_per_step) {
-      const int ntok = min(tokens_per_step, t_hi - t0);
-      const int nent = ntok * K, slot = t0 * K + tid;
-      const bool in = tid < nent;
-      int loff = -1;
-      __syncthreads();  // the step before is done with s.loff and s.bad
-      if (a.fresh) {
-        int e = in ? a.topk[slot] : -1;
-        if (in && (unsigned)e >= (unsigned)E) {
-          record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TOKENS, 2, e, E, slot);
-          e = -1;
-        }
-        if (tid == 0) s.bad = 0;
-        // in-order index among the entries of the same expert: warp by warp, the warps before have moved the cursors on
-        int idx = 0;
-        for (int w = 0; w * 32 < nent; ++w) {
-          if (warp == w) {
-            const unsigned same = __match_any_sync(0xffffffffu, e >= 0 ? e : -1 - lane);
-            if (e >= 0) idx = cur[e] + __popc(same & ((1u << lane) - 1u));
-            __syncwarp();
-            if (e >= 0 && lane == __ffs(same) - 1) cur[e] += __popc(same);
-          }
-          __syncthreads();
-        }
-        if (e >= 0) {
-          if (idx >= cnt[e]) {
-            record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TOKENS, 4, idx, e, slot);
-          } else {
-            loff = off[e] + idx;
-            if (loff < 0 || loff >= NvS) {
-              record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TOKENS, 3, loff, NvS, slot);
-              loff = -1;
-            }
-          }
-        }
-        if (in && loff < 0) s.bad = 1;
-      } else if (in) {
-        const int d = a.dst[slot];
-        loff = d < 0 ? -d - 1 : d;
-        if (loff < 0 || loff >= NvS) {
-          record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_DISPATCH_SEND, 6, d, slot / K, slot % K);
-          loff = -1;
-        }
-      }
-      if (in) s.loff[tid] = loff;
+      lay = {first, nullptr, nullptr, cum, groups};
       __syncthreads();
-      if (a.fresh && in) {
-        const int k = tid % K, base = tid - k, tok = slot / K;
-        // all entries of a token land on this rank: the first is its primary row, the others its duplicates in order
-        int prev = k - 1, next = k + 1;
-        if (s.bad) {  // some entry has no row (recorded above): skip such entries
-          while (prev >= 0 && s.loff[base + prev] < 0) --prev;
-          while (next < K && s.loff[base + next] < 0) ++next;
+    }
+    if (warp >= kPlanWarps) {
+      clear_pads(c, a, lay, s.grab[warp - kPlanWarps], zeros, shard, meta, epoch);
+      if (a.fresh)  // rows behind the last group are unused
+        for (int row = used + blockIdx.x * (kThreads - kEntries) + tid - kEntries; row < NvS;
+             row += gridDim.x * (kThreads - kEntries)) {
+          meta[c.src_info_off + row] = -1;
+          if (a.plan_src_info != nullptr) a.plan_src_info[row] = -1;
+          if (a.plan_link != nullptr) a.plan_link[row] = 0;
         }
-        if (K > 1 && k == 0) {
-          int first = s.loff[base], n = K - 1;
-          if (s.bad) {
-            first = -1, n = -1;
-            for (int q = 0; q < K; ++q) {
-              const int l = s.loff[base + q];
-              if (l < 0) continue;
-              if (n >= 0) a.dup_loffs[tok * (K - 1) + n] = l; else first = l;
-              ++n;
-            }
-            if (n <= 0) first = -1, n = 0;
-          }
-          a.dup_groups[3 * tok] = first;
-          a.dup_groups[3 * tok + 1] = tok * (K - 1);
-          a.dup_groups[3 * tok + 2] = n;
-        }
-        if (loff < 0) {
-          a.dst[slot] = 0;
+    } else {
+      if (t_lo < t_hi) {
+        if (a.fresh) {
+          plan_tokens(c, a, s, cnt, off, cur, meta, t_lo, t_hi);
+          fence_gpu();
+          plan_sync();
+          if (tid == 0) st_release_gpu(a.work + kWorkReady + blockIdx.x, epoch);
         } else {
-          if (k > 0 && !s.bad) a.dup_loffs[tok * (K - 1) + k - 1] = loff;
-          a.dst[slot] = prev >= 0 ? -loff - 1 : loff;
-          const int link = (prev >= 0 ? 0 : MOONEP_LINK_PRIMARY) | (next < K ? MOONEP_LINK_HAS_NEXT | s.loff[base + next] : 0);
-          meta[c.src_info_off + loff] = slot;
-          meta[c.link_off + loff] = link;
-          if (a.plan_src_info != nullptr) a.plan_src_info[loff] = slot;
-          if (a.plan_link != nullptr) a.plan_link[loff] = link;
+          for (int i = t_lo * K + tid; i < t_hi * K; i += kEntries) {
+            const int d = a.dst[i];
+            const int loff = d < 0 ? -d - 1 : d;
+            if (loff < 0 || loff >= NvS)
+              record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_DISPATCH_SEND, 6, d, i / K, i % K);
+            else if (a.weights != nullptr)
+              reinterpret_cast<float*>(meta + c.weights_off)[loff] = a.weights[i];
+          }
         }
       }
-      if (in && loff >= 0 && a.weights != nullptr) wbuf[loff] = a.weights[slot];
-      if (!a.bulk) {
-        copy_plain(c, a, s, t0, ntok, shard);
-      } else if (warp < kCopyWarps && ok) {
-        ok = copy_bulk(c, a, s, t0, ntok, ring, reinterpret_cast<unsigned char*>(shard));
-      }
+      if (!a.bulk)
+        copy_plain(c, a, t_lo, t_hi, shard, meta, epoch);
+      else if (warp < a.copy_warps)
+        ok = copy_bulk(c, a, s, s_dyn, reinterpret_cast<unsigned char*>(shard), meta, epoch);
     }
-    if (a.fresh && t_hi == c.S && t_lo < c.S) {
-      // token counts above what was routed leave rows that nothing landed in
-      __syncthreads();
-      for (int e = tid; e < E; e += kThreads)
-        for (int g = cur[e]; g < cnt[e] && off[e] + g < NvS; ++g) {
-          meta[c.src_info_off + off[e] + g] = -1;
-          if (a.plan_src_info != nullptr) a.plan_src_info[off[e] + g] = -1;
-          if (a.plan_link != nullptr) a.plan_link[off[e] + g] = 0;
-        }
-    }
-    // all rows of this CTA are in memory before the first of their flags goes out
     bulk_wait<0>();
-    fence_gpu();
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;
-    fence_gpu();
-    if (ok) {
-      visit_pads(c, a, s, cnt, off, zeros, shard, meta, epoch, true);
-      for (int i = t_lo * K + tid; i < t_hi * K; i += kThreads) {
-        const int d = a.dst[i];
-        const int loff = d < 0 ? -d - 1 : d;
-        if (loff >= 0 && loff < NvS) st_relaxed_gpu(meta + c.rowflag_off + loff, epoch);
-      }
-    }
     if (tid == 0) stat_phase(c, MOONEP_PH_BUILD_EXPAND, t_begin);
   }
-  // the last CTA publishes what the general kernels' stages publish
-  __syncthreads();
+  // the last CTA resets the counters and publishes what the general kernels' stages publish
+  fence_gpu();
+  ok = __syncthreads_and(ok ? 1 : 0) != 0;
   if (tid == 0) {
     fence_gpu();
-    if (atomicAdd(c.counters + MOONEP_CTR_DISPATCH_ARRIVE, 1) == (int)gridDim.x - 1) {
-      c.counters[MOONEP_CTR_DISPATCH_ARRIVE] = 0;
-      fence_sys();
-      if (ok && !poisoned(c)) {
-        if (a.fresh) {
-          const int plan_epoch = abs_epoch(c, MOONEP_FLAG_PLAN, a.epoch_plan);
-          st_release_gpu(c.counters + MOONEP_CTR_PLAN_DONE, plan_epoch);
-          st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_TPE, 0), abs_epoch(c, MOONEP_FLAG_TPE, a.epoch_tpe));
-          st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_PLAN, 0), plan_epoch);
-        }
-        st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_SENT, 0), abs_epoch(c, MOONEP_FLAG_SENT, a.epoch_sent));
+    s.last = atomicAdd(c.counters + MOONEP_CTR_DISPATCH_ARRIVE, 1) == (int)gridDim.x - 1;
+    fence_gpu();
+  }
+  __syncthreads();
+  if (!s.last) return;
+  for (int i = tid; i < (int)gridDim.x; i += kThreads) a.work[kWorkNext + i] = 0;
+  if (tid == 0) {
+    a.work[kWorkPads] = 0;
+    c.counters[MOONEP_CTR_DISPATCH_ARRIVE] = 0;
+    fence_sys();
+    if (run && ok && !poisoned(c)) {
+      if (a.fresh) {
+        const int plan_epoch = abs_epoch(c, MOONEP_FLAG_PLAN, a.epoch_plan);
+        st_release_gpu(c.counters + MOONEP_CTR_PLAN_DONE, plan_epoch);
+        st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_TPE, 0), abs_epoch(c, MOONEP_FLAG_TPE, a.epoch_tpe));
+        st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_PLAN, 0), plan_epoch);
       }
+      st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_SENT, 0), abs_epoch(c, MOONEP_FLAG_SENT, a.epoch_sent));
     }
   }
 }
@@ -513,6 +663,9 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
 // ---- combine ---------------------------------------------------------------------------------------------------
 
 constexpr int kCombineThreads = 512;
+// At most so many items per warp.  Many short CTAs instead of a resident grid: SMs that are slower to HBM simply run fewer
+// of them.  Below that many items for two CTAs per SM a warp takes fewer, so that a small combine still uses every SM.
+constexpr int kCombineItems = 4;
 constexpr int kCombineRows = 8;  // rows of a token whose loads are in flight together: 128 KB per SM with 32 warps
 
 struct CombineArgs {
@@ -524,6 +677,8 @@ struct CombineArgs {
   const int* ready;         // optional: per 128-row block of in_rows, see moonep_combine_push
   int ready_expect;
   int vec_ok;
+  int items_per_warp;
+  int resident;  // the grid is bounded and strides over the items
 };
 
 __device__ __forceinline__ void add8(float* acc, const int4& v) {
@@ -543,19 +698,20 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(cons
   griddep_wait();
   griddep_launch();
   if (poisoned(c)) return;
-  const unsigned long long t_begin = globaltimer_ns();
   const int lane = threadIdx.x & 31;
   const int K = c.K, H = c.H, NvS = c.NvS;
   const int nvec = H / 8;
   const int npieces = a.vec_ok ? (nvec + 31) / 32 : 1;
-  const int items = c.S * npieces;  // far below 2^31: S * H elements fit the GPU
-  const int step = gridDim.x * (kCombineThreads / 32);
-  int it = blockIdx.x * (kCombineThreads / 32) + (threadIdx.x >> 5);
-  int d_next = it < items && lane < K ? a.dst[it / npieces * K + lane] : 0;
-  for (; it < items; it += step) {
+  const int items = c.S * npieces;  // S * H elements fit the GPU: far below 2^31
+  const int step = a.resident ? gridDim.x * (kCombineThreads / 32) : kCombineThreads / 32;
+  const int first = a.resident ? blockIdx.x * (kCombineThreads / 32) : blockIdx.x * (kCombineThreads / 32) * a.items_per_warp;
+  const int end = a.resident ? items : min(items, first + step * a.items_per_warp);
+  int it = first + (threadIdx.x >> 5);
+  int d_next = it < end && lane < K ? a.dst[it / npieces * K + lane] : 0;
+  for (; it < end; it += step) {
     const int tok = it / npieces, p = it - tok * npieces;
     const int d = d_next;
-    if (it + step < items && lane < K) d_next = a.dst[(it + step) / npieces * K + lane];  // not a dependent load then
+    if (it + step < end && lane < K) d_next = a.dst[(it + step) / npieces * K + lane];  // not a dependent load then
     int row = d < 0 ? -d - 1 : d;
     const bool valid = lane < K && row >= 0 && row < NvS;
     if (lane < K && !valid) record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_COMBINE_PUSH, 6, d, tok, lane);
@@ -633,7 +789,6 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(cons
       }
     }
   }
-  if (threadIdx.x == 0) stat_phase(c, MOONEP_PH_FOLD, t_begin);
 }
 
 }  // namespace
@@ -644,18 +799,20 @@ using namespace moonep;
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-extern "C" int moonep_single_supported(int E, int S, int K) {
-  return E <= kMaxExperts && (long long)S * K <= kMaxEntries ? 1 : 0;
+extern "C" int moonep_single_supported(int E, int B, int S, int K) {
+  return E <= kMaxGroups && B <= kMaxGroups && (long long)S * K <= kMaxEntries ? 1 : 0;
 }
+
+extern "C" int moonep_single_work_words(void) { return kWorkReady + kMaxCtas; }
 
 extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, const int* tpe, int* dst, int* cu_seqlens,
                                       int* experts_to_copy, int* zero_fill, int* remote_stats, int* dup_groups,
                                       int* dup_loffs, int* dup_counts, int* plan_src_info, int* plan_link,
                                       const void* hidden, const float* weights, int with_weights, int epoch_tpe,
-                                      int epoch_plan, int epoch_sent, int n_ctas, void* stream) {
+                                      int epoch_plan, int epoch_sent, int n_ctas, int* work, void* stream) {
   auto* h = (HostCtx*)ctx;
   const MoonepDevCtx& c = h->dev;
-  if (c.R != 1 || (fresh && !moonep_single_supported(c.E, c.S, c.K))) {
+  if (c.R != 1 || !moonep_single_supported(c.E, c.B, c.S, c.K)) {
     set_error("moonep_dispatch_single: needs a single rank, at most 4096 experts and 262144 routing entries");
     return 1;
   }
@@ -673,6 +830,7 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
   a.plan_src_info = plan_src_info;
   a.plan_link = plan_link;
   a.hidden = (const uint16_t*)hidden;
+  a.work = work;
   a.weights = weights;
   a.with_weights = with_weights;
   a.fresh = fresh;
@@ -684,21 +842,29 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
   a.epoch_sent = epoch_sent;
   const size_t static_bytes = sizeof(SingleShared) + 1024;
   const size_t limit = (size_t)imax(0, h->max_smem_optin - (int)static_bytes);
-  const size_t tables = fresh ? (size_t)3 * c.E * sizeof(int) : 0;
-  a.piece_bytes = 0;
-  a.npieces = 1;
+  const size_t tables = (fresh ? (size_t)4 * c.E : (size_t)2 * (c.E + c.B)) * sizeof(int);
+  const long long row_bytes = (long long)c.H * 2;
+  a.stage_bytes = 0;
+  a.npieces = a.tokens_per_unit = 1;
+  a.copy_warps = 0;
   if (a.bulk) {
-    const long long row_bytes = (long long)c.H * 2;
-    const long long room = (long long)(limit - tables) / (kCopyWarps * kRing + 1) / 16 * 16;
-    const long long most = room < kMaxPiece ? room : kMaxPiece;
+    const long long room = (long long)(limit - tables - kZeroBytes);
+    const long long most = room / (4 * kRing) / 16 * 16 < kMaxStage ? room / (4 * kRing) / 16 * 16 : kMaxStage;
     a.npieces = (int)((row_bytes + most - 1) / most);
-    a.piece_bytes = (int)(((row_bytes + a.npieces - 1) / a.npieces + 15) / 16 * 16);
+    if (a.npieces > 1) {
+      a.stage_bytes = (int)(((row_bytes + a.npieces - 1) / a.npieces + 15) / 16 * 16);
+    } else {  // rows below 4 KB share a stage of about that size
+      a.tokens_per_unit = imax(1, imin(16, (int)(4096 / row_bytes)));
+      a.stage_bytes = (int)(a.tokens_per_unit * row_bytes);
+    }
+    a.copy_warps = imin(kCopyWarps, (int)(room / ((long long)kRing * a.stage_bytes)));
   }
-  const size_t smem = (size_t)(kCopyWarps * kRing + 1) * a.piece_bytes + tables;
+  a.pads_per_grab = imax(1, imin(32, (int)(28672 / row_bytes)));
+  const size_t smem = a.bulk ? (size_t)a.copy_warps * kRing * a.stage_bytes + kZeroBytes + tables : tables;
   if (int rc = check_cuda(cudaFuncSetAttribute(dispatch_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit),
                           "cudaFuncSetAttribute(dispatch_single_kernel)"))
     return rc;
-  int grid = imax(1, imin(c.local_sms, h->sm_count));
+  int grid = imax(1, imin(imin(c.local_sms, h->sm_count), kMaxCtas));
   if (n_ctas > 0) grid = imin(grid, n_ctas);
   a.tokens_per_cta = (c.S + grid - 1) / grid;
   if (int rc = check_cuda(launch_maybe_pdl(dispatch_single_kernel, grid, kThreads, smem, (cudaStream_t)stream,
@@ -726,9 +892,12 @@ extern "C" int moonep_combine_single(void* ctx, const int* dst, const void* in_r
   a.ready_expect = ready_expect;
   a.vec_ok = (c.H % 8 == 0 && aligned16(in_rows) && aligned16(out)) ? 1 : 0;
   const long long items = (long long)c.S * (a.vec_ok ? (c.H / 8 + 31) / 32 : 1);
-  const long long need = (items + kCombineThreads / 32 - 1) / (kCombineThreads / 32);
-  const int most = 2 * imax(1, imin(c.local_sms, h->sm_count));
-  const int grid = need < most ? (int)need : most;
+  a.items_per_warp = (int)(items / (2 * kCombineThreads / 32 * h->sm_count));
+  a.items_per_warp = imax(1, imin(kCombineItems, a.items_per_warp));
+  const int per_cta = kCombineThreads / 32 * a.items_per_warp;
+  int grid = (int)((items + per_cta - 1) / per_cta);
+  a.resident = c.local_sms < h->sm_count ? 1 : 0;
+  if (a.resident) grid = imin(grid, 2 * imax(1, c.local_sms));
   if (int rc = check_cuda(launch_maybe_pdl(combine_single_kernel, grid, kCombineThreads, 0, (cudaStream_t)stream,
                                            h->enable_pdl != 0, c, a),
                           "launch combine_single_kernel"))

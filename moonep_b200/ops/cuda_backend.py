@@ -107,7 +107,8 @@ class CudaBackend:
         # rank that is launched later, so they run the dispatch and combine kernels one role per phase.
         self.phased = (bool(getattr(world, "emulated", False)) and world.size > 1) or config.force_phased()
         # one rank: dispatch and combine are kernels of their own (csrc/single_rank.cu)
-        self.single = R == 1 and bool(self.lib.moonep_single_supported(E, S, K)) and not self.phased
+        self.single = R == 1 and bool(self.lib.moonep_single_supported(E, B, S, K)) and not self.phased
+        self.single_work = i32(self.lib.moonep_single_work_words()) if self.single else None
         self.combine_mode = config.combine_mode()
         self.n_expand = 0  # CTAs of the dispatch kernel's destination-side role; 0 = every SM the senders leave free
 
@@ -436,7 +437,7 @@ class CudaBackend:
             _ptr(plan.experts_to_copy), _ptr(plan.zero_fill_ranges), _ptr(plan.remote_stats), _ptr(plan.dup_groups),
             _ptr(plan.dup_loffs), _ptr(plan.dup_counts), _ptr(plan.src_info), _ptr(plan.link), _ptr(hidden), _ptr(weights),
             int(weights is not None), self._cur(FLAG_TPE), self._cur(FLAG_PLAN), self._next(FLAG_SENT), self.n_expand,
-            _stream(), tag="dispatch_single",
+            _ptr(self.single_work), _stream(), tag="dispatch_single",
         )  # fmt: skip
 
     def copy_out(self, out_hidden, out_weights):
