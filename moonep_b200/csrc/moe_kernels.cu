@@ -10,6 +10,8 @@
 //                       projection's weight gradient) and dgate.
 //
 //   sgd_update          w (bf16) -= lr * g (fp32), vectorised.
+//   adamw_update        one AdamW step of up to kAdamTensors weights in one pass: fp32 master, moments and gradient in,
+//                       master, moments and the rounded bf16 weight out.
 //
 // The reference has no expert computation; these serve the MoE training-step configuration.
 #include <cuda_bf16.h>
@@ -22,6 +24,7 @@ namespace moonep {
 namespace {
 
 constexpr int kTile = 64;
+constexpr int kAdamTensors = 3;
 
 __global__ void __launch_bounds__(256)
     transpose_experts_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int d0, int d1,
@@ -115,11 +118,94 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// One AdamW step.  Bound by HBM: 16 bytes in and 14 out per element, where a pass per operation moved 86.  Three weights
+// of 33.5 M elements: 1350 us as 30 elementwise launches, 509 us here (5.9 TB/s).  Four elements per thread and step, a
+// stride of the whole grid between steps: the four loads of a step are 16 bytes each and independent, and 8 CTAs of 256
+// threads per SM keep 128 KB of them in flight.
+struct AdamTensor {
+  float* p;        // fp32 master
+  float* m;        // first moment
+  float* v;        // second moment
+  const float* g;  // gradient
+  uint16_t* w;     // bf16 weight
+  long long n4;    // groups of four elements
+};
+struct AdamArgs {
+  AdamTensor t[kAdamTensors];
+  int count;
+  float decay;            // 1 - lr * weight_decay
+  float b1, b2;           // decay rates of the moments
+  float one_b1, one_b2;   // 1 - b1, 1 - b2
+  float inv_c2, eps;      // 1 / bias correction of the second moment
+  float step;             // lr / bias correction of the first moment
+};
+
+__global__ void __launch_bounds__(256) adamw_kernel(const AdamArgs a) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (int k = 0; k < a.count; ++k) {
+    const AdamTensor t = a.t[k];
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < t.n4; i += stride) {
+      int4 x[4] = {ld16(t.p + i * 4), ld16(t.m + i * 4), ld16(t.v + i * 4), ld16(t.g + i * 4)};
+      float *p = reinterpret_cast<float*>(&x[0]), *m = reinterpret_cast<float*>(&x[1]), *v = reinterpret_cast<float*>(&x[2]);
+      const float* g = reinterpret_cast<const float*>(&x[3]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        m[q] = m[q] * a.b1 + a.one_b1 * g[q];
+        v[q] = v[q] * a.b2 + a.one_b2 * (g[q] * g[q]);
+        p[q] = p[q] * a.decay - a.step * (m[q] / (sqrtf(v[q] * a.inv_c2) + a.eps));
+      }
+      st16(t.p + i * 4, x[0]);
+      st16(t.m + i * 4, x[1]);
+      st16(t.v + i * 4, x[2]);
+      *reinterpret_cast<uint2*>(t.w + i * 4) = make_uint2(pack_bf16(p[0], p[1]), pack_bf16(p[2], p[3]));
+    }
+  }
+}
+
 }  // namespace
 
 }  // namespace moonep
 
 using namespace moonep;
+
+// count weights: master, m, v, g fp32 and w bf16 of n[i] elements each (a multiple of 4; all 16-byte aligned, w 8-byte).
+// step: lr / bias correction of m; decay: 1 - lr * weight_decay; c2: bias correction of v.
+extern "C" int moonep_adamw_update(int count, void* const* master, void* const* m, void* const* v, void* const* g,
+                                   void* const* w, const long long* n, double step, double b1, double b2, double eps,
+                                   double decay, double c2, void* stream) {
+  if (count < 1 || count > kAdamTensors) {
+    set_error("moonep_adamw_update: 1 to " + std::to_string(kAdamTensors) + " weights per call");
+    return 1;
+  }
+  AdamArgs a;
+  a.count = count;
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    const uintptr_t bits = (uintptr_t)master[i] | (uintptr_t)m[i] | (uintptr_t)v[i] | (uintptr_t)g[i];
+    if (n[i] % 4 != 0 || (bits & 15u) != 0 || ((uintptr_t)w[i] & 7u) != 0) {
+      set_error("moonep_adamw_update: element counts must be multiples of 4 and the tensors 16-byte aligned");
+      return 1;
+    }
+    a.t[i] = {(float*)master[i], (float*)m[i], (float*)v[i], (const float*)g[i], (uint16_t*)w[i], n[i] / 4};
+    most = n[i] > most ? n[i] : most;
+  }
+  if (most == 0) return 0;
+  a.decay = (float)decay;
+  a.b1 = (float)b1;
+  a.b2 = (float)b2;
+  a.one_b1 = (float)(1.0 - b1);
+  a.one_b2 = (float)(1.0 - b2);
+  a.inv_c2 = (float)(1.0 / c2);
+  a.eps = (float)eps;
+  a.step = (float)step;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long need = (most / 4 + 255) / 256;
+  const int grid = (int)(need < sms * 8 ? need : sms * 8);
+  adamw_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
+  return check_launch("adamw_kernel");
+}
 
 // w: [n] bf16, g: [n] fp32, n a multiple of 8: w -= lr * g.
 extern "C" int moonep_sgd_update(void* w, const float* g, long long n, float lr, void* stream) {

@@ -326,6 +326,11 @@ int moonep_transpose_experts(const void* src, void* dst, int n, int d0, int d1, 
                              long long dst_expert_stride, int col0, const int* active, void* stream);
 int moonep_swiglu_bwd(const void* a, const void* u, const void* g, const float* w, const int* total_rows, int rows_cap,
                       int I, void* dadu, void* hsw, float* dgate, void* stream);
+// One AdamW step of `count` weights (at most 3): fp32 master, moments m and v, gradient g, bf16 weight w, n elements each.
+// step = lr / (1 - b1^t), decay = 1 - lr * weight_decay, c2 = 1 - b2^t.
+int moonep_adamw_update(int count, void* const* master, void* const* m, void* const* v, void* const* g, void* const* w,
+                        const long long* n, double step, double b1, double b2, double eps, double decay, double c2,
+                        void* stream);
 int moonep_sgd_update(void* w, const float* g, long long n, float lr, void* stream);
 
 // CUDA VMM symmetric allocator (driver API through cudaGetDriverEntryPoint).

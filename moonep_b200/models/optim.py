@@ -3,7 +3,7 @@
 The experts' bf16 weights live in symmetric memory (peers prefetch them), their fp32 gradients in the layer
 (``ExpertParallelMoE.owner_grads()``, completed by ``reduce_grad``).  ``ExpertAdamW`` keeps fp32 master weights and
 moments for the owned experts only, so optimizer state is sharded exactly like the experts, and writes the rounded
-bf16 result back into the symmetric weights.  ``ExpertParallelMoE.sgd_step`` is the fused plain-SGD alternative.
+bf16 result back into the symmetric weights, in one pass over the state (``ops.moe_ops.adamw_update``).  ``ExpertParallelMoE.sgd_step`` is the fused plain-SGD alternative.
 The reference has no optimizer (it stops at the communication API).
 """
 
@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import torch
 
+from ..ops.moe_ops import adamw_update
 from .moe_layer import ExpertParallelMoE
 
 
@@ -29,14 +30,9 @@ class ExpertAdamW:
         self.steps += 1
         b1, b2 = self.betas
         c1, c2 = 1.0 - b1**self.steps, 1.0 - b2**self.steps
-        for p, g, m, v, w in zip(self.master, self.layer.owner_grads(), self.exp_avg, self.exp_avg_sq,
-                                 self.layer.owner_weights()):  # fmt: skip
-            if self.weight_decay:
-                p.mul_(1.0 - self.lr * self.weight_decay)
-            m.mul_(b1).add_(g, alpha=1.0 - b1)
-            v.mul_(b2).addcmul_(g, g, value=1.0 - b2)
-            p.addcdiv_(m, (v / c2).sqrt_().add_(self.eps), value=-self.lr / c1)
-            w.copy_(p)
+        adamw_update(self.master, self.exp_avg, self.exp_avg_sq, self.layer.owner_grads(), self.layer.owner_weights(),
+                     lr=float(self.lr), b1=float(b1), b2=float(b2), eps=float(self.eps),
+                     weight_decay=float(self.weight_decay), c1=c1, c2=c2)  # fmt: skip
         self.layer.publish_owned()
 
     def zero_grad(self) -> None:

@@ -5,6 +5,8 @@ CUDA tensors run the kernels of ``csrc/moe_kernels.cu``; CPU tensors run the sam
 
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -68,3 +70,31 @@ def sgd_update(w: torch.Tensor, g: torch.Tensor, lr: float) -> None:
         rc = _lib.load().moonep_sgd_update(w.data_ptr(), g.data_ptr(), w.numel(), float(lr),
                                            torch.cuda.current_stream().cuda_stream)  # fmt: skip
     _lib.check(rc, "moonep_sgd_update")
+
+
+def adamw_update(masters, exp_avgs, exp_avg_sqs, grads, weights, *, lr, b1, b2, eps, weight_decay, c1, c2) -> None:
+    """One AdamW step of up to three weights: fp32 ``masters`` and moments are updated from the fp32 ``grads`` and the
+    rounded masters stored to the bf16 ``weights``.  ``c1``, ``c2``: bias corrections ``1 - b**t``."""
+    tensors = [list(ts) for ts in (masters, exp_avgs, exp_avg_sqs, grads, weights)]
+    kernel = all(
+        t.is_cuda and t.is_contiguous() and t.numel() == w.numel() and t.device == weights[0].device
+        and t.dtype == (torch.bfloat16 if ts is tensors[4] else torch.float32)
+        and t.numel() % 4 == 0 and t.data_ptr() % (8 if ts is tensors[4] else 16) == 0
+        for ts in tensors for t, w in zip(ts, weights)
+    )  # fmt: skip
+    if not kernel:
+        for p, m, v, g, w in zip(*tensors):
+            if weight_decay:
+                p.mul_(1.0 - lr * weight_decay)
+            m.mul_(b1).add_(g, alpha=1.0 - b1)
+            v.mul_(b2).addcmul_(g, g, value=1.0 - b2)
+            p.addcdiv_(m, (v / c2).sqrt_().add_(eps), value=-lr / c1)
+            w.copy_(p)
+        return
+    n = len(tensors[4])
+    ptrs = [(ctypes.c_void_p * n)(*[t.data_ptr() for t in ts]) for ts in tensors]
+    sizes = (ctypes.c_longlong * n)(*[t.numel() for t in tensors[4]])
+    with torch.cuda.device(weights[0].device):
+        rc = _lib.load().moonep_adamw_update(n, *ptrs, sizes, lr / c1, b1, b2, eps, 1.0 - lr * weight_decay, c2,
+                                             torch.cuda.current_stream().cuda_stream)  # fmt: skip
+    _lib.check(rc, "moonep_adamw_update")

@@ -1,0 +1,45 @@
+"""The one-pass AdamW kernel against the same step in 64 bits, at sizes around its vectors and grid."""
+
+import pytest
+import torch
+
+from moonep_b200.ops.moe_ops import adamw_update
+
+
+@pytest.mark.parametrize(
+    "device,sizes,shift",
+    [
+        ("cpu", [12], 0),
+        pytest.param("cuda", [4], 0, marks=pytest.mark.gpu),
+        pytest.param("cuda", [1020, 1024, 1028], 0, marks=pytest.mark.gpu),
+        pytest.param("cuda", [148 * 8 * 1024 + 4, 8], 0, marks=pytest.mark.gpu),  # one vector past the grid's first step
+        pytest.param("cuda", [1001, 64], 0, marks=pytest.mark.gpu),  # not whole vectors: elementwise operations
+        pytest.param("cuda", [64, 64], 1, marks=pytest.mark.gpu),  # not 16-byte aligned: elementwise operations
+    ],
+)
+def test_adamw_step(device, sizes, shift):
+    g = torch.Generator(device=device).manual_seed(sum(sizes))
+
+    def make(n, dtype=torch.float32):
+        return torch.empty(n + shift, dtype=dtype, device=device)[shift:].copy_(torch.randn(n, generator=g, device=device))
+
+    p, m, gr = ([make(n) for n in sizes] for _ in range(3))
+    v = [make(n).abs_() for n in sizes]
+    w = [make(n, torch.bfloat16) for n in sizes]
+    gr[0][0] = v[0][0] = m[0][0] = 0.0  # an element that has never had a gradient only decays
+    old = [[t.double().clone() for t in ts] for ts in (p, m, v, gr)]
+    lr, b1, b2, eps, wd, t = 1e-2, 0.9, 0.95, 1e-8, 0.1, 3
+    c1, c2 = 1 - b1**t, 1 - b2**t
+    adamw_update(p, m, v, gr, w, lr=lr, b1=b1, b2=b2, eps=eps, weight_decay=wd, c1=c1, c2=c2)
+    u = 2.0**-24
+    for i in range(len(sizes)):
+        p0, m0, v0, g0 = (ts[i] for ts in old)
+        m1, v1 = b1 * m0 + (1 - b1) * g0, b2 * v0 + (1 - b2) * g0 * g0
+        step = lr / c1 * m1 / ((v1 / c2).sqrt() + eps)
+        p1 = p0 * (1 - lr * wd) - step
+        # a rounding for each coefficient, product and sum; the step adds those of the root, the sum and the quotients
+        dm, dv = 4 * u * ((b1 * m0).abs() + ((1 - b1) * g0).abs()), 5 * u * v1
+        assert bool(((m[i].double() - m1).abs() <= dm).all()) and bool(((v[i].double() - v1).abs() <= dv).all())
+        dstep = 12 * u * step.abs() + lr / c1 * dm / ((v1 / c2).sqrt() + eps)
+        assert bool(((p[i].double() - p1).abs() <= 4 * u * (p0.abs() + step.abs()) + dstep).all())
+        assert torch.equal(w[i], p[i].to(torch.bfloat16))
