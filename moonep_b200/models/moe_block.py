@@ -59,7 +59,9 @@ class TopKRouter(nn.Module):
         top_p, top_i = torch.topk(probs, self.k, dim=-1)
         gates = top_p / top_p.sum(dim=-1, keepdim=True)
         topk = top_i.to(torch.int32)
-        tpe = torch.bincount(top_i.reshape(-1), minlength=self.num_experts).to(torch.int32)
+        # counted without torch.bincount, which waits for the GPU to learn the largest index
+        tpe = torch.zeros(self.num_experts, dtype=torch.int32, device=x.device)
+        tpe.scatter_add_(0, top_i.reshape(-1), torch.ones_like(topk).reshape(-1))
         return gates.contiguous(), topk.contiguous(), tpe
 
 

@@ -134,8 +134,9 @@ class ExpertParallelMoE:
         combine's push role consumes.  Nothing is copied and nothing synchronises with the host."""
         buf = self.buffer
         x_nvs, w_nvs, cu, plan = buf.dispatch(x, gates, topk, tokens_per_expert, zero_copy=True)
-        fetched = buf.prefetch_weight(plan, async_finish=True, full_gate_weight=self.w_gate,
-                                      full_up_weight=self.w_up, full_down_weight=self.w_down)  # fmt: skip
+        alone = self.R == 1  # no expert is remote, and every kernel of the step follows the one before on this stream
+        fetched = None if alone else buf.prefetch_weight(plan, async_finish=True, full_gate_weight=self.w_gate,
+                                                         full_up_weight=self.w_up, full_down_weight=self.w_down)  # fmt: skip
         rows, dev = int(x_nvs.shape[0]), x_nvs.device
         if self._y is None:
             self._y = torch.empty(rows, self.H, dtype=torch.bfloat16, device=dev)
@@ -146,8 +147,8 @@ class ExpertParallelMoE:
             a = torch.empty(rows, self.I, dtype=torch.bfloat16, device=dev)
             u = torch.empty_like(a)
         # the hand-off hooks need the CTA-pair kernel's tiling; other shapes run after the prefetch, in stream order
-        hooked = rows >= 128 and self.H % 256 == 0 and self.I % 128 == 0
-        if not hooked:
+        hooked = not alone and rows >= 128 and self.H % 256 == 0 and self.I % 128 == 0
+        if fetched is not None and not hooked:
             torch.cuda.current_stream().wait_event(fetched)
         h = grouped_gemm(x_nvs, self.w_gate, cu, w_up=self.w_up, mode="swiglu", status=status,
                          save_pre=None if a is None else (a, u),
@@ -173,8 +174,8 @@ class ExpertParallelMoE:
             return self._forward_fast(x, gates, topk, tokens_per_expert, save_for_backward)
         x_nvs, w_nvs, cu, plan = buf.dispatch(x, gates, topk, tokens_per_expert, zero_copy=True)
         # the weight copies run on the communication stream while this stream saves the dispatched rows
-        fetched = buf.prefetch_weight(plan, async_finish=True, full_gate_weight=self.w_gate,
-                                      full_up_weight=self.w_up, full_down_weight=self.w_down)  # fmt: skip
+        fetched = None if self.R == 1 else buf.prefetch_weight(plan, async_finish=True, full_gate_weight=self.w_gate,
+                                                               full_up_weight=self.w_up, full_down_weight=self.w_down)  # fmt: skip
         x_saved = x_nvs.clone() if save_for_backward else x_nvs  # training: the shard is reused for the expert output
         if hasattr(fetched, "wait") and x_nvs.is_cuda:
             torch.cuda.current_stream().wait_event(fetched)
@@ -254,7 +255,7 @@ class ExpertParallelMoE:
             sel[i], sel[3 + i] = grads[i], self.red[i]
             reduced.append(self.buffer.reduce_grad(plan, True, *sel, owner_local=True))
 
-        overlap = config.backward_overlap() and x_nvs.is_cuda
+        overlap = self.R > 1 and config.backward_overlap() and x_nvs.is_cuda
         sms = 0
         if overlap:
             total = torch.cuda.get_device_properties(dev).multi_processor_count
@@ -267,7 +268,7 @@ class ExpertParallelMoE:
         if reduced:
             for ev in reduced:  # the gradients are complete, and the reduce slots cleared, for whatever comes next
                 torch.cuda.current_stream().wait_event(ev)
-        else:
+        elif self.R > 1:  # a single rank has no copies of experts, hence no gradients to bring home
             self.buffer.reduce_grad(plan, False, *grads, self.red[0], self.red[1], self.red[2], owner_local=True)
         return dx, dgates
 

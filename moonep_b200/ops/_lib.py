@@ -17,6 +17,8 @@ import subprocess
 import threading
 from pathlib import Path
 
+import torch
+
 _PKG = Path(__file__).resolve().parent.parent
 CSRC = _PKG / "csrc"
 LIBDIR = _PKG / "lib"
@@ -159,6 +161,29 @@ def load():
                 fn.argtypes = args
             _lib = lib
     return _lib
+
+
+def current_stream() -> int:
+    """Handle of the current stream of the current device (``torch.cuda.current_stream().cuda_stream`` without the
+    Stream object, whose construction costs several microseconds)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+class on_device:
+    """``torch.cuda.device(dev)`` that does nothing when ``dev`` is already the current device."""
+
+    __slots__ = ("guard",)
+
+    def __init__(self, dev: torch.device):
+        self.guard = None if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+
+    def __enter__(self):
+        if self.guard is not None:
+            self.guard.__enter__()
+
+    def __exit__(self, *exc):
+        if self.guard is not None:
+            self.guard.__exit__(*exc)
 
 
 class NativeError(RuntimeError):

@@ -59,7 +59,7 @@ def _ptr(t: torch.Tensor | None) -> int | None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _lib.current_stream()
 
 
 class CudaBackend:
@@ -130,7 +130,7 @@ class CudaBackend:
             self.tpe_prev.data_ptr(), self.tables.data_ptr(), self.stats_buf.data_ptr(), self.block_hist.data_ptr(),
         ]  # fmt: skip
         arr = (ctypes.c_longlong * len(params))(*params)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             self.handle = self.lib.moonep_ctx_create(arr, len(params), hp, mp, sp)
         if not self.handle:
             raise _lib.NativeError("moonep_ctx_create failed: " + self.lib.moonep_last_error().decode())
@@ -208,7 +208,7 @@ class CudaBackend:
     # launch, skipped when replays follow each other), so graph replays and ordinary calls can be mixed.
     def _bias_launch(self, values, mode):
         arr = (ctypes.c_int * NUM_FLAG_FAMILIES)(*[int(v) for v in values])
-        with torch.cuda.device(self.ctx["device"]):
+        with _lib.on_device(self.ctx["device"]):
             _lib.check(self.lib.moonep_epoch_bias(self.handle, arr, int(mode), _stream()), "moonep_epoch_bias")
 
     def capture_begin(self):
@@ -250,7 +250,7 @@ class CudaBackend:
         self._quiesced = end["quiesced"]
 
     def _call(self, name, *args, tag=None):
-        with torch.cuda.device(self.ctx["device"]):
+        with _lib.on_device(self.ctx["device"]):
             if self._nvtx:
                 torch.cuda.nvtx.range_push(tag or name)
                 try:

@@ -113,7 +113,7 @@ def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", o
     lib = _lib.load()
     use_pair = config.gemm_on_cta_pairs() if pair is None else pair
     assert hooks is None or use_pair, "hooks need the CTA-pair kernel"
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         args = (
             x.data_ptr(), w.data_ptr(), None if w_up is None else w_up.data_ptr(), out.data_ptr(),
             None if row_scale is None else row_scale.data_ptr(), cu_seqlens.data_ptr(), G, int(x.shape[0]), K, N,
@@ -121,7 +121,7 @@ def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", o
             None if group_map is None else group_map.data_ptr(), W,
             None if save_pre is None else save_pre[0].data_ptr(), None if save_pre is None else save_pre[1].data_ptr(),
         )  # fmt: skip
-        st = torch.cuda.current_stream().cuda_stream
+        st = _lib.current_stream()
         if hooks is not None:
             rc = lib.moonep_grouped_gemm_pair_hooked(*args, ctypes.byref(hooks), st)
         else:
@@ -171,11 +171,11 @@ def grouped_gemm_kn(x, ws, cu_seqlens, *, out=None, status=None, num_sms=0):
         out = torch.empty(x.shape[0], N, dtype=torch.bfloat16, device=x.device)
     assert out.is_contiguous() and out.shape == (x.shape[0], N) and out.dtype == torch.bfloat16
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         rc = lib.moonep_grouped_gemm_pair_kn(
             x.data_ptr(), ws[0].data_ptr(), Ks[0], ws[1].data_ptr() if len(ws) == 2 else None, Ks[1] if len(ws) == 2 else 0,
             out.data_ptr(), cu_seqlens.data_ptr(), G, int(x.shape[0]), N, G, None if status is None else status.data_ptr(),
-            config.timeout_ms(), int(num_sms), torch.cuda.current_stream().cuda_stream,
+            config.timeout_ms(), int(num_sms), _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_grouped_gemm_pair_kn")
     return out
@@ -229,11 +229,11 @@ def grouped_wgrad(left_t, right_t, cu_seqlens, out_ptrs, flags, *, status=None, 
     assert flags.dtype == torch.int32 and flags.numel() == G and flags.is_cuda and flags.is_contiguous()
     assert cu_seqlens.dtype == torch.int32 and cu_seqlens.is_contiguous() and cu_seqlens.is_cuda
     lib = _lib.load()
-    with torch.cuda.device(left_t.device):
+    with _lib.on_device(left_t.device):
         rc = lib.moonep_grouped_wgrad(
             left_t.data_ptr(), right_t.data_ptr(), ld, P, Q, cu_seqlens.data_ptr(), G, out_ptrs.data_ptr(),
             flags.data_ptr(), ld, None if status is None else status.data_ptr(), config.timeout_ms(), int(num_sms),
-            torch.cuda.current_stream().cuda_stream,
+            _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_grouped_wgrad")
 
@@ -254,11 +254,11 @@ def grouped_wgrad_rows(left, right, cu_seqlens, out_ptrs, flags, *, status=None,
     assert flags.dtype == torch.int32 and flags.numel() == G and flags.is_cuda and flags.is_contiguous()
     assert cu_seqlens.dtype == torch.int32 and cu_seqlens.is_contiguous() and cu_seqlens.is_cuda
     lib = _lib.load()
-    with torch.cuda.device(left.device):
+    with _lib.on_device(left.device):
         rc = lib.moonep_grouped_wgrad_rows(
             left.data_ptr(), ldl, right.data_ptr(), ldr, rows, P, Q, cu_seqlens.data_ptr(), G, out_ptrs.data_ptr(),
             flags.data_ptr(), None if status is None else status.data_ptr(), config.timeout_ms(), int(num_sms),
-            torch.cuda.current_stream().cuda_stream,
+            _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_grouped_wgrad_rows")
 

@@ -25,10 +25,10 @@ def transpose_experts(src: torch.Tensor, dst: torch.Tensor, col0: int = 0, activ
                 dst[i, :, col0 : col0 + d0] = src[i].transpose(0, 1)
         return dst
     assert src.is_contiguous() and src.dtype == torch.bfloat16 and dst.dtype == torch.bfloat16
-    with torch.cuda.device(src.device):
+    with _lib.on_device(src.device):
         rc = _lib.load().moonep_transpose_experts(
             src.data_ptr(), dst.data_ptr(), n, d0, d1, int(dst.shape[2]), int(dst.shape[1]) * int(dst.shape[2]), int(col0),
-            None if active is None else active.data_ptr(), torch.cuda.current_stream().cuda_stream,
+            None if active is None else active.data_ptr(), _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_transpose_experts")
     return dst
@@ -51,10 +51,10 @@ def swiglu_bwd(a, u, g, w, total_rows, dadu, hsw, dgate) -> None:
     for t in (a, u, g, dadu, hsw):
         assert t.is_contiguous() and t.dtype == torch.bfloat16
     assert w.dtype == torch.float32 and dgate.dtype == torch.float32 and w.is_contiguous() and dgate.is_contiguous()
-    with torch.cuda.device(a.device):
+    with _lib.on_device(a.device):
         rc = _lib.load().moonep_swiglu_bwd(
             a.data_ptr(), u.data_ptr(), g.data_ptr(), w.data_ptr(), None if total_rows is None else total_rows.data_ptr(),
-            rows, I, dadu.data_ptr(), hsw.data_ptr(), dgate.data_ptr(), torch.cuda.current_stream().cuda_stream,
+            rows, I, dadu.data_ptr(), hsw.data_ptr(), dgate.data_ptr(), _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_swiglu_bwd")
 
@@ -66,9 +66,9 @@ def sgd_update(w: torch.Tensor, g: torch.Tensor, lr: float) -> None:
         w.add_(g, alpha=-lr)
         return
     assert w.is_contiguous() and g.is_contiguous() and w.dtype == torch.bfloat16 and g.dtype == torch.float32
-    with torch.cuda.device(w.device):
+    with _lib.on_device(w.device):
         rc = _lib.load().moonep_sgd_update(w.data_ptr(), g.data_ptr(), w.numel(), float(lr),
-                                           torch.cuda.current_stream().cuda_stream)  # fmt: skip
+                                           _lib.current_stream())  # fmt: skip
     _lib.check(rc, "moonep_sgd_update")
 
 
@@ -94,7 +94,7 @@ def adamw_update(masters, exp_avgs, exp_avg_sqs, grads, weights, *, lr, b1, b2, 
     n = len(tensors[4])
     ptrs = [(ctypes.c_void_p * n)(*[t.data_ptr() for t in ts]) for ts in tensors]
     sizes = (ctypes.c_longlong * n)(*[t.numel() for t in tensors[4]])
-    with torch.cuda.device(weights[0].device):
+    with _lib.on_device(weights[0].device):
         rc = _lib.load().moonep_adamw_update(n, *ptrs, sizes, lr / c1, b1, b2, eps, 1.0 - lr * weight_decay, c2,
-                                             torch.cuda.current_stream().cuda_stream)  # fmt: skip
+                                             _lib.current_stream())  # fmt: skip
     _lib.check(rc, "moonep_adamw_update")

@@ -111,7 +111,9 @@ def _round4(n: int) -> int:
 
 
 def _i32(n: int, dev) -> torch.Tensor:
-    # Over-allocated to a multiple of four words so kernels may use 16-byte accesses.
+    # A multiple of four words so kernels may use 16-byte accesses; CUDA's allocators round up by themselves.
+    if n % 4 == 0 or dev.type == "cuda":
+        return torch.empty(n, dtype=torch.int32, device=dev)
     return torch.empty(_round4(n), dtype=torch.int32, device=dev)[:n]
 
 
@@ -159,10 +161,11 @@ def check_plan_for_ctx(ctx: dict, plan: MoonEPCommPlan, device) -> None:
         "dst": (N,), "experts_to_copy": (R, B), "zero_fill_ranges": (E + B, 2), "remote_stats": (2,),
         "dup_groups": (NvS, 3), "dup_loffs": (NvS,), "dup_counts": (2,), "src_info": (NvS,), "link": (NvS,),
     }  # fmt: skip
+    device = torch.device(device)
     for name, shape in shapes.items():
         t = getattr(plan, name)
         if t is None:  # the two optional trailing fields
             continue
         assert t.dtype == torch.int32 and t.is_contiguous(), f"plan.{name} must be contiguous int32"
         assert tuple(t.shape) == shape, f"plan.{name} must have shape {shape}, got {tuple(t.shape)}"
-        assert t.device == torch.device(device), f"plan.{name} is on the wrong device"
+        assert t.device == device, f"plan.{name} is on the wrong device"
