@@ -281,9 +281,9 @@ class Buffer:
                       *, inter_rank_sync, zero_copy):  # fmt: skip
         be = ctx["_backend"]
         if hasattr(be, "dispatch_all"):  # CUDA: fused launches (one role per phase for emulated ranks)
-            be.dispatch_all(hidden_sh, route_weights_sk, plan, planning_args, inter_rank_sync)
-            if not zero_copy:
-                be.copy_out(hidden_nvsh, route_weights_nvs)
+            copy_to = None if zero_copy else (hidden_nvsh, route_weights_nvs)
+            if not be.dispatch_all(hidden_sh, route_weights_sk, plan, planning_args, inter_rank_sync, copy_to) and copy_to:
+                be.copy_out(*copy_to)
             return
         wait = None
         if planning_args is not None:

@@ -217,14 +217,15 @@ int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk, const int*
 
 // Dispatch of a Buffer with one rank: one launch, fresh (planner arguments as above, tpe [E]) or replayed (dst and
 // zero_fill come from the plan).  n_ctas bounds the grid (<= 0: every SM of local_sms).  Fresh plans need
-// moonep_single_supported(E, B, S, K); work is local scratch of moonep_single_work_words() zeros.  See single_rank.cu.
+// moonep_single_supported(E, B, S, K); work is local scratch of moonep_single_work_words() zeros.
+// out / out_w (optional, fresh plans): [NvS, H] and [NvS], receive the shard and its weights as they are afterwards.  See single_rank.cu.
 int moonep_single_supported(int E, int B, int S, int K);
 int moonep_single_work_words(void);
 int moonep_dispatch_single(void* ctx, int fresh, const int* topk, const int* tpe, int* dst, int* cu_seqlens,
                            int* experts_to_copy, int* zero_fill, int* remote_stats, int* dup_groups, int* dup_loffs,
                            int* dup_counts, int* plan_src_info, int* plan_link, const void* hidden, const float* weights,
                            int with_weights, int epoch_tpe, int epoch_plan, int epoch_sent, int n_ctas, int* work,
-                           void* stream);
+                           void* out, float* out_w, void* stream);
 // Combine of a Buffer with one rank: out[token] = the sum of the token's rows in ascending k (fp32, rounded once),
 // out_w[token, k] = in_w of the entry's row.  ready / ready_expect as in moonep_combine_push.
 int moonep_combine_single(void* ctx, const int* dst, const void* in_rows, const float* in_w, void* out, float* out_w,

@@ -364,17 +364,20 @@ class CudaBackend:
             tag=tag,
         )  # fmt: skip
 
-    def dispatch_all(self, hidden_sh, route_weights_sk, plan, planning_args, inter_rank_sync):
+    def dispatch_all(self, hidden_sh, route_weights_sk, plan, planning_args, inter_rank_sync, copy_to=None):
         """The whole dispatch.  Fresh plan: ``plan_publish`` plus one fused launch (planner tables, token planning, row
         push, and on the destination side zero fill, duplicate map and duplicate expansion as rows arrive).  Replayed
-        plan: an optional READY round plus one launch (push and expansion).  Emulated ranks run one role per phase."""
+        plan: an optional READY round plus one launch (push and expansion).  Emulated ranks run one role per phase.
+        ``copy_to``: tensors that receive the shard and (or None) its weights; True is returned when this call has seen
+        to it, otherwise ``copy_out`` is left to the caller."""
         with_w = route_weights_sk is not None
         self._sent_weights = with_w
         lr = ROLE_LOCAL_ROWS if config.local_rows_by_expand() else 0
         if self.single and lr and (planning_args is None or config.planner_on_gpu()):
-            self._dispatch_single(hidden_sh, route_weights_sk, plan, planning_args)
+            fused = copy_to if planning_args is not None else None
+            self._dispatch_single(hidden_sh, route_weights_sk, plan, planning_args, fused)
             self._quiesced = True
-            return
+            return fused is not None
         if planning_args is not None:
             topk_flat, tpe, cu_seqlens = planning_args
             on_dev = config.planner_on_gpu()
@@ -424,10 +427,12 @@ class CudaBackend:
                 self.world.step()
                 self._dispatch_launch(ROLE_EXPAND | lr, False, plan, tag="dispatch_expand", **kw)
         self.world.step()
+        return False
 
-    def _dispatch_single(self, hidden, weights, plan, planning_args):
+    def _dispatch_single(self, hidden, weights, plan, planning_args, copy_to=None):
         """Fresh or replayed dispatch of a single rank: one launch, no READY round (there are no peers to wait for)."""
         topk, tpe, cu = planning_args if planning_args is not None else (None, None, None)
+        out, out_w = copy_to if copy_to is not None else (None, None)
         if topk is not None:
             self._topk = topk
             self._next(FLAG_TPE)
@@ -437,7 +442,7 @@ class CudaBackend:
             _ptr(plan.experts_to_copy), _ptr(plan.zero_fill_ranges), _ptr(plan.remote_stats), _ptr(plan.dup_groups),
             _ptr(plan.dup_loffs), _ptr(plan.dup_counts), _ptr(plan.src_info), _ptr(plan.link), _ptr(hidden), _ptr(weights),
             int(weights is not None), self._cur(FLAG_TPE), self._cur(FLAG_PLAN), self._next(FLAG_SENT), self.n_expand,
-            _ptr(self.single_work), _stream(), tag="dispatch_single",
+            _ptr(self.single_work), _ptr(out), _ptr(out_w), _stream(), tag="dispatch_single",
         )  # fmt: skip
 
     def copy_out(self, out_hidden, out_weights):

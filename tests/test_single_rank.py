@@ -52,7 +52,13 @@ def test_replay_and_unaligned_inputs(S, H, K, E, pad, shift):
     buf = Buffer(S, H, K, E, 1, token_padding=pad)
     x, topk, tpe = _inputs(S, H, K, E, shift)
     gates = torch.rand(S, K, device="cuda")
-    rows, _, cu, plan = buf.dispatch(x, gates, topk, tpe)
+    ctx = buf._require_ctx()
+    ctx["hidden_buf_local"].fill_(7.0)
+    ctx["weights_buf_local"].fill_(3)
+    rows, w, cu, plan = buf.dispatch(x, gates, topk, tpe)
+    # a staged dispatch returns the whole shard and its weights, rows that no group uses included
+    assert torch.equal(rows, ctx["hidden_buf_local"]) and torch.equal(w.view(torch.int32), ctx["weights_buf_local"])
+    assert bool((rows[int(cu[-1]) :] == 7.0).all())
     x2 = torch.empty_like(x).copy_(-x)
     buf._require_ctx()["hidden_buf_local"].fill_(7.0)
     rows2, w2, _, _ = buf.dispatch(x2, gates, plan=plan, zero_copy=True)
@@ -78,8 +84,10 @@ def test_counts_that_do_not_match_the_routing():
     S, H, K, E = 200, 64, 2, 6
     buf = Buffer(S, H, K, E, 1, token_padding=8)
     x, topk, tpe = _inputs(S, H, K, E, 0)
-    plan = buf.dispatch(x, None, topk, tpe + torch.tensor([0, 3, 0, 0, 0, 1], dtype=torch.int32, device="cuda"))[3]
+    buf._require_ctx()["hidden_buf_local"].fill_(7.0)
+    rows, _, _, plan = buf.dispatch(x, None, topk, tpe + torch.tensor([0, 3, 0, 0, 0, 1], dtype=torch.int32, device="cuda"))
     buf.synchronize()
+    assert torch.equal(rows, buf._require_ctx()["hidden_buf_local"])
     assert int((plan.src_info >= 0).sum()) == S * K
     for bad_topk, bad_tpe in ((topk, tpe - (tpe > 0).int()), (torch.where(topk == 2, E, topk), tpe)):
         buf.dispatch(x, None, bad_topk.contiguous(), bad_tpe)
