@@ -542,11 +542,13 @@ __device__ void plan_tokens(const MoonepDevCtx& c, const SingleArgs& a, SingleSh
     // token counts above what was routed leave rows that nothing landed in
     plan_sync();
     for (int e = tid; e < E; e += kEntries)
-      for (int g = cur[e]; g < cnt[e] && off[e] + g < NvS; ++g) {
-        meta[c.src_info_off + off[e] + g] = -1;
-        if (a.plan_src_info != nullptr) a.plan_src_info[off[e] + g] = -1;
-        if (a.plan_link != nullptr) a.plan_link[off[e] + g] = 0;
-        if (a.out != nullptr) copy_tail(c, a, meta, off[e] + g, off[e] + g + 1, 0, 1);
+      for (int g = cur[e]; g < cnt[e]; ++g) {
+        const int row = off[e] + g;
+        if (row < 0 || row >= NvS) break;  // absurd counts: recorded by CTA 0
+        meta[c.src_info_off + row] = -1;
+        if (a.plan_src_info != nullptr) a.plan_src_info[row] = -1;
+        if (a.plan_link != nullptr) a.plan_link[row] = 0;
+        if (a.out != nullptr) copy_tail(c, a, meta, row, row + 1, 0, 1);
       }
   }
 }
