@@ -1,0 +1,440 @@
+// Weight gradients of every group on CTA pairs (tcgen05 cta_group::2, sm_100a): contraction over the rows of a group,
+//
+//   dW[g] (P x Q, fp32) (=, +=) L[rows of g, :P]^T  @  R[rows of g, :Q]
+//
+// The operands are taken as stored (L: [rows, P], R: [rows, Q]; tiles are staged MN-major, see make_smem_desc_mn) or
+// transposed (Lt: [P, ld], Rt: [Q, ld], the row index contiguous, K-major tiles as in the forward kernel).  The K loop
+// of a tile runs over the group's rows (k0 = first row of the group, any multiple of 16 rows long; the last 64-row
+// block issues only the MMAs that lie inside the group).  The groups that have anything to do are listed once per CTA in
+// shared memory (in group order, the same list in every CTA), so empty groups cost nothing.  Per group, flags[g]
+// selects: 0 store (and store zeros if the group has no rows), 1 add to what is there, 2 store, leave the target alone
+// if the group has no rows.  A null out_ptrs[g] skips the group; rows without a target are reported through the status
+// block.
+//
+// A cluster of two CTAs computes a 256 x 256 tile (as in grouped_gemm_pair.cu): 32 KB of operands per CTA and 64 rows
+// instead of the 48 KB of one CTA per 128 x 256 tile.  The accumulator is dW^T: TMEM lanes (the M index, 128 per CTA) run
+// along Q, columns along P, so the 32 lanes of a warp hold 32 neighbours of a row of dW and every store instruction of the
+// epilogue fills one 128-byte line straight from registers.  Lanes along P instead cost four times the L1 cycles (a sector
+// per lane), or a turn through shared memory, whose slots the MMAs need.  When P is an odd multiple of 128 the last tile
+// has 128 columns that are computed from zeros and not stored.
+//
+// Bound by the tensor pipe and the fp32 results together: a tile of 1024 rows is 16 K blocks of MMAs and 256 KB of output.
+// 8 groups x 1024 rows, 2048 x 7168: 258 us with one CTA per tile, 241 us here (985 TFLOP/s); adding to the old values 301
+// and 262; 16 groups x 512 rows, 1024 x 2048: 53.6 and 49.5.  (Lanes along P, 32-byte stores: 236, 369, 57.7; results
+// through shared memory in 512-byte bulk stores: 242 and 50 in a training step, an SM takes 15 clocks per bulk store.)
+//
+// Every mbarrier wait is bounded; on expiry the role records a status word and leaves its loop (see
+// grouped_gemm_pair.cu for how a pair is torn down).
+//
+// No counterpart in the reference, which has no GEMM.
+#include "umma.cuh"
+
+namespace moonep {
+
+namespace {
+
+constexpr int kStages = 6;
+constexpr int kThreads = 192;
+constexpr int kTmemCols = 512;
+constexpr unsigned kHalfBytes = 128 * BK * 2;     // 16 KB: this CTA's columns of L, its half of R
+constexpr unsigned kStageBytes = 2 * kHalfBytes;  // 32 KB per CTA and stage
+constexpr int kWgradMaxGroups = 512;  // groups per launch (their work list lives in shared memory)
+
+struct WgradArgs {
+  float* const* out_ptrs;  // [G] device array
+  const int* flags;        // [G]
+  const int* cu_seqlens;   // [G] inclusive padded ends
+  int* status;
+  unsigned long long timeout_ns;
+  int G, P, Q, p_tiles, q_tiles, rows_cap;
+  int row_major;  // operands are L [rows, P] and R [rows, Q] as they are (MN-major tiles) instead of their transposes
+};
+
+
+struct WgradGroups {  // per listed group: which group, its first row, its rows, target and mode
+  int n;
+  short g[kWgradMaxGroups];
+  int start[kWgradMaxGroups];
+  int krows[kWgradMaxGroups];
+  int flag[kWgradMaxGroups];
+  float* out[kWgradMaxGroups];
+};
+
+// Warp-collective: list the groups with rows, and the empty ones whose target must be zeroed, in group order.
+__device__ __forceinline__ void wgrad_list_groups(const WgradArgs& a, WgradGroups& sg, int lane) {
+  int n = 0;
+  for (int base = 0; base < a.G; base += 32) {
+    const int g = base + lane;
+    bool listed = false;
+    int start = 0, krows = 0, flag = 0;
+    float* out = nullptr;
+    if (g < a.G) {
+      start = g > 0 ? min(a.cu_seqlens[g - 1], a.rows_cap) : 0;
+      const int end = min(a.cu_seqlens[g], a.rows_cap);
+      krows = end > start ? end - start : 0;
+      out = a.out_ptrs[g];
+      flag = a.flags[g];
+      // the K coordinate of a TMA copy must be a multiple of 8 elements and the MMAs take 16 rows at a time:
+      // a group that does not start and end on a multiple of 16 is refused (reported as rows without a target)
+      if (((start | end) & 15) != 0) out = nullptr;
+      listed = krows > 0 || (out != nullptr && flag == 0);
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, listed);
+    const int pos = n + __popc(mask & ((1u << lane) - 1u));
+    if (listed && pos < kWgradMaxGroups) {
+      sg.g[pos] = (short)g;
+      sg.start[pos] = start;
+      sg.krows[pos] = krows;
+      sg.flag[pos] = flag;
+      sg.out[pos] = out;
+    }
+    n += __popc(mask);
+  }
+  if (lane == 0) sg.n = min(n, kWgradMaxGroups);
+}
+
+struct WgradTile {
+  int g, pb, qb, k0, krows, flag;
+  float* out;
+};
+
+__device__ __forceinline__ WgradTile wgrad_tile(const WgradArgs& a, const WgradGroups& sg, long long t) {
+  WgradTile w;
+  const int per_group = a.p_tiles * a.q_tiles;
+  const int idx = (int)(t / per_group);
+  const int rem = (int)(t % per_group);
+  w.pb = rem / a.q_tiles;
+  w.qb = rem % a.q_tiles;
+  w.g = sg.g[idx];
+  w.k0 = sg.start[idx];
+  w.krows = sg.krows[idx];
+  w.flag = sg.flag[idx];
+  w.out = sg.out[idx];
+  return w;
+}
+
+// 32 accumulator columns (rows of dW, ld apart) of this lane's column of dW: stored, or added to what is there.
+__device__ __forceinline__ void put_cols(float* dst, long long ld, const unsigned (&v)[32], bool add) {
+  if (add) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + j * ld), "f"(__uint_as_float(v[j])) : "memory");
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      asm volatile("st.global.L1::no_allocate.b32 [%0], %1;" ::"l"(dst + j * ld), "r"(v[j]) : "memory");
+  }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_l, const __grid_constant__ CUtensorMap tmap_r,
+                         const WgradArgs a) {
+  extern __shared__ unsigned char s_raw[];
+  __shared__ __align__(8) unsigned long long s_full[kStages], s_empty[kStages], s_tfull[2], s_tempty[2], s_done;
+  __shared__ unsigned s_tmem_base;
+  __shared__ WgradGroups s_groups;
+  unsigned char* s_tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned rank = cluster_ctarank();  // 0: leader (issues the MMAs), 1: its peer
+  if (warp == 0) wgrad_list_groups(a, s_groups, lane);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(s_full + s, 1);   // used in the leader: its own arrive.expect_tx; both CTAs' copies complete the bytes
+      mbar_init(s_empty + s, 1);  // one commit of the leader's MMA lane, delivered to both CTAs
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(s_tfull + b, 1);   // one commit, delivered to both CTAs
+      mbar_init(s_tempty + b, 8);  // used in the leader: four epilogue warps of each CTA
+    }
+    mbar_init(&s_done, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&s_tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the peer's barriers exist before anything is delivered to them
+  tc_fence_after();
+  const unsigned tmem_base = s_tmem_base;
+  // both CTAs own their whole TMEM, so the accumulators start at column 0 in both
+  const bool tmem_ok = (tmem_base & 0xFFFFu) == 0;
+  if (!tmem_ok && threadIdx.x == 0) gemm_fail(a.status, 14, 9, (int)tmem_base, 0);
+  const long long pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const long long num_tiles = (long long)s_groups.n * a.p_tiles * a.q_tiles;
+
+  if (warp == 0) {
+    // ---------------- TMA producer (both CTAs) ----------------
+    if (lane == 0 && tmem_ok) {
+      int stage = 0;
+      unsigned phase = 0;
+      bool failed = false;
+      for (long long t = pair; t < num_tiles && !failed; t += npairs) {
+        const WgradTile w = wgrad_tile(a, s_groups, t);
+        if (w.krows == 0 || w.out == nullptr) continue;
+        const int kbs = (w.krows + BK - 1) / BK;
+        const int q0 = w.qb * BN + (int)rank * 128, p0 = w.pb * BN + (int)rank * 128;  // p0 may lie past P: zeros
+        for (int kb = 0; kb < kbs; ++kb) {
+          if (!mbar_wait_cluster(s_empty + stage, phase ^ 1u, a.timeout_ns)) {
+            gemm_fail(a.status, 14, 1, stage, kb);
+            failed = true;
+            break;
+          }
+          unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
+          if (rank == 0) mbar_expect_tx(s_full + stage, 2 * kStageBytes);
+          const unsigned full_of_leader = mapa_u32(s_full + stage, 0);
+          const int k = w.k0 + kb * BK;
+          if (a.row_major) {  // boxes of 64 columns x 64 rows, two for R and two for L
+            tma_load_2d_pair(st, &tmap_r, q0, k, full_of_leader);
+            tma_load_2d_pair(st + kMnBoxBytes, &tmap_r, q0 + 64, k, full_of_leader);
+            tma_load_2d_pair(st + kHalfBytes, &tmap_l, p0, k, full_of_leader);
+            tma_load_2d_pair(st + kHalfBytes + kMnBoxBytes, &tmap_l, p0 + 64, k, full_of_leader);
+          } else {
+            tma_load_2d_pair(st, &tmap_r, k, q0, full_of_leader);
+            tma_load_2d_pair(st + kHalfBytes, &tmap_l, k, p0, full_of_leader);
+          }
+          if (++stage == kStages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (leader only) ----------------
+    if (lane == 0 && rank == 0 && tmem_ok) {
+      constexpr unsigned idesc = make_idesc(2 * BM, BN);
+      constexpr unsigned idesc_mn = make_idesc(2 * BM, BN, true, true);
+      const unsigned kstep = a.row_major ? kDescStepMn : kDescStepK;
+      int stage = 0;
+      unsigned phase = 0;
+      unsigned tphase[2] = {0, 0};
+      int it = 0;
+      bool failed = false;
+      for (long long t = pair; t < num_tiles && !failed; t += npairs) {
+        const WgradTile w = wgrad_tile(a, s_groups, t);
+        if (w.krows == 0 || w.out == nullptr) continue;
+        const int buf = it & 1;
+        ++it;
+        if (!mbar_wait_cluster(s_tempty + buf, tphase[buf] ^ 1u, a.timeout_ns)) {
+          gemm_fail(a.status, 14, 2, buf, it);
+          break;
+        }
+        tphase[buf] ^= 1u;
+        tc_fence_after();
+        const unsigned d_tmem = tmem_base + (unsigned)(buf * BN);
+        const int kbs = (w.krows + BK - 1) / BK;
+        for (int kb = 0; kb < kbs; ++kb) {
+          if (!mbar_wait_cluster(s_full + stage, phase, a.timeout_ns)) {
+            gemm_fail(a.status, 14, 3, stage, kb);
+            failed = true;
+            break;
+          }
+          tc_fence_after();
+          const unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
+          const unsigned long long adesc = a.row_major ? make_smem_desc_mn(st) : make_smem_desc(st);
+          const unsigned long long bdesc = a.row_major ? make_smem_desc_mn(st + kHalfBytes) : make_smem_desc(st + kHalfBytes);
+          const int nkk = min(BK / UMMA_K, (w.krows - kb * BK) / UMMA_K);  // MMAs inside the group
+          for (int kk = 0; kk < nkk; ++kk)
+            umma_bf16_pair(d_tmem, adesc + (unsigned long long)(kk * kstep), bdesc + (unsigned long long)(kk * kstep),
+                      a.row_major ? idesc_mn : idesc, (kb | kk) != 0 ? 1u : 0u);
+          umma_commit_pair(s_empty + stage, 3);
+          if (++stage == kStages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+        if (!failed) umma_commit_pair(s_tfull + buf, 3);
+      }
+      // the pair must not be torn down under a running MMA: wait for everything issued so far
+      umma_commit_pair(&s_done, 1);
+      if (!mbar_wait_cluster(&s_done, 0, a.timeout_ns)) gemm_fail(a.status, 14, 5, 0, 0);
+    }
+    __syncwarp();
+  } else {
+    // ---------------- epilogue (warps 2..5, both CTAs): one column of dW per thread ----------------
+    const int q = warp & 3;
+    const unsigned tempty_of_leader[2] = {mapa_u32(s_tempty + 0, 0), mapa_u32(s_tempty + 1, 0)};
+    unsigned tphase[2] = {0, 0};
+    int it = 0;
+    for (long long t = pair; tmem_ok && t < num_tiles; t += npairs) {
+      const WgradTile w = wgrad_tile(a, s_groups, t);
+      const int flag = w.flag;
+      if (w.out == nullptr) {
+        if (w.krows != 0 && rank == 0 && q == 0 && lane == 0 && w.pb == 0 && w.qb == 0 && a.status != nullptr &&
+            atomicCAS(a.status + MOONEP_ST_CODE, 0, MOONEP_STATUS_BAD_INDEX) == 0) {
+          a.status[MOONEP_ST_KERNEL] = 14;
+          a.status[MOONEP_ST_FAMILY] = 100;  // kind: rows of a group whose gradient has no target
+          a.status[MOONEP_ST_PEER] = w.g;
+          a.status[MOONEP_ST_EXPECT] = 0;
+          a.status[MOONEP_ST_SEEN] = w.krows;
+          __threadfence();
+        }
+        continue;
+      }
+      float* out = w.out + (long long)w.pb * BN * a.Q + w.qb * BN + (int)rank * 128 + q * 32 + lane;
+      const int cols = min(BN, a.P - w.pb * BN);  // rows of dW in this tile: 256, or 128 in the last tile of an odd P
+      if (w.krows == 0) {
+        if (flag == 0)
+          for (int c = 0; c < cols; ++c) out[(long long)c * a.Q] = 0.f;
+        continue;
+      }
+      const int buf = it & 1;
+      ++it;
+      int got = 1;
+      if (lane == 0) got = mbar_wait_cluster(s_tfull + buf, tphase[buf], a.timeout_ns) ? 1 : 0;
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (!got) {
+        if (lane == 0) gemm_fail(a.status, 14, 4, buf, it);
+        break;
+      }
+      tphase[buf] ^= 1u;
+      tc_fence_after();
+      const unsigned taddr = tmem_base + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN);
+      const bool add = flag == 1;
+      unsigned v[32], u[32];
+      tmem_ld32(taddr, v);
+#pragma unroll 1
+      for (int c0 = 0; c0 < cols; c0 += 64) {  // the load of 32 columns overlaps the stores of the 32 before
+        tmem_ld_wait();
+        tmem_ld32(taddr + (unsigned)(c0 + 32), u);
+        put_cols(out + (long long)c0 * a.Q, a.Q, v, add);
+        tmem_ld_wait();
+        if (c0 + 64 < cols) tmem_ld32(taddr + (unsigned)(c0 + 64), v);
+        put_cols(out + (long long)(c0 + 32) * a.Q, a.Q, u, add);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(tempty_of_leader[buf]);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // nobody delivers to, or computes on, a CTA that has left
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+}  // namespace
+
+}  // namespace moonep
+
+using namespace moonep;
+
+static int launch_wgrad(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs& a, int num_sms, void* stream) {
+  a.p_tiles = (a.P + BN - 1) / BN;  // the last tile of an odd P computes 128 columns that are not stored
+  const size_t smem = (size_t)kStages * kStageBytes + 1024;
+  static int max_pairs = -1;  // pairs of these CTAs the device runs at once
+  if (max_pairs < 0) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(grouped_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem),
+                            "cudaFuncSetAttribute(grouped_wgrad_kernel)"))
+      return rc;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (int rc = check_cuda(cudaOccupancyMaxActiveClusters(&n, grouped_wgrad_kernel, &cfg),
+                            "cudaOccupancyMaxActiveClusters(grouped_wgrad_kernel)"))
+      return rc;
+    max_pairs = n;
+  }
+  if (max_pairs < 1) {
+    set_error("moonep_grouped_wgrad: the device cannot run a pair of these CTAs");
+    return 1;
+  }
+  int pairs = max_pairs;
+  if (num_sms > 0) pairs = imax(1, imin(pairs, num_sms / 2));
+  grouped_wgrad_kernel<<<2 * pairs, kThreads, smem, (cudaStream_t)stream>>>(tl, tr, a);
+  return check_launch("grouped_wgrad_kernel");
+}
+
+// lt: [P, ld] bf16 = L^T, rt: [Q, ld] bf16 = R^T (ld elements per row, a multiple of 8; the column index is the
+// row of the dispatched shard).  For every group g with rows [cu[g-1], cu[g]) (a multiple of 16 long):
+// out_ptrs[g][P, Q] fp32 = or += L_g^T R_g according to flags[g] (see the kernel).  out_ptrs and flags are
+// device arrays of G entries.  P % 128 == 0, Q % 256 == 0.
+extern "C" int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld, int P, int Q, const int* cu_seqlens,
+                                    int G, void* const* out_ptrs, const int* flags, int rows_cap, int* status,
+                                    long long timeout_ms, int num_sms, void* stream) {
+  if (P <= 0 || Q <= 0 || P % BM != 0 || Q % BN != 0) {
+    set_error("moonep_grouped_wgrad: P must be a multiple of 128 and Q a multiple of 256");
+    return 1;
+  }
+  if (G < 1 || G > kWgradMaxGroups) {
+    set_error("moonep_grouped_wgrad: at most " + std::to_string(kWgradMaxGroups) + " groups per launch");
+    return 1;
+  }
+  if (ld <= 0 || ld % 8 != 0 || rows_cap > ld) {
+    set_error("moonep_grouped_wgrad: ld must be a multiple of 8 and at least rows_cap");
+    return 1;
+  }
+  CUtensorMap tl, tr;
+  if (int rc = make_tmap(&tl, lt, (unsigned long long)P, (unsigned long long)ld, 128)) return rc;
+  if (int rc = make_tmap(&tr, rt, (unsigned long long)Q, (unsigned long long)ld, 128)) return rc;
+  WgradArgs a;
+  a.out_ptrs = (float* const*)out_ptrs;
+  a.flags = flags;
+  a.cu_seqlens = cu_seqlens;
+  a.status = status;
+  a.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 10000) * 1000000ull;
+  a.G = G;
+  a.P = P;
+  a.Q = Q;
+  a.q_tiles = Q / BN;
+  a.rows_cap = rows_cap;
+  a.row_major = 0;
+  return launch_wgrad(tl, tr, a, num_sms, stream);
+}
+
+// The same with the operands as they are: l = L [rows, P] and r = R [rows, Q] bf16, rows ldl / ldr elements apart
+// (multiples of 8), so that column slices of wider tensors can be passed.  No transposed copies are needed: the
+// tiles are staged MN-major (see make_smem_desc_mn).
+extern "C" int moonep_grouped_wgrad_rows(const void* l, long long ldl, const void* r, long long ldr, int rows, int P,
+                                         int Q, const int* cu_seqlens, int G, void* const* out_ptrs, const int* flags,
+                                         int* status, long long timeout_ms, int num_sms, void* stream) {
+  if (P <= 0 || Q <= 0 || P % BM != 0 || Q % BN != 0) {
+    set_error("moonep_grouped_wgrad_rows: P must be a multiple of 128 and Q a multiple of 256");
+    return 1;
+  }
+  if (G < 1 || G > kWgradMaxGroups) {
+    set_error("moonep_grouped_wgrad_rows: at most " + std::to_string(kWgradMaxGroups) + " groups per launch");
+    return 1;
+  }
+  if (ldl < P || ldr < Q || ldl % 8 != 0 || ldr % 8 != 0 || rows <= 0) {
+    set_error("moonep_grouped_wgrad_rows: row strides must be multiples of 8 and at least the matrix width");
+    return 1;
+  }
+  CUtensorMap tl, tr;
+  if (int rc = make_tmap(&tl, l, (unsigned long long)rows, (unsigned long long)P, 64, (unsigned long long)ldl)) return rc;
+  if (int rc = make_tmap(&tr, r, (unsigned long long)rows, (unsigned long long)Q, 64, (unsigned long long)ldr)) return rc;
+  WgradArgs a;
+  a.out_ptrs = (float* const*)out_ptrs;
+  a.flags = flags;
+  a.cu_seqlens = cu_seqlens;
+  a.status = status;
+  a.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 10000) * 1000000ull;
+  a.G = G;
+  a.P = P;
+  a.Q = Q;
+  a.q_tiles = Q / BN;
+  a.rows_cap = rows;
+  a.row_major = 1;
+  return launch_wgrad(tl, tr, a, num_sms, stream);
+}
