@@ -9,8 +9,8 @@
 //   dispatch   one launch whose CTAs wait for nobody.  Every CTA derives the whole group layout itself (E counts, one
 //              prefix sum).  Four warps clear pad rows with bulk stores from a piece of zeros, handed out from one
 //              counter; the others count the routing entries before the CTA's own contiguous range of tokens, give its
-//              entries their rows and publish "planned"; then four of them stream tokens through shared memory, one
-//              bulk load and K bulk stores per row.  A CTA that is done with its tokens takes rows over from CTAs that
+//              entries their rows and publish "planned"; then up to six of them stream tokens through shared memory,
+//              one bulk load and K bulk stores per row.  A CTA that is done with its tokens takes rows over from CTAs that
 //              have planned theirs: SMs reach HBM at rates that differ by a quarter, and with a fixed share per SM the
 //              kernel took 138 (426) us at S=4096 (16384) where its average CTA was done after 117 (363); now 131 (400).
 //   combine    a warp per 512-byte piece of an output row, straight from the token's K destinations: no work counter,
@@ -78,7 +78,7 @@ struct SingleArgs {
   int stage_bytes, npieces;  // a row is moved in npieces pieces of at most stage_bytes
   int copy_warps;            // warps that stream rows, each through a ring of its own
   int tokens_per_unit;       // whole rows that share a stage (npieces == 1)
-  int pads_per_grab;
+  int pads_per_grab;         // at least
   int tokens_per_cta;
   int* work;
   int epoch_tpe, epoch_plan, epoch_sent;
@@ -145,15 +145,18 @@ struct Layout {
 };
 
 // Warps kPlanWarps.. : clear pad rows (and their weights), mark them unused in a fresh plan.  Rows are handed out from
-// one counter, pads_per_grab at a time, a lane per row.  Their row flags are released at the end, behind one wait and one
+// one counter, some at a time, a lane per row.  Their row flags are released at the end, behind one wait and one
 // fence: a fence per grab held the clears of S=128, H=7168, E=256 (31 K pad rows) to 5.3 TB/s.
 __device__ void clear_pads(const MoonepDevCtx& c, const SingleArgs& a, const Layout& lay, int* grabs,
                            const unsigned char* zeros, uint16_t* shard, int* meta, int epoch) {
   const int lane = threadIdx.x & 31;
   const long long row_bytes = (long long)c.H * 2;
   const int total = lay.groups > 0 ? lay.cum[lay.groups - 1] : 0;
+  // a sixth of a warp's share at a time where there are many: the grabs of 592 warps meet at one address (two rows per
+  // grab: 100 us per round trip at S=128, H=7168, E=256 with 31 K pad rows; eight: 91)
+  const int per = max(a.pads_per_grab, min(32, total / ((int)gridDim.x * (kWarps - kPlanWarps) * 6)));
   auto row_of = [&](int j) {
-    const int row = lane < a.pads_per_grab && j + lane < total ? lay.pad_row(j + lane) : -1;
+    const int row = lane < per && j + lane < total ? lay.pad_row(j + lane) : -1;
     return row < c.NvS ? row : -1;
   };
   int held = 0;
@@ -170,7 +173,7 @@ __device__ void clear_pads(const MoonepDevCtx& c, const SingleArgs& a, const Lay
   };
   for (;;) {
     int j = 0;
-    if (lane == 0) j = atomicAdd(a.work + kWorkPads, a.pads_per_grab);
+    if (lane == 0) j = atomicAdd(a.work + kWorkPads, per);
     j = __shfl_sync(0xffffffffu, j, 0);
     if (j >= total) break;
     const int row = row_of(j);
@@ -195,7 +198,7 @@ __device__ void clear_pads(const MoonepDevCtx& c, const SingleArgs& a, const Lay
     bulk_commit();
     bulk_wait_read<3>();  // what an SM has queued stays small, so that the rows go to the SMs that are fastest
     if (!a.bulk) {
-      for (int q = 0; q < a.pads_per_grab; ++q) {  // a warp per row
+      for (int q = 0; q < per; ++q) {  // a warp per row
         const int r = __shfl_sync(0xffffffffu, row, q);
         if (r < 0) continue;
         for (uint16_t* base : {shard, a.out}) {
