@@ -97,3 +97,23 @@ def test_counts_that_do_not_match_the_routing():
     buf.synchronize()
     assert torch.equal(buf.combine(plan, rows)[0], (x.float() * K).to(torch.bfloat16))
     buf.destroy()
+
+
+@pytest.mark.parametrize("S", [1, 128, 129, 400])
+def test_layer_forward_on_each_side_of_the_pair_rule(S):
+    """One rank: up to 128 rows per expert the expert GEMMs run with one CTA per tile, above on CTA pairs."""
+    from moonep_b200.models.moe_layer import ExpertParallelMoE, dense_reference
+
+    H, K, E, inter = 256, 2, 2, 256
+    buf = Buffer(S, H, K, E, 1, token_padding=128)
+    layer = ExpertParallelMoE(buf, inter, init_std=0.05, seed=4)
+    x, topk, tpe = _inputs(S, H, K, E, 0)
+    gates = torch.rand(S, K, device="cuda")
+    for save in (False, True):
+        out, _ = layer.forward(x, gates, topk, tpe, save_for_backward=save)
+        layer.check()
+        ref = dense_reference(x.float().cpu(), gates.cpu(), topk.cpu(), *(w[:E].float().cpu() for w in (layer.w_gate, layer.w_up, layer.w_down)))
+        # bf16 roundings of h, of every row and of the sum, each 2^-9 of values no larger than twice the largest result
+        assert float((out.float().cpu() - ref).abs().max()) <= 8 * 2.0**-9 * float(ref.abs().max())
+    layer.destroy()
+    buf.destroy()
