@@ -25,6 +25,7 @@ namespace {
 
 constexpr int kTile = 64;
 constexpr int kAdamTensors = 3;
+constexpr int kUpdateSteps = 4;  // vectors per thread of the weight updates
 
 __global__ void __launch_bounds__(256)
     transpose_experts_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int d0, int d1,
@@ -103,10 +104,14 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// w (bf16) -= lr * g (fp32), 8 elements per thread and step
+// w (bf16) -= lr * g (fp32), 8 elements per thread and step.  Short CTAs as in adamw_kernel: 117 M elements 158 -> 142 us.
 __global__ void __launch_bounds__(256)
     sgd_update_kernel(uint16_t* __restrict__ w, const float* __restrict__ g, long long n8, float lr) {
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n8; v += (long long)gridDim.x * blockDim.x) {
+  const long long first = (long long)blockIdx.x * (256 * kUpdateSteps) + threadIdx.x;
+#pragma unroll 1
+  for (int s = 0; s < kUpdateSteps; ++s) {
+    const long long v = first + s * 256;
+    if (v >= n8) break;
     int4 wv = ld16(w + v * 8);
     const int4 g0 = ld16(g + v * 8), g1 = ld16(g + v * 8 + 4);
     uint16_t* we = reinterpret_cast<uint16_t*>(&wv);
@@ -119,9 +124,9 @@ __global__ void __launch_bounds__(256)
 }
 
 // One AdamW step.  Bound by HBM: 16 bytes in and 14 out per element, where a pass per operation moved 86.  Three weights
-// of 33.5 M elements: 1350 us as 30 elementwise launches, 509 us here (5.9 TB/s).  Four elements per thread and step, a
-// stride of the whole grid between steps: the four loads of a step are 16 bytes each and independent, and 8 CTAs of 256
-// threads per SM keep 128 KB of them in flight.
+// of 33.5 M elements: 1350 us as 30 elementwise launches, 478 us here (6.3 TB/s).  The four loads of a step are 16 bytes
+// each and independent.  CTAs are short (kUpdateSteps vectors per thread) and scheduled as they fit: SMs reach HBM at
+// rates that differ by a quarter, and a resident grid that strode over the elements took 515 us.
 struct AdamTensor {
   float* p;        // fp32 master
   float* m;        // first moment
@@ -141,24 +146,25 @@ struct AdamArgs {
 };
 
 __global__ void __launch_bounds__(256) adamw_kernel(const AdamArgs a) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (int k = 0; k < a.count; ++k) {
-    const AdamTensor t = a.t[k];
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < t.n4; i += stride) {
-      int4 x[4] = {ld16(t.p + i * 4), ld16(t.m + i * 4), ld16(t.v + i * 4), ld16(t.g + i * 4)};
-      float *p = reinterpret_cast<float*>(&x[0]), *m = reinterpret_cast<float*>(&x[1]), *v = reinterpret_cast<float*>(&x[2]);
-      const float* g = reinterpret_cast<const float*>(&x[3]);
+  const AdamTensor t = a.t[blockIdx.y];
+  const long long first = (long long)blockIdx.x * (256 * kUpdateSteps) + threadIdx.x;
+#pragma unroll 1
+  for (int s = 0; s < kUpdateSteps; ++s) {
+    const long long i = first + s * 256;
+    if (i >= t.n4) break;
+    int4 x[4] = {ld16(t.p + i * 4), ld16(t.m + i * 4), ld16(t.v + i * 4), ld16(t.g + i * 4)};
+    float *p = reinterpret_cast<float*>(&x[0]), *m = reinterpret_cast<float*>(&x[1]), *v = reinterpret_cast<float*>(&x[2]);
+    const float* g = reinterpret_cast<const float*>(&x[3]);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        m[q] = m[q] * a.b1 + a.one_b1 * g[q];
-        v[q] = v[q] * a.b2 + a.one_b2 * (g[q] * g[q]);
-        p[q] = p[q] * a.decay - a.step * (m[q] / (sqrtf(v[q] * a.inv_c2) + a.eps));
-      }
-      st16(t.p + i * 4, x[0]);
-      st16(t.m + i * 4, x[1]);
-      st16(t.v + i * 4, x[2]);
-      *reinterpret_cast<uint2*>(t.w + i * 4) = make_uint2(pack_bf16(p[0], p[1]), pack_bf16(p[2], p[3]));
+    for (int q = 0; q < 4; ++q) {
+      m[q] = m[q] * a.b1 + a.one_b1 * g[q];
+      v[q] = v[q] * a.b2 + a.one_b2 * (g[q] * g[q]);
+      p[q] = p[q] * a.decay - a.step * (m[q] / (sqrtf(v[q] * a.inv_c2) + a.eps));
     }
+    st16(t.p + i * 4, x[0]);
+    st16(t.m + i * 4, x[1]);
+    st16(t.v + i * 4, x[2]);
+    *reinterpret_cast<uint2*>(t.w + i * 4) = make_uint2(pack_bf16(p[0], p[1]), pack_bf16(p[2], p[3]));
   }
 }
 
@@ -198,11 +204,8 @@ extern "C" int moonep_adamw_update(int count, void* const* master, void* const* 
   a.inv_c2 = (float)(1.0 / c2);
   a.eps = (float)eps;
   a.step = (float)step;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long need = (most / 4 + 255) / 256;
-  const int grid = (int)(need < sms * 8 ? need : sms * 8);
+  const long long per_cta = 256 * 4 * kUpdateSteps;
+  const dim3 grid((unsigned)((most + per_cta - 1) / per_cta), (unsigned)count);
   adamw_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
   return check_launch("adamw_kernel");
 }
@@ -214,10 +217,8 @@ extern "C" int moonep_sgd_update(void* w, const float* g, long long n, float lr,
     return 1;
   }
   if (n == 0) return 0;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  sgd_update_kernel<<<imax(1, sms * 8), 256, 0, (cudaStream_t)stream>>>((uint16_t*)w, g, n / 8, lr);
+  const long long per_cta = 256 * 8 * kUpdateSteps;
+  sgd_update_kernel<<<(unsigned)((n + per_cta - 1) / per_cta), 256, 0, (cudaStream_t)stream>>>((uint16_t*)w, g, n / 8, lr);
   return check_launch("sgd_update_kernel");
 }
 
