@@ -19,7 +19,7 @@ MOONEP_SUM_SLOTS      ``2``: a warp of combine's sum role holds two tokens and s
                       the native library; default 1: measured equal or slower on 2 GPUs, not measured on more).
 MOONEP_BWD_OVERLAP    ``1``: the MoE layer reduces each weight's gradients beside the remaining backward GEMMs (default 0).
 MOONEP_EXPAND_PATH    ``bulk`` (default) or ``ldst``: how the destination side of dispatch copies duplicate rows and clears
-                      pad rows (read by the native library).
+                      pad rows (several ranks; read by the native library).
 MOONEP_COMBINE        ``push`` (default: the expert side folds duplicates and pushes rows to the tokens' home ranks,
                       which sum them as they arrive) or ``pull`` (fold pass, then the home ranks pull).
 MOONEP_PHASED         ``1``: launch the dispatch and combine kernels one role at a time even on real multi-GPU worlds
@@ -28,7 +28,8 @@ MOONEP_PDL            ``0`` turns programmatic dependent launch off even for Buf
 MOONEP_LOCAL_SMS      CTAs of the kernels that only touch local memory (default: all SMs); ``num_sms`` of
                       the Buffer bounds the kernels that move data between ranks.
 MOONEP_NUM_SMS_DEDUP  CTAs of the dispatch kernel's destination-side role (zero fill, dedup builder, duplicate
-                      expansion); validated, 1..SM count; default: every SM the senders leave free.
+                      expansion; with one rank: of the whole dispatch); validated, 1..SM count; default: every SM the
+                      senders leave free.
 MOONEP_NVTX           ``1`` wraps every native call in an NVTX range.
 MOONEP_GEMM_PAIR      ``1`` (default): grouped GEMMs on CTA pairs (tcgen05 cta_group::2); ``0``: one CTA per tile.
 MOONEP_WGRAD          ``kernel`` (default) or ``torch``: weight gradients of the MoE layer.
