@@ -13,7 +13,7 @@
 //              one bulk load and K bulk stores per row.  A CTA that is done with its tokens takes rows over from CTAs that
 //              have planned theirs: SMs reach HBM at rates that differ by a quarter, and with a fixed share per SM the
 //              kernel took 138 (426) us at S=4096 (16384) where its average CTA was done after 117 (363); now 131 (400).
-//   combine    a warp per 512-byte piece of an output row, straight from the token's K destinations: no work counter,
+//   combine    a warp per 512-byte piece of an output row (several at once where a token has few rows), straight from the token's K destinations: no work counter,
 //              no lists.
 //
 // Both are bound by HBM traffic: the rows are written (read) once, the tokens read (written) once.
@@ -723,7 +723,7 @@ constexpr int kCombineThreads = 512;
 // At most so many items per warp.  Many short CTAs instead of a resident grid: SMs that are slower to HBM simply run fewer
 // of them.  Below that many items for two CTAs per SM a warp takes fewer, so that a small combine still uses every SM.
 constexpr int kCombineItems = 4;
-constexpr int kCombineRows = 8;  // rows of a token whose loads are in flight together: 128 KB per SM with 32 warps
+constexpr int kCombineLoads = 8;  // 16-byte loads of a lane in flight together: 128 KB per SM with 32 warps
 
 struct CombineArgs {
   const int* dst;           // [N]
@@ -749,29 +749,44 @@ __device__ __forceinline__ void add8(float* acc, const int4& v) {
   acc[7] += bf16hi((unsigned)v.w);
 }
 
-// A warp per item: 512 bytes of a token's row (vec_ok) or the whole row.  The rows of a token are added in fp32 in
-// ascending k and rounded once; a token with one row is copied as it is.
+__device__ __forceinline__ int4 pack8(const float* acc) {
+  return make_int4((int)pack_bf16(acc[0], acc[1]), (int)pack_bf16(acc[2], acc[3]), (int)pack_bf16(acc[4], acc[5]),
+                   (int)pack_bf16(acc[6], acc[7]));
+}
+
+// An item is 256 elements (512 bytes) of a token's row; a warp has kItems of them in hand.  Their rows are added in fp32 in
+// ascending k and rounded once; a token with one row is copied as it is.  Bound by HBM, hence by the loads in flight: with
+// one item in hand a lane has only K of them, so tokens of up to 4, 2 or 1 rows come 2, 4 or 8 items at a time (kItems > 1
+// needs K <= kCombineLoads / kItems and 16-byte rows).  One item in hand -> this: S=65536, H=2048, K=1 244 -> 96 us
+// (5.6 TB/s), S=4096, H=7168: K=1 61 -> 27, K=2 65 -> 39, K=4 72 -> 57; on one SM, S=1024, H=4096, K=1 724 -> 160.
+template <int kItems>
 __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(const MoonepDevCtx c, const CombineArgs a) {
+  constexpr int kRows = kCombineLoads / kItems;  // rows of an item whose loads are in flight together
   griddep_wait();
   griddep_launch();
   if (poisoned(c)) return;
   const int lane = threadIdx.x & 31;
   const int K = c.K, H = c.H, NvS = c.NvS;
-  const int nvec = H / 8;
-  const int npieces = a.vec_ok ? (nvec + 31) / 32 : 1;
+  const int npieces = (H + 255) / 256;
   const int items = c.S * npieces;  // S * H elements fit the GPU: far below 2^31
   const int step = a.resident ? gridDim.x * (kCombineThreads / 32) : kCombineThreads / 32;
   const int first = a.resident ? blockIdx.x * (kCombineThreads / 32) : blockIdx.x * (kCombineThreads / 32) * a.items_per_warp;
   const int end = a.resident ? items : min(items, first + step * a.items_per_warp);
+  // this lane looks up row k of the warp's item j
+  const int j_of = kItems > 1 ? lane / kRows : 0, k_of = kItems > 1 ? lane % kRows : lane;
+  const bool looks = j_of < kItems && k_of < K;
   int it = first + (threadIdx.x >> 5);
-  int d_next = it < end && lane < K ? a.dst[it / npieces * K + lane] : 0;
-  for (; it < end; it += step) {
-    const int tok = it / npieces, p = it - tok * npieces;
+  auto lookup = [&](int i) { return looks && i < end ? a.dst[i / npieces * K + k_of] : 0; };
+  int d_next = lookup(it + j_of * step);
+  for (; it < end; it += kItems * step) {
+    const int mine = it + j_of * step;
+    const int my_tok = mine / npieces, my_piece = mine - my_tok * npieces;
     const int d = d_next;
-    if (it + step < end && lane < K) d_next = a.dst[(it + step) / npieces * K + lane];  // not a dependent load then
+    d_next = lookup(mine + kItems * step);  // not a dependent load then
     int row = d < 0 ? -d - 1 : d;
-    const bool valid = lane < K && row >= 0 && row < NvS;
-    if (lane < K && !valid) record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_COMBINE_PUSH, 6, d, tok, lane);
+    const bool here = looks && mine < end;
+    const bool valid = here && row >= 0 && row < NvS;
+    if (here && !valid) record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_COMBINE_PUSH, 6, d, my_tok, k_of);
     if (!valid) row = -1;
     if (a.ready != nullptr) {
       int got = 1;
@@ -790,59 +805,82 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(cons
       }
       if (!__all_sync(0xffffffffu, got)) return;
     }
-    if (p == 0 && a.in_w != nullptr && a.out_w != nullptr && lane < K)
-      a.out_w[(long long)tok * K + lane] = valid ? a.in_w[row] : 0.f;
+    if (here && my_piece == 0 && a.in_w != nullptr && a.out_w != nullptr)
+      a.out_w[(long long)my_tok * K + k_of] = valid ? a.in_w[row] : 0.f;
     const unsigned rows = __ballot_sync(0xffffffffu, valid);
-    const bool one = __popc(rows) == 1;
-    if (a.vec_ok) {
-      const int i = p * 32 + lane;
-      float acc[8];
+    const int nvec = H / 8;
+    if constexpr (kItems > 1) {
+      int4 v[kItems][kRows];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = 0.f;
+      for (int j = 0; j < kItems; ++j) {
+        const int i = __shfl_sync(0xffffffffu, my_piece, j * kRows) * 32 + lane;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          const int from = __shfl_sync(0xffffffffu, row, j * kRows + r);
+          v[j][r] = make_int4(0, 0, 0, 0);
+          if (from >= 0 && i < nvec) v[j][r] = ld16(reinterpret_cast<const int4*>(a.in_rows + (long long)from * H) + i);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kItems; ++j) {
+        const int tok = __shfl_sync(0xffffffffu, my_tok, j * kRows);
+        const int i = __shfl_sync(0xffffffffu, my_piece, j * kRows) * 32 + lane;
+        const unsigned have = (rows >> (j * kRows)) & ((1u << kRows) - 1u);
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        int4 only = make_int4(0, 0, 0, 0);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+          if ((have >> r) & 1u) {
+            add8(acc, v[j][r]);
+            only = v[j][r];
+          }
+        if (i < nvec && it + j * step < end)
+          st16(reinterpret_cast<int4*>(a.out + (long long)tok * H) + i, __popc(have) == 1 ? only : pack8(acc));
+      }
+    } else if (a.vec_ok) {
+      const int i = my_piece * 32 + lane;
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       int4 only = make_int4(0, 0, 0, 0);
-      for (int k0 = 0; k0 < K; k0 += kCombineRows) {
-        int4 v[kCombineRows];
+      for (int k0 = 0; k0 < K; k0 += kRows) {
+        int4 v[kRows];
 #pragma unroll
-        for (int r = 0; r < kCombineRows; ++r) {
+        for (int r = 0; r < kRows; ++r) {
           const int from = __shfl_sync(0xffffffffu, row, (k0 + r) & 31);
           v[r] = make_int4(0, 0, 0, 0);
           if (k0 + r < K && from >= 0 && i < nvec)
             v[r] = ld16(reinterpret_cast<const int4*>(a.in_rows + (long long)from * H) + i);
         }
 #pragma unroll
-        for (int r = 0; r < kCombineRows; ++r) {
+        for (int r = 0; r < kRows; ++r)
           if (k0 + r < K && ((rows >> (k0 + r)) & 1u)) {
             add8(acc, v[r]);
             only = v[r];
           }
+      }
+      if (i < nvec) st16(reinterpret_cast<int4*>(a.out + (long long)my_tok * H) + i, __popc(rows) == 1 ? only : pack8(acc));
+    } else {  // element by element, eight loads of a row in flight (a warp per row, one load at a time: S=4096, H=2044, K=4 113 -> 39 us)
+      const int e0 = my_piece * 256 + lane;
+      float acc[8];
+      uint16_t only[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q] = 0.f, only[q] = 0;
+      for (int k = 0; k < K; ++k) {
+        const int from = __shfl_sync(0xffffffffu, row, k);
+        if (from < 0) continue;
+        uint16_t v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = e0 + q * 32 < H ? a.in_rows[(long long)from * H + e0 + q * 32] : 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          acc[q] += __uint_as_float((unsigned)v[q] << 16);
+          only[q] = v[q];
         }
       }
-      if (i < nvec) {
-        int4 o = only;
-        if (!one) {
-          o.x = (int)pack_bf16(acc[0], acc[1]);
-          o.y = (int)pack_bf16(acc[2], acc[3]);
-          o.z = (int)pack_bf16(acc[4], acc[5]);
-          o.w = (int)pack_bf16(acc[6], acc[7]);
-        }
-        st16(reinterpret_cast<int4*>(a.out + (long long)tok * H) + i, o);
-      }
-    } else {
-      for (int i0 = 0; i0 < H; i0 += 32) {  // whole warps: the shuffles need every lane
-        const int i = i0 + lane;
-        float acc = 0.f;
-        uint16_t only = 0;
-        for (int k = 0; k < K; ++k) {
-          const int from = __shfl_sync(0xffffffffu, row, k);
-          if (from >= 0 && i < H) {
-            only = a.in_rows[(long long)from * H + i];
-            acc += __uint_as_float((unsigned)only << 16);
-          }
-        }
-        if (i < H) {
-          const __nv_bfloat16 b = __float2bfloat16_rn(acc);
-          a.out[(long long)tok * H + i] = one ? only : *reinterpret_cast<const uint16_t*>(&b);
-        }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (e0 + q * 32 >= H) continue;
+        const __nv_bfloat16 b = __float2bfloat16_rn(acc[q]);
+        a.out[(long long)my_tok * H + e0 + q * 32] = __popc(rows) == 1 ? only[q] : *reinterpret_cast<const uint16_t*>(&b);
       }
     }
   }
@@ -951,15 +989,23 @@ extern "C" int moonep_combine_single(void* ctx, const int* dst, const void* in_r
   a.ready = ready;
   a.ready_expect = ready_expect;
   a.vec_ok = (c.H % 8 == 0 && aligned16(in_rows) && aligned16(out)) ? 1 : 0;
-  const long long items = (long long)c.S * (a.vec_ok ? (c.H / 8 + 31) / 32 : 1);
-  a.items_per_warp = (int)(items / (2 * kCombineThreads / 32 * h->sm_count));
-  a.items_per_warp = imax(1, imin(kCombineItems, a.items_per_warp));
+  const long long items = (long long)c.S * ((c.H + 255) / 256);
+  a.resident = c.local_sms < h->sm_count ? 1 : 0;
+  const long long slots = 2 * kCombineThreads / 32 * (long long)imax(1, a.resident ? c.local_sms : h->sm_count);  // warps at once
+  // as many items in hand as fill a lane's loads, as long as every warp slot gets some: below that the latency of one round
+  // trip counts and fewer SMs would do the work
+  int hand = !a.vec_ok || c.K > 4 ? 1 : c.K > 2 ? 2 : c.K > 1 ? 4 : 8;
+  while (hand > 1 && items < hand * slots) hand /= 2;
+  a.items_per_warp = hand * (int)(items / (hand * slots) < 1 ? 1 : items / (hand * slots));
+  a.items_per_warp = imin(imax(kCombineItems, hand), a.items_per_warp);
   const int per_cta = kCombineThreads / 32 * a.items_per_warp;
   int grid = (int)((items + per_cta - 1) / per_cta);
-  a.resident = c.local_sms < h->sm_count ? 1 : 0;
   if (a.resident) grid = imin(grid, 2 * imax(1, c.local_sms));
-  if (int rc = check_cuda(launch_maybe_pdl(combine_single_kernel, grid, kCombineThreads, 0, (cudaStream_t)stream,
-                                           h->enable_pdl != 0, c, a),
+  auto* kernel = hand == 1   ? combine_single_kernel<1>
+                 : hand == 2 ? combine_single_kernel<2>
+                 : hand == 4 ? combine_single_kernel<4>
+                             : combine_single_kernel<8>;
+  if (int rc = check_cuda(launch_maybe_pdl(kernel, grid, kCombineThreads, 0, (cudaStream_t)stream, h->enable_pdl != 0, c, a),
                           "launch combine_single_kernel"))
     return rc;
   return check_launch("combine_single_kernel");

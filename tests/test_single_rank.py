@@ -117,3 +117,33 @@ def test_layer_forward_on_each_side_of_the_pair_rule(S):
         assert float((out.float().cpu() - ref).abs().max()) <= 8 * 2.0**-9 * float(ref.abs().max())
     layer.destroy()
     buf.destroy()
+
+
+@pytest.mark.parametrize("sms", [None, 1, 3])
+@pytest.mark.parametrize("S,H,K", [(40001, 8, 1), (9999, 264, 1), (301, 264, 1), (9999, 520, 2), (150, 2056, 2), (9999, 264, 3),
+                                   (5001, 520, 4), (77, 520, 4), (301, 264, 5), (70, 265, 3), (40, 13, 9)])  # fmt: skip
+def test_combine_with_one_to_eight_pieces_of_rows_in_hand(S, H, K, sms, monkeypatch):
+    """The combine holds 8, 4, 2 or 1 pieces of 256 elements per warp by K and size, on a grid that is bounded or not:
+    fp32 sums in ascending k rounded once, a lone row bit for bit (a negative zero and a NaN among its elements)."""
+    if sms is not None:
+        monkeypatch.setenv("MOONEP_LOCAL_SMS", str(sms))
+    E = max(K, 4)
+    buf = Buffer(S, H, K, E, 1, token_padding=4)
+    x, topk, tpe = _inputs(S, H, K, E, 0)
+    gates = torch.rand(S, K, device="cuda")
+    rows, w, _, plan = buf.dispatch(x, gates, topk, tpe, zero_copy=True)
+    loff = torch.where(plan.dst < 0, -plan.dst - 1, plan.dst).long().view(S, K)
+    assert torch.equal(rows[loff.flatten()], x.repeat_interleave(K, 0))
+    y = torch.randn(buf._require_ctx()["NvS"], H, generator=torch.Generator(device="cuda").manual_seed(K), device="cuda")
+    y = y.to(torch.bfloat16)
+    y[:, 0], y[loff[0], -1] = -0.0, float("nan")
+    for with_weights in (True, False):
+        out, back, _ = buf.combine(plan, y, w if with_weights else None)
+        want = torch.zeros(S, H, device="cuda")
+        for k in range(K):
+            want += y[loff[:, k]].float()
+        want = y[loff[:, 0]] if K == 1 else want.to(torch.bfloat16)
+        same = (out.view(torch.int16) == want.view(torch.int16)) | (out.isnan() & want.isnan() & (K > 1))
+        assert bool(same.all()) and (back is None or torch.equal(back, gates))
+    buf.synchronize()
+    buf.destroy()
