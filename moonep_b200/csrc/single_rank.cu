@@ -73,8 +73,9 @@ struct SingleArgs {
   int with_weights;        // pad rows' weight slots are cleared
   int fresh;
   int topk_vec;  // topk can be read 16 bytes at a time
-  int vec_ok;    // rows can be moved 16 bytes at a time
-  int bulk;      // rows go through shared memory with bulk copies
+  int vec_ok;    // rows of the shard and the copy are whole 16-byte words at 16-byte addresses: pads go out in bulk stores
+  int bulk;      // so are the input's: rows go through shared memory with bulk copies
+  int word;      // bytes per store of a row that does not
   int stage_bytes, npieces;  // a row is moved in npieces pieces of at most stage_bytes
   int copy_warps;            // warps that stream rows, each through a ring of its own
   int tokens_per_unit;       // whole rows that share a stage (npieces == 1)
@@ -144,6 +145,16 @@ struct Layout {
   }
 };
 
+// A warp clears n elements at any address: 16-byte stores between the edges.
+__device__ __forceinline__ void clear_row(uint16_t* p, int n) {
+  const int lane = threadIdx.x & 31;
+  const int head = min(n, (int)((16u - ((unsigned)reinterpret_cast<uintptr_t>(p) & 15u)) & 15u) / 2);
+  const int words = (n - head) / 8, tail = head + words * 8;
+  if (lane < head) p[lane] = 0;
+  for (int i = lane; i < words; i += 32) st16(reinterpret_cast<int4*>(p + head) + i, make_int4(0, 0, 0, 0));
+  if (lane < n - tail) p[tail + lane] = 0;
+}
+
 // Warps kPlanWarps.. : clear pad rows (and their weights), mark them unused in a fresh plan.  Rows are handed out from
 // one counter, some at a time, a lane per row.  Their row flags are released at the end, behind one wait and one
 // fence: a fence per grab held the clears of S=128, H=7168, E=256 (31 K pad rows) to 5.3 TB/s.
@@ -178,7 +189,7 @@ __device__ void clear_pads(const MoonepDevCtx& c, const SingleArgs& a, const Lay
     if (j >= total) break;
     const int row = row_of(j);
     if (row >= 0) {
-      if (a.bulk) {
+      if (a.vec_ok) {
         unsigned char* p = reinterpret_cast<unsigned char*>(shard) + row * row_bytes;
         unsigned char* p2 = reinterpret_cast<unsigned char*>(a.out) + row * row_bytes;
         for (long long o = 0; o < row_bytes; o += kZeroBytes) {
@@ -197,19 +208,12 @@ __device__ void clear_pads(const MoonepDevCtx& c, const SingleArgs& a, const Lay
     }
     bulk_commit();
     bulk_wait_read<3>();  // what an SM has queued stays small, so that the rows go to the SMs that are fastest
-    if (!a.bulk) {
-      for (int q = 0; q < per; ++q) {  // a warp per row
+    if (!a.vec_ok) {
+      for (int q = 0; q < per; ++q) {
         const int r = __shfl_sync(0xffffffffu, row, q);
         if (r < 0) continue;
-        for (uint16_t* base : {shard, a.out}) {
-          if (base == nullptr) continue;
-          uint16_t* p = base + (long long)r * c.H;
-          if (a.vec_ok) {
-            for (int i = lane; i < c.H / 8; i += 32) st16(reinterpret_cast<int4*>(p) + i, make_int4(0, 0, 0, 0));
-          } else {
-            for (int i = lane; i < c.H; i += 32) p[i] = 0;
-          }
-        }
+        clear_row(shard + (long long)r * c.H, c.H);
+        if (a.out != nullptr) clear_row(a.out + (long long)r * c.H, c.H);
       }
       fence_gpu();  // other lanes' stores precede the flag that lane q releases
     }
@@ -379,35 +383,59 @@ __device__ bool copy_bulk(const MoonepDevCtx& c, const SingleArgs& a, SingleShar
   return true;
 }
 
-// The same without bulk copies: a warp per row of this CTA's tokens, 16 bytes or one element at a time.
-__device__ void copy_plain(const MoonepDevCtx& c, const SingleArgs& a, int t_lo, int t_hi, uint16_t* shard, int* meta,
-                           int epoch) {
+// The same without bulk copies: words of D for this CTA's tokens, loaded as they are or (input rows that start anywhere)
+// two bytes at a time.  A warp takes kPlainWords words per lane at a time, so that one token keeps several warps busy and a
+// lane several loads in flight.  Against a warp per row that moved (and cleared) two bytes per lane: S=4096, K=8, H=4096 with
+// an input that is not 16-byte aligned 1059 -> 84 us, S=128, H=7168 609 -> 33, S=4096, K=4, H=4100 665 -> 86.
+constexpr int kPlainWords = 4;
+
+template <typename D, typename T>
+__device__ void copy_words(const MoonepDevCtx& c, const SingleArgs& a, int t_lo, int t_hi, uint16_t* shard) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int tok = t_lo + warp; tok < t_hi; tok += kPlanWarps) {
-    const uint16_t* src = a.hidden + (long long)tok * c.H;
+  const int n = c.H * 2 / (int)sizeof(D), pieces = (n + 32 * kPlainWords - 1) / (32 * kPlainWords);
+  for (int u = warp; u < (t_hi - t_lo) * pieces; u += kPlanWarps) {
+    const int tok = t_lo + u / pieces, i0 = (u % pieces) * 32 * kPlainWords + lane;
+    const T* src = reinterpret_cast<const T*>(a.hidden + (long long)tok * c.H);
     const int d = lane < c.K ? a.dst[tok * c.K + lane] : 0;
     int loff = d < 0 ? -d - 1 : d;
     if (lane >= c.K || loff < 0 || loff >= c.NvS) loff = -1;
-    const int n = a.vec_ok ? c.H / 8 : c.H;
-    for (int i0 = 0; i0 < n; i0 += 32) {  // whole warps: the shuffles need every lane
-      const int i = i0 + lane;
-      int4 v = make_int4(0, 0, 0, 0);
-      uint16_t w = 0;
-      if (i < n) {
-        if (a.vec_ok) v = ld16(reinterpret_cast<const int4*>(src) + i); else w = src[i];
-      }
-      for (int k = 0; k < c.K; ++k) {
-        const int row = __shfl_sync(0xffffffffu, loff, k);
-        if (row < 0 || i >= n) continue;
-        for (uint16_t* base : {shard, a.out}) {
-          if (base == nullptr) continue;
-          if (a.vec_ok) st16(reinterpret_cast<int4*>(base + (long long)row * c.H) + i, v); else base[(long long)row * c.H + i] = w;
-        }
+    D v[kPlainWords];
+#pragma unroll
+    for (int q = 0; q < kPlainWords; ++q) {
+      T* part = reinterpret_cast<T*>(v + q);
+#pragma unroll
+      for (int p = 0; p < (int)(sizeof(D) / sizeof(T)); ++p)
+        if (i0 + q * 32 < n) part[p] = src[(long long)(i0 + q * 32) * (sizeof(D) / sizeof(T)) + p];
+    }
+    for (int k = 0; k < c.K; ++k) {
+      const int row = __shfl_sync(0xffffffffu, loff, k);
+      if (row < 0) continue;
+      for (uint16_t* base : {shard, a.out}) {
+        if (base == nullptr) continue;
+        D* to = reinterpret_cast<D*>(base + (long long)row * c.H) + i0;
+#pragma unroll
+        for (int q = 0; q < kPlainWords; ++q)
+          if (i0 + q * 32 < n) to[q * 32] = v[q];
       }
     }
-    fence_gpu();
-    __syncwarp();
-    if (loff >= 0) st_relaxed_gpu(meta + c.rowflag_off + loff, epoch);
+  }
+}
+
+__device__ void copy_plain(const MoonepDevCtx& c, const SingleArgs& a, int t_lo, int t_hi, uint16_t* shard, int* meta,
+                           int epoch) {
+  switch (a.word) {
+    case 16: copy_words<int4, uint16_t>(c, a, t_lo, t_hi, shard); break;
+    case 8: copy_words<int2, int2>(c, a, t_lo, t_hi, shard); break;
+    case 4: copy_words<int, int>(c, a, t_lo, t_hi, shard); break;
+    default: copy_words<uint16_t, uint16_t>(c, a, t_lo, t_hi, shard);
+  }
+  fence_gpu();
+  plan_sync();  // a row's words come from several warps
+  fence_gpu();
+  for (int e = t_lo * c.K + threadIdx.x; e < t_hi * c.K; e += kEntries) {
+    const int d = a.dst[e];
+    const int loff = d < 0 ? -d - 1 : d;
+    if (loff >= 0 && loff < c.NvS) st_relaxed_gpu(meta + c.rowflag_off + loff, epoch);
   }
 }
 
@@ -562,9 +590,9 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
   const int tid = threadIdx.x, warp = tid >> 5;
   const int E = c.E, K = c.K, NvS = c.NvS;
   unsigned char* zeros = s_dyn + (size_t)a.copy_warps * kRing * a.stage_bytes;
-  int* tables = reinterpret_cast<int*>(zeros + (a.bulk ? kZeroBytes : 0));
+  int* tables = reinterpret_cast<int*>(zeros + (a.vec_ok ? kZeroBytes : 0));
   if (tid < kCopyWarps * kRing) mbar_init(s.bar + tid, 1);
-  if (a.bulk)
+  if (a.vec_ok)
     for (int i = tid; i < kZeroBytes / 16; i += kThreads) reinterpret_cast<int4*>(zeros)[i] = make_int4(0, 0, 0, 0);
   fence_barrier_init();
   fence_proxy_async();
@@ -933,8 +961,11 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
   a.with_weights = with_weights;
   a.fresh = fresh;
   a.topk_vec = aligned16(topk) ? 1 : 0;
-  a.vec_ok = (c.H % 8 == 0 && aligned16(hidden) && aligned16(a.out)) ? 1 : 0;
-  a.bulk = a.vec_ok;
+  a.vec_ok = (c.H % 8 == 0 && aligned16(a.out)) ? 1 : 0;
+  a.bulk = (a.vec_ok && aligned16(hidden)) ? 1 : 0;
+  // rows of 16-byte words take any input (the stores, K per load, stay wide); others move in what all addresses allow
+  const uintptr_t bits = (uintptr_t)(2ll * c.H) | (uintptr_t)a.out | (uintptr_t)hidden | 16u;
+  a.word = a.vec_ok ? 16 : (int)(bits & (~bits + 1));
   a.epoch_tpe = epoch_tpe;
   a.epoch_plan = epoch_plan;
   a.epoch_sent = epoch_sent;
@@ -958,7 +989,7 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
     a.copy_warps = imin(kCopyWarps, (int)(room / ((long long)kRing * a.stage_bytes)));
   }
   a.pads_per_grab = imax(1, imin(32, (int)(28672 / row_bytes)));
-  const size_t smem = a.bulk ? (size_t)a.copy_warps * kRing * a.stage_bytes + kZeroBytes + tables : tables;
+  const size_t smem = (size_t)a.copy_warps * kRing * a.stage_bytes + (a.vec_ok ? kZeroBytes : 0) + tables;
   if (int rc = check_cuda(cudaFuncSetAttribute(dispatch_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit),
                           "cudaFuncSetAttribute(dispatch_single_kernel)"))
     return rc;

@@ -47,7 +47,9 @@ def _inputs(S, H, K, E, shift):
 
 
 @pytest.mark.parametrize("shift", [0, 1, 4])
-@pytest.mark.parametrize("S,H,K,E,pad", [(1, 64, 2, 4, 8), (500, 520, 3, 9, 16), (3000, 64, 6, 12, 1)])
+@pytest.mark.parametrize("S,H,K,E,pad", [(1, 64, 2, 4, 8), (500, 520, 3, 9, 16), (3000, 64, 6, 12, 1),
+                                         # several pieces per row, in words of 16 (or 2, read), 8, 4 and 2 bytes
+                                         (20, 2056, 3, 5, 8), (150, 1028, 2, 4, 8), (33, 1002, 2, 4, 4), (9, 515, 4, 5, 2)])  # fmt: skip
 def test_replay_and_unaligned_inputs(S, H, K, E, pad, shift):
     buf = Buffer(S, H, K, E, 1, token_padding=pad)
     x, topk, tpe = _inputs(S, H, K, E, shift)
