@@ -21,6 +21,9 @@
 // Parity: reference moonep_td/dispatch.py:42-117, moonep_td/_dedup_builder.py:23-108, moonep_td/combine.py:22-68 at one
 // rank; the plan's contents are those of the general kernels (the order of the duplicate groups, which is arbitrary
 // there, is token order here).
+#include <cstdlib>
+#include <cstring>
+
 #include "common.cuh"
 #include "host.h"
 
@@ -73,9 +76,11 @@ struct SingleArgs {
   int with_weights;        // pad rows' weight slots are cleared
   int fresh;
   int topk_vec;  // topk can be read 16 bytes at a time
-  int vec_ok;    // rows of the shard and the copy are whole 16-byte words at 16-byte addresses: pads go out in bulk stores
-  int bulk;      // so are the input's: rows go through shared memory with bulk copies
+  int vec_ok;    // rows of the shard and the copy are whole 16-byte words at 16-byte addresses
+  int bulk_pads; // pads are cleared in bulk stores
+  int bulk;      // rows go through shared memory with bulk copies
   int word;      // bytes per store of a row that does not
+  int narrow;    // its input is read two bytes at a time
   int stage_bytes, npieces;  // a row is moved in npieces pieces of at most stage_bytes
   int copy_warps;            // warps that stream rows, each through a ring of its own
   int tokens_per_unit;       // whole rows that share a stage (npieces == 1)
@@ -189,7 +194,7 @@ __device__ void clear_pads(const MoonepDevCtx& c, const SingleArgs& a, const Lay
     if (j >= total) break;
     const int row = row_of(j);
     if (row >= 0) {
-      if (a.vec_ok) {
+      if (a.bulk_pads) {
         unsigned char* p = reinterpret_cast<unsigned char*>(shard) + row * row_bytes;
         unsigned char* p2 = reinterpret_cast<unsigned char*>(a.out) + row * row_bytes;
         for (long long o = 0; o < row_bytes; o += kZeroBytes) {
@@ -208,7 +213,7 @@ __device__ void clear_pads(const MoonepDevCtx& c, const SingleArgs& a, const Lay
     }
     bulk_commit();
     bulk_wait_read<3>();  // what an SM has queued stays small, so that the rows go to the SMs that are fastest
-    if (!a.vec_ok) {
+    if (!a.bulk_pads) {
       for (int q = 0; q < per; ++q) {
         const int r = __shfl_sync(0xffffffffu, row, q);
         if (r < 0) continue;
@@ -424,7 +429,9 @@ __device__ void copy_words(const MoonepDevCtx& c, const SingleArgs& a, int t_lo,
 __device__ void copy_plain(const MoonepDevCtx& c, const SingleArgs& a, int t_lo, int t_hi, uint16_t* shard, int* meta,
                            int epoch) {
   switch (a.word) {
-    case 16: copy_words<int4, uint16_t>(c, a, t_lo, t_hi, shard); break;
+    case 16:
+      if (a.narrow) copy_words<int4, uint16_t>(c, a, t_lo, t_hi, shard); else copy_words<int4, int4>(c, a, t_lo, t_hi, shard);
+      break;
     case 8: copy_words<int2, int2>(c, a, t_lo, t_hi, shard); break;
     case 4: copy_words<int, int>(c, a, t_lo, t_hi, shard); break;
     default: copy_words<uint16_t, uint16_t>(c, a, t_lo, t_hi, shard);
@@ -590,9 +597,9 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
   const int tid = threadIdx.x, warp = tid >> 5;
   const int E = c.E, K = c.K, NvS = c.NvS;
   unsigned char* zeros = s_dyn + (size_t)a.copy_warps * kRing * a.stage_bytes;
-  int* tables = reinterpret_cast<int*>(zeros + (a.vec_ok ? kZeroBytes : 0));
+  int* tables = reinterpret_cast<int*>(zeros + (a.bulk_pads ? kZeroBytes : 0));
   if (tid < kCopyWarps * kRing) mbar_init(s.bar + tid, 1);
-  if (a.vec_ok)
+  if (a.bulk_pads)
     for (int i = tid; i < kZeroBytes / 16; i += kThreads) reinterpret_cast<int4*>(zeros)[i] = make_int4(0, 0, 0, 0);
   fence_barrier_init();
   fence_proxy_async();
@@ -962,7 +969,12 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
   a.fresh = fresh;
   a.topk_vec = aligned16(topk) ? 1 : 0;
   a.vec_ok = (c.H % 8 == 0 && aligned16(a.out)) ? 1 : 0;
-  a.bulk = (a.vec_ok && aligned16(hidden)) ? 1 : 0;
+  // MOONEP_EXPAND_PATH=ldst selects register copies as it does with several ranks (S=4096, H=7168, K=8, E=32: 126 us
+  // against 112 with bulk copies)
+  const char* xp = getenv("MOONEP_EXPAND_PATH");
+  a.bulk_pads = (a.vec_ok && !(xp != nullptr && strcmp(xp, "ldst") == 0)) ? 1 : 0;
+  a.bulk = (a.bulk_pads && aligned16(hidden)) ? 1 : 0;
+  a.narrow = aligned16(hidden) ? 0 : 1;
   // rows of 16-byte words take any input (the stores, K per load, stay wide); others move in what all addresses allow
   const uintptr_t bits = (uintptr_t)(2ll * c.H) | (uintptr_t)a.out | (uintptr_t)hidden | 16u;
   a.word = a.vec_ok ? 16 : (int)(bits & (~bits + 1));
@@ -989,7 +1001,7 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
     a.copy_warps = imin(kCopyWarps, (int)(room / ((long long)kRing * a.stage_bytes)));
   }
   a.pads_per_grab = imax(1, imin(32, (int)(28672 / row_bytes)));
-  const size_t smem = (size_t)a.copy_warps * kRing * a.stage_bytes + (a.vec_ok ? kZeroBytes : 0) + tables;
+  const size_t smem = (size_t)a.copy_warps * kRing * a.stage_bytes + (a.bulk_pads ? kZeroBytes : 0) + tables;
   if (int rc = check_cuda(cudaFuncSetAttribute(dispatch_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit),
                           "cudaFuncSetAttribute(dispatch_single_kernel)"))
     return rc;
