@@ -175,9 +175,11 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// arrive on an mbarrier of another CTA of the cluster (address from mapa_u32)
+// arrive on an mbarrier of another CTA of the cluster (address from mapa_u32), release at CTA scope: it says that TMEM has been
+// read, which the tcgen05 fences order.  At cluster scope it would also hold until this thread's stores of the results have
+// reached L2, and the next MMAs with it.
 __device__ __forceinline__ void mbar_arrive_cluster(unsigned cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait_cluster(unsigned long long* bar, unsigned parity) {
