@@ -1,4 +1,4 @@
-// Weight gradients of every group on CTA pairs (tcgen05 cta_group::2, sm_100a): contraction over the rows of a group,
+// Weight gradients of every group on tcgen05 tensor cores (sm_100a): contraction over the rows of a group,
 //
 //   dW[g] (P x Q, fp32) (=, +=) L[rows of g, :P]^T  @  R[rows of g, :Q]
 //
@@ -11,17 +11,20 @@
 // if the group has no rows.  A null out_ptrs[g] skips the group; rows without a target are reported through the status
 // block.
 //
-// A cluster of two CTAs computes a 256 x 256 tile (as in grouped_gemm_pair.cu): 32 KB of operands per CTA and 64 rows
-// instead of the 48 KB of one CTA per 128 x 256 tile.  The accumulator is dW^T: TMEM lanes (the M index, 128 per CTA) run
-// along Q, columns along P, so the 32 lanes of a warp hold 32 neighbours of a row of dW and every store instruction of the
-// epilogue fills one 128-byte line straight from registers.  Lanes along P instead cost four times the L1 cycles (a sector
-// per lane), or a turn through shared memory, whose slots the MMAs need.  When P is an odd multiple of 128 the last tile
-// has 128 columns that are computed from zeros and not stored.
+// A cluster of two CTAs computes a 256 x 256 tile (cta_group::2, as in grouped_gemm_pair.cu): 32 KB of operands per CTA and
+// 64 rows.  The accumulator is dW^T: TMEM lanes (the M index, 128 per CTA) run along Q, columns along P, so the 32 lanes of
+// a warp hold 32 neighbours of a row of dW and every store instruction of the epilogue fills one 128-byte line straight from
+// registers.  Lanes along P instead cost four times the L1 cycles (a sector per lane), or a turn through shared memory, whose
+// slots the MMAs need.  When P is an odd multiple of 128 the last tile has 128 columns that are computed from zeros and not
+// stored.  Short groups and a few odd numbers of SMs take one CTA per 256 x 128 tile of the same kernel instead (48 KB per
+// 64 rows; the last tile of an odd P is 128 x 128): moonep_wgrad_single_cta.
 //
 // Bound by the tensor pipe and the fp32 results together: a tile of 1024 rows is 16 K blocks of MMAs and 256 KB of output.
-// 8 groups x 1024 rows, 2048 x 7168: 258 us with one CTA per tile, 241 us here (985 TFLOP/s); adding to the old values 301
-// and 262; 16 groups x 512 rows, 1024 x 2048: 53.6 and 49.5.  (Lanes along P, 32-byte stores: 236, 369, 57.7; results
-// through shared memory in 512-byte bulk stores: 242 and 50 in a training step, an SM takes 15 clocks per bulk store.)
+// 8 groups x 1024 rows, 2048 x 7168: pairs 239 us (1006 TFLOP/s), single CTAs 256; adding to the old values 258 and 296;
+// 16 groups x 512 rows, 1024 x 2048: 47 and 53.  What an accumulator waits for before it is used again is only that TMEM has
+// been read (mbar_arrive_cluster): as long as the arrive also waited for the stores to reach L2, groups of 128 rows took 38.6
+// us where they take 32.2 (16 groups, 1024 x 2048).  (Lanes along P, 32-byte stores: 236, 369, 57.7; results through shared
+// memory in 512-byte bulk stores: 242 and 50 in a training step, an SM takes 15 clocks per bulk store.)
 //
 // Every mbarrier wait is bounded; on expiry the role records a status word and leaves its loop (see
 // grouped_gemm_pair.cu for how a pair is torn down).
@@ -33,11 +36,13 @@ namespace moonep {
 
 namespace {
 
-constexpr int kStages = 6;
 constexpr int kThreads = 192;
 constexpr int kTmemCols = 512;
-constexpr unsigned kHalfBytes = 128 * BK * 2;     // 16 KB: this CTA's columns of L, its half of R
-constexpr unsigned kStageBytes = 2 * kHalfBytes;  // 32 KB per CTA and stage
+constexpr unsigned kHalfBytes = 128 * BK * 2;  // 16 KB: 128 columns of L or R
+// A CTA stages 128 columns of R and, as one of a pair, 128 of L, alone 256: 192 KB of operands either way.
+template <bool kPair> constexpr int kStages = kPair ? 6 : 4;
+template <bool kPair> constexpr unsigned kStageBytes = (kPair ? 2 : 3) * kHalfBytes;
+constexpr size_t kSmemBytes = 12 * kHalfBytes + 1024;
 constexpr int kWgradMaxGroups = 512;  // groups per launch (their work list lives in shared memory)
 
 struct WgradArgs {
@@ -126,16 +131,17 @@ __device__ __forceinline__ void put_cols(float* dst, long long ld, const unsigne
   }
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-    grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_l, const __grid_constant__ CUtensorMap tmap_r,
-                         const WgradArgs a) {
+template <bool kPair>
+__device__ __forceinline__ void wgrad_body(const CUtensorMap* tmap_l, const CUtensorMap* tmap_r, const WgradArgs& a) {
+  constexpr int kStages = moonep::kStages<kPair>;
+  constexpr unsigned kStageBytes = moonep::kStageBytes<kPair>;
   extern __shared__ unsigned char s_raw[];
   __shared__ __align__(8) unsigned long long s_full[kStages], s_empty[kStages], s_tfull[2], s_tempty[2], s_done;
   __shared__ unsigned s_tmem_base;
   __shared__ WgradGroups s_groups;
   unsigned char* s_tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned rank = cluster_ctarank();  // 0: leader (issues the MMAs), 1: its peer
+  const unsigned rank = kPair ? cluster_ctarank() : 0;  // 0: leader (issues the MMAs), 1: its peer
   if (warp == 0) wgrad_list_groups(a, s_groups, lane);
 
   if (threadIdx.x == 0) {
@@ -145,7 +151,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(s_tfull + b, 1);   // one commit, delivered to both CTAs
-      mbar_init(s_tempty + b, 8);  // used in the leader: four epilogue warps of each CTA
+      mbar_init(s_tempty + b, kPair ? 8 : 4);  // used in the leader: four epilogue warps of each CTA
     }
     mbar_init(&s_done, 1);
     fence_barrier_init();
@@ -156,13 +162,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();  // the peer's barriers exist before anything is delivered to them
+  if (kPair) cluster_sync_all();  // the peer's barriers exist before anything is delivered to them
   tc_fence_after();
   const unsigned tmem_base = s_tmem_base;
   // both CTAs own their whole TMEM, so the accumulators start at column 0 in both
   const bool tmem_ok = (tmem_base & 0xFFFFu) == 0;
   if (!tmem_ok && threadIdx.x == 0) gemm_fail(a.status, 14, 9, (int)tmem_base, 0);
-  const long long pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const long long unit = kPair ? blockIdx.x >> 1 : blockIdx.x, nunits = kPair ? gridDim.x >> 1 : gridDim.x;
   const long long num_tiles = (long long)s_groups.n * a.p_tiles * a.q_tiles;
 
   if (warp == 0) {
@@ -171,11 +177,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       int stage = 0;
       unsigned phase = 0;
       bool failed = false;
-      for (long long t = pair; t < num_tiles && !failed; t += npairs) {
+      for (long long t = unit; t < num_tiles && !failed; t += nunits) {
         const WgradTile w = wgrad_tile(a, s_groups, t);
         if (w.krows == 0 || w.out == nullptr) continue;
         const int kbs = (w.krows + BK - 1) / BK;
-        const int q0 = w.qb * BN + (int)rank * 128, p0 = w.pb * BN + (int)rank * 128;  // p0 may lie past P: zeros
+        const int q0 = w.qb * (kPair ? BN : 128) + (int)rank * 128;
+        const int p0 = w.pb * BN + (int)rank * 128;               // of a pair's second CTA it may lie past P: zeros
+        const int cols = kPair ? 128 : min(BN, a.P - w.pb * BN);  // columns of L that this CTA stages
         for (int kb = 0; kb < kbs; ++kb) {
           if (!mbar_wait_cluster(s_empty + stage, phase ^ 1u, a.timeout_ns)) {
             gemm_fail(a.status, 14, 1, stage, kb);
@@ -183,17 +191,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             break;
           }
           unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
-          if (rank == 0) mbar_expect_tx(s_full + stage, 2 * kStageBytes);
-          const unsigned full_of_leader = mapa_u32(s_full + stage, 0);
           const int k = w.k0 + kb * BK;
-          if (a.row_major) {  // boxes of 64 columns x 64 rows, two for R and two for L
-            tma_load_2d_pair(st, &tmap_r, q0, k, full_of_leader);
-            tma_load_2d_pair(st + kMnBoxBytes, &tmap_r, q0 + 64, k, full_of_leader);
-            tma_load_2d_pair(st + kHalfBytes, &tmap_l, p0, k, full_of_leader);
-            tma_load_2d_pair(st + kHalfBytes + kMnBoxBytes, &tmap_l, p0 + 64, k, full_of_leader);
+          if constexpr (kPair) {
+            if (rank == 0) mbar_expect_tx(s_full + stage, 2 * kStageBytes);
+            const unsigned full_of_leader = mapa_u32(s_full + stage, 0);
+            if (a.row_major) {  // boxes of 64 columns x 64 rows, two for R and two for L
+              tma_load_2d_pair(st, tmap_r, q0, k, full_of_leader);
+              tma_load_2d_pair(st + kMnBoxBytes, tmap_r, q0 + 64, k, full_of_leader);
+              tma_load_2d_pair(st + kHalfBytes, tmap_l, p0, k, full_of_leader);
+              tma_load_2d_pair(st + kHalfBytes + kMnBoxBytes, tmap_l, p0 + 64, k, full_of_leader);
+            } else {
+              tma_load_2d_pair(st, tmap_r, k, q0, full_of_leader);
+              tma_load_2d_pair(st + kHalfBytes, tmap_l, k, p0, full_of_leader);
+            }
           } else {
-            tma_load_2d_pair(st, &tmap_r, k, q0, full_of_leader);
-            tma_load_2d_pair(st + kHalfBytes, &tmap_l, k, p0, full_of_leader);
+            mbar_expect_tx(s_full + stage, kHalfBytes + (unsigned)cols * BK * 2);
+            if (a.row_major) {
+              tma_load_2d(st, tmap_r, q0, k, s_full + stage);
+              tma_load_2d(st + kMnBoxBytes, tmap_r, q0 + 64, k, s_full + stage);
+              for (int c = 0; c < cols / 64; ++c)
+                tma_load_2d(st + kHalfBytes + c * kMnBoxBytes, tmap_l, p0 + 64 * c, k, s_full + stage);
+            } else {
+              tma_load_2d(st, tmap_r, k, q0, s_full + stage);
+              for (int c = 0; c < cols / 128; ++c)
+                tma_load_2d(st + (1 + c) * kHalfBytes, tmap_l, k, p0 + 128 * c, s_full + stage);
+            }
           }
           if (++stage == kStages) {
             stage = 0;
@@ -206,15 +228,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader only) ----------------
     if (lane == 0 && rank == 0 && tmem_ok) {
-      constexpr unsigned idesc = make_idesc(2 * BM, BN);
-      constexpr unsigned idesc_mn = make_idesc(2 * BM, BN, true, true);
+      constexpr int M = kPair ? 2 * BM : BM;
       const unsigned kstep = a.row_major ? kDescStepMn : kDescStepK;
       int stage = 0;
       unsigned phase = 0;
       unsigned tphase[2] = {0, 0};
       int it = 0;
       bool failed = false;
-      for (long long t = pair; t < num_tiles && !failed; t += npairs) {
+      for (long long t = unit; t < num_tiles && !failed; t += nunits) {
         const WgradTile w = wgrad_tile(a, s_groups, t);
         if (w.krows == 0 || w.out == nullptr) continue;
         const int buf = it & 1;
@@ -227,6 +248,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         tc_fence_after();
         const unsigned d_tmem = tmem_base + (unsigned)(buf * BN);
         const int kbs = (w.krows + BK - 1) / BK;
+        const bool half = !kPair && a.P - w.pb * BN < BN;  // the last tile of an odd P
+        const unsigned idesc = a.row_major ? (half ? make_idesc(M, 128, true, true) : make_idesc(M, BN, true, true))
+                                           : (half ? make_idesc(M, 128) : make_idesc(M, BN));
         for (int kb = 0; kb < kbs; ++kb) {
           if (!mbar_wait_cluster(s_full + stage, phase, a.timeout_ns)) {
             gemm_fail(a.status, 14, 3, stage, kb);
@@ -238,19 +262,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           const unsigned long long adesc = a.row_major ? make_smem_desc_mn(st) : make_smem_desc(st);
           const unsigned long long bdesc = a.row_major ? make_smem_desc_mn(st + kHalfBytes) : make_smem_desc(st + kHalfBytes);
           const int nkk = min(BK / UMMA_K, (w.krows - kb * BK) / UMMA_K);  // MMAs inside the group
-          for (int kk = 0; kk < nkk; ++kk)
-            umma_bf16_pair(d_tmem, adesc + (unsigned long long)(kk * kstep), bdesc + (unsigned long long)(kk * kstep),
-                      a.row_major ? idesc_mn : idesc, (kb | kk) != 0 ? 1u : 0u);
-          umma_commit_pair(s_empty + stage, 3);
+          for (int kk = 0; kk < nkk; ++kk) {
+            const unsigned long long ad = adesc + (unsigned long long)(kk * kstep), bd = bdesc + (unsigned long long)(kk * kstep);
+            const unsigned add = (kb | kk) != 0 ? 1u : 0u;
+            if (kPair) umma_bf16_pair(d_tmem, ad, bd, idesc, add); else umma_bf16(d_tmem, ad, bd, idesc, add);
+          }
+          if (kPair) umma_commit_pair(s_empty + stage, 3); else umma_commit(s_empty + stage);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (!failed) umma_commit_pair(s_tfull + buf, 3);
+        if (!failed) {
+          if (kPair) umma_commit_pair(s_tfull + buf, 3); else umma_commit(s_tfull + buf);
+        }
       }
-      // the pair must not be torn down under a running MMA: wait for everything issued so far
-      umma_commit_pair(&s_done, 1);
+      // nothing may be torn down under a running MMA: wait for everything issued so far
+      if (kPair) umma_commit_pair(&s_done, 1); else umma_commit(&s_done);
       if (!mbar_wait_cluster(&s_done, 0, a.timeout_ns)) gemm_fail(a.status, 14, 5, 0, 0);
     }
     __syncwarp();
@@ -260,7 +288,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const unsigned tempty_of_leader[2] = {mapa_u32(s_tempty + 0, 0), mapa_u32(s_tempty + 1, 0)};
     unsigned tphase[2] = {0, 0};
     int it = 0;
-    for (long long t = pair; tmem_ok && t < num_tiles; t += npairs) {
+    for (long long t = unit; tmem_ok && t < num_tiles; t += nunits) {
       const WgradTile w = wgrad_tile(a, s_groups, t);
       const int flag = w.flag;
       if (w.out == nullptr) {
@@ -275,7 +303,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         continue;
       }
-      float* out = w.out + (long long)w.pb * BN * a.Q + w.qb * BN + (int)rank * 128 + q * 32 + lane;
+      float* out = w.out + (long long)w.pb * BN * a.Q + w.qb * (kPair ? BN : 128) + (int)rank * 128 + q * 32 + lane;
       const int cols = min(BN, a.P - w.pb * BN);  // rows of dW in this tile: 256, or 128 in the last tile of an odd P
       if (w.krows == 0) {
         if (flag == 0)
@@ -314,11 +342,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();  // nobody delivers to, or computes on, a CTA that has left
+  if (kPair) cluster_sync_all();  // nobody delivers to, or computes on, a CTA that has left
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_l, const __grid_constant__ CUtensorMap tmap_r,
+                         const WgradArgs a) {
+  wgrad_body<true>(&tmap_l, &tmap_r, a);
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+    grouped_wgrad_single_kernel(const __grid_constant__ CUtensorMap tmap_l, const __grid_constant__ CUtensorMap tmap_r,
+                                const WgradArgs a) {
+  wgrad_body<false>(&tmap_l, &tmap_r, a);
 }
 
 }  // namespace
@@ -327,9 +367,39 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
 using namespace moonep;
 
-static int launch_wgrad(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs& a, int num_sms, void* stream) {
-  a.p_tiles = (a.P + BN - 1) / BN;  // the last tile of an odd P computes 128 columns that are not stored
-  const size_t smem = (size_t)kStages * kStageBytes + 1024;
+static int launch_single(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs& a, int num_sms, void* stream) {
+  static int sms = -1;
+  if (sms < 0) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(grouped_wgrad_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)kSmemBytes),
+                            "cudaFuncSetAttribute(grouped_wgrad_single_kernel)"))
+      return rc;
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    sms = n;
+  }
+  a.q_tiles = a.Q / 128;
+  grouped_wgrad_single_kernel<<<num_sms > 0 ? imin(num_sms, sms) : sms, kThreads, kSmemBytes, (cudaStream_t)stream>>>(tl, tr, a);
+  return check_launch("grouped_wgrad_single_kernel");
+}
+
+// One CTA per tile, or pairs: 1 or 0.  rows_per_group: rows of a group that has any, as far as the caller knows.
+// Short groups are epilogue: a CTA's results are half a pair's, and the tail wave is finer.  16 groups, 1024 x 2048, single
+// against pair: 256 rows 36.2 and 37.0 us (adding: 63.0, 65.1), 512 rows 53.3 and 47.2; 64 groups x 128 rows, 640 x 1024: 41.7
+// and 44.4.  A pair cannot use the last of an odd number of SMs, and not one alone: 3 SMs 971 and 1400 us, 9 SMs 332 and 361
+// (16 groups x 128 rows), from there on the pair's rate makes up for it.
+extern "C" int moonep_wgrad_single_cta(int rows_per_group, int num_sms) {
+  return rows_per_group < 384 || (num_sms < 10 && (num_sms & 1) != 0) ? 1 : 0;
+}
+
+static int launch_wgrad(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs& a, int rows_per_group, int num_sms,
+                        void* stream) {
+  a.p_tiles = (a.P + BN - 1) / BN;  // a pair computes 128 columns that are not stored in the last tile of an odd P
+  if (rows_per_group <= 0) rows_per_group = a.rows_cap / a.G;
+  if (moonep_wgrad_single_cta(rows_per_group, imax(0, num_sms))) return launch_single(tl, tr, a, num_sms, stream);
+  a.q_tiles = a.Q / BN;
+  const size_t smem = kSmemBytes;
   static int max_pairs = -1;  // pairs of these CTAs the device runs at once
   if (max_pairs < 0) {
     if (int rc = check_cuda(cudaFuncSetAttribute(grouped_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -361,7 +431,7 @@ static int launch_wgrad(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs&
     return 1;
   }
   int pairs = max_pairs;
-  if (num_sms > 0) pairs = imax(1, imin(pairs, num_sms / 2));
+  if (num_sms > 0) pairs = imin(pairs, num_sms / 2);
   grouped_wgrad_kernel<<<2 * pairs, kThreads, smem, (cudaStream_t)stream>>>(tl, tr, a);
   return check_launch("grouped_wgrad_kernel");
 }
@@ -369,10 +439,10 @@ static int launch_wgrad(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs&
 // lt: [P, ld] bf16 = L^T, rt: [Q, ld] bf16 = R^T (ld elements per row, a multiple of 8; the column index is the
 // row of the dispatched shard).  For every group g with rows [cu[g-1], cu[g]) (a multiple of 16 long):
 // out_ptrs[g][P, Q] fp32 = or += L_g^T R_g according to flags[g] (see the kernel).  out_ptrs and flags are
-// device arrays of G entries.  P % 128 == 0, Q % 256 == 0.
+// device arrays of G entries.  P % 128 == 0, Q % 256 == 0.  rows_per_group: see moonep_wgrad_single_cta (0: rows_cap / G).
 extern "C" int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld, int P, int Q, const int* cu_seqlens,
                                     int G, void* const* out_ptrs, const int* flags, int rows_cap, int* status,
-                                    long long timeout_ms, int num_sms, void* stream) {
+                                    long long timeout_ms, int rows_per_group, int num_sms, void* stream) {
   if (P <= 0 || Q <= 0 || P % BM != 0 || Q % BN != 0) {
     set_error("moonep_grouped_wgrad: P must be a multiple of 128 and Q a multiple of 256");
     return 1;
@@ -397,10 +467,9 @@ extern "C" int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld
   a.G = G;
   a.P = P;
   a.Q = Q;
-  a.q_tiles = Q / BN;
   a.rows_cap = rows_cap;
   a.row_major = 0;
-  return launch_wgrad(tl, tr, a, num_sms, stream);
+  return launch_wgrad(tl, tr, a, rows_per_group, num_sms, stream);
 }
 
 // The same with the operands as they are: l = L [rows, P] and r = R [rows, Q] bf16, rows ldl / ldr elements apart
@@ -408,7 +477,8 @@ extern "C" int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld
 // tiles are staged MN-major (see make_smem_desc_mn).
 extern "C" int moonep_grouped_wgrad_rows(const void* l, long long ldl, const void* r, long long ldr, int rows, int P,
                                          int Q, const int* cu_seqlens, int G, void* const* out_ptrs, const int* flags,
-                                         int* status, long long timeout_ms, int num_sms, void* stream) {
+                                         int* status, long long timeout_ms, int rows_per_group, int num_sms,
+                                         void* stream) {
   if (P <= 0 || Q <= 0 || P % BM != 0 || Q % BN != 0) {
     set_error("moonep_grouped_wgrad_rows: P must be a multiple of 128 and Q a multiple of 256");
     return 1;
@@ -433,8 +503,7 @@ extern "C" int moonep_grouped_wgrad_rows(const void* l, long long ldl, const voi
   a.G = G;
   a.P = P;
   a.Q = Q;
-  a.q_tiles = Q / BN;
   a.rows_cap = rows;
   a.row_major = 1;
-  return launch_wgrad(tl, tr, a, num_sms, stream);
+  return launch_wgrad(tl, tr, a, rows_per_group, num_sms, stream);
 }

@@ -307,12 +307,14 @@ class ExpertParallelMoE:
         ptrs = self._wgrad_ptrs
         done = after if after is not None else (lambda i: None)
         later = num_sms if after is not None else 0
+        # rows of an owned expert, on average; the prefetch slots of a step are mostly empty
+        kw = {"status": status, "rows_per_group": max(1, self.S * self.K // self.epn)}
         if config.wgrad_layout() == "rows":  # the kernel stages MN-major tiles: the activations as they are
-            grouped_wgrad_rows(dy_nvs, hsw, cu, ptrs[2], flags, status=status)  # dW_down = dy^T (h * gate weight)
+            grouped_wgrad_rows(dy_nvs, hsw, cu, ptrs[2], flags, **kw)  # dW_down = dy^T (h * gate weight)
             done(2)
-            grouped_wgrad_rows(dadu[:, :I], x_nvs, cu, ptrs[0], flags, status=status, num_sms=later)  # dW_gate = da^T x
+            grouped_wgrad_rows(dadu[:, :I], x_nvs, cu, ptrs[0], flags, num_sms=later, **kw)  # dW_gate = da^T x
             done(0)
-            grouped_wgrad_rows(dadu[:, I:], x_nvs, cu, ptrs[1], flags, status=status, num_sms=later)  # dW_up   = du^T x
+            grouped_wgrad_rows(dadu[:, I:], x_nvs, cu, ptrs[1], flags, num_sms=later, **kw)  # dW_up   = du^T x
             done(1)
         else:  # K-major tiles from transposed copies
 
@@ -321,11 +323,11 @@ class ExpertParallelMoE:
                 return transpose_experts(t[:rows].unsqueeze(0), out)[0]
 
             xt, dadut, dyt, hswt = transposed(x_nvs), transposed(dadu), transposed(dy_nvs), transposed(hsw)
-            grouped_wgrad(dyt, hswt, cu, ptrs[2], flags, status=status)
+            grouped_wgrad(dyt, hswt, cu, ptrs[2], flags, **kw)
             done(2)
-            grouped_wgrad(dadut[:I], xt, cu, ptrs[0], flags, status=status, num_sms=later)
+            grouped_wgrad(dadut[:I], xt, cu, ptrs[0], flags, num_sms=later, **kw)
             done(0)
-            grouped_wgrad(dadut[I:], xt, cu, ptrs[1], flags, status=status, num_sms=later)
+            grouped_wgrad(dadut[I:], xt, cu, ptrs[1], flags, num_sms=later, **kw)
             done(1)
         self._fresh = False
         return True

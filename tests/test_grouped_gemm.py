@@ -3,6 +3,7 @@
 import pytest
 import torch
 
+from moonep_b200.ops import _lib
 from moonep_b200.ops.grouped_gemm import grouped_gemm, grouped_gemm_reference
 
 
@@ -221,6 +222,47 @@ def test_grouped_wgrad_matches_fp32_reference(rows, P, Q, layout):
     grouped_wgrad_reference(left.cpu(), right.cpu(), cu.cpu(), targets, flag_list)
     excess = ((out.cpu() - want).abs() / (2 * bound)).max().item()
     assert excess <= 1.0, f"second launch: an element is {excess:.2f} times its error bound away"
+
+
+def test_wgrad_rule_keeps_to_the_bound_on_sms():
+    """A pair takes two SMs, so one SM, and a few odd numbers of them, run with one CTA per tile; so do short groups."""
+    single = _lib.load().moonep_wgrad_single_cta
+    assert all(single(rows, sms) for rows in (16, 1024) for sms in (1, 3, 9))
+    assert all(single(128, sms) for sms in (0, 2, 8, 147)) and not any(single(384, sms) for sms in (0, 2, 8, 148))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("num_sms", [0, 1, 2, 3, 5])
+@pytest.mark.parametrize("rows,P,Q", [([16, 0, 208], 128, 256), ([1024, 400, 0, 16], 384, 256), ([80, 1200], 256, 512)])
+def test_grouped_wgrad_on_pairs_and_single_ctas_agree(rows, P, Q, num_sms):
+    """The same operands through both kernels and both layouts, with targets at 4-byte addresses, within the accumulation
+    error of the fp32 reference element by element."""
+    from moonep_b200.ops.grouped_gemm import grouped_wgrad, grouped_wgrad_reference, grouped_wgrad_rows
+
+    G = len(rows)
+    left, right, cu, cap = _wgrad_case(rows, P, Q, seed=P, device="cuda")
+    lt, rt = left.t().contiguous(), right.t().contiguous()
+    flag_list = [1, 0, 0, 2][:G]
+    init = torch.randn(G, P, Q, device="cuda")
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    flags = torch.tensor(flag_list, dtype=torch.int32, device="cuda")
+    want = [t.clone() for t in init.cpu()]
+    grouped_wgrad_reference(left.cpu(), right.cpu(), cu.cpu(), want, flag_list)
+    ends = [0, *cu.tolist()]
+    ad = [left[a:b].float().abs().cpu().t() @ right[a:b].float().abs().cpu() for a, b in zip(ends, ends[1:])]
+    bound = [ACC_REL * d + 2.0**-22 * w.abs() + 1e-30 for d, w in zip(ad, want)]
+    for per_group in (1, 1 << 20):
+        for layout in ("rows", "transposed"):
+            flat = torch.empty(G * P * Q + 1, device="cuda")
+            out = flat[1:].view(G, P, Q).copy_(init)
+            ptrs = torch.tensor([out[g].data_ptr() for g in range(G)], dtype=torch.int64, device="cuda")
+            args = (left, right) if layout == "rows" else (lt, rt)
+            run = grouped_wgrad_rows if layout == "rows" else grouped_wgrad
+            run(*args, cu, ptrs, flags, status=status, num_sms=num_sms, rows_per_group=per_group)
+            torch.cuda.synchronize()
+            assert status.tolist()[0] == 0
+            for g in range(G):
+                assert bool(((out[g].cpu() - want[g]).abs() <= bound[g]).all()), (per_group, layout, g)
 
 
 def test_kn_reference_on_cpu():
