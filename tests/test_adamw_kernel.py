@@ -12,7 +12,11 @@ from moonep_b200.ops.moe_ops import adamw_update
         ("cpu", [12], 0),
         pytest.param("cuda", [4], 0, marks=pytest.mark.gpu),
         pytest.param("cuda", [1020, 1024, 1028], 0, marks=pytest.mark.gpu),
-        pytest.param("cuda", [148 * 8 * 1024 + 4, 8], 0, marks=pytest.mark.gpu),  # one vector past the grid's first step
+        # just short of, at and past one vector per thread of a full GPU, then two and four of them
+        pytest.param("cuda", [148 * 8 * 1024 - 4, 8], 0, marks=pytest.mark.gpu),
+        pytest.param("cuda", [148 * 8 * 1024 + 4, 8], 0, marks=pytest.mark.gpu),
+        pytest.param("cuda", [148 * 16 * 1024 + 4], 0, marks=pytest.mark.gpu),
+        pytest.param("cuda", [148 * 40 * 1024 + 1028], 0, marks=pytest.mark.gpu),
         pytest.param("cuda", [1001, 64], 0, marks=pytest.mark.gpu),  # not whole vectors: elementwise operations
         pytest.param("cuda", [64, 64], 1, marks=pytest.mark.gpu),  # not 16-byte aligned: elementwise operations
     ],
@@ -43,3 +47,19 @@ def test_adamw_step(device, sizes, shift):
         dstep = 12 * u * step.abs() + lr / c1 * dm / ((v1 / c2).sqrt() + eps)
         assert bool(((p[i].double() - p1).abs() <= 4 * u * (p0.abs() + step.abs()) + dstep).all())
         assert torch.equal(w[i], p[i].to(torch.bfloat16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [8, 2040, 148 * 8 * 2048 - 8, 148 * 16 * 2048 + 8, 148 * 40 * 2048 + 2056])
+def test_sgd_update_at_the_edges_of_its_grid(n):
+    from moonep_b200.ops.moe_ops import sgd_update
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    w0 = torch.randn(n, generator=g, device="cuda").to(torch.bfloat16)
+    gr = torch.randn(n, generator=g, device="cuda")
+    w = torch.cat([w0, w0[:8]])
+    sgd_update(w[:n], gr, 0.25)
+    # the product is exact, the difference rounded to fp32 (2^-24) and to bf16, whose 8-bit mantissa gives 2^-8
+    want = w0.double() - 0.25 * gr.double()
+    assert bool(((w[:n].double() - want).abs() <= (2.0**-8 + 2.0**-23) * want.abs()).all())
+    assert torch.equal(w[n:], w0[:8])  # nothing past the end
