@@ -72,14 +72,25 @@ def sgd_update(w: torch.Tensor, g: torch.Tensor, lr: float) -> None:
     _lib.check(rc, "moonep_sgd_update")
 
 
+_ADAM_TENSORS = 3  # weights per launch of the AdamW kernel
+
+
 def adamw_update(masters, exp_avgs, exp_avg_sqs, grads, weights, *, lr, b1, b2, eps, weight_decay, c1, c2) -> None:
-    """One AdamW step of up to three weights: fp32 ``masters`` and moments are updated from the fp32 ``grads`` and the
+    """One AdamW step of any number of weights: fp32 ``masters`` and moments are updated from the fp32 ``grads`` and the
     rounded masters stored to the bf16 ``weights``.  ``c1``, ``c2``: bias corrections ``1 - b**t``."""
     tensors = [list(ts) for ts in (masters, exp_avgs, exp_avg_sqs, grads, weights)]
+    if len({len(ts) for ts in tensors}) != 1:
+        raise ValueError(f"adamw_update: lists of {[len(ts) for ts in tensors]} tensors")
+    for i in range(0, len(tensors[4]), _ADAM_TENSORS):
+        _adamw_step([ts[i : i + _ADAM_TENSORS] for ts in tensors], lr, b1, b2, eps, weight_decay, c1, c2)
+
+
+def _adamw_step(tensors, lr, b1, b2, eps, weight_decay, c1, c2) -> None:
+    weights = tensors[4]
     kernel = all(
         t.is_cuda and t.is_contiguous() and t.numel() == w.numel() and t.device == weights[0].device
-        and t.dtype == (torch.bfloat16 if ts is tensors[4] else torch.float32)
-        and t.numel() % 4 == 0 and t.data_ptr() % (8 if ts is tensors[4] else 16) == 0
+        and t.dtype == (torch.bfloat16 if ts is weights else torch.float32)
+        and t.numel() % 4 == 0 and t.data_ptr() % (8 if ts is weights else 16) == 0
         for ts in tensors for t, w in zip(ts, weights)
     )  # fmt: skip
     if not kernel:
@@ -91,9 +102,9 @@ def adamw_update(masters, exp_avgs, exp_avg_sqs, grads, weights, *, lr, b1, b2, 
             p.addcdiv_(m, (v / c2).sqrt_().add_(eps), value=-lr / c1)
             w.copy_(p)
         return
-    n = len(tensors[4])
+    n = len(weights)
     ptrs = [(ctypes.c_void_p * n)(*[t.data_ptr() for t in ts]) for ts in tensors]
-    sizes = (ctypes.c_longlong * n)(*[t.numel() for t in tensors[4]])
+    sizes = (ctypes.c_longlong * n)(*[t.numel() for t in weights])
     with _lib.on_device(weights[0].device):
         rc = _lib.load().moonep_adamw_update(n, *ptrs, sizes, lr / c1, b1, b2, eps, 1.0 - lr * weight_decay, c2,
                                              _lib.current_stream())  # fmt: skip

@@ -10,8 +10,11 @@ from moonep_b200.ops.moe_ops import adamw_update
     "device,sizes,shift",
     [
         ("cpu", [12], 0),
+        ("cpu", [], 0),
+        ("cpu", [4, 8, 12, 16], 0),
         pytest.param("cuda", [4], 0, marks=pytest.mark.gpu),
         pytest.param("cuda", [1020, 1024, 1028], 0, marks=pytest.mark.gpu),
+        pytest.param("cuda", [8, 4, 1024, 64, 1028, 16, 12], 0, marks=pytest.mark.gpu),  # three launches
         # just short of, at and past one vector per thread of a full GPU, then two and four of them
         pytest.param("cuda", [148 * 8 * 1024 - 4, 8], 0, marks=pytest.mark.gpu),
         pytest.param("cuda", [148 * 8 * 1024 + 4, 8], 0, marks=pytest.mark.gpu),
@@ -30,7 +33,9 @@ def test_adamw_step(device, sizes, shift):
     p, m, gr = ([make(n) for n in sizes] for _ in range(3))
     v = [make(n).abs_() for n in sizes]
     w = [make(n, torch.bfloat16) for n in sizes]
-    gr[0][0] = v[0][0] = m[0][0] = 0.0  # an element that has never had a gradient only decays
+    for ts in (gr, v, m):
+        for t in ts[:1]:
+            t[0] = 0.0  # an element that has never had a gradient only decays
     old = [[t.double().clone() for t in ts] for ts in (p, m, v, gr)]
     lr, b1, b2, eps, wd, t = 1e-2, 0.9, 0.95, 1e-8, 0.1, 3
     c1, c2 = 1 - b1**t, 1 - b2**t
@@ -47,6 +52,12 @@ def test_adamw_step(device, sizes, shift):
         dstep = 12 * u * step.abs() + lr / c1 * dm / ((v1 / c2).sqrt() + eps)
         assert bool(((p[i].double() - p1).abs() <= 4 * u * (p0.abs() + step.abs()) + dstep).all())
         assert torch.equal(w[i], p[i].to(torch.bfloat16))
+
+
+def test_adamw_refuses_lists_that_do_not_match():
+    t = [torch.zeros(4)]
+    with pytest.raises(ValueError):
+        adamw_update(t, t, t, t, t + t, lr=1e-2, b1=0.9, b2=0.95, eps=1e-8, weight_decay=0.0, c1=0.1, c2=0.05)
 
 
 @pytest.mark.gpu
