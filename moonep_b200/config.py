@@ -31,7 +31,8 @@ MOONEP_NUM_SMS_DEDUP  CTAs of the dispatch kernel's destination-side role (zero 
                       expansion; with one rank: of the whole dispatch); validated, 1..SM count; default: every SM the
                       senders leave free.
 MOONEP_NVTX           ``1`` wraps every native call in an NVTX range.
-MOONEP_GEMM_PAIR      ``1`` (default): grouped GEMMs on CTA pairs (tcgen05 cta_group::2); ``0``: one CTA per tile.
+MOONEP_GEMM_PAIR      ``1``: grouped GEMMs on CTA pairs (tcgen05 cta_group::2); ``0``: one CTA per tile.  Unset: pairs, except
+                      that the MoE layer's forward GEMMs on one rank take one CTA per tile up to 128 rows per expert.
 MOONEP_WGRAD          ``kernel`` (default) or ``torch``: weight gradients of the MoE layer.
 MOONEP_WGRAD_LAYOUT   ``rows`` (default: activations as stored, MN-major tiles) or ``transposed``.
 
@@ -151,6 +152,11 @@ def gemm_on_cta_pairs() -> bool:
     """The grouped GEMM runs on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles; measured 9-10 % faster);
     MOONEP_GEMM_PAIR=0 selects the kernel with one CTA per 128 x 256 tile."""
     return os.environ.get("MOONEP_GEMM_PAIR", "1") not in _FALSE
+
+
+def gemm_pair_is_set() -> bool:
+    """True when the environment names the grouped GEMM kernel explicitly."""
+    return bool(os.environ.get("MOONEP_GEMM_PAIR"))
 
 
 def wgrad_layout() -> str:

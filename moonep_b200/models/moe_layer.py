@@ -126,6 +126,19 @@ class ExpertParallelMoE:
             self.bwd_buffer = None
 
     # -- forward -------------------------------------------------------------------------------
+    def forward_gemm_pair(self):
+        """``pair`` of the forward GEMMs: None for the default, False for one CTA per tile.
+
+        Up to 128 rows per expert most groups are one row block, which leaves the second CTA of a pair without work: one
+        CTA per tile takes 0.92 of the pairs' time on average over 420 combinations of 4 to 64 experts, 8 to 128 rows per
+        expert, H 1024 to 7168, I 512 to 2048 with even, Zipf and one-hot routing (0.73 to 1.05 with even routing; at worst
+        1.12, 8 experts of 100 rows with Zipf routing, whose hot experts have several blocks).  From two blocks on the pairs
+        win or are equal where the count is even (8 experts of 512 rows, H=7168: 229 us against 240).  The counts are not
+        known on the host, so their mean decides.  With several ranks the hand-off hooks need the pairs, and
+        MOONEP_GEMM_PAIR, where it is set, is what it says."""
+        short = self.R == 1 and self.S * self.K <= 128 * self.E
+        return False if short and not config.gemm_pair_is_set() else None
+
     def _forward_fast(self, x, gates, topk, tokens_per_expert, save_for_backward):
         """CUDA: dispatch -> prefetch (on the communication stream, beside the GEMMs) -> SwiGLU GEMM -> down projection
         into a separate tensor -> push combine that reads it in place.  The GEMMs take their hand-off from the
@@ -150,11 +163,7 @@ class ExpertParallelMoE:
         hooked = not alone and rows >= 128 and self.H % 256 == 0 and self.I % 128 == 0
         if fetched is not None and not hooked:
             torch.cuda.current_stream().wait_event(fetched)
-        # Up to 128 rows per expert most groups are one row block, which leaves the second CTA of a pair without work: one
-        # CTA per tile is faster (16 experts of 128 rows, H=2048, I=1024: SwiGLU 72 -> 57 us, down 31 -> 27; 8 experts,
-        # H=7168, I=2048: 141 -> 123, 76 -> 64).  From two blocks on the pairs win or are equal where the count is even
-        # (8 experts of 512 rows, H=7168: 229 against 240).  The hand-off hooks need the pairs.
-        pair = False if alone and self.S * self.K <= 128 * self.E else None
+        pair = self.forward_gemm_pair()
         h = grouped_gemm(x_nvs, self.w_gate, cu, w_up=self.w_up, mode="swiglu", status=status, pair=pair,
                          save_pre=None if a is None else (a, u),
                          hooks=buf.gemm_hooks(rows=True, slots=True) if hooked else None)  # fmt: skip

@@ -81,6 +81,26 @@ def _layer_against_dense(device, R, routing):
     lw.run(lambda r: bufs[r].destroy())
 
 
+def test_forward_gemm_kernel_follows_the_switch_where_it_is_set(monkeypatch):
+    def chosen(R, S):
+        lw = LocalWorld(R, "cpu")
+
+        def body(r):
+            buf = Buffer(S, 16, 2, 4, R, token_padding=8, world=lw.view(r))
+            layer = ExpertParallelMoE(buf, 8)
+            pair = layer.forward_gemm_pair()
+            layer.destroy()
+            buf.destroy()
+            return pair
+
+        return lw.run(body)[0]
+
+    monkeypatch.delenv("MOONEP_GEMM_PAIR", raising=False)
+    assert chosen(1, 256) is False and chosen(1, 257) is None and chosen(2, 8) is None
+    monkeypatch.setenv("MOONEP_GEMM_PAIR", "1")
+    assert chosen(1, 256) is None
+
+
 @pytest.mark.parametrize("device", DEVICES)
 def test_moe_helper_ops_match_torch(device):
     """Batched expert transpose, SwiGLU backward and the SGD update against plain torch."""
