@@ -19,7 +19,8 @@ MOONEP_SUM_SLOTS      ``2``: a warp of combine's sum role holds two tokens and s
                       the native library; default 1: measured equal or slower on 2 GPUs, not measured on more).
 MOONEP_BWD_OVERLAP    ``1``: the MoE layer reduces each weight's gradients beside the remaining backward GEMMs (default 0).
 MOONEP_EXPAND_PATH    ``bulk`` (default) or ``ldst``: how the destination side of dispatch copies duplicate rows and clears
-                      pad rows; with one rank, how it moves all rows (read by the native library).
+                      pad rows; with one rank, how it moves all rows (read by the native library, with one rank
+                      when the Buffer is made).
 MOONEP_COMBINE        ``push`` (default: the expert side folds duplicates and pushes rows to the tokens' home ranks,
                       which sum them as they arrive) or ``pull`` (fold pass, then the home ranks pull).
 MOONEP_PHASED         ``1``: launch the dispatch and combine kernels one role at a time even on real multi-GPU worlds

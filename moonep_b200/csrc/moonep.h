@@ -93,6 +93,8 @@
 #define MOONEP_PH_WAIT_PLAN 4     // EXPAND role: wait for every peer's FLAG_PLAN
 #define MOONEP_PH_BUILD_EXPAND 5  // EXPAND role: duplicate map + expansion (includes waiting for rows to land)
 #define MOONEP_PH_WAIT_SENT 6     // EXPAND role: final wait for every peer's FLAG_SENT
+// The single-rank dispatch kernel: TABLES its group layout, TOKENS a CTA's planning, ZERO its pads, SEND its rows, and
+// BUILD_EXPAND a CTA from beginning to end.  The single-rank combine is one phase, which the launch's time is.
 #define MOONEP_PH_FOLD 7          // combine FOLD role
 #define MOONEP_PH_PUSH 8          // combine PUSH role (a copy warp)
 #define MOONEP_PH_SUM 9           // combine SUM role

@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdio>
+#include <cstdlib>
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -109,6 +110,8 @@ extern "C" void* moonep_ctx_create(const long long* p, int nparams, const unsign
     }
     d.stage_peer = (unsigned char* const*)((char*)tab + 2 * tbytes);
   }
+  const char* xp = getenv("MOONEP_EXPAND_PATH");
+  h->expand_ldst = xp != nullptr && strcmp(xp, "ldst") == 0 ? 1 : 0;
   cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, 0);
   int devid = 0;
   cudaGetDevice(&devid);

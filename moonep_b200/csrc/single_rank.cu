@@ -21,9 +21,6 @@
 // Parity: reference moonep_td/dispatch.py:42-117, moonep_td/_dedup_builder.py:23-108, moonep_td/combine.py:22-68 at one
 // rank; the plan's contents are those of the general kernels (the order of the duplicate groups, which is arbitrary
 // there, is token order here).
-#include <cstdlib>
-#include <cstring>
-
 #include "common.cuh"
 #include "host.h"
 
@@ -970,9 +967,8 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
   a.topk_vec = aligned16(topk) ? 1 : 0;
   a.vec_ok = (c.H % 8 == 0 && aligned16(a.out)) ? 1 : 0;
   // MOONEP_EXPAND_PATH=ldst selects register copies as it does with several ranks (S=4096, H=7168, K=8, E=32: 126 us
-  // against 112 with bulk copies)
-  const char* xp = getenv("MOONEP_EXPAND_PATH");
-  a.bulk_pads = (a.vec_ok && !(xp != nullptr && strcmp(xp, "ldst") == 0)) ? 1 : 0;
+  // against 112 with bulk copies); looked up once, a lookup per launch costs 0.8 us
+  a.bulk_pads = (a.vec_ok && !h->expand_ldst) ? 1 : 0;
   a.bulk = (a.bulk_pads && aligned16(hidden)) ? 1 : 0;
   a.narrow = aligned16(hidden) ? 0 : 1;
   // rows of 16-byte words take any input (the stores, K per load, stay wide); others move in what all addresses allow
