@@ -90,8 +90,11 @@ __device__ __forceinline__ void record_status(const MoonepDevCtx& c, int code, i
 }
 
 // Phase statistics: one thread of a CTA reports how long a phase took; the longest one over the CTAs is kept.
+__device__ __forceinline__ void stat_phase(const MoonepDevCtx& c, int phase, unsigned long long t0, unsigned long long t1) {
+  atomicMax(reinterpret_cast<unsigned long long*>(c.stats) + MOONEP_STAT_PHASE_NS + phase, t1 - t0);
+}
 __device__ __forceinline__ void stat_phase(const MoonepDevCtx& c, int phase, unsigned long long t0) {
-  atomicMax(reinterpret_cast<unsigned long long*>(c.stats) + MOONEP_STAT_PHASE_NS + phase, globaltimer_ns() - t0);
+  stat_phase(c, phase, t0, globaltimer_ns());
 }
 
 // Programmatic dependent launch: everything before this call may run while the previous kernel of the stream is

@@ -682,8 +682,12 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
       lay = {first, nullptr, nullptr, cum, groups};
       __syncthreads();
     }
+    unsigned long long t_laid = 0, t_planned = 0;  // kept by the two threads that report the phases
+    if (tid == 0 || tid == kEntries) t_laid = globaltimer_ns();
+    if (tid == 0 && a.fresh) stat_phase(c, MOONEP_PH_TABLES, t_begin, t_laid);
     if (warp >= kPlanWarps) {
       clear_pads(c, a, lay, s.grab[warp - kPlanWarps], zeros, shard, meta, epoch);
+      if (tid == kEntries) stat_phase(c, MOONEP_PH_ZERO, t_laid);
       if (a.fresh)  // rows behind the last group are unused
         for (int row = used + blockIdx.x * (kThreads - kEntries) + tid - kEntries; row < NvS;
              row += gridDim.x * (kThreads - kEntries)) {
@@ -697,7 +701,10 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
           plan_tokens(c, a, s, cnt, off, cur, meta, t_lo, t_hi);
           fence_gpu();
           plan_sync();
-          if (tid == 0) st_release_gpu(a.work + kWorkReady + blockIdx.x, epoch);
+          if (tid == 0) {
+            st_release_gpu(a.work + kWorkReady + blockIdx.x, epoch);
+            stat_phase(c, MOONEP_PH_TOKENS, t_laid);
+          }
         } else {
           for (int i = t_lo * K + tid; i < t_hi * K; i += kEntries) {
             const int d = a.dst[i];
@@ -709,10 +716,12 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
           }
         }
       }
+      if (tid == 0) t_planned = globaltimer_ns();
       if (!a.bulk)
         copy_plain(c, a, t_lo, t_hi, shard, meta, epoch);
       else if (warp < a.copy_warps)
         ok = copy_bulk(c, a, s, s_dyn, reinterpret_cast<unsigned char*>(shard), meta, epoch);
+      if (tid == 0) stat_phase(c, MOONEP_PH_SEND, t_planned);
       // rows behind the last group go into the copy as they are; the warps that do not stream rows see to it
       const int w0 = a.bulk ? a.copy_warps : 0;
       if (a.out != nullptr && a.fresh && warp >= w0)

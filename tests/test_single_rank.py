@@ -149,3 +149,19 @@ def test_combine_with_one_to_eight_pieces_of_rows_in_hand(S, H, K, sms, monkeypa
         assert bool(same.all()) and (back is None or torch.equal(back, gates))
     buf.synchronize()
     buf.destroy()
+
+
+def test_phases_of_the_dispatch_are_reported():
+    S, H, K, E = 300, 512, 4, 8
+    buf = Buffer(S, H, K, E, 1, token_padding=16)
+    x, topk, tpe = _inputs(S, H, K, E, 0)
+    _, _, _, plan = buf.dispatch(x, None, topk, tpe)
+    be = buf._require_ctx()["_backend"]
+    for args, names in (((x, None, topk, tpe), {"tables", "tokens", "send", "zero_fill", "build_expand"}),
+                        ((x, None, None, None, plan), {"send", "zero_fill", "build_expand"})):  # fmt: skip
+        be.reset_wait_stats()
+        buf.dispatch(*args)
+        buf.synchronize()
+        phases = buf.stats()["kernel_phase_max_us"]
+        assert set(phases) == names
+    buf.destroy()
