@@ -7,7 +7,7 @@
 // read both CTAs' shared memory and write 128 x 256 fp32 accumulators into both CTAs' TMEM.  Compared
 // with one CTA per 128 x 256 tile this halves the W bytes every SM moves through shared memory (32 KB
 // instead of 48 KB per K block for the same MMA work), which is what bounds the single-CTA kernel, and
-// leaves room for a 5-stage ring and the output pieces.
+// leaves room for a ring of five or six stages and the output pieces.
 //
 // Per CTA, 192 threads:
 //   warp 0      TMA producer (both CTAs): X tile and W half tile of this CTA per K block; the bytes of
@@ -15,8 +15,9 @@
 //   warp 1      allocates this CTA's 512 TMEM columns; in the leader one lane issues four
 //               tcgen05.mma.cta_group::2 (M=256, N=256, K=16) per stage and commits to the stage's
 //               "empty" barrier in both CTAs, and after the last K block to both "accumulator full" barriers.
-//   warps 2..5  epilogue of this CTA's 128 rows (same epilogues as the single-CTA kernel, stored 32 rows x 64 columns
-//               at a time by tensor copies from shared memory); one arrival per warp on the leader's "accumulator empty" barrier, which counts both CTAs' warps.
+//   warps 2..5  epilogue of this CTA's 128 rows (same epilogues as the single-CTA kernel, stored 32 rows x 64 or 32
+//               columns at a time by tensor copies from shared memory); one arrival per warp on the leader's
+//               "accumulator empty" barrier, which counts both CTAs' warps.
 //
 // Tiles: the 128-row blocks of a group are taken two at a time.  When a group has an odd number of
 // blocks the second CTA of its last pair has no rows of that group: it still feeds the MMA (with rows
@@ -36,20 +37,25 @@ namespace moonep {
 
 namespace {
 
-constexpr int kPairStages = 5;
 constexpr int kPairThreads = 192;
 constexpr int kPairTmemCols = 512;
 constexpr unsigned kPairATileBytes = BM * BK * 2;                         // 16 KB: this CTA's rows of X
 constexpr unsigned kPairBHalfBytes = 128 * BK * 2;                        // 16 KB: this CTA's half of the W tile
 constexpr unsigned kPairStageBytes = kPairATileBytes + kPairBHalfBytes;   // 32 KB per CTA and stage
-// The results leave through shared memory: 32 rows x 64 columns per warp and tensor store, in the 128-byte swizzle.
-// Three pieces per warp: in flight one behind the other, or one per output of SwiGLU with its two pre-activations.
-// Against 16-byte stores from registers (a row per lane, two half-written sectors per lane and instruction pair) and a
-// sixth stage: 16 groups of 1024 rows, H=4096, I=1024, down projection 125 -> 117 us, [da|du] times the weights 232 -> 220,
-// SwiGLU with pre-activations 230 -> 226; 8 groups, H=7168, I=2048: 207 -> 193, 410 -> 396, 388 -> 386.
+// The results leave through shared memory: 32 rows x kCols columns per warp and tensor store, swizzled over the row; three
+// such pieces per warp are in flight one behind the other.  Shared memory holds six stages of operands with pieces of 32
+// columns, or five with pieces of 64.  The sixth stage counts where loads bound the kernel, the wide pieces where the
+// epilogue does; the line is drawn at K = 1024 (launch_pair).  Five stages against six, us: 8 groups x 512 rows, K=4096,
+// N=1024: SwiGLU 79.3 and 77.7, plain 54.2 and 52.3; 16 x 128, K=2048, N=1024: SwiGLU 53.7 and 52.3; 16 x 1024, K=4096,
+// N=512: plain 76.0 and 73.7; 16 x 1024, K=1024, N=4096: SwiGLU 302 and 305, with pre-activations 313 and 342; 1 x 16384,
+// K=512, N=2048: 138 and 141, 148 and 159.  16-byte stores from registers with six stages (a row per lane, two half-written
+// sectors per lane and instruction pair): 78.2, 54.3; 52.7; 76.1; 307, 329; 142, 155, plain at the last 47.6 where five
+// stages take 39.1.
 constexpr int kPairPieces = 3;
-constexpr unsigned kPairPieceBytes = 32 * 128;
-constexpr unsigned kPairWarpPieces = kPairPieces * kPairPieceBytes;
+template <int kCols>
+constexpr unsigned kPairWarpPieces = kPairPieces * 32 * kCols * 2;
+template <int kStages, int kCols>
+constexpr size_t kPairSmem = (size_t)kStages * kPairStageBytes + 1024 + 4 * kPairWarpPieces<kCols>;
 constexpr int kPairKernelId = 15;
 constexpr int kPairGroupsInSmem = 2048;  // group ends are walked from shared memory up to this many groups
 
@@ -122,14 +128,6 @@ __device__ __forceinline__ bool rows_arrived(const MoonepGemmHooks& h, int row0,
   }
 }
 
-// Four bf16x8 chunks (32 columns, chunk0 .. chunk0 + 3 of the row's eight) of this lane's row of a piece.
-__device__ __forceinline__ void put_chunks(unsigned char* piece, int lane, int chunk0, const unsigned (&o)[16]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    *reinterpret_cast<uint4*>(piece + lane * 128 + (((chunk0 + j) ^ (lane & 7)) << 4)) =
-        make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-}
-
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, const void* smem_src, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                    reinterpret_cast<unsigned long long>(tmap)),
@@ -137,13 +135,14 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, const void
                : "memory");
 }
 
+template <int kStages, int kCols>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                              const __grid_constant__ CUtensorMap tmap_b1, const __grid_constant__ CUtensorMap tmap_o,
                              const __grid_constant__ CUtensorMap tmap_pg, const __grid_constant__ CUtensorMap tmap_pu,
                              const GemmArgs a) {
   extern __shared__ unsigned char s_raw[];
-  __shared__ __align__(8) unsigned long long s_full[kPairStages], s_empty[kPairStages], s_tfull[2], s_tempty[2], s_done;
+  __shared__ __align__(8) unsigned long long s_full[kStages], s_empty[kStages], s_tfull[2], s_tempty[2], s_done;
   __shared__ unsigned s_tmem_base;
   __shared__ int s_cu[kPairGroupsInSmem];
   unsigned char* s_tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
@@ -167,7 +166,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   const long long pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kPairStages; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       mbar_init(s_full + s, 1);   // used in the leader: its own arrive.expect_tx; both CTAs' copies complete the bytes
       mbar_init(s_empty + s, 1);  // one commit of the leader's MMA lane, delivered to both CTAs
     }
@@ -266,7 +265,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
               tma_load_2d_pair(st + kPairATileBytes, tb, kb * BK, brow, full_of_leader);
             }
           }
-          if (++stage == kPairStages) {
+          if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -312,7 +311,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             umma_bf16_pair(d_tmem, adesc + (unsigned long long)(kk * kDescStepK), bdesc + (unsigned long long)(kk * bstep),
                            a.b_kn ? idesc_kn : idesc, (kb | kk) != 0 ? 1u : 0u);
           umma_commit_pair(s_empty + stage, 3);
-          if (++stage == kPairStages) {
+          if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -328,7 +327,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     // ---------------- epilogue (warps 2..5, both CTAs) ----------------
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     const unsigned tempty_of_leader[2] = {mapa_u32(s_tempty + 0, 0), mapa_u32(s_tempty + 1, 0)};
-    unsigned char* pieces = s_tiles + (size_t)kPairStages * kPairStageBytes + (warp - 2) * kPairWarpPieces;
+    unsigned char* pieces = s_tiles + (size_t)kStages * kPairStageBytes + (warp - 2) * kPairWarpPieces<kCols>;
     int piece = 0;
     PairSched sched(a, cu);
     unsigned tphase[2] = {0, 0};
@@ -350,76 +349,65 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       if (valid) {
         const int row0 = (sched.blk0 + blk_in_group) * BM + q * 32;
         const unsigned taddr = tmem_base + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN);
+        // kCols columns of one output: `value(j)` is the bf16 pair of elements 2j and 2j + 1 of this lane's row
+        auto emit = [&](const CUtensorMap* tmap, int col, auto value) {
+          constexpr int kRowBytes = kCols * 2;
+          unsigned char* p = pieces + piece * 32 * kRowBytes;
+          if (lane == 0) bulk_wait_read<kPairPieces - 1>();
+          __syncwarp();
+          const int swizzle = kCols == 64 ? lane & 7 : (lane >> 1) & 3;
+#pragma unroll
+          for (int j = 0; j < kCols / 8; ++j)
+            *reinterpret_cast<uint4*>(p + lane * kRowBytes + ((j ^ swizzle) << 4)) =
+                make_uint4(value(4 * j), value(4 * j + 1), value(4 * j + 2), value(4 * j + 3));
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(tmap, p, col, row0);
+            bulk_commit();
+          }
+          if (++piece == kPairPieces) piece = 0;
+        };
+        constexpr int kLoads = kCols / 32;  // TMEM loads of 32 columns per piece
         if (a.mode == kSwiglu) {
-          const bool pre = a.pre_gate != nullptr;
 #pragma unroll 1
-          for (int c0 = 0; c0 < 128; c0 += 64) {
-            unsigned char* ph = pieces + piece * kPairPieceBytes;  // pre: piece stays 0 and all three are used
-            if (lane == 0) {
-              if (pre) bulk_wait_read<0>(); else bulk_wait_read<kPairPieces - 1>();
+          for (int c0 = 0; c0 < 128; c0 += kCols) {
+            unsigned g[kLoads][32], u[kLoads][32];
+#pragma unroll
+            for (int l = 0; l < kLoads; ++l) {
+              tmem_ld32(taddr + (unsigned)(c0 + 32 * l), g[l]);
+              tmem_ld32(taddr + (unsigned)(128 + c0 + 32 * l), u[l]);
             }
-            __syncwarp();
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              unsigned g[32], u[32];
-              tmem_ld32(taddr + (unsigned)(c0 + 32 * hh), g);
-              tmem_ld32(taddr + (unsigned)(128 + c0 + 32 * hh), u);
-              tmem_ld_wait();
-              unsigned o[16];
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float y0 = silu(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]);
-                const float y1 = silu(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]);
-                o[j] = pack_bf16(y0, y1);
-              }
-              put_chunks(ph, lane, 4 * hh, o);
-              if (pre) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) o[j] = pack_bf16(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]));
-                put_chunks(ph + kPairPieceBytes, lane, 4 * hh, o);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) o[j] = pack_bf16(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1]));
-                put_chunks(ph + 2 * kPairPieceBytes, lane, 4 * hh, o);
-              }
+            tmem_ld_wait();
+            const int col = nb * 128 + c0;
+            emit(&tmap_o, col, [&](int j) {
+              const unsigned *gj = g[j / 16] + 2 * (j % 16), *uj = u[j / 16] + 2 * (j % 16);
+              return pack_bf16(silu(__uint_as_float(gj[0])) * __uint_as_float(uj[0]),
+                               silu(__uint_as_float(gj[1])) * __uint_as_float(uj[1]));
+            });
+            if (a.pre_gate != nullptr) {
+              emit(&tmap_pg, col, [&](int j) {
+                return pack_bf16(__uint_as_float(g[j / 16][2 * (j % 16)]), __uint_as_float(g[j / 16][2 * (j % 16) + 1]));
+              });
+              emit(&tmap_pu, col, [&](int j) {
+                return pack_bf16(__uint_as_float(u[j / 16][2 * (j % 16)]), __uint_as_float(u[j / 16][2 * (j % 16) + 1]));
+              });
             }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmap_o, ph, nb * 128 + c0, row0);
-              if (pre) {
-                tma_store_2d(&tmap_pg, ph + kPairPieceBytes, nb * 128 + c0, row0);
-                tma_store_2d(&tmap_pu, ph + 2 * kPairPieceBytes, nb * 128 + c0, row0);
-              }
-              bulk_commit();
-            }
-            if (!pre && ++piece == kPairPieces) piece = 0;
           }
         } else {
           const float scale = (a.mode == kScale && a.row_scale != nullptr) ? a.row_scale[row0 + lane] : 1.f;
 #pragma unroll 1
           for (int c0 = 0; c0 < BN; c0 += 64) {
-            unsigned char* ph = pieces + piece * kPairPieceBytes;
             unsigned v[2][32];
             tmem_ld32(taddr + (unsigned)c0, v[0]);
             tmem_ld32(taddr + (unsigned)(c0 + 32), v[1]);
-            if (lane == 0) bulk_wait_read<kPairPieces - 1>();
-            __syncwarp();
             tmem_ld_wait();
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              unsigned o[16];
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                o[j] = pack_bf16(__uint_as_float(v[hh][2 * j]) * scale, __uint_as_float(v[hh][2 * j + 1]) * scale);
-              put_chunks(ph, lane, 4 * hh, o);
-            }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmap_o, ph, nb * BN + c0, row0);
-              bulk_commit();
-            }
-            if (++piece == kPairPieces) piece = 0;
+            for (int e = 0; e < 64 / kCols; ++e)
+              emit(&tmap_o, nb * BN + c0 + kCols * e, [&](int j) {
+                const unsigned* x = v[(j + kCols / 2 * e) / 16] + 2 * (j % 16);
+                return pack_bf16(__uint_as_float(x[0]) * scale, __uint_as_float(x[1]) * scale);
+              });
           }
         }
       }
@@ -562,50 +550,31 @@ extern "C" int moonep_grouped_gemm_pair_kn(const void* x, const void* w0, int K0
   return launch_pair(ta, tb0, tb1, a, num_sms, stream);
 }
 
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const GemmArgs& a,
+template <int kStages, int kCols>
+static int launch_pair_of(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const GemmArgs& a,
                        int num_sms, void* stream) {
   CUtensorMap to, tg, tu;
-  if (int rc = make_tmap(&to, a.out, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32)) return rc;
+  if (int rc = make_tmap(&to, a.out, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32, 0, kCols)) return rc;
   tg = tu = to;
   if (a.pre_gate != nullptr) {
-    if (int rc = make_tmap(&tg, a.pre_gate, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32)) return rc;
-    if (int rc = make_tmap(&tu, a.pre_up, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32)) return rc;
+    if (int rc = make_tmap(&tg, a.pre_gate, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32, 0, kCols)) return rc;
+    if (int rc = make_tmap(&tu, a.pre_up, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32, 0, kCols)) return rc;
   }
-  const size_t smem = (size_t)kPairStages * kPairStageBytes + 1024 + 4 * kPairWarpPieces;
+  constexpr auto* kernel = grouped_gemm_pair_kernel<kStages, kCols>;
+  constexpr size_t smem = kPairSmem<kStages, kCols>;
   static int max_pairs = -1;  // pairs of these CTAs the device runs at once
-  if (max_pairs < 0) {
-    if (int rc = check_cuda(cudaFuncSetAttribute(grouped_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem),
-                            "cudaFuncSetAttribute(grouped_gemm_pair_kernel)"))
-      return rc;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
-    cfg.blockDim = dim3(kPairThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (int rc = check_cuda(cudaOccupancyMaxActiveClusters(&n, grouped_gemm_pair_kernel, &cfg),
-                            "cudaOccupancyMaxActiveClusters(grouped_gemm_pair_kernel)"))
-      return rc;
-    max_pairs = n;
-  }
-  if (max_pairs < 1) {
-    set_error("moonep_grouped_gemm_pair: the device cannot run a pair of these CTAs");
-    return 1;
-  }
+  if (max_pairs < 0)
+    if (int rc = pairs_at_once(kernel, kPairThreads, smem, "grouped_gemm_pair_kernel", &max_pairs)) return rc;
   int pairs = max_pairs;
   if (num_sms > 0) pairs = imax(1, imin(pairs, num_sms / 2));
-  grouped_gemm_pair_kernel<<<2 * pairs, kPairThreads, smem, (cudaStream_t)stream>>>(ta, tb0, tb1, to, tg, tu, a);
+  kernel<<<2 * pairs, kPairThreads, smem, (cudaStream_t)stream>>>(ta, tb0, tb1, to, tg, tu, a);
   return check_launch("grouped_gemm_pair_kernel");
+}
+
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const GemmArgs& a,
+                       int num_sms, void* stream) {
+  return a.k_blocks <= 1024 / BK ? launch_pair_of<5, 64>(ta, tb0, tb1, a, num_sms, stream)
+                                 : launch_pair_of<6, 32>(ta, tb0, tb1, a, num_sms, stream);
 }
 
 // Host-side walk of the tile schedule of one CTA pair (for tests): writes, for every tile that pair `pair` of

@@ -399,40 +399,12 @@ static int launch_wgrad(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs&
   if (rows_per_group <= 0) rows_per_group = a.rows_cap / a.G;
   if (moonep_wgrad_single_cta(rows_per_group, imax(0, num_sms))) return launch_single(tl, tr, a, num_sms, stream);
   a.q_tiles = a.Q / BN;
-  const size_t smem = kSmemBytes;
   static int max_pairs = -1;  // pairs of these CTAs the device runs at once
-  if (max_pairs < 0) {
-    if (int rc = check_cuda(cudaFuncSetAttribute(grouped_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem),
-                            "cudaFuncSetAttribute(grouped_wgrad_kernel)"))
-      return rc;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (int rc = check_cuda(cudaOccupancyMaxActiveClusters(&n, grouped_wgrad_kernel, &cfg),
-                            "cudaOccupancyMaxActiveClusters(grouped_wgrad_kernel)"))
-      return rc;
-    max_pairs = n;
-  }
-  if (max_pairs < 1) {
-    set_error("moonep_grouped_wgrad: the device cannot run a pair of these CTAs");
-    return 1;
-  }
+  if (max_pairs < 0)
+    if (int rc = pairs_at_once(grouped_wgrad_kernel, kThreads, kSmemBytes, "grouped_wgrad_kernel", &max_pairs)) return rc;
   int pairs = max_pairs;
   if (num_sms > 0) pairs = imin(pairs, num_sms / 2);
-  grouped_wgrad_kernel<<<2 * pairs, kThreads, smem, (cudaStream_t)stream>>>(tl, tr, a);
+  grouped_wgrad_kernel<<<2 * pairs, kThreads, kSmemBytes, (cudaStream_t)stream>>>(tl, tr, a);
   return check_launch("grouped_wgrad_kernel");
 }
 

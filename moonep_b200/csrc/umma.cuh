@@ -261,10 +261,10 @@ inline EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// 2-D bf16 row-major [rows, cols] tensor (rows ld elements apart; 0 = cols), box = 64 columns x box_rows rows,
-// 128-byte swizzle.
+// 2-D bf16 row-major [rows, cols] tensor (rows ld elements apart; 0 = cols), box = box_cols (64, or 32) columns x box_rows
+// rows, swizzled over the bytes of a box row.
 inline int make_tmap(CUtensorMap* m, const void* base, unsigned long long rows, unsigned long long cols,
-                     unsigned box_rows, unsigned long long ld = 0) {
+                     unsigned box_rows, unsigned long long ld = 0, unsigned box_cols = BK) {
   EncodeTiledFn fn = encode_tiled();
   if (fn == nullptr) {
     set_error("cuTensorMapEncodeTiled is not available (no CUDA driver?)");
@@ -272,15 +272,44 @@ inline int make_tmap(CUtensorMap* m, const void* base, unsigned long long rows, 
   }
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {(ld ? ld : cols) * 2};
-  cuuint32_t box[2] = {(cuuint32_t)BK, box_rows};
+  cuuint32_t box[2] = {box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed with CUresult " + std::to_string((int)r));
     return (int)r;
   }
+  return 0;
+}
+
+// How many clusters of two CTAs of this kernel the device runs at once (an error when it is none); allows the kernel its
+// dynamic shared memory.
+template <typename Kernel>
+int pairs_at_once(Kernel* kernel, int threads, size_t smem, const char* name, int* pairs) {
+  if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), name)) return rc;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (int rc = check_cuda(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg), name)) return rc;
+  if (n < 1) {
+    set_error(std::string(name) + ": the device cannot run a pair of these CTAs");
+    return 1;
+  }
+  *pairs = n;
   return 0;
 }
 

@@ -92,6 +92,7 @@ def test_reference_on_cpu_matches_dense():
         (2, [128, 256], 256, 512),
         (5, [256, 0, 128, 384, 0], 512, 256),
         (8, [1024, 128, 0, 640, 256, 128, 0, 512], 1024, 768),
+        (3, [128, 384, 256], 1088, 256),  # the pair kernel takes another split of shared memory above K = 1024
         (36, [128 * ((i * 7) % 5) for i in range(36)], 2048, 512),
     ],
 )
@@ -285,6 +286,7 @@ def test_kn_reference_on_cpu():
         ([128], [64], 256),
         ([256, 0, 128], [128, 64], 256),
         ([384, 128, 0, 640], [512], 512),
+        ([128, 640], [704, 384], 256),  # above K = 1024
         ([128 * ((i * 3) % 4) for i in range(12)], [256, 256], 768),
     ],
 )
