@@ -304,8 +304,8 @@ __device__ inline void plan_tokens_block(const MoonepDevCtx& c, const int* __res
     if (part < parts) {
       for (int e = col0; e < E; e += cols) {
         int sum = 0;
-  #pragma unroll 8
-      for (int r = part; r < block; r += parts) sum += c.block_hist[(long long)r * E + e];
+#pragma unroll 8
+        for (int r = part; r < block; r += parts) sum += c.block_hist[(long long)r * E + e];
         if (sum) atomicAdd(s_hist + e, sum);
       }
     }
@@ -317,23 +317,23 @@ __device__ inline void plan_tokens_block(const MoonepDevCtx& c, const int* __res
     s.e[i] = valid ? e : -1;
   }
   __syncthreads();
-  // In-order index of every entry among the entries of its expert: 32 entries at a time, s_hist moves on as a cursor.
-  // (A scan of the entries before each entry made this the longest part of the stage: up to 512 steps per thread
-  // against at most 16 rounds of one match and a barrier.  Two emulated ranks, S=4096, K=8, E=64: 1291 -> 1212 us per
-  // pass of dispatch, prefetch, combine and reduce_grad.)
-  const int lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
-  for (int w = 0; w * 32 < nent; ++w) {
-    if (warp == w % nwarps) {
-      const int i = w * 32 + lane;
+  // In-order index of every entry among the entries of its expert: 32 entries at a time, s_hist moves on as a cursor.  One
+  // warp takes the at most 16 rounds, a match each; with the warps taking turns behind a barrier every round cost more than
+  // it saved where a CTA has one block.  The stage with a scan of the entries before each entry (up to 512 steps per
+  // thread), warps in turn, one warp, us: R=2, S=16384, K=8, E=16 70, 61, 54; S=4096, E=64 19.6, 20.4, 15.9 to 17.9; S=64,
+  // E=256 9.3, 10.1, 9.3.
+  if (tid < 32) {
+    for (int i = tid; i - tid < nent; i += 32) {
       const int e = i < nent ? s.e[i] : -1;
-      const unsigned same = __match_any_sync(0xffffffffu, e >= 0 ? e : -1 - lane);
+      const unsigned same = __match_any_sync(0xffffffffu, e >= 0 ? e : -1 - tid);
       const int before = e >= 0 ? s_hist[e] : 0;
       __syncwarp();
-      if (e >= 0 && lane == __ffs(same) - 1) s_hist[e] = before + __popc(same);
-      if (i < nent) s.lc[i] = before + __popc(same & ((1u << lane) - 1u));
+      if (e >= 0 && tid == __ffs(same) - 1) s_hist[e] = before + __popc(same);
+      if (i < nent) s.lc[i] = before + __popc(same & ((1u << tid) - 1u));
+      __syncwarp();
     }
-    __syncthreads();
   }
+  __syncthreads();
   for (int i = tid; i < nent; i += blockDim.x) {
     const int e = s.e[i];
     int dstv = -1, dest = -1;
