@@ -10,7 +10,8 @@ MOONEP_COPY_PATH      ``bulk`` (default: TMA bulk copies through shared memory) 
 MOONEP_RING_STAGES    2..6 (default 4): 2 KB stages per warp of the prefetch kernel's cp.async ring (read by the native
                       library).
 MOONEP_FUSE_PUBLISH   ``1``: ``plan_publish`` runs as the first step of the dispatch kernel, so a fresh dispatch is one launch
-                      (default 0: measured the same as the separate kernel).
+                      (default 0: measured the same as the separate kernel; no effect with one rank, whose dispatch is one
+                      launch).
 MOONEP_LOCAL_ROWS     ``0``: the send role of dispatch also writes the rows that stay on the rank (default: the
                       destination-side role writes them from the input).
 MOONEP_LOCAL_HOME     ``0``: the push role of combine also moves the rows whose token lives on the rank (default: the fold

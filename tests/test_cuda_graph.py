@@ -14,10 +14,15 @@ def _expected(x, K):
     return (x.float() * K).to(torch.bfloat16)
 
 
-@pytest.mark.parametrize("fuse_publish", ["0", "1"], ids=["publish_kernel", "publish_fused"])
-def test_captured_round_trip_replays_and_mixes_with_eager_calls(fuse_publish, monkeypatch):
-    # with MOONEP_FUSE_PUBLISH=1 the tokens-per-expert exchange is the first step of the dispatch kernel
-    monkeypatch.setenv("MOONEP_FUSE_PUBLISH", fuse_publish)
+@pytest.mark.parametrize("env,launches", [
+    ({}, {"dispatch_single", "combine_single"}),
+    # the general kernels: with MOONEP_FUSE_PUBLISH=1 the tokens-per-expert exchange is the first step of the dispatch kernel
+    ({"MOONEP_LOCAL_ROWS": "0", "MOONEP_FUSE_PUBLISH": "0"}, {"plan_publish", "dispatch_fused", "combine_single"}),
+    ({"MOONEP_LOCAL_ROWS": "0", "MOONEP_FUSE_PUBLISH": "1"}, {"dispatch_fused", "combine_single"}),
+], ids=["single_rank", "publish_kernel", "publish_fused"])  # fmt: skip
+def test_captured_round_trip_replays_and_mixes_with_eager_calls(env, launches, monkeypatch):
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
     S, H, K, E = 256, 512, 4, 8
     buf = Buffer(S, H, K, E, 1, num_sms=8, token_padding=16, explicitly_destroy=True)
     be = buf._require_ctx()["_backend"]
@@ -30,6 +35,10 @@ def test_captured_round_trip_replays_and_mixes_with_eager_calls(fuse_publish, mo
         out, wb, _ = buf.combine(plan, xn, wn, zero_copy=True)
         return out, wb, cu
 
+    be.profile(True)
+    step()
+    assert set(be.phase_times()) == launches
+    be.profile(False)
     graph_step = buf.capture(step)
     epochs_before = list(be.epoch)
     for i in range(3):

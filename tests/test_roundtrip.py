@@ -114,7 +114,8 @@ def test_round_trip_on_the_alternative_copy_paths(case, paths, monkeypatch):
 def test_round_trip_with_local_rows_written_by_either_role(case, R, expand, local_rows, monkeypatch):
     """The rows of a rank's own tokens come from the destination-side role (straight from the input, primary row and
     duplicates from one read; ``MOONEP_LOCAL_ROWS=1``) or from the send role like every other row (``0``); both on
-    the bulk-copy and the register variant of the expansion, with one rank (every row is local) and several.  On the
+    the bulk-copy and the register variant of the expansion.  With one rank every row is local: the single-rank kernel moves
+    them in either way (``1``), or the general kernels do (``0``).  On the
     way back the same rows reach the local staging chunk through the fold role (``MOONEP_LOCAL_HOME=1``) or the push
     role."""
     if not case.supports(R):

@@ -1,12 +1,14 @@
 """Dispatch and combine kernels of a single rank (csrc/single_rank.cu) at the edges of their tiling, against the host
-planner and the two-rounding model: pieces of rows, tokens per CTA, steps of 512 entries, lists of 1024 groups, rows and
-routing that are not 16-byte aligned, replayed plans, token counts that do not match the routing."""
+planner and the two-rounding model: pieces of rows, tokens per CTA, steps of 384 entries, 512 groups scanned at a time, rows
+and routing that are not 16-byte aligned, tokens handed out between CTAs, replayed plans, token counts that do not match the
+routing, sizes that take the general kernels."""
 
 import pytest
 import torch
 
 from moonep_b200 import Buffer
-from moonep_b200.errors import MoonEPIndexError
+from moonep_b200.constants import FLAG_SENT
+from moonep_b200.errors import MoonEPIndexError, MoonEPTimeoutError
 from tests.harness import Case, assert_within_ulp, check_dispatch_records, expected_combine, run_round_trip
 
 pytestmark = pytest.mark.gpu
@@ -15,10 +17,13 @@ CASES = [
     Case("one_token_many_pads", S=1, K=1, epn=3, H=8, token_padding=128, routing="single_expert"),
     Case("fewer_tokens_than_ctas", S=147, K=3, epn=5, H=264, token_padding=16, routing="biased"),
     Case("one_cta_with_one_token", S=149, K=2, epn=8, H=4104, token_padding=1, routing="softmax"),
-    Case("three_pieces_per_row", S=40, K=4, epn=6, H=8200, token_padding=32, routing="zipf"),
+    Case("two_pieces_per_row", S=40, K=4, epn=6, H=8200, token_padding=32, routing="zipf"),
+    Case("three_pieces_per_row", S=40, K=4, epn=6, H=16392, token_padding=32, routing="zipf"),
     Case("several_steps_per_cta", S=12000, K=8, epn=16, H=64, token_padding=64, routing="zipf"),
-    Case("step_of_16_tokens", S=300, K=32, epn=40, H=32, token_padding=8, routing="softmax"),
-    Case("two_lists_of_groups", S=700, K=2, epn=1100, H=16, token_padding=4, routing="softmax", B=1),
+    Case("twelve_tokens_per_step", S=300, K=32, epn=40, H=32, token_padding=8, routing="softmax"),
+    Case("one_entry_past_a_step", S=149 * 129, K=3, epn=8, H=16, token_padding=4, routing="softmax"),  # 130 tokens per CTA
+    Case("one_scan_of_groups", S=700, K=2, epn=512, H=16, token_padding=4, routing="softmax", B=1),
+    Case("three_scans_of_groups", S=700, K=2, epn=1100, H=16, token_padding=4, routing="softmax", B=1),
     Case("rows_of_40_bytes", S=333, K=5, epn=7, H=20, token_padding=16, routing="biased"),
     Case("odd_rows", S=50, K=2, epn=4, H=13, token_padding=4, routing="softmax"),
 ]
@@ -76,6 +81,119 @@ def test_replay_and_unaligned_inputs(S, H, K, E, pad, shift):
     for k in range(K):  # the kernel's order: fp32, ascending k, rounded once
         want += y[loff.view(S, K)[:, k]].float()
     assert torch.equal(out, want.to(torch.bfloat16)) and torch.equal(back, gates)
+    buf.synchronize()
+    buf.destroy()
+
+
+@pytest.mark.parametrize("ctas", ["1", "2", "3", None])
+@pytest.mark.parametrize("var", ["MOONEP_NUM_SMS_DEDUP", "MOONEP_LOCAL_SMS"])
+@pytest.mark.parametrize("S,H,K,E,pad,shift,hot", [
+    (2000, 2056, 2, 9, 4, 0, True),   # more units of a copy warp than it remembers, and tokens to hand out on every grid
+    (250, 16392, 3, 8, 8, 0, False),  # the same with rows of three pieces
+    (100, 2056, 2, 100, 128, 0, False),  # more grabs of pad rows than a warp remembers
+    (1500, 1032, 2, 9, 16, 1, True),  # without bulk copies
+])  # fmt: skip
+def test_tokens_and_pads_handed_out_between_ctas(S, H, K, E, pad, shift, hot, var, ctas, monkeypatch):
+    """Fresh, staged and replayed dispatches in a row on one Buffer: every row, pad row and row flag, on grids of one to
+    three CTAs and of every SM."""
+    if ctas is None and var == "MOONEP_LOCAL_SMS":
+        pytest.skip("the same as the other switch unset")
+    if ctas is not None:
+        monkeypatch.setenv(var, ctas)
+    buf = Buffer(S, H, K, E, 1, token_padding=pad)
+    ctx = buf._require_ctx()
+    be = ctx["_backend"]
+    g = torch.Generator(device="cuda").manual_seed(S)
+    flags = ctx["meta_buf"][ctx["ROWFLAG_OFF"] :][: ctx["NvS"]]
+    plan = None
+    for turn in range(6):
+        fresh, staged = turn % 3 != 2, turn % 3 == 1
+        if fresh:
+            lg = torch.rand(S, E, generator=g, device="cuda") * (torch.arange(E, device="cuda") < 4 + turn if hot else 1)
+            topk = lg.topk(K, dim=1).indices.to(torch.int32)
+            tpe = torch.bincount(topk.flatten().long(), minlength=E).to(torch.int32)
+        x = torch.empty(S * H + shift, dtype=torch.bfloat16, device="cuda")[shift:].view(S, H)
+        x.copy_(torch.randn(S, H, generator=g, device="cuda"))
+        gates = torch.rand(S, K, generator=g, device="cuda")
+        ctx["hidden_buf_local"].fill_(7.0)
+        if fresh:
+            rows, w, cu, plan = buf.dispatch(x, gates, topk, tpe, zero_copy=not staged)
+        else:
+            rows, w, _, _ = buf.dispatch(x, gates, plan=plan, zero_copy=True)
+        end = int(cu[-1])
+        loff = torch.where(plan.dst < 0, -plan.dst - 1, plan.dst).long()
+        assert torch.equal(rows[loff], x.repeat_interleave(K, 0)) and torch.equal(w[loff], gates.flatten())
+        assert int(torch.unique(loff).numel()) == S * K and torch.equal(plan.src_info[loff].long(), torch.arange(S * K, device="cuda"))
+        pads = torch.ones(end, dtype=torch.bool, device="cuda")
+        pads[loff] = False
+        assert not bool(rows[:end][pads].any()) and not bool(w[:end][pads].any()) and bool((rows[end:] == 7.0).all())
+        assert bool((flags[:end] == be.epoch[FLAG_SENT]).all())
+        out, back, _ = buf.combine(plan, rows, w)
+        want = torch.zeros(S, H, device="cuda")
+        for _ in range(K):
+            want += x.float()
+        assert torch.equal(out, want.to(torch.bfloat16)) and torch.equal(back, gates)
+        buf.synchronize()
+    buf.destroy()
+
+
+@pytest.mark.parametrize("S,K,E,single", [(32768, 8, 16, True), (32769, 8, 16, False), (64, 1, 4096, True), (64, 1, 4097, False)])
+def test_on_each_side_of_the_single_rank_limits(S, K, E, single):
+    """262144 routing entries and 4096 experts are the most the single-rank dispatch takes; beyond, the general kernels
+    make the same plan, which the single-rank combine reads."""
+    H = 8
+    buf = Buffer(S, H, K, E, 1, token_padding=2, B=1)
+    be = buf._require_ctx()["_backend"]
+    x, topk, tpe = _inputs(S, H, K, E, 0)
+    gates = torch.rand(S, K, device="cuda")
+    be.profile(True)
+    rows, w, cu, plan = buf.dispatch(x, gates, topk, tpe)
+    loff = torch.where(plan.dst < 0, -plan.dst - 1, plan.dst).long()
+    rows2, w2, _, _ = buf.dispatch(-x, gates, plan=plan, zero_copy=True)
+    out, back, _ = buf.combine(plan, rows2, w2, zero_copy=True)
+    tags = set(be.phase_times())
+    assert ("dispatch_single" in tags) == single and ("dispatch_fused" in tags) != single and "combine_single" in tags
+    # rows of an expert in the order of the routing entries
+    flat = topk.flatten().long()
+    padded = (tpe.long() + 1) // 2 * 2
+    first = padded.cumsum(0) - padded
+    order = torch.sort(flat, stable=True).indices
+    want = torch.empty(S * K, dtype=torch.long, device="cuda")
+    want[order] = torch.arange(S * K, device="cuda") - (tpe.long().cumsum(0) - tpe)[flat[order]] + first[flat[order]]
+    assert torch.equal(loff, want) and int(cu[-1]) == int(padded.sum())
+    assert torch.equal(rows[loff], x.repeat_interleave(K, 0)) and torch.equal(w[loff], gates.flatten())
+    assert torch.equal(rows2[loff], -x.repeat_interleave(K, 0))
+    acc = torch.zeros(S, H, device="cuda")
+    for _ in range(K):
+        acc -= x.float()
+    assert torch.equal(out, acc.to(torch.bfloat16)) and torch.equal(back, gates)
+    buf.synchronize()
+    buf.destroy()
+
+
+@pytest.mark.parametrize("K", [1, 3, 6])
+def test_combine_takes_rows_as_their_blocks_are_finished(K):
+    """``combine(ready=...)`` on one rank: behind a product that counts its row blocks, and behind one that never finishes
+    the last count, which is a timeout after which the Buffer works again."""
+    from moonep_b200.ops.grouped_gemm import grouped_gemm
+
+    S, H, E = 300, 256, 8
+    buf = Buffer(S, H, K, E, 1, token_padding=128, B=1)
+    be = buf._require_ctx()["_backend"]
+    x, topk, tpe = _inputs(S, H, K, E, 0)
+    rows, _, cu, plan = buf.dispatch(x, None, topk, tpe, zero_copy=True)
+    w = (torch.randn(E + 1, H, H, device="cuda") * 0.05).to(torch.bfloat16)
+    done = torch.zeros(rows.shape[0] // 128 + 1, dtype=torch.int32, device="cuda")
+    y = grouped_gemm(rows, w, cu, hooks=buf.gemm_hooks(done_counter=done))
+    out, _, _ = buf.combine(plan, y, None, ready=(done, 4 * (H // 256)))
+    buf.synchronize()
+    want, _, _ = buf.combine(plan, y, None)
+    assert torch.equal(out, want) and bool((done[: int(cu[-1]) // 128] == 4).all())
+    be.set_timeout_ms(100)
+    buf.combine(plan, y, None, ready=(done, 4 * (H // 256) + 1))
+    with pytest.raises(MoonEPTimeoutError):
+        buf.synchronize()
+    assert torch.equal(buf.combine(plan, y, None)[0], want)
     buf.synchronize()
     buf.destroy()
 
