@@ -150,15 +150,16 @@ def backward_overlap() -> bool:
     return os.environ.get("MOONEP_BWD_OVERLAP", "0") not in _FALSE
 
 
+def gemm_pair_switch() -> bool | None:
+    """MOONEP_GEMM_PAIR where it is set, None where it is not."""
+    raw = os.environ.get("MOONEP_GEMM_PAIR")
+    return None if raw is None else raw not in _FALSE
+
+
 def gemm_on_cta_pairs() -> bool:
     """The grouped GEMM runs on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles; measured 9-10 % faster);
     MOONEP_GEMM_PAIR=0 selects the kernel with one CTA per 128 x 256 tile."""
-    return os.environ.get("MOONEP_GEMM_PAIR", "1") not in _FALSE
-
-
-def gemm_pair_is_set() -> bool:
-    """True when the environment names the grouped GEMM kernel explicitly."""
-    return bool(os.environ.get("MOONEP_GEMM_PAIR"))
+    return gemm_pair_switch() is not False
 
 
 def wgrad_layout() -> str:

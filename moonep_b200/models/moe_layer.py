@@ -127,7 +127,8 @@ class ExpertParallelMoE:
 
     # -- forward -------------------------------------------------------------------------------
     def forward_gemm_pair(self):
-        """``pair`` of the forward GEMMs: None for the default, False for one CTA per tile.
+        """``pair`` of the forward GEMMs on the kernels: True for CTA pairs, False for one CTA per tile; None where
+        ``MOONEP_GEMM_PAIR=0`` asks for the forward pass without hand-offs.
 
         Up to 128 rows per expert most groups are one row block, which leaves the second CTA of a pair without work: one
         CTA per tile takes 0.92 of the pairs' time on average over 420 combinations of 4 to 64 experts, 8 to 128 rows per
@@ -135,11 +136,13 @@ class ExpertParallelMoE:
         1.12, 8 experts of 100 rows with Zipf routing, whose hot experts have several blocks).  From two blocks on the pairs
         win or are equal where the count is even (8 experts of 512 rows, H=7168: 229 us against 240).  The counts are not
         known on the host, so their mean decides.  With several ranks the hand-off hooks need the pairs, and
-        MOONEP_GEMM_PAIR, where it is set, is what it says."""
-        short = self.R == 1 and self.S * self.K <= 128 * self.E
-        return False if short and not config.gemm_pair_is_set() else None
+        ``MOONEP_GEMM_PAIR=1``, where it is set, means pairs."""
+        switch = config.gemm_pair_switch()
+        if switch is None:
+            return self.R > 1 or self.S * self.K > 128 * self.E
+        return True if switch else None
 
-    def _forward_fast(self, x, gates, topk, tokens_per_expert, save_for_backward):
+    def _forward_fast(self, x, gates, topk, tokens_per_expert, save_for_backward, pair):
         """CUDA: dispatch -> prefetch (on the communication stream, beside the GEMMs) -> SwiGLU GEMM -> down projection
         into a separate tensor -> push combine that reads it in place.  The GEMMs take their hand-off from the
         communication kernels tile by tile: row flags of the dispatch, per-slot flags of the prefetch (so only the
@@ -163,7 +166,6 @@ class ExpertParallelMoE:
         hooked = not alone and rows >= 128 and self.H % 256 == 0 and self.I % 128 == 0
         if fetched is not None and not hooked:
             torch.cuda.current_stream().wait_event(fetched)
-        pair = self.forward_gemm_pair()
         h = grouped_gemm(x_nvs, self.w_gate, cu, w_up=self.w_up, mode="swiglu", status=status, pair=pair,
                          save_pre=None if a is None else (a, u),
                          hooks=buf.gemm_hooks(rows=True, slots=True) if hooked else None)  # fmt: skip
@@ -184,8 +186,10 @@ class ExpertParallelMoE:
         """Returns ``(out[S, H], saved)``.  ``save_for_backward=False`` (inference): nothing is kept, the expert
         GEMMs read the dispatched rows in place, ``saved`` is None."""
         buf = self.buffer
-        if self.fast and (self.bwd_buffer is not None or not save_for_backward) and config.gemm_on_cta_pairs():
-            return self._forward_fast(x, gates, topk, tokens_per_expert, save_for_backward)
+        if self.fast and (self.bwd_buffer is not None or not save_for_backward):
+            pair = self.forward_gemm_pair()
+            if pair is not None:
+                return self._forward_fast(x, gates, topk, tokens_per_expert, save_for_backward, pair)
         x_nvs, w_nvs, cu, plan = buf.dispatch(x, gates, topk, tokens_per_expert, zero_copy=True)
         # the weight copies run on the communication stream while this stream saves the dispatched rows
         fetched = None if self.R == 1 else buf.prefetch_weight(plan, async_finish=True, full_gate_weight=self.w_gate,

@@ -96,8 +96,10 @@ def test_forward_gemm_kernel_follows_the_switch_where_it_is_set(monkeypatch):
         return lw.run(body)[0]
 
     monkeypatch.delenv("MOONEP_GEMM_PAIR", raising=False)
-    assert chosen(1, 256) is False and chosen(1, 257) is None and chosen(2, 8) is None
+    assert chosen(1, 256) is False and chosen(1, 257) is True and chosen(2, 8) is True
     monkeypatch.setenv("MOONEP_GEMM_PAIR", "1")
+    assert chosen(1, 256) is True
+    monkeypatch.setenv("MOONEP_GEMM_PAIR", "0")
     assert chosen(1, 256) is None
 
 
