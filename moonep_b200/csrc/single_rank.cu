@@ -1007,9 +1007,12 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
   }
   a.pads_per_grab = imax(1, imin(32, (int)(28672 / row_bytes)));
   const size_t smem = (size_t)a.copy_warps * kRing * a.stage_bytes + (a.bulk_pads ? kZeroBytes : 0) + tables;
-  if (int rc = check_cuda(cudaFuncSetAttribute(dispatch_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit),
-                          "cudaFuncSetAttribute(dispatch_single_kernel)"))
-    return rc;
+  if (!h->single_smem_set) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(dispatch_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit),
+                            "cudaFuncSetAttribute(dispatch_single_kernel)"))
+      return rc;
+    h->single_smem_set = 1;
+  }
   int grid = imax(1, imin(imin(c.local_sms, h->sm_count), kMaxCtas));
   if (n_ctas > 0) grid = imin(grid, n_ctas);
   a.tokens_per_cta = (c.S + grid - 1) / grid;
