@@ -42,8 +42,9 @@ constexpr int kEntries = kPlanWarps * 32;  // routing entries planned at a time 
 constexpr int kUnits = 64;         // units remembered per copy warp: those loaded and those not flagged yet
 constexpr int kGrabs = 64;         // grabs of pad rows remembered per warp
 constexpr int kMaxGroups = 4096;   // experts, and prefetch slots: up to four words of shared memory each
-// Every CTA reads the routing before its own tokens: at 32 K entries that is 3 us for the last CTA, at 256 K about
-// 25 us, where the general kernel's per-block histograms are the better way.
+// Every CTA reads the routing before its own tokens, beside the copies of the CTAs that are ahead.  The line is how far the
+// kernel is tested, not where the general kernels catch up: S=32768, K=8, H=1024 (at the line) takes 165 us here and 363
+// there, and with the line out of the way S=65536 takes 302 and 725, S=262144, H=64 498 and 2816.
 constexpr int kMaxEntries = 1 << 18;
 // work[]: pad rows handed out, then per CTA the tokens handed out, then per CTA the epoch at which its tokens were planned
 constexpr int kMaxCtas = 256;

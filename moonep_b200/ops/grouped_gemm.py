@@ -73,6 +73,7 @@ def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", o
     ``group_map`` (int32 ``[G]``) group ``g`` uses ``w[group_map[g]]`` and ``w`` may hold fewer experts
     than there are groups (e.g. only the experts a rank owns or has prefetched).  ``save_pre=(a, u)`` (SwiGLU
     only, two ``[rows, N]`` bf16 tensors) also stores the pre-activations ``x @ w.T`` and ``x @ w_up.T``.
+    ``num_sms`` bounds the SMs (0: all; a CTA pair takes two, also where the bound is one).
     ``pair`` selects the kernel: True = CTA pairs (``cta_group::2``), False = one CTA per tile, None = ``MOONEP_GEMM_PAIR``.
     ``hooks`` (a ``GemmHooks``, CTA-pair kernel only) lets the kernel run beside the communication kernels: it waits
     per row block / weight slot for their flags and counts finished output tiles per row block.
