@@ -923,11 +923,11 @@ extern "C" long long moonep_stage_layout(int S, int K, int H, int kp, long long*
   return rows + flags + w;
 }
 
-// roles: MOONEP_ROLE_FOLD | MOONEP_ROLE_PUSH | MOONEP_ROLE_SUM.  src_info / link: the plan's copies ([NvS] each); dup_groups / dup_loffs / dup_counts: the plan's
-// duplicate map.  in_rows: the local expert output rows [NvS, H] (the shard or any other local tensor), in_w: their gate
-// weights [NvS] or null.  fold_buf [fold_rows, H] bf16 and fold_flag [fold_rows] int32 (zero-initialised once) are
-// local scratch of the Buffer; fold_rows bounds the number of duplicate groups.  ready / ready_expect: optional
-// per-128-row-block counters bumped by the producer of in_rows (see moonep_grouped_gemm_pair).
+// roles: MOONEP_ROLE_FOLD | MOONEP_ROLE_PUSH | MOONEP_ROLE_SUM.  src_info / link: the plan's copies ([NvS] each);
+// dup_groups / dup_loffs / dup_counts: the plan's duplicate map.  in_rows: the local expert output rows [NvS, H] (the shard
+// or any other local tensor), in_w: their gate weights [NvS] or null.  fold_buf [fold_rows, H] bf16 and fold_flag [fold_rows]
+// int32 (zero-initialised once) are local scratch of the Buffer; fold_rows bounds the number of duplicate groups.  ready /
+// ready_expect: optional per-128-row-block counters bumped by the producer of in_rows (see moonep_grouped_gemm_pair).
 extern "C" int moonep_combine_push(void* ctx, int roles, const int* src_info, const int* link, const int* dst,
                                    const void* in_rows, const float* in_w, void* out_hidden, float* out_weights,
                                    int wait_family, int wait_epoch, int epoch_comb, const int* ready, int ready_expect,
