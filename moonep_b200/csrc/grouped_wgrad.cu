@@ -380,7 +380,8 @@ static int launch_single(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs
     sms = n;
   }
   a.q_tiles = a.Q / 128;
-  grouped_wgrad_single_kernel<<<num_sms > 0 ? imin(num_sms, sms) : sms, kThreads, kSmemBytes, (cudaStream_t)stream>>>(tl, tr, a);
+  const int grid = num_sms > 0 ? imin(num_sms, sms) : sms;
+  grouped_wgrad_single_kernel<<<grid, kThreads, kSmemBytes, (cudaStream_t)stream>>>(tl, tr, a);
   return check_launch("grouped_wgrad_single_kernel");
 }
 

@@ -220,7 +220,8 @@ int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk, const int*
 // Dispatch of a Buffer with one rank: one launch, fresh (planner arguments as above, tpe [E]) or replayed (dst and
 // zero_fill come from the plan).  n_ctas bounds the grid (<= 0: every SM of local_sms).  Fresh plans need
 // moonep_single_supported(E, B, S, K); work is local scratch of moonep_single_work_words() zeros.
-// out / out_w (optional, fresh plans): [NvS, H] and [NvS], receive the shard and its weights as they are afterwards.  See single_rank.cu.
+// out / out_w (optional, fresh plans): [NvS, H] and [NvS], receive the shard and its weights as they are afterwards.  See
+// single_rank.cu.
 int moonep_single_supported(int E, int B, int S, int K);
 int moonep_single_work_words(void);
 int moonep_dispatch_single(void* ctx, int fresh, const int* topk, const int* tpe, int* dst, int* cu_seqlens,

@@ -13,8 +13,8 @@
 //              one bulk load and K bulk stores per row.  A CTA that is done with its tokens takes rows over from CTAs that
 //              have planned theirs: SMs reach HBM at rates that differ by a quarter, and with a fixed share per SM the
 //              kernel took 138 (426) us at S=4096 (16384) where its average CTA was done after 117 (363); now 131 (400).
-//   combine    a warp per 512-byte piece of an output row (several at once where a token has few rows), straight from the token's K destinations: no work counter,
-//              no lists.
+//   combine    a warp per 512-byte piece of an output row (several at once where a token has few rows), straight from the
+//              token's K destinations: no work counter, no lists.
 //
 // Both are bound by HBM traffic: the rows are written (read) once, the tokens read (written) once.
 //
@@ -900,7 +900,8 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(cons
           }
       }
       if (i < nvec) st16(reinterpret_cast<int4*>(a.out + (long long)my_tok * H) + i, __popc(rows) == 1 ? only : pack8(acc));
-    } else {  // element by element, eight loads of a row in flight (a warp per row, one load at a time: S=4096, H=2044, K=4 113 -> 39 us)
+    } else {
+      // element by element, eight loads of a row in flight (a warp per row, one load at a time: S=4096, H=2044, K=4 113 -> 39 us)
       const int e0 = my_piece * 256 + lane;
       float acc[8];
       uint16_t only[8];
