@@ -168,6 +168,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   } else {
     // ---------------- epilogue (warps 2..5) ----------------
     const int q = warp & 3;  // TMEM lane quarter this warp may read
+    if (blockIdx.x == 0)  // while the first accumulator is being filled
+      for (int g = threadIdx.x - 64; g < a.G; g += kGemmThreads - 64) gemm_check_end(a.status, 13, g, a.cu_seqlens[g]);
     unsigned tphase[2] = {0, 0};
     int it = 0;
     for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {

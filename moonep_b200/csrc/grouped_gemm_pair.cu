@@ -161,8 +161,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     }
   }
   __syncthreads();
-  if (a.G <= kPairGroupsInSmem)
-    for (int g = threadIdx.x; g < a.G; g += blockDim.x) s_cu[g] = a.cu_seqlens[g];
+  if (a.G <= kPairGroupsInSmem || blockIdx.x == 0)
+    for (int g = threadIdx.x; g < a.G; g += blockDim.x) {
+      const int end = a.cu_seqlens[g];
+      if (a.G <= kPairGroupsInSmem) s_cu[g] = end;
+      if (blockIdx.x == 0 && s_hook_ok) gemm_check_end(a.status, kPairKernelId, g, end);
+    }
   const long long pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {

@@ -38,6 +38,11 @@ __device__ __forceinline__ void gemm_bad_index(int* status, int kernel, int kind
   }
 }
 
+// The kernels tile whole blocks of BM rows: a group that ends inside one would be computed in part, an index error.
+__device__ __forceinline__ void gemm_check_end(int* status, int kernel, int g, int end) {
+  if (end % BM != 0) gemm_bad_index(status, kernel, 14, g, end);
+}
+
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* tmap, int c0, int c1,
                                             unsigned long long* bar) {
   asm volatile(

@@ -197,16 +197,17 @@ class ExpertParallelMoE:
         x_saved = x_nvs.clone() if save_for_backward else x_nvs  # training: the shard is reused for the expert output
         if hasattr(fetched, "wait") and x_nvs.is_cuda:
             torch.cuda.current_stream().wait_event(fetched)
+        status = buf._require_ctx()["_backend"].status if x_nvs.is_cuda else None
         if not save_for_backward:
-            h = grouped_gemm(x_nvs, self.w_gate, cu, w_up=self.w_up, mode="swiglu")
-            grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=x_nvs)
+            h = grouped_gemm(x_nvs, self.w_gate, cu, w_up=self.w_up, mode="swiglu", status=status)
+            grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=x_nvs, status=status)
             out, _, _ = buf.combine(plan, x_nvs, None, zero_copy=True)
             return out, None
         # the pre-activations are kept for the backward pass (two bf16 [NvS, I] tensors instead of two more GEMMs)
         a = torch.empty(x_saved.shape[0], self.I, dtype=torch.bfloat16, device=x_saved.device)
         u = torch.empty_like(a)
-        h = grouped_gemm(x_saved, self.w_gate, cu, w_up=self.w_up, mode="swiglu", save_pre=(a, u))
-        grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=x_nvs)
+        h = grouped_gemm(x_saved, self.w_gate, cu, w_up=self.w_up, mode="swiglu", save_pre=(a, u), status=status)
+        grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=x_nvs, status=status)
         out, _, _ = buf.combine(plan, x_nvs, None, zero_copy=True)
         saved = {"plan": plan, "cu": cu, "x_nvs": x_saved, "w_nvs": w_nvs.clone(), "h": h, "a": a, "u": u}
         return out, saved

@@ -69,7 +69,8 @@ def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", o
                  group_map=None, save_pre=None, pair=None, hooks=None):
     """See module docstring.  ``x``: ``[rows, K]`` bf16, ``w``: ``[G, N, K]`` bf16, returns ``[rows, N]`` bf16.
 
-    Rows beyond ``cu_seqlens[-1]`` are not written.  Group ends must be multiples of 128.  With
+    Rows beyond ``cu_seqlens[-1]`` are not written.  Group ends must be multiples of 128 (the kernels record an index
+    error in ``status`` where one is not).  With
     ``group_map`` (int32 ``[G]``) group ``g`` uses ``w[group_map[g]]`` and ``w`` may hold fewer experts
     than there are groups (e.g. only the experts a rank owns or has prefetched).  ``save_pre=(a, u)`` (SwiGLU
     only, two ``[rows, N]`` bf16 tensors) also stores the pre-activations ``x @ w.T`` and ``x @ w_up.T``.

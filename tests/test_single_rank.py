@@ -283,3 +283,34 @@ def test_phases_of_the_dispatch_are_reported():
         phases = buf.stats()["kernel_phase_max_us"]
         assert set(phases) == names
     buf.destroy()
+
+
+@pytest.mark.parametrize("S", [64, 400])
+@pytest.mark.parametrize("switch", [None, "0", "1"])
+def test_layer_reports_groups_that_are_not_whole_row_blocks(S, switch, monkeypatch):
+    """The expert GEMMs take whole blocks of 128 rows.  A smaller padding works where the counts happen to fill them and is
+    an index error otherwise, on one CTA per tile, on pairs and without hand-offs."""
+    from moonep_b200.models.moe_layer import ExpertParallelMoE, dense_reference
+
+    if switch is not None:
+        monkeypatch.setenv("MOONEP_GEMM_PAIR", switch)
+    H, E, inter = 256, 2, 256
+    for K, rows, ok in ((1, 128, True), (2, S, False)):
+        n = E * rows if ok else S
+        buf = Buffer(n, H, K, E, 1, token_padding=16 if not ok else 64)
+        layer = ExpertParallelMoE(buf, inter, init_std=0.05, seed=4)
+        topk = ((torch.arange(n, device="cuda")[:, None] + torch.arange(K, device="cuda")) % E).to(torch.int32)
+        tpe = torch.bincount(topk.flatten().long(), minlength=E).to(torch.int32)
+        x = torch.randn(n, H, generator=torch.Generator(device="cuda").manual_seed(S), device="cuda").to(torch.bfloat16)
+        gates = torch.ones(n, K, device="cuda")
+        out, _ = layer.forward(x, gates, topk, tpe, save_for_backward=False)
+        if ok:
+            layer.check()
+            ref = dense_reference(x.float().cpu(), gates.cpu(), topk.cpu(), *(w[:E].float().cpu() for w in (layer.w_gate, layer.w_up, layer.w_down)))
+            # bf16 roundings of h, of every row and of the sum, each 2^-9 of values no larger than twice the largest result
+            assert float((out.float().cpu() - ref).abs().max()) <= 8 * 2.0**-9 * float(ref.abs().max())
+        else:
+            with pytest.raises(MoonEPIndexError):
+                layer.check()
+        layer.destroy()
+        buf.destroy()
