@@ -220,11 +220,12 @@ int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk, const int*
 // Dispatch of a Buffer with one rank: one launch, fresh (planner arguments as above, tpe [E]) or replayed (dst and
 // zero_fill come from the plan).  n_ctas bounds the grid (<= 0: every SM of local_sms).  Fresh plans need
 // moonep_single_supported(E, B, S, K); work is local scratch of moonep_single_work_words() zeros.
+// exact (fresh plans): token counts above what was routed are an index error; otherwise they leave rows unused.
 // out / out_w (optional, fresh plans): [NvS, H] and [NvS], receive the shard and its weights as they are afterwards.  See
 // single_rank.cu.
 int moonep_single_supported(int E, int B, int S, int K);
 int moonep_single_work_words(void);
-int moonep_dispatch_single(void* ctx, int fresh, const int* topk, const int* tpe, int* dst, int* cu_seqlens,
+int moonep_dispatch_single(void* ctx, int fresh, int exact, const int* topk, const int* tpe, int* dst, int* cu_seqlens,
                            int* experts_to_copy, int* zero_fill, int* remote_stats, int* dup_groups, int* dup_loffs,
                            int* dup_counts, int* plan_src_info, int* plan_link, const void* hidden, const float* weights,
                            int with_weights, int epoch_tpe, int epoch_plan, int epoch_sent, int n_ctas, int* work,

@@ -73,6 +73,7 @@ struct SingleArgs {
   const float* weights;    // [S, K] or null
   int with_weights;        // pad rows' weight slots are cleared
   int fresh;
+  int exact;     // fresh: counts that do not add up to the routing entries are an index error, not rows left unused
   int topk_vec;  // topk can be read 16 bytes at a time
   int vec_ok;    // rows of the shard and the copy are whole 16-byte words at 16-byte addresses
   int bulk_pads; // pads are cleared in bulk stores
@@ -660,6 +661,8 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
           a.dup_counts[tid] = K > 1 ? (tid == 0 ? c.S : c.S * (K - 1)) : 0;
         }
         if (tid == 0 && carry > NvS) record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TABLES, 1, carry, NvS, 0);
+        if (tid == 0 && a.exact && carry - pads != c.S * K)
+          record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TABLES, 5, carry - pads, c.S * K, 0);
         __syncthreads();
         if (tid == 0) {
           __threadfence();
@@ -943,7 +946,7 @@ extern "C" int moonep_single_supported(int E, int B, int S, int K) {
 
 extern "C" int moonep_single_work_words(void) { return kWorkReady + kMaxCtas; }
 
-extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, const int* tpe, int* dst, int* cu_seqlens,
+extern "C" int moonep_dispatch_single(void* ctx, int fresh, int exact, const int* topk, const int* tpe, int* dst, int* cu_seqlens,
                                       int* experts_to_copy, int* zero_fill, int* remote_stats, int* dup_groups,
                                       int* dup_loffs, int* dup_counts, int* plan_src_info, int* plan_link,
                                       const void* hidden, const float* weights, int with_weights, int epoch_tpe,
@@ -975,6 +978,7 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, const int* topk, con
   a.weights = weights;
   a.with_weights = with_weights;
   a.fresh = fresh;
+  a.exact = exact;
   a.topk_vec = aligned16(topk) ? 1 : 0;
   a.vec_ok = (c.H % 8 == 0 && aligned16(a.out)) ? 1 : 0;
   // MOONEP_EXPAND_PATH=ldst selects register copies as it does with several ranks (S=4096, H=7168, K=8, E=32: 126 us

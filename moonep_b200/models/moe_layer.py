@@ -149,34 +149,41 @@ class ExpertParallelMoE:
         groups that use a prefetched expert wait for it), and a per-row-block counter of finished output tiles that the
         combine's push role consumes.  Nothing is copied and nothing synchronises with the host."""
         buf = self.buffer
-        x_nvs, w_nvs, cu, plan = buf.dispatch(x, gates, topk, tokens_per_expert, zero_copy=True)
         alone = self.R == 1  # no expert is remote, and every kernel of the step follows the one before on this stream
+        be = buf._require_ctx()["_backend"]
+        be.exact_counts = alone
+        try:
+            x_nvs, w_nvs, cu, plan = buf.dispatch(x, gates, topk, tokens_per_expert, zero_copy=True)
+        finally:
+            be.exact_counts = False
         fetched = None if alone else buf.prefetch_weight(plan, async_finish=True, full_gate_weight=self.w_gate,
                                                          full_up_weight=self.w_up, full_down_weight=self.w_down)  # fmt: skip
         rows, dev = int(x_nvs.shape[0]), x_nvs.device
         if self._y is None:
             self._y = torch.empty(rows, self.H, dtype=torch.bfloat16, device=dev)
             self._done = torch.zeros(-(-rows // 128), dtype=torch.int32, device=dev)
-        status = buf._require_ctx()["_backend"].status
+        status = be.status
         a = u = None
         if save_for_backward:
             a = torch.empty(rows, self.I, dtype=torch.bfloat16, device=dev)
             u = torch.empty_like(a)
-        # the hand-off hooks need the CTA-pair kernel's tiling; other shapes run after the prefetch, in stream order
-        hooked = not alone and rows >= 128 and self.H % 256 == 0 and self.I % 128 == 0
+        # The hand-off hooks need the CTA-pair kernel's tiling; other shapes run after the prefetch, in stream order.  Alone
+        # there is nothing to wait for, as long as the dispatch has seen that every row of a group is one that lands.
+        hooked = not (alone and be.counts_checked) and rows >= 128 and self.H % 256 == 0 and self.I % 128 == 0
+        pair = pair or hooked
         if fetched is not None and not hooked:
             torch.cuda.current_stream().wait_event(fetched)
         h = grouped_gemm(x_nvs, self.w_gate, cu, w_up=self.w_up, mode="swiglu", status=status, pair=pair,
                          save_pre=None if a is None else (a, u),
-                         hooks=buf.gemm_hooks(rows=True, slots=True) if hooked else None)  # fmt: skip
+                         hooks=buf.gemm_hooks(rows=True, slots=not alone) if hooked else None)  # fmt: skip
         ready = None
         if hooked:
             self._down_calls += 1
             ready = (self._done, self._down_calls * 4 * (self.H // 256))
         grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=self._y, status=status, pair=pair,
-                     hooks=buf.gemm_hooks(slots=True, done_counter=self._done) if hooked else None)  # fmt: skip
+                     hooks=buf.gemm_hooks(slots=not alone, done_counter=self._done) if hooked else None)  # fmt: skip
         out, _, _ = buf.combine(plan, self._y, None, ready=ready)
-        if hooked:
+        if hooked and fetched is not None:
             torch.cuda.current_stream().wait_event(fetched)  # later users of the weight slots come after the copy
         if not save_for_backward:
             return out, None

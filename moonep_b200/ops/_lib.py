@@ -114,7 +114,7 @@ _SIGNATURES = {
     "moonep_dispatch": (_i, [_vp, _i, _i] + [_vp] * 9 + [_i] + [_vp] * 5 + [_i] * 9 + [_vp, _vp]),
     "moonep_single_supported": (_i, [_i, _i, _i, _i]),
     "moonep_single_work_words": (_i, []),
-    "moonep_dispatch_single": (_i, [_vp, _i] + [_vp] * 14 + [_i] * 5 + [_vp] * 4),
+    "moonep_dispatch_single": (_i, [_vp, _i, _i] + [_vp] * 14 + [_i] * 5 + [_vp] * 4),
     "moonep_combine_single": (_i, [_vp] * 7 + [_i, _vp]),
     "moonep_peer_store_bench": (_i, [_vp, _vp, _ll, _i, _i, _vp, _ll, _i, _vp, _vp]),
     "moonep_stage_layout": (_ll, [_i, _i, _i, _i, ctypes.POINTER(_ll), ctypes.POINTER(_ll)]),

@@ -109,6 +109,10 @@ class CudaBackend:
         # one rank: dispatch and combine are kernels of their own (csrc/single_rank.cu)
         self.single = R == 1 and bool(self.lib.moonep_single_supported(E, B, S, K)) and not self.phased
         self.single_work = i32(self.lib.moonep_single_work_words()) if self.single else None
+        # set around a dispatch whose rows are used whether or not something landed in them (the MoE layer's products without
+        # row flags): counts above what was routed are then an index error, if the dispatch that runs can tell
+        self.exact_counts = False
+        self.counts_checked = False  # the last dispatch could
         self.combine_mode = config.combine_mode()
         self.n_expand = 0  # CTAs of the dispatch kernel's destination-side role; 0 = every SM the senders leave free
 
@@ -373,7 +377,9 @@ class CudaBackend:
         with_w = route_weights_sk is not None
         self._sent_weights = with_w
         lr = ROLE_LOCAL_ROWS if config.local_rows_by_expand() else 0
+        self.counts_checked = False
         if self.single and lr and (planning_args is None or config.planner_on_gpu()):
+            self.counts_checked = self.exact_counts
             fused = copy_to if planning_args is not None else None
             self._dispatch_single(hidden_sh, route_weights_sk, plan, planning_args, fused)
             self._quiesced = True
@@ -438,7 +444,7 @@ class CudaBackend:
             self._next(FLAG_TPE)
             self._next(FLAG_PLAN)
         self._call(
-            "moonep_dispatch_single", int(topk is not None), _ptr(topk), _ptr(tpe), _ptr(plan.dst), _ptr(cu),
+            "moonep_dispatch_single", int(topk is not None), int(self.exact_counts), _ptr(topk), _ptr(tpe), _ptr(plan.dst), _ptr(cu),
             _ptr(plan.experts_to_copy), _ptr(plan.zero_fill_ranges), _ptr(plan.remote_stats), _ptr(plan.dup_groups),
             _ptr(plan.dup_loffs), _ptr(plan.dup_counts), _ptr(plan.src_info), _ptr(plan.link), _ptr(hidden), _ptr(weights),
             int(weights is not None), self._cur(FLAG_TPE), self._cur(FLAG_PLAN), self._next(FLAG_SENT), self.n_expand,

@@ -314,3 +314,36 @@ def test_layer_reports_groups_that_are_not_whole_row_blocks(S, switch, monkeypat
                 layer.check()
         layer.destroy()
         buf.destroy()
+
+
+@pytest.mark.parametrize("general", [False, True], ids=["single", "general"])
+def test_layer_refuses_counts_above_what_was_routed(general, monkeypatch):
+    """Rows of a group in which nothing landed would enter the weight gradients: an error in the layer (the general kernels'
+    products wait for such rows in vain), although ``Buffer.dispatch`` takes such counts; the layer works again after it."""
+    from moonep_b200.models.moe_layer import ExpertParallelMoE, dense_reference
+
+    if general:
+        monkeypatch.setenv("MOONEP_LOCAL_ROWS", "0")
+        monkeypatch.setenv("MOONEP_TIMEOUT_MS", "200")
+    S, H, K, E, inter = 200, 256, 2, 4, 256
+    buf = Buffer(S, H, K, E, 1, token_padding=128)
+    layer = ExpertParallelMoE(buf, inter, init_std=0.05, seed=4)
+    x, topk, tpe = _inputs(S, H, K, E, 0)
+    gates = torch.rand(S, K, device="cuda")
+    for extra in (3, 128):
+        more = tpe + torch.tensor([0, extra, 0, 0], dtype=torch.int32, device="cuda")
+        for save in (False, True):
+            layer.forward(x, gates, topk, more, save_for_backward=save)
+            with pytest.raises(MoonEPTimeoutError if general else MoonEPIndexError):
+                layer.check()
+    buf.dispatch(x, gates, topk, more)
+    buf.synchronize()
+    out, saved = layer.forward(x, gates, topk, tpe)
+    layer.check()
+    ref = dense_reference(x.float().cpu(), gates.cpu(), topk.cpu(), *(w[:E].float().cpu() for w in (layer.w_gate, layer.w_up, layer.w_down)))
+    # bf16 roundings of h, of every row and of the sum, each 2^-9 of values no larger than twice the largest result
+    assert float((out.float().cpu() - ref).abs().max()) <= 8 * 2.0**-9 * float(ref.abs().max())
+    layer.backward(saved, x)
+    layer.check()
+    layer.destroy()
+    buf.destroy()
