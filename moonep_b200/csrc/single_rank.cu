@@ -686,9 +686,11 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
       lay = {first, nullptr, nullptr, cum, groups};
       __syncthreads();
     }
-    unsigned long long t_laid = 0, t_planned = 0;  // kept by the two threads that report the phases
-    if (tid == 0 || tid == kEntries) t_laid = globaltimer_ns();
-    if (tid == 0 && a.fresh) stat_phase(c, MOONEP_PH_TABLES, t_begin, t_laid);
+    // The phases' times: of the planning from a warp that streams no rows, of the rows from one that does.
+    const bool times_plan = tid == kEntries - 32;
+    unsigned long long t_laid = 0, t_planned = 0;
+    if (times_plan || tid == kEntries) t_laid = globaltimer_ns();
+    if (times_plan && a.fresh) stat_phase(c, MOONEP_PH_TABLES, t_begin, t_laid);
     if (warp >= kPlanWarps) {
       clear_pads(c, a, lay, s.grab[warp - kPlanWarps], zeros, shard, meta, epoch);
       if (tid == kEntries) stat_phase(c, MOONEP_PH_ZERO, t_laid);
@@ -705,10 +707,8 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
           plan_tokens(c, a, s, cnt, off, cur, meta, t_lo, t_hi);
           fence_gpu();
           plan_sync();
-          if (tid == 0) {
-            st_release_gpu(a.work + kWorkReady + blockIdx.x, epoch);
-            stat_phase(c, MOONEP_PH_TOKENS, t_laid);
-          }
+          if (tid == 0) st_release_gpu(a.work + kWorkReady + blockIdx.x, epoch);
+          if (times_plan) stat_phase(c, MOONEP_PH_TOKENS, t_laid);
         } else {
           for (int i = t_lo * K + tid; i < t_hi * K; i += kEntries) {
             const int d = a.dst[i];
@@ -725,7 +725,6 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
         copy_plain(c, a, t_lo, t_hi, shard, meta, epoch);
       else if (warp < a.copy_warps)
         ok = copy_bulk(c, a, s, s_dyn, reinterpret_cast<unsigned char*>(shard), meta, epoch);
-      if (tid == 0) stat_phase(c, MOONEP_PH_SEND, t_planned);
       // rows behind the last group go into the copy as they are; the warps that do not stream rows see to it
       const int w0 = a.bulk ? a.copy_warps : 0;
       if (a.out != nullptr && a.fresh && warp >= w0)
@@ -733,7 +732,11 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
                   (int)gridDim.x * (kEntries - 32 * w0));
     }
     bulk_wait<0>();
-    if (tid == 0) stat_phase(c, MOONEP_PH_BUILD_EXPAND, t_begin);
+    if (tid == 0) {
+      const unsigned long long t_end = globaltimer_ns();
+      stat_phase(c, MOONEP_PH_SEND, t_planned, t_end);
+      stat_phase(c, MOONEP_PH_BUILD_EXPAND, t_begin, t_end);
+    }
   }
   // the last CTA resets the counters and publishes what the general kernels' stages publish
   fence_gpu();
@@ -804,7 +807,7 @@ __device__ __forceinline__ int4 pack8(const float* acc) {
 // one item in hand a lane has only K of them, so tokens of up to 4, 2 or 1 rows come 2, 4 or 8 items at a time (kItems > 1
 // needs K <= kCombineLoads / kItems and 16-byte rows).  One item in hand -> this: S=65536, H=2048, K=1 244 -> 96 us
 // (5.6 TB/s), S=4096, H=7168: K=1 61 -> 27, K=2 65 -> 39, K=4 72 -> 57; on one SM, S=1024, H=4096, K=1 724 -> 160.
-template <int kItems>
+template <int kItems, bool kVec = true>
 __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(const MoonepDevCtx c, const CombineArgs a) {
   constexpr int kRows = kCombineLoads / kItems;  // rows of an item whose loads are in flight together
   griddep_wait();
@@ -882,7 +885,7 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(cons
         if (i < nvec && it + j * step < end)
           st16(reinterpret_cast<int4*>(a.out + (long long)tok * H) + i, __popc(have) == 1 ? only : pack8(acc));
       }
-    } else if (a.vec_ok) {
+    } else if constexpr (kVec) {
       const int i = my_piece * 32 + lane;
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       int4 only = make_int4(0, 0, 0, 0);
@@ -1058,7 +1061,8 @@ extern "C" int moonep_combine_single(void* ctx, const int* dst, const void* in_r
   const int per_cta = kCombineThreads / 32 * a.items_per_warp;
   int grid = (int)((items + per_cta - 1) / per_cta);
   if (a.resident) grid = imin(grid, 2 * imax(1, c.local_sms));
-  auto* kernel = hand == 1   ? combine_single_kernel<1>
+  auto* kernel = !a.vec_ok   ? combine_single_kernel<1, false>
+                 : hand == 1 ? combine_single_kernel<1>
                  : hand == 2 ? combine_single_kernel<2>
                  : hand == 4 ? combine_single_kernel<4>
                              : combine_single_kernel<8>;
