@@ -1,0 +1,336 @@
+// Top-k router of a MoE block (sm_100a, plain CUDA cores): logits, selection, gates and token counts in one launch, all
+// gradients in another.
+//
+//   forward    logits[s, e] = x[s, :] . w[e, :]   (bf16 x fp32, fp32 sums);  topk[s, :] = the K largest, in order (equal ones
+//              by index);  gates[s, :] = softmax over those K, which is the softmax over all experts renormalised to the K;
+//              tokens_per_expert[e] += 1
+//   backward   dl[s, k] = gates[s, k] (dg[s, k] - sum_j gates[s, j] dg[s, j])   (the others' logits have no gradient)
+//              dx[s, :] = sum_k dl[s, k] w[topk[s, k], :]   (fp32, rounded to bf16 once)
+//              dw[e, :] = sum_s dl[s, e] x[s, :]            (fixed order: bitwise reproducible)
+//
+// As library calls the router of a block of S=2048 tokens, H=2048, 16 experts, K=4 is 17 launches forward and 13 backward
+// (fp32 copies of x and dx, three SIMT matrix products, softmax, top-k with its sort, gather, scatter, count): 148 us of
+// device time for 8 MB of x, 8 MB of dx and two passes over 128 KB of w.  Here: 13 us forward and 20 us backward (the sums of
+// the first form, 64 CTAs with 16 experts of all columns each and a load at a time, took 64).  Both are bound by the latency of
+// their few rounds of loads.
+//
+// No counterpart in the reference, whose callers bring the routing.
+#include "common.cuh"
+#include "host.h"
+
+namespace moonep {
+
+namespace {
+
+constexpr int kRouterExperts = 64;  // at most: a row of logits is two values per lane
+constexpr int kRouterTopK = 32;     // at most: a lane per selected expert
+
+// ---- forward ---------------------------------------------------------------------------------------------------
+// A CTA takes eight tokens: two groups of four, for each of which four warps share the columns.  A warp holds 4 tokens x 8
+// experts of partial sums per lane, so a 16-byte load of w serves 16 FMAs, and the two groups find each other's w in L1.
+constexpr int kFwdWarps = 8, kFwdTokens = 4, kFwdSplit = 4, kFwdExperts = 8;
+constexpr int kFwdCtaTokens = kFwdWarps / kFwdSplit * kFwdTokens;
+
+// Sums v[i] over the lanes for all i (N = 32); afterwards v[0] of a lane holds the total of entry `lane`: every step gives half
+// of the entries away, the top lane bit decides about the top half.
+template <int N>
+__device__ __forceinline__ void reduce_scatter(float (&v)[N], int lane) {
+  int n = N / 2;
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      if (i >= n) break;
+      const float keep = upper ? v[i + n] : v[i], give = upper ? v[i] : v[i + n];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+    n /= 2;
+  }
+}
+
+// Order of logits as unsigned numbers: NaN above everything, 0 is below everything (taken already).
+__device__ __forceinline__ unsigned rank_key(float f) {
+  const unsigned u = __float_as_uint(f);
+  if (f != f) return 0xffffffffu;
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+__global__ void __launch_bounds__(kFwdWarps * 32, 2)
+    router_fwd_kernel(const uint16_t* __restrict__ x, const float* __restrict__ w, int S, int H, int E, int K,
+                      float* __restrict__ gates, int* __restrict__ topk, int* __restrict__ tpe) {
+  __shared__ float s_part[kFwdSplit][kFwdCtaTokens][kFwdExperts];
+  __shared__ float s_logit[kFwdCtaTokens][kRouterExperts];
+  __shared__ int s_count[kRouterExperts];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int group = warp / kFwdSplit, part = warp % kFwdSplit;
+  const int tok0 = blockIdx.x * kFwdCtaTokens;
+  if (threadIdx.x < kRouterExperts) s_count[threadIdx.x] = 0;
+  for (int e0 = 0; e0 < E; e0 += kFwdExperts) {
+    float acc[kFwdTokens * kFwdExperts];
+#pragma unroll
+    for (int i = 0; i < kFwdTokens * kFwdExperts; ++i) acc[i] = 0.f;
+    for (int h = (part * 32 + lane) * 4; h < H; h += kFwdSplit * 128) {
+      float xf[kFwdTokens][4];
+#pragma unroll
+      for (int t = 0; t < kFwdTokens; ++t) {  // tokens and experts past the end repeat the last one and are dropped later
+        const int tok = min(tok0 + group * kFwdTokens + t, S - 1);
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(x + (long long)tok * H + h));
+        xf[t][0] = bf16lo(v.x), xf[t][1] = bf16hi(v.x), xf[t][2] = bf16lo(v.y), xf[t][3] = bf16hi(v.y);
+      }
+#pragma unroll
+      for (int e = 0; e < kFwdExperts; ++e) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(w + (long long)min(e0 + e, E - 1) * H + h));
+#pragma unroll
+        for (int t = 0; t < kFwdTokens; ++t) {
+          float& a = acc[t * kFwdExperts + e];
+          a = fmaf(xf[t][0], v.x, a);
+          a = fmaf(xf[t][1], v.y, a);
+          a = fmaf(xf[t][2], v.z, a);
+          a = fmaf(xf[t][3], v.w, a);
+        }
+      }
+    }
+    reduce_scatter(acc, lane);
+    static_assert(kFwdTokens * kFwdExperts == 32, "a lane per sum");
+    s_part[part][group * kFwdTokens + lane / kFwdExperts][lane % kFwdExperts] = acc[0];
+    __syncthreads();
+    for (int i = threadIdx.x; i < kFwdCtaTokens * kFwdExperts; i += kFwdWarps * 32) {
+      const int t = i / kFwdExperts, e = i % kFwdExperts;
+      float sum = s_part[0][t][e];
+#pragma unroll
+      for (int p = 1; p < kFwdSplit; ++p) sum += s_part[p][t][e];
+      s_logit[t][e0 + e] = sum;
+    }
+    __syncthreads();
+  }
+  // a warp per token: lane l looks after experts l and l + 32
+  const int tok = tok0 + warp;
+  if (tok < S) {
+    const float l0 = lane < E ? s_logit[warp][lane] : 0.f, l1 = lane + 32 < E ? s_logit[warp][lane + 32] : 0.f;
+    unsigned k0 = lane < E ? rank_key(l0) : 0u, k1 = lane + 32 < E ? rank_key(l1) : 0u;
+    const bool nan = __any_sync(0xffffffffu, (lane < E && l0 != l0) || (lane + 32 < E && l1 != l1));
+    int mine = 0;  // lane k keeps selection k
+    for (int k = 0; k < K; ++k) {
+      const unsigned best = __reduce_max_sync(0xffffffffu, k0 > k1 ? k0 : k1);
+      const unsigned lo = __ballot_sync(0xffffffffu, k0 == best), hi = __ballot_sync(0xffffffffu, k1 == best);
+      const int e = lo ? __ffs(lo) - 1 : 32 + __ffs(hi) - 1;
+      if (e == lane) k0 = 0u;
+      if (e == lane + 32) k1 = 0u;
+      if (lane == k) mine = e;
+    }
+    const float l = s_logit[warp][mine];
+    const float top = __shfl_sync(0xffffffffu, l, 0);
+    const float ex = lane < K ? expf(l - top) : 0.f;
+    float sum = ex;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane < K) {
+      gates[(long long)tok * K + lane] = nan ? __int_as_float(0x7fc00000) : ex / sum;
+      topk[(long long)tok * K + lane] = mine;
+      atomicAdd(s_count + mine, 1);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < E && s_count[threadIdx.x] != 0) atomicAdd(tpe + threadIdx.x, s_count[threadIdx.x]);
+}
+
+// ---- backward --------------------------------------------------------------------------------------------------
+// Clusters of eight CTAs.  The first n_dw clusters make 128 columns of dw for 16 experts each: the four quarters of their CTAs
+// share the tokens, every thread holds 2 columns x 16 experts of partial sums, and the partial sums are added through the
+// cluster's shared memory in a fixed order.  The CTAs of the others take eight tokens of dx at a time, a warp each.
+constexpr int kBwdThreads = 256, kBwdCluster = 8, kBwdExperts = 16;
+constexpr int kBwdParts = 4, kBwdPart = kBwdThreads / kBwdParts;  // quarters of a CTA, threads of one
+constexpr int kBwdCols = 2 * kBwdPart;
+constexpr int kBwdBatch = 64;  // tokens whose dl a quarter has in hand
+static_assert(kBwdBatch == kBwdPart, "a thread per token of a batch");
+constexpr int kBwdRows = 8;    // rows of x, or 16-byte loads of w, that a thread has in flight
+
+struct RouterBwdArgs {
+  const uint16_t* x;    // [S, H]
+  const float* w;       // [E, H]
+  const float* gates;   // [S, K]
+  const int* topk;      // [S, K]
+  const float* dgates;  // [S, K]
+  uint16_t* dx;         // [S, H] or null
+  float* dw;            // [E, H] or null
+  int S, H, E, K, n_dw;
+};
+
+__device__ void router_dw(const RouterBwdArgs& a, float (*s_dl)[kBwdBatch][kBwdExperts], float* s_sum) {
+  const int rank = (int)(blockIdx.x % kBwdCluster), job = (int)(blockIdx.x / kBwdCluster);
+  const int nchunks = (a.H + kBwdCols - 1) / kBwdCols;
+  const int e0 = job / nchunks * kBwdExperts, col0 = job % nchunks * kBwdCols;
+  const int part = threadIdx.x / kBwdPart, t = threadIdx.x % kBwdPart;
+  const int col = min(col0 + 2 * t, a.H - 2);  // H is even; columns past the end repeat the last ones and are dropped
+  const int share = (a.S + kBwdParts * kBwdCluster - 1) / (kBwdParts * kBwdCluster);
+  const int lo = min(a.S, (rank * kBwdParts + part) * share), hi = min(a.S, lo + share);
+  float acc[2][kBwdExperts];
+#pragma unroll
+  for (int e = 0; e < kBwdExperts; ++e) acc[0][e] = acc[1][e] = 0.f;
+  for (int b = 0; b < share; b += kBwdBatch) {
+    const int n = max(0, min(kBwdBatch, hi - lo - b));
+    const long long at = (long long)(lo + b + t) * a.K;
+    float dot = 0.f;
+    if (t < n)
+#pragma unroll 4
+      for (int k = 0; k < a.K; ++k) dot = fmaf(__ldg(a.gates + at + k), __ldg(a.dgates + at + k), dot);
+    __syncthreads();  // the batch before has been used
+#pragma unroll
+    for (int e = 0; e < kBwdExperts; e += 4) *reinterpret_cast<float4*>(&s_dl[part][t][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < n)
+#pragma unroll 4
+      for (int k = 0; k < a.K; ++k) {
+        const int e = __ldg(a.topk + at + k) - e0;
+        const float dl = __ldg(a.gates + at + k) * (__ldg(a.dgates + at + k) - dot);
+        if ((unsigned)e < (unsigned)kBwdExperts) s_dl[part][t][e] = dl;
+      }
+    __syncthreads();
+    const uint16_t* src = a.x + (long long)(lo + b) * a.H + col;
+    for (int i0 = 0; i0 < n; i0 += kBwdRows) {
+      unsigned v[kBwdRows];
+#pragma unroll
+      for (int i = 0; i < kBwdRows; ++i)
+        v[i] = i0 + i < n ? __ldg(reinterpret_cast<const unsigned*>(src + (long long)(i0 + i) * a.H)) : 0u;
+#pragma unroll
+      for (int i = 0; i < kBwdRows; ++i) {
+        if (i0 + i >= n) break;
+        const float x0 = bf16lo(v[i]), x1 = bf16hi(v[i]);
+#pragma unroll
+        for (int q = 0; q < kBwdExperts / 4; ++q) {
+          const float4 d = *reinterpret_cast<const float4*>(&s_dl[part][i0 + i][4 * q]);
+          acc[0][4 * q] = fmaf(d.x, x0, acc[0][4 * q]);
+          acc[1][4 * q] = fmaf(d.x, x1, acc[1][4 * q]);
+          acc[0][4 * q + 1] = fmaf(d.y, x0, acc[0][4 * q + 1]);
+          acc[1][4 * q + 1] = fmaf(d.y, x1, acc[1][4 * q + 1]);
+          acc[0][4 * q + 2] = fmaf(d.z, x0, acc[0][4 * q + 2]);
+          acc[1][4 * q + 2] = fmaf(d.z, x1, acc[1][4 * q + 2]);
+          acc[0][4 * q + 3] = fmaf(d.w, x0, acc[0][4 * q + 3]);
+          acc[1][4 * q + 3] = fmaf(d.w, x1, acc[1][4 * q + 3]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < kBwdExperts; ++e)
+    *reinterpret_cast<float2*>(s_sum + (part * kBwdExperts + e) * kBwdCols + 2 * t) = make_float2(acc[0][e], acc[1][e]);
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  // a CTA adds up two experts' columns of all quarters of all eight
+  const unsigned base = (unsigned)__cvta_generic_to_shared(s_sum);
+  const int e = rank * 2 + threadIdx.x / kBwdCols, c = threadIdx.x % kBwdCols;
+  static_assert(2 * kBwdCols == kBwdThreads && 2 * kBwdCluster == kBwdExperts, "a thread per sum");
+  float sum = 0.f;
+#pragma unroll
+  for (int r = 0; r < kBwdCluster; ++r) {
+    float v[kBwdParts];
+#pragma unroll
+    for (int p = 0; p < kBwdParts; ++p) {
+      unsigned from;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                   : "=r"(from)
+                   : "r"(base + (unsigned)((p * kBwdExperts + e) * kBwdCols + c) * 4u), "r"(r));
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[p]) : "r"(from) : "memory");
+    }
+#pragma unroll
+    for (int p = 0; p < kBwdParts; ++p) sum += v[p];
+  }
+  if (e0 + e < a.E && col0 + c < a.H) a.dw[(long long)(e0 + e) * a.H + col0 + c] = sum;
+  // the others' sums are read out of this CTA's shared memory until here
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ void router_dx(const RouterBwdArgs& a) {
+  constexpr int kHand = kBwdRows / 2;  // selections whose rows of w are in flight together
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ctas = (int)gridDim.x - a.n_dw * kBwdCluster, cta = (int)blockIdx.x - a.n_dw * kBwdCluster;
+  for (int tok = cta * (kBwdThreads / 32) + warp; tok < a.S; tok += ctas * (kBwdThreads / 32)) {
+    const long long at = (long long)tok * a.K + lane;
+    const float g = lane < a.K ? a.gates[at] : 0.f, dg = lane < a.K ? a.dgates[at] : 0.f;
+    const int e = lane < a.K ? a.topk[at] : 0;
+    float dot = g * dg;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+    const float dl = g * (dg - dot);
+    for (int h0 = 0; h0 < a.H; h0 += 256) {
+      const int h = min(h0 + lane * 8, a.H - 8);  // H is a multiple of 8; lanes past the end repeat the last columns
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int k0 = 0; k0 < a.K; k0 += kHand) {
+        float4 v[kHand][2];
+#pragma unroll
+        for (int k = 0; k < kHand; ++k) {
+          const float* row = a.w + (long long)__shfl_sync(0xffffffffu, e, min(k0 + k, a.K - 1)) * a.H + h;
+          v[k][0] = __ldg(reinterpret_cast<const float4*>(row));
+          v[k][1] = __ldg(reinterpret_cast<const float4*>(row) + 1);
+        }
+#pragma unroll
+        for (int k = 0; k < kHand; ++k) {
+          const float d = __shfl_sync(0xffffffffu, dl, min(k0 + k, a.K - 1));
+          if (k0 + k >= a.K) break;
+          acc[0] = fmaf(d, v[k][0].x, acc[0]);
+          acc[1] = fmaf(d, v[k][0].y, acc[1]);
+          acc[2] = fmaf(d, v[k][0].z, acc[2]);
+          acc[3] = fmaf(d, v[k][0].w, acc[3]);
+          acc[4] = fmaf(d, v[k][1].x, acc[4]);
+          acc[5] = fmaf(d, v[k][1].y, acc[5]);
+          acc[6] = fmaf(d, v[k][1].z, acc[6]);
+          acc[7] = fmaf(d, v[k][1].w, acc[7]);
+        }
+      }
+      if (h0 + lane * 8 < a.H)
+        st16(reinterpret_cast<int4*>(a.dx + (long long)tok * a.H + h),
+             make_int4((int)pack_bf16(acc[0], acc[1]), (int)pack_bf16(acc[2], acc[3]), (int)pack_bf16(acc[4], acc[5]),
+                       (int)pack_bf16(acc[6], acc[7])));
+    }
+  }
+}
+
+__global__ void __cluster_dims__(kBwdCluster, 1, 1) __launch_bounds__(kBwdThreads) router_bwd_kernel(const RouterBwdArgs a) {
+  __shared__ __align__(16) float s_dl[kBwdParts][kBwdBatch][kBwdExperts];
+  __shared__ __align__(16) float s_sum[kBwdParts * kBwdExperts * kBwdCols];
+  if ((int)blockIdx.x < a.n_dw * kBwdCluster) router_dw(a, s_dl, s_sum); else router_dx(a);
+}
+
+}  // namespace
+
+}  // namespace moonep
+
+using namespace moonep;
+
+static int router_sizes_ok(const char* what, int S, int H, int E, int K, const void* const* aligned, int n) {
+  if (S < 1 || H < 8 || H % 8 != 0 || E < 1 || E > kRouterExperts || K < 1 || K > E || K > kRouterTopK) {
+    set_error(std::string(what) + ": needs S >= 1, H a multiple of 8, E <= " + std::to_string(kRouterExperts) + " and K <= min(E, " +
+              std::to_string(kRouterTopK) + ")");
+    return 0;
+  }
+  for (int i = 0; i < n; ++i)
+    if ((reinterpret_cast<uintptr_t>(aligned[i]) & 15u) != 0) {
+      set_error(std::string(what) + ": x, w and dx must be 16-byte aligned");
+      return 0;
+    }
+  return 1;
+}
+
+// x: [S, H] bf16, w: [E, H] fp32 -> gates [S, K] fp32, topk [S, K], tpe [E] (overwritten).
+extern "C" int moonep_router_fwd(const void* x, const float* w, int S, int H, int E, int K, float* gates, int* topk, int* tpe,
+                                 void* stream) {
+  const void* aligned[] = {x, w};
+  if (!router_sizes_ok("moonep_router_fwd", S, H, E, K, aligned, 2)) return 1;
+  if (int rc = check_cuda(cudaMemsetAsync(tpe, 0, sizeof(int) * (size_t)E, (cudaStream_t)stream), "moonep_router_fwd")) return rc;
+  router_fwd_kernel<<<(S + kFwdCtaTokens - 1) / kFwdCtaTokens, kFwdWarps * 32, 0, (cudaStream_t)stream>>>(
+      (const uint16_t*)x, w, S, H, E, K, gates, topk, tpe);
+  return check_launch("router_fwd_kernel");
+}
+
+// dgates: [S, K] fp32 -> dx [S, H] bf16 and dw [E, H] fp32 (either may be null); gates and topk from the forward pass.
+extern "C" int moonep_router_bwd(const void* x, const float* w, const float* gates, const int* topk, const float* dgates, int S,
+                                 int H, int E, int K, void* dx, float* dw, void* stream) {
+  const void* aligned[] = {x, w, dx};
+  if (!router_sizes_ok("moonep_router_bwd", S, H, E, K, aligned, 3)) return 1;
+  RouterBwdArgs a = {(const uint16_t*)x, w, gates, topk, dgates, (uint16_t*)dx, dw, S, H, E, K, 0};
+  if (dw != nullptr) a.n_dw = (H + kBwdCols - 1) / kBwdCols * ((E + kBwdExperts - 1) / kBwdExperts);
+  const int per_cluster = kBwdCluster * kBwdThreads / 32;  // tokens a cluster takes at a time
+  const int n_dx = dx != nullptr ? imin((S + per_cluster - 1) / per_cluster, 64) : 0;
+  if (a.n_dw + n_dx == 0) return 0;
+  router_bwd_kernel<<<(a.n_dw + n_dx) * kBwdCluster, kBwdThreads, 0, (cudaStream_t)stream>>>(a);
+  return check_launch("router_bwd_kernel");
+}

@@ -21,8 +21,10 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.autograd import forward_ad
 
 from ..api import Buffer
+from ..ops.moe_ops import router_backward, router_forward, router_kernel_supports
 from .moe_layer import ExpertParallelMoE
 
 
@@ -42,6 +44,43 @@ class MoEFunction(torch.autograd.Function):
         return dx, dgates, None, None, None
 
 
+class RouterFunction(torch.autograd.Function):
+    """``gates, topk, tokens_per_expert = RouterFunction.apply(x, weight, k)`` on ``csrc/router.cu``; differentiable in ``x``
+    and ``weight`` through the gates."""
+
+    @staticmethod
+    def forward(ctx, x, weight, k):
+        gates, topk, tpe = router_forward(x, weight, k)
+        ctx.save_for_backward(x, weight, gates, topk)
+        ctx.mark_non_differentiable(topk, tpe)
+        ctx.set_materialize_grads(False)
+        return gates, topk, tpe
+
+    @staticmethod
+    def backward(ctx, dgates, _topk, _tpe):
+        if dgates is None:
+            return None, None, None
+        x, weight, gates, topk = ctx.saved_tensors
+        want_dx, want_dw = ctx.needs_input_grad[:2]
+        if torch.is_grad_enabled():  # a graph of the gradients is wanted: the same in differentiable operations
+            g = torch.softmax((x.float() @ weight.t()).gather(1, topk.long()), dim=-1)
+            wrt = [t for t, want in ((x, want_dx), (weight, want_dw)) if want]
+            grads = list(torch.autograd.grad(g, wrt, dgates, create_graph=True))
+            return grads.pop(0) if want_dx else None, grads.pop(0) if want_dw else None, None
+        dx, dw = router_backward(x, weight, gates, topk, dgates.float().contiguous(), want_dx, want_dw)
+        return dx, dw, None
+
+
+def _plain_eager_call(x, weight) -> bool:
+    """No transform, trace or dispatch mode sees the call, so an autograd function may stand in for the operations."""
+    return (
+        type(x) is torch.Tensor and type(weight) in (torch.Tensor, nn.Parameter)
+        and not torch.compiler.is_compiling() and not torch.jit.is_tracing() and not torch.is_autocast_enabled("cuda")
+        and torch._C._functorch.peek_interpreter_stack() is None and forward_ad._current_level < 0
+        and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+    )  # fmt: skip
+
+
 class TopKRouter(nn.Module):
     """Softmax router: ``gates`` are the top-k probabilities renormalised to sum to one (fp32), ``topk`` the expert
     ids (int32), ``tokens_per_expert`` this rank's count per expert (int32, what the planner exchanges)."""
@@ -54,6 +93,8 @@ class TopKRouter(nn.Module):
         self.k, self.num_experts = k, num_experts
 
     def forward(self, x):
+        if _plain_eager_call(x, self.weight) and router_kernel_supports(x, self.weight, self.k):
+            return RouterFunction.apply(x, self.weight, self.k)
         logits = x.float() @ self.weight.t()
         probs = torch.softmax(logits, dim=-1)
         top_p, top_i = torch.topk(probs, self.k, dim=-1)

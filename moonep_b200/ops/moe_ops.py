@@ -1,6 +1,6 @@
-"""Dense helpers of the MoE layer's backward pass: batched expert transposes and the SwiGLU backward.
+"""Dense helpers of the MoE layer and block: batched expert transposes, the SwiGLU backward, weight updates, the router.
 
-CUDA tensors run the kernels of ``csrc/moe_kernels.cu``; CPU tensors run the same arithmetic in torch.
+CUDA tensors run the kernels of ``csrc/moe_kernels.cu`` and ``csrc/router.cu``; CPU tensors run the same arithmetic in torch.
 """
 
 from __future__ import annotations
@@ -109,3 +109,45 @@ def _adamw_step(tensors, lr, b1, b2, eps, weight_decay, c1, c2) -> None:
         rc = _lib.load().moonep_adamw_update(n, *ptrs, sizes, lr / c1, b1, b2, eps, 1.0 - lr * weight_decay, c2,
                                              _lib.current_stream())  # fmt: skip
     _lib.check(rc, "moonep_adamw_update")
+
+
+ROUTER_MAX_EXPERTS, ROUTER_MAX_TOPK = 64, 32  # of the router kernels
+
+
+def router_kernel_supports(x: torch.Tensor, weight: torch.Tensor, k: int) -> bool:
+    """Whether ``csrc/router.cu`` takes this call.  Up to 64 experts its one launch replaces a dozen; with more, the matrix
+    product dominates and a tiled one wins."""
+    return (
+        x.is_cuda and weight.is_cuda and x.device == weight.device and x.dim() == 2 and weight.dim() == 2
+        and x.dtype == torch.bfloat16 and weight.dtype == torch.float32 and x.is_contiguous() and weight.is_contiguous()
+        and x.shape[0] >= 1 and x.shape[1] == weight.shape[1] and x.shape[1] >= 8 and x.shape[1] % 8 == 0
+        and 1 <= k <= min(int(weight.shape[0]), ROUTER_MAX_TOPK) and weight.shape[0] <= ROUTER_MAX_EXPERTS
+        and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+    )  # fmt: skip
+
+
+def router_forward(x: torch.Tensor, weight: torch.Tensor, k: int):
+    """``(gates [S, k] fp32, topk [S, k] int32, tokens_per_expert [E] int32)`` of logits ``x @ weight.T``."""
+    (S, H), E = x.shape, int(weight.shape[0])
+    gates = torch.empty(S, k, dtype=torch.float32, device=x.device)
+    topk = torch.empty(S, k, dtype=torch.int32, device=x.device)
+    tpe = torch.empty(E, dtype=torch.int32, device=x.device)
+    with _lib.on_device(x.device):
+        rc = _lib.load().moonep_router_fwd(x.data_ptr(), weight.data_ptr(), S, H, E, k, gates.data_ptr(), topk.data_ptr(),
+                                           tpe.data_ptr(), _lib.current_stream())  # fmt: skip
+    _lib.check(rc, "moonep_router_fwd")
+    return gates, topk, tpe
+
+
+def router_backward(x, weight, gates, topk, dgates, want_dx: bool, want_dw: bool):
+    """Gradients of ``router_forward``'s gates: ``(dx [S, H] bf16 or None, dweight [E, H] fp32 or None)``."""
+    (S, H), E = x.shape, int(weight.shape[0])
+    dx = torch.empty_like(x) if want_dx else None
+    dw = torch.empty_like(weight) if want_dw else None
+    with _lib.on_device(x.device):
+        rc = _lib.load().moonep_router_bwd(
+            x.data_ptr(), weight.data_ptr(), gates.data_ptr(), topk.data_ptr(), dgates.data_ptr(), S, H, E, int(topk.shape[1]),
+            None if dx is None else dx.data_ptr(), None if dw is None else dw.data_ptr(), _lib.current_stream(),
+        )  # fmt: skip
+    _lib.check(rc, "moonep_router_bwd")
+    return dx, dw

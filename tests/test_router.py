@@ -1,0 +1,116 @@
+"""The router kernels (csrc/router.cu) against 64-bit arithmetic, and the calls that keep the differentiable operations."""
+
+import pytest
+import torch
+
+from moonep_b200.models.moe_block import TopKRouter
+
+gpu = pytest.mark.gpu
+
+
+def _case(S, H, E, K, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    router = TopKRouter(H, E, K, init_std=0.05, seed=seed, device="cuda")
+    x = torch.randn(S, H, generator=g).to(torch.bfloat16).cuda().requires_grad_(True)
+    return router, x, torch.randn(S, K, generator=g).cuda()
+
+
+# one token, one expert; a token group that is not full; 16-column remainders of the warps' shares of H; experts beyond a chunk
+# of 16; the most experts and selections the kernels take; more tokens than the backward's CTAs hold at a time
+@gpu
+@pytest.mark.parametrize("S,H,E,K", [(1, 8, 1, 1), (7, 264, 3, 3), (8, 128, 16, 4), (33, 2048, 17, 4), (130, 520, 64, 32),
+                                     (9, 7168, 48, 8), (4100, 256, 16, 2)])  # fmt: skip
+def test_router_kernels_match_64_bit(S, H, E, K):
+    router, x, dg = _case(S, H, E, K)
+    gates, topk, tpe = router(x)
+    assert gates.grad_fn is not None and "RouterFunction" in type(gates.grad_fn).__name__
+    xd, wd = x.detach().double(), router.weight.detach().double()
+    logits = xd @ wd.t()
+    # 32-bit sums: a lane adds H / 128 products (whole groups of four), then five lanes' and three warps' sums are added; each
+    # rounding is at most 2^-24 of the sum of the products' sizes
+    bound = ((H / 128 + 12) * 2.0**-24) * (xd.abs() @ wd.abs().t()).max().item()
+    idx = topk.long()
+    assert topk.dtype == torch.int32 and (idx.sort(dim=1).values.diff(dim=1) > 0).all() and idx.min() >= 0 and idx.max() < E
+    picked = logits.gather(1, idx)
+    assert (picked.diff(dim=1) <= 2 * bound).all(), "selections out of order"
+    rest = logits.scatter(1, idx, float("-inf")).max(dim=1).values
+    assert (picked.min(dim=1).values >= rest - 2 * bound).all(), "a larger logit was left out"
+    assert torch.equal(tpe, torch.bincount(idx.flatten(), minlength=E).to(torch.int32))
+    gd = torch.softmax(picked, dim=1)
+    # a gate moves by at most twice its logits' error, and is rounded a few times
+    assert (gates.double() - gd).abs().max() <= 2 * bound + 8 * 2.0**-24
+    gates.backward(dg)
+    dl = torch.zeros_like(logits).scatter(1, idx, gd * (dg.double() - (gd * dg.double()).sum(dim=1, keepdim=True)))
+    dx, dw = dl @ wd, dl.t() @ xd
+    rel = 4 * bound + (K + 16) * 2.0**-24  # of dl, whose terms are gates times differences of dg
+    scale = dg.abs().max().item()
+    # dx: K terms, rounded to bf16 once; dw: sixteen shares of the tokens one after the other, then added
+    assert ((x.grad.double() - dx).abs() <= 2.0**-8 * dx.abs() + 2 * rel * scale * K * wd.abs().max()).all()
+    slack = rel * scale * xd.abs().sum(dim=0) + (S / 16 + 20) * 2.0**-24 * (dl.abs().t() @ xd.abs())
+    assert ((router.weight.grad.double() - dw).abs() <= 2 * slack).all()
+
+
+@gpu
+def test_router_ties_and_non_finite_logits():
+    router, x, _ = _case(5, 16, 6, 3)
+    with torch.no_grad():
+        router.weight.zero_()
+        router.weight[4, 0] = float("inf")
+        router.weight[5, 1] = float("-inf")
+        x.zero_()  # row 0: inf * 0 and -inf * 0 are NaN
+        x[1:, 0], x[1:, 1] = 1, 1  # +inf and -inf
+        x[2:, 0] = 0  # expert 4 is NaN
+        x[3:, 1] = 0
+        router.weight[:, 2] = 1.0
+    gates, topk, _ = router(x)
+    assert torch.isnan(gates).all() and (topk >= 0).all() and (topk < 6).all()
+    assert (topk.long().sort(dim=1).values.diff(dim=1) > 0).all()
+    with torch.no_grad():
+        router.weight.fill_(0.25)
+        x.fill_(1)
+    gates, topk, tpe = router(x)
+    assert topk.tolist() == [[0, 1, 2]] * 5 and torch.equal(gates, torch.full_like(gates, 1 / 3))
+    assert tpe.tolist() == [5, 5, 5, 0, 0, 0]
+    with torch.no_grad():  # one expert is impossible
+        router.weight[0] = float("-inf")
+    gates, topk, _ = router(x)
+    assert topk.tolist() == [[1, 2, 3]] * 5 and torch.isfinite(gates).all()
+
+
+@gpu
+def test_router_gradients_of_parts_and_of_gradients():
+    router, x, dg = _case(12, 64, 8, 2)
+    gates, _, _ = router(x.detach())
+    gates.backward(dg)
+    want = router.weight.grad.clone()
+    router.weight.grad = None
+    gates, _, _ = router(x)
+    (dx,) = torch.autograd.grad(gates, x, dg, create_graph=True)  # a graph of the gradient
+    assert dx.grad_fn is not None
+    dx.float().square().sum().backward()
+    assert torch.isfinite(router.weight.grad).all() and router.weight.grad.abs().sum() > 0
+    router.weight.grad = None
+    gates, _, _ = router(x)
+    gates.backward(dg)
+    assert torch.equal(router.weight.grad, want), "not reproducible"
+
+
+@gpu
+@pytest.mark.parametrize("what", ["experts", "strided", "fp32", "autocast", "dual"])
+def test_router_keeps_the_general_operations(what):
+    router, x, _ = _case(16, 64, 65 if what == "experts" else 8, 2)
+    if what == "strided":
+        x = torch.randn(16, 128, device="cuda").to(torch.bfloat16)[:, ::2]
+    if what == "fp32":
+        x = x.float()
+    if what == "dual":
+        import torch.autograd.forward_ad as fw
+
+        with fw.dual_level():
+            gates, _, _ = router(fw.make_dual(x.detach(), torch.ones_like(x)))
+            assert fw.unpack_dual(gates).tangent is not None
+        return
+    with torch.autocast("cuda", dtype=torch.bfloat16, enabled=what == "autocast"):
+        gates, topk, tpe = router(x)
+    assert "RouterFunction" not in type(gates.grad_fn).__name__
+    assert gates.shape == (16, 2) and int(tpe.sum()) == 32
