@@ -90,6 +90,10 @@ def _create_context(S, H, K, E, num_ep_ranks, num_sms=None, token_padding=128, B
     return ctx
 
 
+def _contiguous_i32(t: torch.Tensor) -> torch.Tensor:
+    return t if t.dtype is torch.int32 and t.is_contiguous() else t.to(torch.int32).contiguous()
+
+
 class Buffer:
     """Communication buffer of one EP rank (see module docstring)."""
 
@@ -330,8 +334,8 @@ class Buffer:
                 "a fresh dispatch needs topk_experts_sk and tokens_per_expert"
             )
             assert topk_experts_sk.numel() == S * K, "topk_experts_sk shape mismatch"
-            topk_flat = topk_experts_sk.reshape(-1).to(torch.int32).contiguous()
-            tpe = tokens_per_expert.to(torch.int32).contiguous()
+            topk_flat = _contiguous_i32(topk_experts_sk.reshape(-1))
+            tpe = _contiguous_i32(tokens_per_expert)
             assert tpe.numel() in (ctx["E"], ctx["R"] * ctx["E"]), "tokens_per_expert must be [E] or [R, E]"
             plan, cu_seqlens = allocate_planning_outputs(ctx)
             check_planning_outputs(ctx, cu_seqlens, plan)

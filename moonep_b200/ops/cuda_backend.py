@@ -443,10 +443,13 @@ class CudaBackend:
             self._topk = topk
             self._next(FLAG_TPE)
             self._next(FLAG_PLAN)
+        # a fresh plan of this Buffer comes as one allocation; its tensors are made when somebody asks for them
+        dst, etc, zf, rs, dg, dl, dc, si, lk = (plan._addresses() if topk is not None else None) or [
+            _ptr(t) for t in (plan.dst, plan.experts_to_copy, plan.zero_fill_ranges, plan.remote_stats, plan.dup_groups,
+                              plan.dup_loffs, plan.dup_counts, plan.src_info, plan.link)]  # fmt: skip
         self._call(
-            "moonep_dispatch_single", int(topk is not None), int(self.exact_counts), _ptr(topk), _ptr(tpe), _ptr(plan.dst), _ptr(cu),
-            _ptr(plan.experts_to_copy), _ptr(plan.zero_fill_ranges), _ptr(plan.remote_stats), _ptr(plan.dup_groups),
-            _ptr(plan.dup_loffs), _ptr(plan.dup_counts), _ptr(plan.src_info), _ptr(plan.link), _ptr(hidden), _ptr(weights),
+            "moonep_dispatch_single", int(topk is not None), int(self.exact_counts), _ptr(topk), _ptr(tpe), dst, _ptr(cu),
+            etc, zf, rs, dg, dl, dc, si, lk, _ptr(hidden), _ptr(weights),
             int(weights is not None), self._cur(FLAG_TPE), self._cur(FLAG_PLAN), self._next(FLAG_SENT), self.n_expand,
             _ptr(self.single_work), _ptr(out), _ptr(out_w), _stream(), tag="dispatch_single",
         )  # fmt: skip
@@ -486,8 +489,9 @@ class CudaBackend:
 
     # -- combine -------------------------------------------------------------------------
     def can_push(self, plan) -> bool:
-        return (self.combine_mode == "push" and (self.ctx.get("stage_buf") is not None or self.ctx["R"] == 1)
-                and plan.src_info is not None and plan.link is not None)  # fmt: skip
+        if self.combine_mode != "push" or (self.ctx.get("stage_buf") is None and self.ctx["R"] != 1):
+            return False
+        return getattr(plan, "_pack", None) is not None or (plan.src_info is not None and plan.link is not None)
 
     def combine_all(self, plan, hidden_nvsh, route_weights_nvs, out_hidden, out_weights_sk, inter_rank_sync,
                     zero_copy, ready=None, ready_expect=0):  # fmt: skip

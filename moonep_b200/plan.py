@@ -36,8 +36,47 @@ import torch
 from .layout import check_encoding_bounds
 
 
+_FIELDS = ("dst", "experts_to_copy", "zero_fill_ranges", "remote_stats", "dup_groups", "dup_loffs", "dup_counts", "src_info", "link")
+_ALIGN = 128  # words: what a tensor of its own would start on
+
+
+def _field_shapes(N, R, E, B, NvS) -> dict:
+    return {
+        "dst": (N,), "experts_to_copy": (R, B), "zero_fill_ranges": (E + B, 2), "remote_stats": (2,),
+        "dup_groups": (NvS, 3), "dup_loffs": (NvS,), "dup_counts": (2,), "src_info": (NvS,), "link": (NvS,),
+    }  # fmt: skip
+
+
+class _PlanLayout:
+    """Where the fields of a plan lie in one int32 allocation (words), and their shapes and strides."""
+
+    __slots__ = ("fields", "offsets", "words")
+
+    def __init__(self, N, R, E, B, NvS):
+        self.fields, self.offsets, self.words = {}, [], 0
+        for name, shape in _field_shapes(N, R, E, B, NvS).items():
+            strides = (1,) if len(shape) == 1 else (shape[1], 1)
+            self.fields[name] = (shape, strides, self.words)
+            self.offsets.append(self.words)
+            self.words += -(-max(1, shape[0] * (shape[1] if len(shape) == 2 else 1)) // _ALIGN) * _ALIGN
+
+
+class _Packed:
+    """What a plan from ``allocate_planning_outputs`` on a GPU keeps in the place of its tensors until they are asked for:
+    the allocation, its layout and the tensors made so far."""
+
+    __slots__ = ("base", "layout", "made")
+
+    def __init__(self, base, layout):
+        self.base, self.layout, self.made = base, layout, {}
+
+
+class _PackSlot:
+    __slots__ = ("_pack",)
+
+
 @dataclass(frozen=True, slots=True)
-class MoonEPCommPlan:
+class MoonEPCommPlan(_PackSlot):
     dst: torch.Tensor
     experts_to_copy: torch.Tensor
     zero_fill_ranges: torch.Tensor
@@ -58,19 +97,46 @@ class MoonEPCommPlan:
         N, R, E, B, NvS = int(self.N), int(self.R), int(self.E), int(self.B), int(self.NvS)
         assert self.dst.dtype == torch.int32 and self.dst.is_contiguous(), "dst must be contiguous int32"
         assert self.dst.numel() == N, "dst must hold one entry per (token, k)"
-        for name, shape in (
-            ("experts_to_copy", (R, B)),
-            ("zero_fill_ranges", (E + B, 2)),
-            ("remote_stats", (2,)),
-            ("dup_groups", (NvS, 3)),
-            ("dup_loffs", (NvS,)),
-            ("dup_counts", (2,)),
-        ):
-            got = tuple(getattr(self, name).shape)
-            assert got == shape, f"{name} has shape {got}, expected {shape}"
-        for name in ("src_info", "link"):
+        for name, shape in _field_shapes(N, R, E, B, NvS).items():
             t = getattr(self, name)
-            assert t is None or tuple(t.shape) == (NvS,), f"{name} must have shape ({NvS},)"
+            if name == "dst" or (t is None and name in ("src_info", "link")):
+                continue
+            assert tuple(t.shape) == shape, f"{name} has shape {tuple(t.shape)}, expected {shape}"
+
+    def __getattr__(self, name):
+        """A field of a packed plan that nobody has used yet: a view of the plan's allocation, made once."""
+        try:
+            pack = object.__getattribute__(self, "_pack")
+            shape, strides, offset = pack.layout.fields[name]
+        except (AttributeError, KeyError):
+            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}") from None
+        t = pack.base.as_strided(shape, strides, offset)
+        object.__setattr__(self, name, t)
+        pack.made[name] = t
+        return t
+
+    @classmethod
+    def _packed(cls, base, layout, N, R, E, B, NvS, K) -> "MoonEPCommPlan":
+        """A plan whose tensors are views of ``base``.  A round trip uses one of the nine; the others cost what they
+        cost only where they are used, and the allocation is one call instead of nine (18 us of host time)."""
+        plan = object.__new__(cls)
+        put = object.__setattr__
+        put(plan, "_pack", _Packed(base, layout))
+        put(plan, "N", N)
+        put(plan, "R", R)
+        put(plan, "E", E)
+        put(plan, "B", B)
+        put(plan, "NvS", NvS)
+        put(plan, "K", K)
+        return plan
+
+    def _addresses(self):
+        """Addresses of the fields, in order, of a plan that has just been allocated; None if it is not packed."""
+        pack = getattr(self, "_pack", None)
+        if pack is None:
+            return None
+        p = pack.base.data_ptr()
+        return [p + 4 * o for o in pack.layout.offsets]
 
     def tensors(self):
         """The tensors a stream must keep alive while it uses this plan."""
@@ -121,6 +187,13 @@ def allocate_planning_outputs(ctx: dict) -> tuple[MoonEPCommPlan, torch.Tensor]:
     """Allocate an empty plan and the ``cu_seqlens[E+B]`` tensor for ``ctx``."""
     E, B, N, NvS, R, K = ctx["E"], ctx["B"], ctx["N"], ctx["NvS"], ctx["R"], ctx["K"]
     dev = ctx["meta_buf"].device
+    if dev.type == "cuda":
+        layout = ctx.get("_plan_layout")
+        if layout is None:
+            layout = ctx["_plan_layout"] = _PlanLayout(N, R, E, B, NvS)
+        base = torch.empty(layout.words, dtype=torch.int32, device=dev)
+        # a tensor of its own: it may be kept long after the plan
+        return MoonEPCommPlan._packed(base, layout, N, R, E, B, NvS, K), torch.empty(E + B, dtype=torch.int32, device=dev)
     plan = MoonEPCommPlan(
         dst=_i32(N, dev),
         experts_to_copy=_i32(R * B, dev).view(R, B),
@@ -156,16 +229,17 @@ def check_plan_for_ctx(ctx: dict, plan: MoonEPCommPlan, device) -> None:
     assert isinstance(plan, MoonEPCommPlan), "plan must be a MoonEPCommPlan"
     assert plan.N == ctx["N"] and plan.R == ctx["R"] and plan.K == ctx["K"] and plan.NvS == ctx["NvS"]
     assert plan.E == ctx["E"] and plan.B == ctx["B"]
-    E, B, N, NvS, R = ctx["E"], ctx["B"], ctx["N"], ctx["NvS"], ctx["R"]
-    shapes = {
-        "dst": (N,), "experts_to_copy": (R, B), "zero_fill_ranges": (E + B, 2), "remote_stats": (2,),
-        "dup_groups": (NvS, 3), "dup_loffs": (NvS,), "dup_counts": (2,), "src_info": (NvS,), "link": (NvS,),
-    }  # fmt: skip
+    shapes = _field_shapes(plan.N, plan.R, plan.E, plan.B, plan.NvS)
     device = torch.device(device)
-    for name, shape in shapes.items():
-        t = getattr(plan, name)
+    pack = getattr(plan, "_pack", None)
+    if pack is not None:  # fields not used so far are views yet to be made, in the layout of these sizes
+        assert pack.base.device == device, "plan is on the wrong device"
+        items = list(pack.made.items())
+    else:
+        items = [(name, getattr(plan, name)) for name in _FIELDS]
+    for name, t in items:
         if t is None:  # the two optional trailing fields
             continue
         assert t.dtype == torch.int32 and t.is_contiguous(), f"plan.{name} must be contiguous int32"
-        assert tuple(t.shape) == shape, f"plan.{name} must have shape {shape}, got {tuple(t.shape)}"
+        assert t.shape == shapes[name], f"plan.{name} must have shape {shapes[name]}, got {tuple(t.shape)}"
         assert t.device == device, f"plan.{name} is on the wrong device"
