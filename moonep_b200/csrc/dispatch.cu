@@ -52,6 +52,10 @@ constexpr int kMaxChunkBytes = 16 * 1024;
 constexpr int kExpandVec = 14;   // int4 per lane in flight while a row is expanded (a 14 KB row in two steps)
 constexpr int kExpandCopyWarps = 12;  // warps of an expander CTA that own a shared-memory piece for bulk copies
 constexpr int kExpandSlice = 2048;  // rows whose duplicate groups an expander CTA lists in shared memory at a time
+// Expander CTAs are dealt the rows of the shard this many at a time, in turn.  A token's copies are made where its primary row
+// is listed, and top-k order puts most primary rows into the experts that most tokens like best: with a contiguous share of
+// the shard each, the CTAs whose shares were those experts made nearly all copies.
+constexpr int kExpandDeal = 4;
 
 // Base addresses of every rank's shard and meta chunk, copied into shared memory at kernel start: the copy loops
 // look them up per destination, and a lookup in global memory is a dependent load of several hundred nanoseconds.
@@ -785,6 +789,14 @@ __device__ bool expand_as_rows_arrive(const MoonepDevCtx& c, const DispatchArgs&
   return true;
 }
 
+// Row i of the share of expander CTA xidx of xcnt, and the size of a share of n rows (its last rows may lie past n).
+__device__ __forceinline__ int dealt_row(int i, int xidx, int xcnt) {
+  return (i / kExpandDeal * xcnt + xidx) * kExpandDeal + i % kExpandDeal;
+}
+__device__ __forceinline__ int dealt_rows(int n, int xcnt) {
+  return (n + kExpandDeal * xcnt - 1) / (kExpandDeal * xcnt) * kExpandDeal;
+}
+
 // xidx of xcnt expander CTAs.  Returns false after a failed wait.
 //
 // With a.expand_bulk the copies go through shared memory with bulk copies: warps 0..kExpandCopyWarps-1 own one piece
@@ -836,17 +848,16 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
       if (a.plan_src_info != nullptr) a.plan_src_info[loff] = -1;
       if (a.plan_link != nullptr) a.plan_link[loff] = 0;
     }
-    const int per_cta = (used + xcnt - 1) / xcnt;
-    const int lo = xidx * per_cta, hi = min(used, lo + per_cta);
-    for (int s0 = lo; s0 < hi && ok; s0 += kExpandSlice) {
-      const int s1 = min(hi, s0 + kExpandSlice);
+    const int share = dealt_rows(used, xcnt);
+    for (int s0 = 0; s0 < share && ok; s0 += kExpandSlice) {
+      const int s1 = min(share, s0 + kExpandSlice);
       if (threadIdx.x == 0) s_ngroups = 0;
       __syncthreads();
       for (int base = s0; base < s1; base += blockDim.x) {  // uniform trip count: the ballots need whole warps
-        const int loff = base + threadIdx.x;
+        const int loff = dealt_row(base + threadIdx.x, xidx, xcnt);
         int dup_n = 0, first = -1;
         bool single = false;  // a primary row without duplicates whose token lives on this rank
-        if (loff < s1) {
+        if (base + (int)threadIdx.x < s1 && loff < used) {
           const int si = src_info[loff];
           const int l = si >= 0 ? link[loff] : 0;
           if (a.plan_src_info != nullptr) a.plan_src_info[loff] = si;
@@ -934,14 +945,15 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
     if (a.local_rows && a.plan_src_info != nullptr && a.plan_link != nullptr) {
       // the lone primary rows of this rank's own tokens: found in the plan's copy of the link words, a slice of rows
       // per CTA and round
-      const int per_cta = (NvS + xcnt - 1) / xcnt;
-      const int lo = xidx * per_cta, hi = min(NvS, lo + per_cta);
-      for (int s0 = lo; s0 < hi && ok; s0 += kExpandSlice) {
-        const int s1 = min(hi, s0 + kExpandSlice);
+      const int share = dealt_rows(NvS, xcnt);
+      for (int s0 = 0; s0 < share && ok; s0 += kExpandSlice) {
+        const int s1 = min(share, s0 + kExpandSlice);
         __syncthreads();
         if (threadIdx.x == 0) s_ngroups = 0;
         __syncthreads();
-        for (int loff = s0 + threadIdx.x; loff < s1; loff += blockDim.x) {
+        for (int i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
+          const int loff = dealt_row(i, xidx, xcnt);
+          if (loff >= NvS) continue;
           const int si = a.plan_src_info[loff];
           const int l = si >= 0 ? a.plan_link[loff] : 0;
           if (si >= 0 && (l & MOONEP_LINK_PRIMARY) && !(l & MOONEP_LINK_HAS_NEXT) && si / NvS == c.rank)
