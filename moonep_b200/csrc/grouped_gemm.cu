@@ -122,9 +122,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    // ---------------- MMA issuer: the whole warp waits, one lane issues ----------------
+    {
       constexpr unsigned idesc = make_idesc(BM, BN);
+      // descriptors of stage 0; those of another lie a stage's bytes further, in 16-byte units
+      const unsigned long long adesc0 = make_smem_desc(s_tiles), bdesc0 = make_smem_desc(s_tiles + kATileBytes);
       int stage = 0;
       unsigned phase = 0;
       unsigned tphase[2] = {0, 0};
@@ -132,36 +134,37 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       bool failed = false;
       for (long long t = blockIdx.x; t < num_tiles && !failed; t += gridDim.x, ++it) {
         const int buf = it & 1;
-        if (!mbar_wait(s_tempty + buf, tphase[buf] ^ 1u, a.timeout_ns)) {
-          gemm_fail(a.status, 13, 2, buf, it);
+        if (!mbar_wait_warp(s_tempty + buf, tphase[buf] ^ 1u, a.timeout_ns)) {
+          if (lane == 0) gemm_fail(a.status, 13, 2, buf, it);
           break;
         }
         tphase[buf] ^= 1u;
-        tc_fence_after();
         const unsigned d_tmem = tmem_base + (unsigned)(buf * BN);
         for (int kb = 0; kb < a.k_blocks; ++kb) {
-          if (!mbar_wait(s_full + stage, phase, a.timeout_ns)) {
-            gemm_fail(a.status, 13, 3, stage, kb);
+          if (!mbar_wait_warp(s_full + stage, phase, a.timeout_ns)) {
+            if (lane == 0) gemm_fail(a.status, 13, 3, stage, kb);
             failed = true;
             break;
           }
           tc_fence_after();
-          const unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
-          const unsigned long long adesc = make_smem_desc(st);
-          const unsigned long long bdesc = make_smem_desc(st + kATileBytes);
+          const unsigned long long off = (unsigned long long)(stage * (int)(kStageBytes >> 4));
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            // 16 bf16 = 32 bytes further along K inside the swizzled 128-byte rows
-            umma_bf16(d_tmem, adesc + (unsigned long long)(kk * 2), bdesc + (unsigned long long)(kk * 2), idesc,
-                      (kb | kk) != 0 ? 1u : 0u);
+            for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+              // 16 bf16 = 32 bytes further along K inside the swizzled 128-byte rows
+              umma_bf16(d_tmem, adesc0 + off + (unsigned long long)(kk * kDescStepK), bdesc0 + off + (unsigned long long)(kk * kDescStepK),
+                        idesc, (kb | kk) != 0 ? 1u : 0u);
+            }
+            umma_commit(s_empty + stage);
           }
-          umma_commit(s_empty + stage);
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (!failed) umma_commit(s_tfull + buf);
+        if (!failed && elect_one()) umma_commit(s_tfull + buf);
+        __syncwarp();
       }
     }
     __syncwarp();
@@ -287,9 +290,9 @@ extern "C" int moonep_grouped_gemm(const void* x, const void* w0, const void* w1
   CUtensorMap ta, tb0, tb1;
   if (int rc = make_tmap(&ta, x, (unsigned long long)rows_cap, (unsigned long long)K, BM)) return rc;
   if (int rc = make_tmap(&tb0, w0, (unsigned long long)w_slots * n_per_group, (unsigned long long)K, 128)) return rc;
-  if (int rc = make_tmap(&tb1, mode == kSwiglu ? w1 : w0, (unsigned long long)w_slots * n_per_group,
-                         (unsigned long long)K, 128))
-    return rc;
+  tb1 = tb0;
+  if (mode == kSwiglu)
+    if (int rc = make_tmap(&tb1, w1, (unsigned long long)w_slots * n_per_group, (unsigned long long)K, 128)) return rc;
   GemmArgs a;
   a.out = (uint16_t*)out;
   a.row_scale = row_scale;

@@ -278,11 +278,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer (leader only) ----------------
-    if (lane == 0 && rank == 0 && tmem_ok) {
-      constexpr unsigned idesc = make_idesc(2 * BM, BN);
-      constexpr unsigned idesc_kn = make_idesc(2 * BM, BN, false, true);
+    // ---------------- MMA issuer (leader only): the whole warp waits, one lane issues ----------------
+    // The rate of this warp bounds the kernel where K is long: as code of one lane it took 685 clocks per K block, whose MMAs
+    // take 512, with and without the loads running.  8 groups x 1024 rows, K=7168, N=2048, before and after: plain 194 and 168
+    // us, SwiGLU with pre-activations 354 and 315; 1 x 16384, K=N=4096: 376 and 332.
+    if (rank == 0 && tmem_ok) {
+      const unsigned idesc = a.b_kn ? make_idesc(2 * BM, BN, false, true) : make_idesc(2 * BM, BN);
       const unsigned bstep = a.b_kn ? kDescStepMn : kDescStepK;
+      // descriptors of stage 0; those of another lie a stage's bytes further, in 16-byte units
+      const unsigned long long adesc0 = make_smem_desc(s_tiles);
+      const unsigned long long bdesc0 = a.b_kn ? make_smem_desc_mn(s_tiles + kPairATileBytes) : make_smem_desc(s_tiles + kPairATileBytes);
       PairSched sched(a, cu);
       int stage = 0;
       unsigned phase = 0;
@@ -292,39 +297,42 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       int pig, nb;
       for (long long t = pair; !failed && sched.locate(t, pig, nb); t += npairs, ++it) {
         const int buf = it & 1;
-        if (!mbar_wait_cluster(s_tempty + buf, tphase[buf] ^ 1u, pipe_timeout_ns)) {
-          gemm_fail(a.status, kPairKernelId, 2, buf, it);
+        if (!mbar_wait_warp(s_tempty + buf, tphase[buf] ^ 1u, pipe_timeout_ns)) {
+          if (lane == 0) gemm_fail(a.status, kPairKernelId, 2, buf, it);
           failed = true;
           break;
         }
         tphase[buf] ^= 1u;
-        tc_fence_after();
         const unsigned d_tmem = tmem_base + (unsigned)(buf * BN);
         for (int kb = 0; kb < a.k_blocks; ++kb) {
-          if (!mbar_wait_cluster(s_full + stage, phase, pipe_timeout_ns)) {
-            gemm_fail(a.status, kPairKernelId, 3, stage, kb);
+          if (!mbar_wait_warp(s_full + stage, phase, pipe_timeout_ns)) {
+            if (lane == 0) gemm_fail(a.status, kPairKernelId, 3, stage, kb);
             failed = true;
             break;
           }
           tc_fence_after();
-          const unsigned char* st = s_tiles + (size_t)stage * kPairStageBytes;
-          const unsigned long long adesc = make_smem_desc(st);
-          const unsigned long long bdesc = a.b_kn ? make_smem_desc_mn(st + kPairATileBytes) : make_smem_desc(st + kPairATileBytes);
+          const unsigned long long off = (unsigned long long)(stage * (int)(kPairStageBytes >> 4));
+          const unsigned long long adesc = adesc0 + off, bdesc = bdesc0 + off;
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BK / UMMA_K; ++kk)
-            umma_bf16_pair(d_tmem, adesc + (unsigned long long)(kk * kDescStepK), bdesc + (unsigned long long)(kk * bstep),
-                           a.b_kn ? idesc_kn : idesc, (kb | kk) != 0 ? 1u : 0u);
-          umma_commit_pair(s_empty + stage, 3);
+            for (int kk = 0; kk < BK / UMMA_K; ++kk)
+              umma_bf16_pair(d_tmem, adesc + (unsigned long long)(kk * kDescStepK), bdesc + (unsigned long long)(kk * bstep), idesc,
+                             (kb | kk) != 0 ? 1u : 0u);
+            umma_commit_pair(s_empty + stage, 3);
+          }
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (!failed) umma_commit_pair(s_tfull + buf, 3);
+        if (!failed && elect_one()) umma_commit_pair(s_tfull + buf, 3);
+        __syncwarp();
       }
       // the pair must not be torn down under a running MMA: wait for everything issued so far
-      umma_commit_pair(&s_done, 1);
-      if (!mbar_wait_cluster(&s_done, 0, pipe_timeout_ns)) gemm_fail(a.status, kPairKernelId, 5, 0, 0);
+      if (elect_one()) umma_commit_pair(&s_done, 1);
+      __syncwarp();
+      if (!mbar_wait_warp(&s_done, 0, pipe_timeout_ns) && lane == 0) gemm_fail(a.status, kPairKernelId, 5, 0, 0);
     }
     __syncwarp();
   } else {
@@ -484,9 +492,9 @@ extern "C" int moonep_grouped_gemm_pair_hooked(const void* x, const void* w0, co
   CUtensorMap ta, tb0, tb1;
   if (int rc = make_tmap(&ta, x, (unsigned long long)rows_cap, (unsigned long long)K, BM)) return rc;
   if (int rc = make_tmap(&tb0, w0, (unsigned long long)w_slots * n_per_group, (unsigned long long)K, 128)) return rc;
-  if (int rc = make_tmap(&tb1, mode == kSwiglu ? w1 : w0, (unsigned long long)w_slots * n_per_group,
-                         (unsigned long long)K, 128))
-    return rc;
+  tb1 = tb0;
+  if (mode == kSwiglu)
+    if (int rc = make_tmap(&tb1, w1, (unsigned long long)w_slots * n_per_group, (unsigned long long)K, 128)) return rc;
   GemmArgs a;
   a.out = (uint16_t*)out;
   a.row_scale = row_scale;
@@ -529,8 +537,9 @@ extern "C" int moonep_grouped_gemm_pair_kn(const void* x, const void* w0, int K0
   CUtensorMap ta, tb0, tb1;
   if (int rc = make_tmap(&ta, x, (unsigned long long)rows_cap, (unsigned long long)(K0 + K1), BM)) return rc;
   if (int rc = make_tmap(&tb0, w0, (unsigned long long)w_slots * K0, (unsigned long long)N, 64)) return rc;
-  if (int rc = make_tmap(&tb1, K1 ? w1 : w0, (unsigned long long)w_slots * (K1 ? K1 : K0), (unsigned long long)N, 64))
-    return rc;
+  tb1 = tb0;
+  if (K1)
+    if (int rc = make_tmap(&tb1, w1, (unsigned long long)w_slots * K1, (unsigned long long)N, 64)) return rc;
   GemmArgs a;
   a.out = (uint16_t*)out;
   a.row_scale = nullptr;

@@ -20,8 +20,9 @@
 // 64 rows; the last tile of an odd P is 128 x 128): moonep_wgrad_single_cta.
 //
 // Bound by the tensor pipe and the fp32 results together: a tile of 1024 rows is 16 K blocks of MMAs and 256 KB of output.
-// 8 groups x 1024 rows, 2048 x 7168: pairs 239 us (1006 TFLOP/s), single CTAs 256; adding to the old values 258 and 296;
-// 16 groups x 512 rows, 1024 x 2048: 47 and 53.  What an accumulator waits for before it is used again is only that TMEM has
+// 8 groups x 1024 rows, 2048 x 7168: 205 us (1174 TFLOP/s), adding to the old values 235; 16 groups x 512 rows, 1024 x 2048:
+// 43.  With the MMAs issued by a lane on its own instead of an elected lane of a warp that stays together: 239, 253, 47 (and
+// single CTAs 256, 296, 53).  What an accumulator waits for before it is used again is only that TMEM has
 // been read (mbar_arrive_cluster): as long as the arrive also waited for the stores to reach L2, groups of 128 rows took 38.6
 // us where they take 32.2 (16 groups, 1024 x 2048).  (Lanes along P, 32-byte stores: 236, 369, 57.7; results through shared
 // memory in 512-byte bulk stores: 242 and 50 in a training step, an SM takes 15 clocks per bulk store.)
@@ -226,10 +227,15 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap* tmap_l, const CUte
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer (leader only) ----------------
-    if (lane == 0 && rank == 0 && tmem_ok) {
+    // ---------------- MMA issuer (leader only): the whole warp waits, one lane issues ----------------
+    if (rank == 0 && tmem_ok) {
       constexpr int M = kPair ? 2 * BM : BM;
       const unsigned kstep = a.row_major ? kDescStepMn : kDescStepK;
+      const unsigned idesc_full = make_idesc(M, BN, a.row_major != 0, a.row_major != 0);
+      const unsigned idesc_half = make_idesc(M, 128, a.row_major != 0, a.row_major != 0);
+      // descriptors of stage 0; those of another lie a stage's bytes further, in 16-byte units
+      const unsigned long long adesc0 = a.row_major ? make_smem_desc_mn(s_tiles) : make_smem_desc(s_tiles);
+      const unsigned long long bdesc0 = a.row_major ? make_smem_desc_mn(s_tiles + kHalfBytes) : make_smem_desc(s_tiles + kHalfBytes);
       int stage = 0;
       unsigned phase = 0;
       unsigned tphase[2] = {0, 0};
@@ -240,46 +246,51 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap* tmap_l, const CUte
         if (w.krows == 0 || w.out == nullptr) continue;
         const int buf = it & 1;
         ++it;
-        if (!mbar_wait_cluster(s_tempty + buf, tphase[buf] ^ 1u, a.timeout_ns)) {
-          gemm_fail(a.status, 14, 2, buf, it);
+        if (!mbar_wait_warp(s_tempty + buf, tphase[buf] ^ 1u, a.timeout_ns)) {
+          if (lane == 0) gemm_fail(a.status, 14, 2, buf, it);
           break;
         }
         tphase[buf] ^= 1u;
-        tc_fence_after();
         const unsigned d_tmem = tmem_base + (unsigned)(buf * BN);
         const int kbs = (w.krows + BK - 1) / BK;
-        const bool half = !kPair && a.P - w.pb * BN < BN;  // the last tile of an odd P
-        const unsigned idesc = a.row_major ? (half ? make_idesc(M, 128, true, true) : make_idesc(M, BN, true, true))
-                                           : (half ? make_idesc(M, 128) : make_idesc(M, BN));
+        const unsigned idesc = !kPair && a.P - w.pb * BN < BN ? idesc_half : idesc_full;  // half: the last tile of an odd P
         for (int kb = 0; kb < kbs; ++kb) {
-          if (!mbar_wait_cluster(s_full + stage, phase, a.timeout_ns)) {
-            gemm_fail(a.status, 14, 3, stage, kb);
+          if (!mbar_wait_warp(s_full + stage, phase, a.timeout_ns)) {
+            if (lane == 0) gemm_fail(a.status, 14, 3, stage, kb);
             failed = true;
             break;
           }
           tc_fence_after();
-          const unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
-          const unsigned long long adesc = a.row_major ? make_smem_desc_mn(st) : make_smem_desc(st);
-          const unsigned long long bdesc = a.row_major ? make_smem_desc_mn(st + kHalfBytes) : make_smem_desc(st + kHalfBytes);
-          const int nkk = min(BK / UMMA_K, (w.krows - kb * BK) / UMMA_K);  // MMAs inside the group
-          for (int kk = 0; kk < nkk; ++kk) {
-            const unsigned long long ad = adesc + (unsigned long long)(kk * kstep), bd = bdesc + (unsigned long long)(kk * kstep);
-            const unsigned add = (kb | kk) != 0 ? 1u : 0u;
-            if (kPair) umma_bf16_pair(d_tmem, ad, bd, idesc, add); else umma_bf16(d_tmem, ad, bd, idesc, add);
+          const unsigned long long off = (unsigned long long)(stage * (int)(kStageBytes >> 4));
+          const unsigned long long adesc = adesc0 + off, bdesc = bdesc0 + off;
+          const int left = w.krows - kb * BK;
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+              if (kk * UMMA_K >= left) break;  // MMAs inside the group
+              const unsigned long long ad = adesc + (unsigned long long)(kk * kstep), bd = bdesc + (unsigned long long)(kk * kstep);
+              const unsigned add = (kb | kk) != 0 ? 1u : 0u;
+              if (kPair) umma_bf16_pair(d_tmem, ad, bd, idesc, add); else umma_bf16(d_tmem, ad, bd, idesc, add);
+            }
+            if (kPair) umma_commit_pair(s_empty + stage, 3); else umma_commit(s_empty + stage);
           }
-          if (kPair) umma_commit_pair(s_empty + stage, 3); else umma_commit(s_empty + stage);
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (!failed) {
+        if (!failed && elect_one()) {
           if (kPair) umma_commit_pair(s_tfull + buf, 3); else umma_commit(s_tfull + buf);
         }
+        __syncwarp();
       }
       // nothing may be torn down under a running MMA: wait for everything issued so far
-      if (kPair) umma_commit_pair(&s_done, 1); else umma_commit(&s_done);
-      if (!mbar_wait_cluster(&s_done, 0, a.timeout_ns)) gemm_fail(a.status, 14, 5, 0, 0);
+      if (elect_one()) {
+        if (kPair) umma_commit_pair(&s_done, 1); else umma_commit(&s_done);
+      }
+      __syncwarp();
+      if (!mbar_wait_warp(&s_done, 0, a.timeout_ns) && lane == 0) gemm_fail(a.status, 14, 5, 0, 0);
     }
     __syncwarp();
   } else {

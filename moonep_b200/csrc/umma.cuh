@@ -65,6 +65,20 @@ __device__ __forceinline__ void tmem_dealloc(unsigned taddr, unsigned ncols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// True in one lane of a whole warp, the same one every time.  MMAs are issued under it and not under `lane == 0`: the warp
+// stays together up to the issue, so that descriptors and barriers are the warp's common values, which the instructions want.
+__device__ __forceinline__ bool elect_one() {
+  unsigned p;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void umma_bf16(unsigned d_tmem, unsigned long long adesc, unsigned long long bdesc,
                                           unsigned idesc, unsigned accumulate) {
   asm volatile(
@@ -209,6 +223,16 @@ __device__ __forceinline__ bool mbar_wait_cluster(unsigned long long* bar, unsig
   while (!mbar_try_wait_cluster(bar, parity)) {
     if ((++spins & 255u) == 0 && globaltimer_ns() - t0 > timeout_ns) return false;
   }
+  return true;
+}
+
+// The same for a whole warp, which goes on together.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long* bar, unsigned parity, unsigned long long timeout_ns) {
+  if (__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity))) return true;
+  const unsigned long long t0 = globaltimer_ns();
+  unsigned spins = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity)))
+    if ((++spins & 255u) == 0 && __any_sync(0xffffffffu, globaltimer_ns() - t0 > timeout_ns)) return false;
   return true;
 }
 
