@@ -752,15 +752,18 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
   if (tid == 0) {
     a.work[kWorkPads] = 0;
     c.counters[MOONEP_CTR_DISPATCH_ARRIVE] = 0;
-    fence_sys();
     if (run && ok && !poisoned(c)) {
+      // whoever reads these is on this GPU: one fence for all of them (a release at system scope each held the kernel's end
+      // back by several microseconds)
+      const int plan_epoch = abs_epoch(c, MOONEP_FLAG_PLAN, a.epoch_plan), tpe_epoch = abs_epoch(c, MOONEP_FLAG_TPE, a.epoch_tpe);
+      const int sent_epoch = abs_epoch(c, MOONEP_FLAG_SENT, a.epoch_sent);
+      fence_gpu();
       if (a.fresh) {
-        const int plan_epoch = abs_epoch(c, MOONEP_FLAG_PLAN, a.epoch_plan);
-        st_release_gpu(c.counters + MOONEP_CTR_PLAN_DONE, plan_epoch);
-        st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_TPE, 0), abs_epoch(c, MOONEP_FLAG_TPE, a.epoch_tpe));
-        st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_PLAN, 0), plan_epoch);
+        st_relaxed_gpu(c.counters + MOONEP_CTR_PLAN_DONE, plan_epoch);
+        st_relaxed_sys(flag_ptr(c, 0, MOONEP_FLAG_TPE, 0), tpe_epoch);
+        st_relaxed_sys(flag_ptr(c, 0, MOONEP_FLAG_PLAN, 0), plan_epoch);
       }
-      st_release_sys(flag_ptr(c, 0, MOONEP_FLAG_SENT, 0), abs_epoch(c, MOONEP_FLAG_SENT, a.epoch_sent));
+      st_relaxed_sys(flag_ptr(c, 0, MOONEP_FLAG_SENT, 0), sent_epoch);
     }
   }
 }

@@ -48,7 +48,10 @@ struct BiasValues {
   int v[MOONEP_NUM_FLAG_FAMILIES];
 };
 
+// A step of one decode batch is as short as a few launches, so this one is launched like the kernels it follows
+// (enable_pdl) and is in place when they end.
 __global__ void epoch_bias_kernel(const MoonepDevCtx c, const BiasValues b, int mode) {
+  griddep_wait();
   const int f = threadIdx.x;
   if (f < MOONEP_NUM_FLAG_FAMILIES) c.counters[MOONEP_BIAS_OFF + f] = (mode ? c.counters[MOONEP_BIAS_OFF + f] : 0) + b.v[f];
 }
@@ -547,7 +550,9 @@ extern "C" int moonep_epoch_bias(void* ctx, const int* values, int mode, void* s
   auto* h = (HostCtx*)ctx;
   BiasValues b;
   for (int f = 0; f < MOONEP_NUM_FLAG_FAMILIES; ++f) b.v[f] = values[f];
-  epoch_bias_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(h->dev, b, mode);
+  if (int rc = check_cuda(launch_maybe_pdl(epoch_bias_kernel, 1, 32, 0, (cudaStream_t)stream, h->enable_pdl != 0, h->dev, b, mode),
+                          "launch epoch_bias_kernel"))
+    return rc;
   return check_launch("epoch_bias_kernel");
 }
 
