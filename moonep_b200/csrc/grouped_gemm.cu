@@ -68,6 +68,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     tmem_alloc(&s_tmem_base, kTmemCols);
     tmem_relinquish();
   }
+  griddep_wait();  // what the kernels before wrote is read from here on
+  griddep_launch();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -326,6 +328,9 @@ extern "C" int moonep_grouped_gemm(const void* x, const void* w0, const void* w1
       return rc;
     attr_set = true;
   }
-  grouped_gemm_kernel<<<grid, kGemmThreads, smem, (cudaStream_t)stream>>>(ta, tb0, tb1, a);
+  if (int rc = check_cuda(launch_maybe_pdl(grouped_gemm_kernel, grid, kGemmThreads, smem, (cudaStream_t)stream, expert_pdl(num_sms), ta, tb0,
+                                           tb1, a),
+                          "launch grouped_gemm_kernel"))
+    return rc;
   return check_launch("grouped_gemm_kernel");
 }

@@ -59,6 +59,12 @@ constexpr size_t kPairSmem = (size_t)kStages * kPairStageBytes + 1024 + 4 * kPai
 constexpr int kPairKernelId = 15;
 constexpr int kPairGroupsInSmem = 2048;  // group ends are walked from shared memory up to this many groups
 
+// A launch that waits for, or is waited for by, the communication kernels keeps the next kernel off the SMs until it ends: they
+// may still be needed by the kernels it waits for.
+__host__ __device__ inline bool has_hooks(const MoonepGemmHooks& h) {
+  return h.row_flags != nullptr || h.tables_ready != nullptr || h.slot_flags != nullptr || h.done_counter != nullptr;
+}
+
 // Walks the pair tiles in order: group-major, then pairs of row blocks, then column tiles (fastest).
 struct PairSched {
   const GemmArgs& a;
@@ -135,7 +141,7 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, const void
                : "memory");
 }
 
-template <int kStages, int kCols>
+template <int kStages, int kCols, bool kKn>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                              const __grid_constant__ CUtensorMap tmap_b1, const __grid_constant__ CUtensorMap tmap_o,
@@ -150,6 +156,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   const unsigned rank = cluster_ctarank();  // 0: leader (issues the MMAs), 1: its peer
   // every role walks the groups once; from shared memory a group costs a few cycles instead of an L2 round trip
   const int* cu = a.G <= kPairGroupsInSmem ? s_cu : a.cu_seqlens;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(s_full + s, 1);   // used in the leader: its own arrive.expect_tx; both CTAs' copies complete the bytes
+      mbar_init(s_empty + s, 1);  // one commit of the leader's MMA lane, delivered to both CTAs
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(s_tfull + b, 1);   // one commit, delivered to both CTAs
+      mbar_init(s_tempty + b, 8);  // used in the leader: four epilogue warps of each CTA
+    }
+    mbar_init(&s_done, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&s_tmem_base, kPairTmemCols);
+    tmem_relinquish();
+  }
+  griddep_wait();  // what the kernels before wrote is read from here on
+  if (!has_hooks(a.hooks)) griddep_launch();
   __shared__ int s_hook_ok;
   if (threadIdx.x == 0) {
     s_hook_ok = 1;
@@ -169,22 +193,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     }
   const long long pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(s_full + s, 1);   // used in the leader: its own arrive.expect_tx; both CTAs' copies complete the bytes
-      mbar_init(s_empty + s, 1);  // one commit of the leader's MMA lane, delivered to both CTAs
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(s_tfull + b, 1);   // one commit, delivered to both CTAs
-      mbar_init(s_tempty + b, 8);  // used in the leader: four epilogue warps of each CTA
-    }
-    mbar_init(&s_done, 1);
-    fence_barrier_init();
-  }
-  if (warp == 1) {
-    tmem_alloc(&s_tmem_base, kPairTmemCols);
-    tmem_relinquish();
-  }
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // the peer's barriers exist before anything is delivered to them
@@ -213,8 +221,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       int checked_blk = -1, checked_slot = -1;
       for (long long t = pair; !failed && sched.locate(t, pig, nb); t += npairs) {
         const int blk = sched.blk0 + 2 * pig + (int)rank;
-        const int row0 = blk * BM;  // beyond the group for the odd last block: loaded, never stored
-        if (a.hooks.row_flags != nullptr && 2 * pig + (int)rank < sched.nblk && blk != checked_blk) {
+        // An odd last block leaves the second CTA without rows: its tile is filled with zeros (a box past the end of X), which
+        // costs neither loads nor, nearly, power, and the clock under a long step is set by power.
+        const bool mine = 2 * pig + (int)rank < sched.nblk;
+        const int row0 = mine ? blk * BM : a.rows_cap;
+        if (a.hooks.row_flags != nullptr && mine && blk != checked_blk) {
           if (!rows_arrived(a.hooks, row0, lane, a.timeout_ns)) {
             if (lane == 0) gemm_fail(a.status, kPairKernelId, 11, blk, sched.g);
             failed = true;
@@ -256,7 +267,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             if (rank == 0) mbar_expect_tx(s_full + stage, 2 * kPairStageBytes);
             const unsigned full_of_leader = mapa_u32(s_full + stage, 0);
             tma_load_2d_pair(st, &tmap_a, kb * BK, row0, full_of_leader);
-            if (a.b_kn) {
+            if constexpr (kKn) {
               // W is [slots, K, N]: this CTA's 128 columns of the tile as two boxes of 64 columns x 64 k
               const bool second = kb >= a.k_split;
               const int kdim = (second ? a.k_blocks - a.k_split : a.k_split) * BK;  // K rows per expert in that tensor
@@ -283,11 +294,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     // take 512, with and without the loads running.  8 groups x 1024 rows, K=7168, N=2048, before and after: plain 194 and 168
     // us, SwiGLU with pre-activations 354 and 315; 1 x 16384, K=N=4096: 376 and 332.
     if (rank == 0 && tmem_ok) {
-      const unsigned idesc = a.b_kn ? make_idesc(2 * BM, BN, false, true) : make_idesc(2 * BM, BN);
-      const unsigned bstep = a.b_kn ? kDescStepMn : kDescStepK;
+      constexpr unsigned idesc = make_idesc(2 * BM, BN, false, kKn);
+      constexpr unsigned bstep = kKn ? kDescStepMn : kDescStepK;
       // descriptors of stage 0; those of another lie a stage's bytes further, in 16-byte units
       const unsigned long long adesc0 = make_smem_desc(s_tiles);
-      const unsigned long long bdesc0 = a.b_kn ? make_smem_desc_mn(s_tiles + kPairATileBytes) : make_smem_desc(s_tiles + kPairATileBytes);
+      const unsigned long long bdesc0 = kKn ? make_smem_desc_mn(s_tiles + kPairATileBytes) : make_smem_desc(s_tiles + kPairATileBytes);
       PairSched sched(a, cu);
       int stage = 0;
       unsigned phase = 0;
@@ -381,7 +392,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
           if (++piece == kPairPieces) piece = 0;
         };
         constexpr int kLoads = kCols / 32;  // TMEM loads of 32 columns per piece
-        if (a.mode == kSwiglu) {
+        if (!kKn && a.mode == kSwiglu) {
 #pragma unroll 1
           for (int c0 = 0; c0 < 128; c0 += kCols) {
             unsigned g[kLoads][32], u[kLoads][32];
@@ -563,7 +574,7 @@ extern "C" int moonep_grouped_gemm_pair_kn(const void* x, const void* w0, int K0
   return launch_pair(ta, tb0, tb1, a, num_sms, stream);
 }
 
-template <int kStages, int kCols>
+template <int kStages, int kCols, bool kKn>
 static int launch_pair_of(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const GemmArgs& a,
                        int num_sms, void* stream) {
   CUtensorMap to, tg, tu;
@@ -573,21 +584,27 @@ static int launch_pair_of(const CUtensorMap& ta, const CUtensorMap& tb0, const C
     if (int rc = make_tmap(&tg, a.pre_gate, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32, 0, kCols)) return rc;
     if (int rc = make_tmap(&tu, a.pre_up, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32, 0, kCols)) return rc;
   }
-  constexpr auto* kernel = grouped_gemm_pair_kernel<kStages, kCols>;
+  constexpr auto* kernel = grouped_gemm_pair_kernel<kStages, kCols, kKn>;
   constexpr size_t smem = kPairSmem<kStages, kCols>;
   static int max_pairs = -1;  // pairs of these CTAs the device runs at once
   if (max_pairs < 0)
     if (int rc = pairs_at_once(kernel, kPairThreads, smem, "grouped_gemm_pair_kernel", &max_pairs)) return rc;
   int pairs = max_pairs;
   if (num_sms > 0) pairs = imax(1, imin(pairs, num_sms / 2));
-  kernel<<<2 * pairs, kPairThreads, smem, (cudaStream_t)stream>>>(ta, tb0, tb1, to, tg, tu, a);
+  if (int rc = check_cuda(launch_maybe_pdl(kernel, 2 * pairs, kPairThreads, smem, (cudaStream_t)stream,
+                                           !has_hooks(a.hooks) && expert_pdl(num_sms), ta, tb0, tb1, to, tg, tu, a),
+                          "launch grouped_gemm_pair_kernel"))
+    return rc;
   return check_launch("grouped_gemm_pair_kernel");
 }
 
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const GemmArgs& a,
                        int num_sms, void* stream) {
-  return a.k_blocks <= 1024 / BK ? launch_pair_of<5, 64>(ta, tb0, tb1, a, num_sms, stream)
-                                 : launch_pair_of<6, 32>(ta, tb0, tb1, a, num_sms, stream);
+  if (a.b_kn)
+    return a.k_blocks <= 1024 / BK ? launch_pair_of<5, 64, true>(ta, tb0, tb1, a, num_sms, stream)
+                                   : launch_pair_of<6, 32, true>(ta, tb0, tb1, a, num_sms, stream);
+  return a.k_blocks <= 1024 / BK ? launch_pair_of<5, 64, false>(ta, tb0, tb1, a, num_sms, stream)
+                                 : launch_pair_of<6, 32, false>(ta, tb0, tb1, a, num_sms, stream);
 }
 
 // Host-side walk of the tile schedule of one CTA pair (for tests): writes, for every tile that pair `pair` of

@@ -143,8 +143,6 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap* tmap_l, const CUte
   unsigned char* s_tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned rank = kPair ? cluster_ctarank() : 0;  // 0: leader (issues the MMAs), 1: its peer
-  if (warp == 0) wgrad_list_groups(a, s_groups, lane);
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(s_full + s, 1);   // used in the leader: its own arrive.expect_tx; both CTAs' copies complete the bytes
@@ -161,6 +159,9 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap* tmap_l, const CUte
     tmem_alloc(&s_tmem_base, kTmemCols);
     tmem_relinquish();
   }
+  griddep_wait();  // what the kernels before wrote is read from here on
+  griddep_launch();
+  if (warp == 0) wgrad_list_groups(a, s_groups, lane);
   tc_fence_before();
   __syncthreads();
   if (kPair) cluster_sync_all();  // the peer's barriers exist before anything is delivered to them
@@ -392,7 +393,10 @@ static int launch_single(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs
   }
   a.q_tiles = a.Q / 128;
   const int grid = num_sms > 0 ? imin(num_sms, sms) : sms;
-  grouped_wgrad_single_kernel<<<grid, kThreads, kSmemBytes, (cudaStream_t)stream>>>(tl, tr, a);
+  if (int rc = check_cuda(launch_maybe_pdl(grouped_wgrad_single_kernel, grid, kThreads, kSmemBytes, (cudaStream_t)stream,
+                                           expert_pdl(num_sms), tl, tr, a),
+                          "launch grouped_wgrad_single_kernel"))
+    return rc;
   return check_launch("grouped_wgrad_single_kernel");
 }
 
@@ -416,7 +420,10 @@ static int launch_wgrad(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs&
     if (int rc = pairs_at_once(grouped_wgrad_kernel, kThreads, kSmemBytes, "grouped_wgrad_kernel", &max_pairs)) return rc;
   int pairs = max_pairs;
   if (num_sms > 0) pairs = imin(pairs, num_sms / 2);
-  grouped_wgrad_kernel<<<2 * pairs, kThreads, kSmemBytes, (cudaStream_t)stream>>>(tl, tr, a);
+  if (int rc = check_cuda(launch_maybe_pdl(grouped_wgrad_kernel, 2 * pairs, kThreads, kSmemBytes, (cudaStream_t)stream,
+                                           expert_pdl(num_sms), tl, tr, a),
+                          "launch grouped_wgrad_kernel"))
+    return rc;
   return check_launch("grouped_wgrad_kernel");
 }
 

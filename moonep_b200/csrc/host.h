@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cstdlib>
+#include <cstring>
 #include <string>
 #include <utility>
 
@@ -48,6 +50,15 @@ inline cudaError_t launch_maybe_pdl(void (*kernel)(KArgs...), int grid, int bloc
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// The kernels of the expert computation are launched the same way unless MOONEP_PDL=0: their barriers and TMEM are set up
+// while the kernel before drains (about 2 us between one and the next otherwise).  Not where they leave SMs to another stream
+// (num_sms > 0): the next kernel in line would take them.
+inline bool expert_pdl(int num_sms) {
+  if (num_sms > 0) return false;
+  const char* v = getenv("MOONEP_PDL");
+  return v == nullptr || !(v[0] == 0 || strcmp(v, "0") == 0 || strcmp(v, "false") == 0 || strcmp(v, "False") == 0);
 }
 
 inline int imin(int a, int b) { return a < b ? a : b; }

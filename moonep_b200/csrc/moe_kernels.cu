@@ -68,6 +68,8 @@ __global__ void __launch_bounds__(256)
                       const float* __restrict__ w, const int* __restrict__ total_rows_ptr, int rows_cap, int I,
                       uint16_t* __restrict__ dadu, uint16_t* __restrict__ hsw, float* __restrict__ dgate) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  griddep_wait();
+  griddep_launch();
   int rows = total_rows_ptr != nullptr ? *total_rows_ptr : rows_cap;
   if (rows > rows_cap) rows = rows_cap;
   for (int r = blockIdx.x * nwarps + warp; r < rows; r += gridDim.x * nwarps) {
@@ -258,8 +260,10 @@ extern "C" int moonep_swiglu_bwd(const void* a, const void* u, const void* g, co
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  swiglu_bwd_kernel<<<imax(1, sms * 4), 256, 0, (cudaStream_t)stream>>>((const uint16_t*)a, (const uint16_t*)u,
-                                                                        (const uint16_t*)g, w, total_rows, rows_cap, I,
-                                                                        (uint16_t*)dadu, (uint16_t*)hsw, dgate);
+  if (int rc = check_cuda(launch_maybe_pdl(swiglu_bwd_kernel, imax(1, sms * 4), 256, 0, (cudaStream_t)stream, expert_pdl(0),
+                                           (const uint16_t*)a, (const uint16_t*)u, (const uint16_t*)g, w, total_rows, rows_cap, I,
+                                           (uint16_t*)dadu, (uint16_t*)hsw, dgate),
+                          "launch swiglu_bwd_kernel"))
+    return rc;
   return check_launch("swiglu_bwd_kernel");
 }
