@@ -210,7 +210,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
-    // Lane 0 issues the copies; the whole warp takes part in the (bounded) waits for rows that the dispatch kernel is
+    // One lane issues the copies; the whole warp takes part in the (bounded) waits, also for rows that the dispatch kernel is
     // still delivering and for weight slots the prefetch kernel is still filling.
     if (tmem_ok) {
       PairSched sched(a, cu);
@@ -255,31 +255,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         const CUtensorMap* tb = (a.mode == kSwiglu && rank == 1) ? &tmap_b1 : &tmap_b0;
         const int brow = (a.mode == kSwiglu) ? wrow0 : wrow0 + (int)rank * 128;
         for (int kb = 0; kb < a.k_blocks; ++kb) {
-          int got = 1;
-          if (lane == 0) got = mbar_wait_cluster(s_empty + stage, phase ^ 1u, pipe_timeout_ns) ? 1 : 0;
-          if (!__shfl_sync(0xffffffffu, got, 0)) {
+          if (!mbar_wait_warp(s_empty + stage, phase ^ 1u, pipe_timeout_ns)) {
             if (lane == 0) gemm_fail(a.status, kPairKernelId, 1, stage, kb);
             failed = true;
             break;
           }
-          if (lane == 0) {
+          if (elect_one()) {
             unsigned char* st = s_tiles + (size_t)stage * kPairStageBytes;
             if (rank == 0) mbar_expect_tx(s_full + stage, 2 * kPairStageBytes);
             const unsigned full_of_leader = mapa_u32(s_full + stage, 0);
             tma_load_2d_pair(st, &tmap_a, kb * BK, row0, full_of_leader);
             if constexpr (kKn) {
-              // W is [slots, K, N]: this CTA's 128 columns of the tile as two boxes of 64 columns x 64 k
+              // W is [slots, K, N]: this CTA's 128 columns of the tile
               const bool second = kb >= a.k_split;
               const int kdim = (second ? a.k_blocks - a.k_split : a.k_split) * BK;  // K rows per expert in that tensor
               const int y = wslot * kdim + (second ? kb - a.k_split : kb) * BK;
-              const int x0 = nb * BN + (int)rank * 128;
-              const CUtensorMap* tw = second ? &tmap_b1 : &tmap_b0;
-              tma_load_2d_pair(st + kPairATileBytes, tw, x0, y, full_of_leader);
-              tma_load_2d_pair(st + kPairATileBytes + kMnBoxBytes, tw, x0 + 64, y, full_of_leader);
+              tma_load_mn_pair(st + kPairATileBytes, second ? &tmap_b1 : &tmap_b0, (nb * BN + (int)rank * 128) / 64, y, full_of_leader);
             } else {
               tma_load_2d_pair(st + kPairATileBytes, tb, kb * BK, brow, full_of_leader);
             }
           }
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -547,10 +543,10 @@ extern "C" int moonep_grouped_gemm_pair_kn(const void* x, const void* w0, int K0
   }
   CUtensorMap ta, tb0, tb1;
   if (int rc = make_tmap(&ta, x, (unsigned long long)rows_cap, (unsigned long long)(K0 + K1), BM)) return rc;
-  if (int rc = make_tmap(&tb0, w0, (unsigned long long)w_slots * K0, (unsigned long long)N, 64)) return rc;
+  if (int rc = make_tmap_mn(&tb0, w0, (unsigned long long)w_slots * K0, (unsigned long long)N)) return rc;
   tb1 = tb0;
   if (K1)
-    if (int rc = make_tmap(&tb1, w1, (unsigned long long)w_slots * K1, (unsigned long long)N, 64)) return rc;
+    if (int rc = make_tmap_mn(&tb1, w1, (unsigned long long)w_slots * K1, (unsigned long long)N)) return rc;
   GemmArgs a;
   a.out = (uint16_t*)out;
   a.row_scale = nullptr;

@@ -20,9 +20,9 @@
 // 64 rows; the last tile of an odd P is 128 x 128): moonep_wgrad_single_cta.
 //
 // Bound by the tensor pipe and the fp32 results together: a tile of 1024 rows is 16 K blocks of MMAs and 256 KB of output.
-// 8 groups x 1024 rows, 2048 x 7168: 205 us (1174 TFLOP/s), adding to the old values 235; 16 groups x 512 rows, 1024 x 2048:
-// 43.  With the MMAs issued by a lane on its own instead of an elected lane of a warp that stays together: 239, 253, 47 (and
-// single CTAs 256, 296, 53).  What an accumulator waits for before it is used again is only that TMEM has
+// 8 groups x 1024 rows, 2048 x 7168: 183 us (1315 TFLOP/s), adding to the old values 224; 16 groups x 512 rows, 1024 x 2048:
+// 41.  With MMAs and loads issued by a lane on its own instead of an elected lane of a warp that stays together: 239, 253, 47
+// (and single CTAs 256, 296, 53).  What an accumulator waits for before it is used again is only that TMEM has
 // been read (mbar_arrive_cluster): as long as the arrive also waited for the stores to reach L2, groups of 128 rows took 38.6
 // us where they take 32.2 (16 groups, 1024 x 2048).  (Lanes along P, 32-byte stores: 236, 369, 57.7; results through shared
 // memory in 512-byte bulk stores: 242 and 50 in a training step, an SM takes 15 clocks per bulk store.)
@@ -175,7 +175,7 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap* tmap_l, const CUte
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
-    if (lane == 0 && tmem_ok) {
+    if (tmem_ok) {
       int stage = 0;
       unsigned phase = 0;
       bool failed = false;
@@ -187,38 +187,38 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap* tmap_l, const CUte
         const int p0 = w.pb * BN + (int)rank * 128;               // of a pair's second CTA it may lie past P: zeros
         const int cols = kPair ? 128 : min(BN, a.P - w.pb * BN);  // columns of L that this CTA stages
         for (int kb = 0; kb < kbs; ++kb) {
-          if (!mbar_wait_cluster(s_empty + stage, phase ^ 1u, a.timeout_ns)) {
-            gemm_fail(a.status, 14, 1, stage, kb);
+          if (!mbar_wait_warp(s_empty + stage, phase ^ 1u, a.timeout_ns)) {
+            if (lane == 0) gemm_fail(a.status, 14, 1, stage, kb);
             failed = true;
             break;
           }
-          unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
-          const int k = w.k0 + kb * BK;
-          if constexpr (kPair) {
-            if (rank == 0) mbar_expect_tx(s_full + stage, 2 * kStageBytes);
-            const unsigned full_of_leader = mapa_u32(s_full + stage, 0);
-            if (a.row_major) {  // boxes of 64 columns x 64 rows, two for R and two for L
-              tma_load_2d_pair(st, tmap_r, q0, k, full_of_leader);
-              tma_load_2d_pair(st + kMnBoxBytes, tmap_r, q0 + 64, k, full_of_leader);
-              tma_load_2d_pair(st + kHalfBytes, tmap_l, p0, k, full_of_leader);
-              tma_load_2d_pair(st + kHalfBytes + kMnBoxBytes, tmap_l, p0 + 64, k, full_of_leader);
+          if (elect_one()) {
+            unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
+            const int k = w.k0 + kb * BK;
+            if constexpr (kPair) {
+              if (rank == 0) mbar_expect_tx(s_full + stage, 2 * kStageBytes);
+              const unsigned full_of_leader = mapa_u32(s_full + stage, 0);
+              if (a.row_major) {
+                tma_load_mn_pair(st, tmap_r, q0 / 64, k, full_of_leader);
+                tma_load_mn_pair(st + kHalfBytes, tmap_l, p0 / 64, k, full_of_leader);
+              } else {
+                tma_load_2d_pair(st, tmap_r, k, q0, full_of_leader);
+                tma_load_2d_pair(st + kHalfBytes, tmap_l, k, p0, full_of_leader);
+              }
             } else {
-              tma_load_2d_pair(st, tmap_r, k, q0, full_of_leader);
-              tma_load_2d_pair(st + kHalfBytes, tmap_l, k, p0, full_of_leader);
-            }
-          } else {
-            mbar_expect_tx(s_full + stage, kHalfBytes + (unsigned)cols * BK * 2);
-            if (a.row_major) {
-              tma_load_2d(st, tmap_r, q0, k, s_full + stage);
-              tma_load_2d(st + kMnBoxBytes, tmap_r, q0 + 64, k, s_full + stage);
-              for (int c = 0; c < cols / 64; ++c)
-                tma_load_2d(st + kHalfBytes + c * kMnBoxBytes, tmap_l, p0 + 64 * c, k, s_full + stage);
-            } else {
-              tma_load_2d(st, tmap_r, k, q0, s_full + stage);
-              for (int c = 0; c < cols / 128; ++c)
-                tma_load_2d(st + (1 + c) * kHalfBytes, tmap_l, k, p0 + 128 * c, s_full + stage);
+              mbar_expect_tx(s_full + stage, kHalfBytes + (unsigned)cols * BK * 2);
+              if (a.row_major) {
+                tma_load_mn(st, tmap_r, q0 / 64, k, s_full + stage);
+                for (int c = 0; c < cols / 128; ++c)
+                  tma_load_mn(st + (1 + c) * kHalfBytes, tmap_l, p0 / 64 + 2 * c, k, s_full + stage);
+              } else {
+                tma_load_2d(st, tmap_r, k, q0, s_full + stage);
+                for (int c = 0; c < cols / 128; ++c)
+                  tma_load_2d(st + (1 + c) * kHalfBytes, tmap_l, k, p0 + 128 * c, s_full + stage);
+              }
             }
           }
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -483,8 +483,8 @@ extern "C" int moonep_grouped_wgrad_rows(const void* l, long long ldl, const voi
     return 1;
   }
   CUtensorMap tl, tr;
-  if (int rc = make_tmap(&tl, l, (unsigned long long)rows, (unsigned long long)P, 64, (unsigned long long)ldl)) return rc;
-  if (int rc = make_tmap(&tr, r, (unsigned long long)rows, (unsigned long long)Q, 64, (unsigned long long)ldr)) return rc;
+  if (int rc = make_tmap_mn(&tl, l, (unsigned long long)rows, (unsigned long long)P, (unsigned long long)ldl)) return rc;
+  if (int rc = make_tmap_mn(&tr, r, (unsigned long long)rows, (unsigned long long)Q, (unsigned long long)ldr)) return rc;
   WgradArgs a;
   a.out_ptrs = (float* const*)out_ptrs;
   a.flags = flags;

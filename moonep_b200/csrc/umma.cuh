@@ -124,7 +124,7 @@ __device__ __forceinline__ unsigned long long make_smem_desc(const void* tile) {
 }
 
 // Descriptor of an MN-major tile (the M or N index is contiguous in memory, e.g. a [k, n] row-major slice)
-// stored with the 128-byte swizzle as TMA writes it from boxes of 64 columns x 64 rows: a 128-byte line holds
+// stored with the 128-byte swizzle as TMA writes it (make_tmap_mn): a 128-byte line holds
 // 64 consecutive M/N elements of one k, eight consecutive k form a 1024-byte swizzle atom, the next eight k
 // follow 1024 bytes later (stride byte offset) and the next 64 M/N elements start one box (8192 bytes) later
 // (leading byte offset).  One MMA (K = 16) consumes two atoms, so its successor starts 2048 bytes further.
@@ -140,7 +140,6 @@ __device__ __forceinline__ unsigned long long make_smem_desc_mn(const void* tile
 }
 constexpr unsigned kDescStepK = 2;       // K-major: 16 elements = 32 bytes along the swizzled row, in 16-byte units
 constexpr unsigned kDescStepMn = 128;    // MN-major: 16 k = two 1024-byte atoms, in 16-byte units
-constexpr unsigned kMnBoxBytes = 64 * 64 * 2;  // one 64 x 64 bf16 box
 
 // kind::f16 instruction descriptor: bf16 x bf16 -> fp32, M x N; a_mn / b_mn: that operand is MN-major.
 __host__ __device__ constexpr unsigned make_idesc(int m, int n, bool a_mn = false, bool b_mn = false) {
@@ -247,6 +246,22 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       : "memory");
 }
 
+// 128 columns x 64 rows of a row-major matrix (make_tmap_mn) as an MN-major tile: column block c (of 64), row r.
+__device__ __forceinline__ void tma_load_mn_pair(void* smem_dst, const CUtensorMap* tmap, int c, int r, unsigned bar_cluster_addr) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+          smem_u32(smem_dst)),
+      "l"(reinterpret_cast<unsigned long long>(tmap)), "r"(bar_cluster_addr), "r"(0), "r"(r), "r"(c)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_mn(void* smem_dst, const CUtensorMap* tmap, int c, int r, unsigned long long* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+          smem_u32(smem_dst)),
+      "l"(reinterpret_cast<unsigned long long>(tmap)), "r"(smem_u32(bar)), "r"(0), "r"(r), "r"(c)
+      : "memory");
+}
+
 // One MMA over both CTAs of the pair (M = 256: 128 rows per CTA; each CTA holds half of the B tile).
 __device__ __forceinline__ void umma_bf16_pair(unsigned d_tmem, unsigned long long adesc, unsigned long long bdesc,
                                                unsigned idesc, unsigned accumulate) {
@@ -306,6 +321,31 @@ inline int make_tmap(CUtensorMap* m, const void* base, unsigned long long rows, 
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed with CUresult " + std::to_string((int)r));
+    return (int)r;
+  }
+  return 0;
+}
+
+// The same matrix for MN-major tiles: [cols / 64, rows, 64] with boxes of 2 x 64 x 64, which is 128 columns x 64 rows in one
+// copy, 64 columns after the other in shared memory, each swizzled over its 128-byte lines.  As two copies of 64 columns, each
+// issued by lane 0 on its own: [K, N] products of 1 x 16384 rows, K=N=4096, 425 us, now 338; 8 x 1024, K=7168, N=2048, 182 and
+// 155; weight gradients 8 x 1024 rows, 2048 x 7168, 197 and 183.
+inline int make_tmap_mn(CUtensorMap* m, const void* base, unsigned long long rows, unsigned long long cols,
+                        unsigned long long ld = 0) {
+  EncodeTiledFn fn = encode_tiled();
+  if (fn == nullptr) {
+    set_error("cuTensorMapEncodeTiled is not available (no CUDA driver?)");
+    return 1;
+  }
+  cuuint64_t dims[3] = {64, rows, cols / 64};
+  cuuint64_t strides[2] = {(ld ? ld : cols) * 2, 128};
+  cuuint32_t box[3] = {64, 64, 2};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed with CUresult " + std::to_string((int)r));
     return (int)r;
