@@ -7,7 +7,7 @@
 // exactly one group.  The number of row blocks is read from cu_seqlens on the device; the host never
 // synchronises.
 //
-// Persistent kernel, one CTA per SM, 192 threads:
+// Persistent kernel, one CTA per SM, 320 threads:
 //   warp 0      TMA producer: per 64-wide K block one 128x64 tile of X and two 128x64 tiles of W
 //               (cp.async.bulk.tensor.2d, 128-byte swizzle, every CTA loads its own tiles) into a 4-stage ring; the
 //               transaction bytes complete the stage's "full" mbarrier.
@@ -15,9 +15,9 @@
 //               one lane: four tcgen05.mma (M=128, N=256, K=16, bf16 -> fp32) per stage;
 //               tcgen05.commit releases the stage and, after the last K block, publishes the
 //               accumulator to the epilogue.
-//   warps 2..5  epilogue: tcgen05.ld 32 columns at a time from their 32 TMEM lanes, apply the
-//               epilogue, convert to bf16, store.  While they drain one accumulator the MMA warp
-//               fills the other.
+//   warps 2..9  epilogue: tcgen05.ld 32 columns at a time from their 32 TMEM lanes and their half of the
+//               columns, apply the epilogue, convert to bf16, store.  While they drain one accumulator the
+//               MMA warp fills the other.
 // Epilogues: PLAIN  y = acc                                   (256 output columns per tile)
 //            SWIGLU y = silu(acc[:, :128]) * acc[:, 128:]      (W tiles come from W_gate and W_up;
 //                                                              128 output columns per tile)
@@ -38,7 +38,10 @@ namespace moonep {
 namespace {
 
 constexpr int kStages = 4;
-constexpr int kGemmThreads = 192;
+// Two epilogue warps per quarter of the TMEM lanes: a decode step is one tile per CTA, whose epilogue nothing hides (SwiGLU of
+// 16 groups x 128 rows, K=2048, N=1024: 38.2 us with one warp per quarter, 34.8 with two; K=512, N=256: 19.8 and 16.4).
+constexpr int kEpilogueWarps = 8;
+constexpr int kGemmThreads = 64 + 32 * kEpilogueWarps;
 constexpr int kTmemCols = 512;
 constexpr unsigned kATileBytes = BM * BK * 2;        // 16 KB
 constexpr unsigned kBHalfBytes = 128 * BK * 2;       // 16 KB
@@ -60,7 +63,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(s_tfull + b, 1);
-      mbar_init(s_tempty + b, 4);
+      mbar_init(s_tempty + b, kEpilogueWarps);
     }
     fence_barrier_init();
   }
@@ -82,7 +85,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    {
       int stage = 0;
       unsigned phase = 0;
       bool failed = false;
@@ -97,24 +100,27 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         int wslot = a.group_map != nullptr ? a.group_map[lo] : lo;
         if (wslot < 0 || wslot >= a.w_slots) {
           // a group whose weights this rank does not hold: reported, computed with slot 0 (in bounds), never trusted
-          gemm_bad_index(a.status, 13, 13, lo, wslot);
+          if (lane == 0) gemm_bad_index(a.status, 13, 13, lo, wslot);
           wslot = 0;
         }
         const int wrow0 = wslot * a.n_per_group + nb * b_rows_per_tile;
         for (int kb = 0; kb < a.k_blocks; ++kb) {
-          if (!mbar_wait(s_empty + stage, phase ^ 1u, a.timeout_ns)) {
-            gemm_fail(a.status, 13, 1, stage, kb);
+          if (!mbar_wait_warp(s_empty + stage, phase ^ 1u, a.timeout_ns)) {
+            if (lane == 0) gemm_fail(a.status, 13, 1, stage, kb);
             failed = true;
             break;
           }
-          unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
-          mbar_expect_tx(s_full + stage, kStageBytes);
-          tma_load_2d(st, &tmap_a, kb * BK, row0, s_full + stage);
-          tma_load_2d(st + kATileBytes, &tmap_b0, kb * BK, wrow0, s_full + stage);
-          if (a.mode == kSwiglu)
-            tma_load_2d(st + kATileBytes + kBHalfBytes, &tmap_b1, kb * BK, wrow0, s_full + stage);
-          else
-            tma_load_2d(st + kATileBytes + kBHalfBytes, &tmap_b0, kb * BK, wrow0 + 128, s_full + stage);
+          if (elect_one()) {
+            unsigned char* st = s_tiles + (size_t)stage * kStageBytes;
+            mbar_expect_tx(s_full + stage, kStageBytes);
+            tma_load_2d(st, &tmap_a, kb * BK, row0, s_full + stage);
+            tma_load_2d(st + kATileBytes, &tmap_b0, kb * BK, wrow0, s_full + stage);
+            if (a.mode == kSwiglu)
+              tma_load_2d(st + kATileBytes + kBHalfBytes, &tmap_b1, kb * BK, wrow0, s_full + stage);
+            else
+              tma_load_2d(st + kATileBytes + kBHalfBytes, &tmap_b0, kb * BK, wrow0 + 128, s_full + stage);
+          }
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -171,8 +177,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     __syncwarp();
   } else {
-    // ---------------- epilogue (warps 2..5) ----------------
-    const int q = warp & 3;  // TMEM lane quarter this warp may read
+    // ---------------- epilogue (warps 2..9) ----------------
+    const int q = warp & 3;            // TMEM lane quarter this warp may read
+    const int half = (warp - 2) >> 2;  // which half of the columns is this warp's
     if (blockIdx.x == 0)  // while the first accumulator is being filled
       for (int g = threadIdx.x - 64; g < a.G; g += kGemmThreads - 64) gemm_check_end(a.status, 13, g, a.cu_seqlens[g]);
     unsigned tphase[2] = {0, 0};
@@ -194,7 +201,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (a.mode == kSwiglu) {
         uint16_t* orow = a.out + (long long)row * a.ldo + (long long)nb * 128;
 #pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
+        for (int c0 = half * 64; c0 < half * 64 + 64; c0 += 32) {
           unsigned g[32], u[32];
           tmem_ld32(taddr + (unsigned)c0, g);
           tmem_ld32(taddr + (unsigned)(128 + c0), u);
@@ -227,7 +234,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const float scale = (a.mode == kScale && a.row_scale != nullptr) ? a.row_scale[row] : 1.f;
         uint16_t* orow = a.out + (long long)row * a.ldo + (long long)nb * BN;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
+        for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 32) {
           unsigned v[32];
           tmem_ld32(taddr + (unsigned)c0, v);
           tmem_ld_wait();
