@@ -443,10 +443,7 @@ class CudaBackend:
             self._topk = topk
             self._next(FLAG_TPE)
             self._next(FLAG_PLAN)
-        # a fresh plan of this Buffer comes as one allocation; its tensors are made when somebody asks for them
-        dst, etc, zf, rs, dg, dl, dc, si, lk = (plan._addresses() if topk is not None else None) or [
-            _ptr(t) for t in (plan.dst, plan.experts_to_copy, plan.zero_fill_ranges, plan.remote_stats, plan.dup_groups,
-                              plan.dup_loffs, plan.dup_counts, plan.src_info, plan.link)]  # fmt: skip
+        dst, etc, zf, rs, dg, dl, dc, si, lk = plan._addresses()
         self._call(
             "moonep_dispatch_single", int(topk is not None), int(self.exact_counts), _ptr(topk), _ptr(tpe), dst, _ptr(cu),
             etc, zf, rs, dg, dl, dc, si, lk, _ptr(hidden), _ptr(weights),
@@ -510,7 +507,7 @@ class CudaBackend:
             return
         self._quiesced = False
         if self.ctx["R"] == 1:  # nothing to stage or fold: the rows of a token are summed where they are
-            self._call("moonep_combine_single", _ptr(plan.dst), _ptr(hidden_nvsh), _ptr(route_weights_nvs), _ptr(out_hidden),
+            self._call("moonep_combine_single", plan._dst_address(), _ptr(hidden_nvsh), _ptr(route_weights_nvs), _ptr(out_hidden),
                        _ptr(out_weights_sk), _ptr(ready), int(ready_expect), _stream(), tag="combine_single")  # fmt: skip
             return
         comb = self._next(FLAG_COMB)

@@ -50,10 +50,11 @@ def _field_shapes(N, R, E, B, NvS) -> dict:
 class _PlanLayout:
     """Where the fields of a plan lie in one int32 allocation (words), and their shapes and strides."""
 
-    __slots__ = ("fields", "offsets", "words")
+    __slots__ = ("fields", "index", "offsets", "words")
 
     def __init__(self, N, R, E, B, NvS):
         self.fields, self.offsets, self.words = {}, [], 0
+        self.index = {name: i for i, name in enumerate(_FIELDS)}
         for name, shape in _field_shapes(N, R, E, B, NvS).items():
             strides = (1,) if len(shape) == 1 else (shape[1], 1)
             self.fields[name] = (shape, strides, self.words)
@@ -131,12 +132,20 @@ class MoonEPCommPlan(_PackSlot):
         return plan
 
     def _addresses(self):
-        """Addresses of the fields, in order, of a plan that has just been allocated; None if it is not packed."""
+        """Addresses of the fields in the order of ``_FIELDS`` (None for an absent one), without making a packed plan's
+        tensors."""
         pack = getattr(self, "_pack", None)
         if pack is None:
-            return None
+            return [None if t is None else t.data_ptr() for t in (getattr(self, name) for name in _FIELDS)]
         p = pack.base.data_ptr()
-        return [p + 4 * o for o in pack.layout.offsets]
+        out = [p + 4 * o for o in pack.layout.offsets]
+        for name, t in pack.made.items():
+            out[pack.layout.index[name]] = t.data_ptr()
+        return out
+
+    def _dst_address(self) -> int:
+        pack = getattr(self, "_pack", None)
+        return self.dst.data_ptr() if pack is None or "dst" in pack.made else pack.base.data_ptr()  # dst comes first
 
     def tensors(self):
         """The tensors a stream must keep alive while it uses this plan."""

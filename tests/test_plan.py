@@ -1,0 +1,63 @@
+"""Plans whose tensors are views of one allocation (what a Buffer on a GPU hands out) behave like plans made of tensors."""
+
+import copy
+import dataclasses
+import pickle
+
+import pytest
+import torch
+
+from moonep_b200.plan import MoonEPCommPlan, _PlanLayout, check_plan_for_ctx
+
+FIELDS = ("dst", "experts_to_copy", "zero_fill_ranges", "remote_stats", "dup_groups", "dup_loffs", "dup_counts", "src_info", "link")
+
+
+def _packed(N=15, R=2, E=6, B=3, NvS=40, K=5):
+    layout = _PlanLayout(N, R, E, B, NvS)
+    base = torch.arange(layout.words, dtype=torch.int32)
+    return MoonEPCommPlan._packed(base, layout, N, R, E, B, NvS, K), base
+
+
+@pytest.mark.parametrize("sizes", [dict(), dict(N=1, R=1, E=1, B=0, NvS=1, K=1), dict(N=129, E=128, NvS=300)])
+def test_fields_are_disjoint_aligned_views(sizes):
+    plan, base = _packed(**sizes)
+    addresses, dst = plan._addresses(), plan._dst_address()
+    assert dst == addresses[0] == base.data_ptr()
+    for name, at in zip(FIELDS, addresses):
+        t = getattr(plan, name)
+        assert (t.numel() == 0 or t.data_ptr() == at) and (at - base.data_ptr()) % 512 == 0 and t.is_contiguous() and t.dtype == torch.int32
+        assert getattr(plan, name) is t, "made once"
+        t.view(-1).fill_(-1)
+    used = base == -1
+    assert int(used.sum()) == sum(getattr(plan, n).numel() for n in FIELDS), "fields overlap"
+    assert plan.dst.shape == (plan.N,) and plan.experts_to_copy.shape == (plan.R, plan.B)
+    assert plan.zero_fill_ranges.shape == (plan.E + plan.B, 2) and plan.dup_groups.shape == (plan.NvS, 3)
+    assert [a for n, a in zip(FIELDS, plan._addresses()) if getattr(plan, n).numel()] == \
+        [a for n, a in zip(FIELDS, addresses) if getattr(plan, n).numel()] and plan._dst_address() == dst
+    # the ordinary constructor accepts them
+    MoonEPCommPlan(**{f.name: getattr(plan, f.name) for f in dataclasses.fields(plan)})
+
+
+def test_copies_and_attributes():
+    plan, base = _packed()
+    twin = plan.clone()
+    assert twin._addresses() == [getattr(twin, n).data_ptr() for n in FIELDS] and all(torch.equal(getattr(twin, n), getattr(plan, n)) for n in FIELDS)
+    assert all(getattr(twin, n).data_ptr() != getattr(plan, n).data_ptr() for n in FIELDS)
+    for other in (copy.copy(plan), copy.deepcopy(plan), pickle.loads(pickle.dumps(plan)), dataclasses.replace(plan, K=5)):
+        assert torch.equal(other.link, plan.link) and other.NvS == plan.NvS and len(other.tensors()) == 9
+    assert not hasattr(plan, "nothing")
+    with pytest.raises(dataclasses.FrozenInstanceError):
+        plan.dst = base
+
+
+def test_checks_see_what_was_handed_out():
+    plan, _ = _packed()
+    ctx = {k: getattr(plan, k) for k in ("N", "R", "E", "B", "NvS", "K")}
+    check_plan_for_ctx(ctx, plan, "cpu")
+    with pytest.raises(AssertionError):
+        check_plan_for_ctx({**ctx, "NvS": 41}, plan, "cpu")
+    with pytest.raises(AssertionError, match="wrong device"):
+        check_plan_for_ctx(ctx, plan, "cuda:0")
+    plan.link.unsqueeze_(0)
+    with pytest.raises(AssertionError, match="plan.link"):
+        check_plan_for_ctx(ctx, plan, "cpu")
