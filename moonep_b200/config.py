@@ -26,7 +26,8 @@ MOONEP_COMBINE        ``push`` (default: the expert side folds duplicates and pu
                       which sum them as they arrive) or ``pull`` (fold pass, then the home ranks pull).
 MOONEP_PHASED         ``1``: launch the dispatch and combine kernels one role at a time even on real multi-GPU worlds
                       (what emulated ranks always do); for per-role timing and debugging.
-MOONEP_PDL            ``0`` turns programmatic dependent launch off even for Buffers created with ``enable_pdl=True``.
+MOONEP_PDL            ``0`` turns programmatic dependent launch off even for Buffers created with ``enable_pdl=True``, and for the
+                      expert kernels (GEMMs, weight gradients, SwiGLU backward), which no Buffer launches.
 MOONEP_LOCAL_SMS      CTAs of the kernels that only touch local memory (default: all SMs); ``num_sms`` of
                       the Buffer bounds the kernels that move data between ranks.
 MOONEP_NUM_SMS_DEDUP  CTAs of the dispatch kernel's destination-side role (zero fill, dedup builder, duplicate
