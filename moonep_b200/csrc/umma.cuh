@@ -147,8 +147,14 @@ __host__ __device__ constexpr unsigned make_idesc(int m, int n, bool a_mn = fals
          ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
 }
 
-__device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
-
+// x / (1 + exp(-x)).  A zero numerator takes the division off its fast path, for all lanes of the warp, and the pad rows at a
+// group's end are all zeros; so zeros divide a one and are put back.
+__device__ __forceinline__ float silu(float x) {
+  float n = x == 0.f ? 1.f : x;
+  asm("" : "+f"(n));  // or the two selects are folded into the plain division
+  const float q = n / (1.f + __expf(-x));
+  return x == 0.f ? x : q;
+}
 
 enum GemmMode { kPlain = 0, kSwiglu = 1, kScale = 2 };
 
