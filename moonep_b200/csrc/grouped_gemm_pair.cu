@@ -9,19 +9,19 @@
 // instead of 48 KB per K block for the same MMA work), which is what bounds the single-CTA kernel, and
 // leaves room for a ring of five or six stages and the output pieces.
 //
-// Per CTA, 192 threads:
+// Per CTA, 192 or 320 threads:
 //   warp 0      TMA producer (both CTAs): X tile and W half tile of this CTA per K block; the bytes of
 //               both CTAs complete the transaction of the LEADER's "full" barrier of the stage.
 //   warp 1      allocates this CTA's 512 TMEM columns; in the leader one lane issues four
 //               tcgen05.mma.cta_group::2 (M=256, N=256, K=16) per stage and commits to the stage's
 //               "empty" barrier in both CTAs, and after the last K block to both "accumulator full" barriers.
-//   warps 2..5  epilogue of this CTA's 128 rows (same epilogues as the single-CTA kernel, stored 32 rows x 64 or 32
-//               columns at a time by tensor copies from shared memory); one arrival per warp on the leader's
-//               "accumulator empty" barrier, which counts both CTAs' warps.
+//   warps 2..   epilogue of this CTA's 128 rows, four warps or eight (same epilogues as the single-CTA kernel,
+//               stored 32 rows x 64 or 32 columns at a time by tensor copies from shared memory); one arrival
+//               per warp on the leader's "accumulator empty" barrier, which counts both CTAs' warps.
 //
 // Tiles: the 128-row blocks of a group are taken two at a time.  When a group has an odd number of
-// blocks the second CTA of its last pair has no rows of that group: it still feeds the MMA (with rows
-// that are simply not stored) and skips its stores.  SwiGLU: the leader's W half is the gate tile, the
+// blocks the second CTA of its last pair has no rows of that group: it still feeds the MMA (with zeros)
+// and skips its stores.  SwiGLU: the leader's W half is the gate tile, the
 // other CTA's the up tile, so accumulator columns 0-127 / 128-255 are gate / up as in the single-CTA kernel.
 //
 // Every mbarrier wait is bounded; on expiry the role records a status word and leaves its loop.  Both
@@ -37,25 +37,21 @@ namespace moonep {
 
 namespace {
 
-constexpr int kPairThreads = 192;
+template <int kEpi>
+constexpr int kPairThreads = 64 + 32 * kEpi;  // producer, MMA issuer, epilogue warps
 constexpr int kPairTmemCols = 512;
 constexpr unsigned kPairATileBytes = BM * BK * 2;                         // 16 KB: this CTA's rows of X
 constexpr unsigned kPairBHalfBytes = 128 * BK * 2;                        // 16 KB: this CTA's half of the W tile
 constexpr unsigned kPairStageBytes = kPairATileBytes + kPairBHalfBytes;   // 32 KB per CTA and stage
 // The results leave through shared memory: 32 rows x kCols columns per warp and tensor store, swizzled over the row; three
-// such pieces per warp are in flight one behind the other.  Shared memory holds six stages of operands with pieces of 32
-// columns, or five with pieces of 64.  The sixth stage counts where loads bound the kernel, the wide pieces where the
-// epilogue does; the line is drawn at K = 1024 (launch_pair).  Five stages against six, us: 8 groups x 512 rows, K=4096,
-// N=1024: SwiGLU 79.3 and 77.7, plain 54.2 and 52.3; 16 x 128, K=2048, N=1024: SwiGLU 53.7 and 52.3; 16 x 1024, K=4096,
-// N=512: plain 76.0 and 73.7; 16 x 1024, K=1024, N=4096: SwiGLU 302 and 305, with pre-activations 313 and 342; 1 x 16384,
-// K=512, N=2048: 138 and 141, 148 and 159.  16-byte stores from registers with six stages (a row per lane, two half-written
-// sectors per lane and instruction pair): 78.2, 54.3; 52.7; 76.1; 307, 329; 142, 155, plain at the last 47.6 where five
-// stages take 39.1.
+// such pieces per warp are in flight one behind the other.  Shared memory holds six stages of operands and pieces of 32
+// columns of four epilogue warps, or five stages and either pieces of 64 columns or eight such warps.  Which of them takes a
+// call is decided in launch_pair.
 constexpr int kPairPieces = 3;
 template <int kCols>
 constexpr unsigned kPairWarpPieces = kPairPieces * 32 * kCols * 2;
-template <int kStages, int kCols>
-constexpr size_t kPairSmem = (size_t)kStages * kPairStageBytes + 1024 + 4 * kPairWarpPieces<kCols>;
+template <int kStages, int kCols, int kEpi>
+constexpr size_t kPairSmem = (size_t)kStages * kPairStageBytes + 1024 + kEpi * kPairWarpPieces<kCols>;
 constexpr int kPairKernelId = 15;
 constexpr int kPairGroupsInSmem = 2048;  // group ends are walked from shared memory up to this many groups
 
@@ -141,8 +137,8 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, const void
                : "memory");
 }
 
-template <int kStages, int kCols, bool kKn>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+template <int kStages, int kCols, int kEpi, bool kKn>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads<kEpi>, 1)
     grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                              const __grid_constant__ CUtensorMap tmap_b1, const __grid_constant__ CUtensorMap tmap_o,
                              const __grid_constant__ CUtensorMap tmap_pg, const __grid_constant__ CUtensorMap tmap_pu,
@@ -163,7 +159,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(s_tfull + b, 1);   // one commit, delivered to both CTAs
-      mbar_init(s_tempty + b, 8);  // used in the leader: four epilogue warps of each CTA
+      mbar_init(s_tempty + b, 2 * kEpi);  // used in the leader: the epilogue warps of both CTAs
     }
     mbar_init(&s_done, 1);
     fence_barrier_init();
@@ -343,8 +339,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     }
     __syncwarp();
   } else {
-    // ---------------- epilogue (warps 2..5, both CTAs) ----------------
-    const int q = warp & 3;  // TMEM lane quarter this warp may read
+    // ---------------- epilogue (warps 2.., both CTAs) ----------------
+    const int q = warp & 3;                            // TMEM lane quarter this warp may read
+    constexpr int kShares = kEpi / 4;                  // warps of a quarter, which share its columns
+    const int share = kShares > 1 ? (warp - 2) >> 2 : 0;
     const unsigned tempty_of_leader[2] = {mapa_u32(s_tempty + 0, 0), mapa_u32(s_tempty + 1, 0)};
     unsigned char* pieces = s_tiles + (size_t)kStages * kPairStageBytes + (warp - 2) * kPairWarpPieces<kCols>;
     int piece = 0;
@@ -390,7 +388,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         constexpr int kLoads = kCols / 32;  // TMEM loads of 32 columns per piece
         if (!kKn && a.mode == kSwiglu) {
 #pragma unroll 1
-          for (int c0 = 0; c0 < 128; c0 += kCols) {
+          for (int c0 = share * (128 / kShares); c0 < (share + 1) * (128 / kShares); c0 += kCols) {
             unsigned g[kLoads][32], u[kLoads][32];
 #pragma unroll
             for (int l = 0; l < kLoads; ++l) {
@@ -416,7 +414,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         } else {
           const float scale = (a.mode == kScale && a.row_scale != nullptr) ? a.row_scale[row0 + lane] : 1.f;
 #pragma unroll 1
-          for (int c0 = 0; c0 < BN; c0 += 64) {
+          for (int c0 = share * (BN / kShares); c0 < (share + 1) * (BN / kShares); c0 += 64) {
             unsigned v[2][32];
             tmem_ld32(taddr + (unsigned)c0, v[0]);
             tmem_ld32(taddr + (unsigned)(c0 + 32), v[1]);
@@ -570,7 +568,7 @@ extern "C" int moonep_grouped_gemm_pair_kn(const void* x, const void* w0, int K0
   return launch_pair(ta, tb0, tb1, a, num_sms, stream);
 }
 
-template <int kStages, int kCols, bool kKn>
+template <int kStages, int kCols, int kEpi, bool kKn>
 static int launch_pair_of(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const GemmArgs& a,
                        int num_sms, void* stream) {
   CUtensorMap to, tg, tu;
@@ -580,14 +578,14 @@ static int launch_pair_of(const CUtensorMap& ta, const CUtensorMap& tb0, const C
     if (int rc = make_tmap(&tg, a.pre_gate, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32, 0, kCols)) return rc;
     if (int rc = make_tmap(&tu, a.pre_up, (unsigned long long)a.rows_cap, (unsigned long long)a.ldo, 32, 0, kCols)) return rc;
   }
-  constexpr auto* kernel = grouped_gemm_pair_kernel<kStages, kCols, kKn>;
-  constexpr size_t smem = kPairSmem<kStages, kCols>;
+  constexpr auto* kernel = grouped_gemm_pair_kernel<kStages, kCols, kEpi, kKn>;
+  constexpr size_t smem = kPairSmem<kStages, kCols, kEpi>;
   static int max_pairs = -1;  // pairs of these CTAs the device runs at once
   if (max_pairs < 0)
-    if (int rc = pairs_at_once(kernel, kPairThreads, smem, "grouped_gemm_pair_kernel", &max_pairs)) return rc;
+    if (int rc = pairs_at_once(kernel, kPairThreads<kEpi>, smem, "grouped_gemm_pair_kernel", &max_pairs)) return rc;
   int pairs = max_pairs;
   if (num_sms > 0) pairs = imax(1, imin(pairs, num_sms / 2));
-  if (int rc = check_cuda(launch_maybe_pdl(kernel, 2 * pairs, kPairThreads, smem, (cudaStream_t)stream,
+  if (int rc = check_cuda(launch_maybe_pdl(kernel, 2 * pairs, kPairThreads<kEpi>, smem, (cudaStream_t)stream,
                                            !has_hooks(a.hooks) && expert_pdl(num_sms), ta, tb0, tb1, to, tg, tu, a),
                           "launch grouped_gemm_pair_kernel"))
     return rc;
@@ -596,11 +594,21 @@ static int launch_pair_of(const CUtensorMap& ta, const CUtensorMap& tb0, const C
 
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const GemmArgs& a,
                        int num_sms, void* stream) {
+  // The sixth stage counts where loads bound the kernel, eight epilogue warps where the SwiGLU epilogue does (a division per
+  // element, and two more outputs with pre-activations: a tile's epilogue is as long as 32 K blocks), wide pieces where K is so
+  // short that the stores do.  us, five stages with four warps / six stages / five stages with eight warps:
+  //   plain, 16 groups x 1024 rows, N=4096: K=256 41.0 / 47.1 / 42.6, K=512 57.2 / 55.1 / 59.3, K=1024 92.1 / 86.3 / 94.0
+  //   SwiGLU, 16 x 1024: K=512, N=4096 256 / 264 / 158; K=2048, N=2048 166 / 164 / 162; K=4096, N=1024 169 / 164 / 165
+  //   with pre-activations: K=512, N=4096 283 / 306 / 182; K=2048, N=2048 179 / 187 / 174; K=3072, N=1024 137 / 129 / 134
+  // The count of finished tiles that a consumer waits for is one per warp of four, so with it the eight warps stay out.
+  const bool short_k = a.k_blocks < 512 / BK || (a.mode == kSwiglu && a.k_blocks <= 1024 / BK);
   if (a.b_kn)
-    return a.k_blocks <= 1024 / BK ? launch_pair_of<5, 64, true>(ta, tb0, tb1, a, num_sms, stream)
-                                   : launch_pair_of<6, 32, true>(ta, tb0, tb1, a, num_sms, stream);
-  return a.k_blocks <= 1024 / BK ? launch_pair_of<5, 64, false>(ta, tb0, tb1, a, num_sms, stream)
-                                 : launch_pair_of<6, 32, false>(ta, tb0, tb1, a, num_sms, stream);
+    return short_k ? launch_pair_of<5, 64, 4, true>(ta, tb0, tb1, a, num_sms, stream)
+                   : launch_pair_of<6, 32, 4, true>(ta, tb0, tb1, a, num_sms, stream);
+  if (a.mode == kSwiglu && a.k_blocks <= 2048 / BK && a.hooks.done_counter == nullptr)
+    return launch_pair_of<5, 32, 8, false>(ta, tb0, tb1, a, num_sms, stream);
+  return short_k ? launch_pair_of<5, 64, 4, false>(ta, tb0, tb1, a, num_sms, stream)
+                 : launch_pair_of<6, 32, 4, false>(ta, tb0, tb1, a, num_sms, stream);
 }
 
 // Host-side walk of the tile schedule of one CTA pair (for tests): writes, for every tile that pair `pair` of
