@@ -1091,6 +1091,10 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const Moo
   bool is_sender = (roles & (MOONEP_ROLE_TOKENS | MOONEP_ROLE_SEND)) != 0;
   bool is_expander = (roles & MOONEP_ROLE_EXPAND) != 0;
   int scnt = gridDim.x, xidx = blockIdx.x, xcnt = gridDim.x;
+  if (!mixed && (roles & MOONEP_ROLE_SEND)) {  // CTAs beyond the senders only plan
+    is_sender = (int)blockIdx.x < a.n_send;
+    scnt = a.n_send;
+  }
   if (mixed) {
     is_sender = (int)blockIdx.x >= s0 && (int)blockIdx.x < s0 + a.n_send;
     is_expander = !is_sender;
@@ -1277,6 +1281,8 @@ extern "C" int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk,
     // a single rank whose rows are all written by the EXPAND role: the senders only store gate weights
     if (c.R == 1 && a.local_rows && expanders) a.n_send = imin(a.n_send, 4);
     grid = a.n_send;
+    // planning is local work: as many CTAs as there are blocks of tokens (S=4096, K=8 on 32 CTAs: 19 us of planning each way, 10 on 64)
+    if (!expanders && (roles & MOONEP_ROLE_TOKENS)) grid = imax(grid, imin(a.n_blocks, imin(c.local_sms, h->sm_count)));
   }
   if (expanders) {
     const int room = imax(1, imin(c.local_sms, h->sm_count) - a.n_send);
