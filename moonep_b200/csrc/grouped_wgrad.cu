@@ -401,12 +401,14 @@ static int launch_single(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs
 }
 
 // One CTA per tile, or pairs: 1 or 0.  rows_per_group: rows of a group that has any, as far as the caller knows.
-// Short groups are epilogue: a CTA's results are half a pair's, and the tail wave is finer.  16 groups, 1024 x 2048, single
-// against pair: 256 rows 36.2 and 37.0 us (adding: 63.0, 65.1), 512 rows 53.3 and 47.2; 64 groups x 128 rows, 640 x 1024: 41.7
-// and 44.4.  A pair cannot use the last of an odd number of SMs, and not one alone: 3 SMs 971 and 1400 us, 9 SMs 332 and 361
-// (16 groups x 128 rows), from there on the pair's rate makes up for it.
+// Short groups are epilogue: a CTA's results are half a pair's, and the tail wave is finer.  Single against pair, us (adding):
+// 8 groups, 2048 x 7168: 256 rows 97.5 and 100.4 (193, 195), 320 rows 109 and 98 (194, 196), 512 rows 141 and 117 (196, 195);
+// 64 groups, 640 x 1024: 128 rows 40.0 and 39.0 (65.5, 67.1), 256 rows 45.0 and 45.1 (66.3, 68.1), 320 rows 51.1 and 47.3
+// (67.0, 69.5); 16 groups, 1024 x 2048: 256 rows 34.7 and 34.1 (52.7, 52.2), 384 rows 41.8 and 36.9 (53.3, 54.3).  A pair
+// cannot use the last of an odd number of SMs, and not one alone: 3 SMs 971 and 1400 us, 9 SMs 332 and 361 (16 groups x 128
+// rows), from there on the pair's rate makes up for it.
 extern "C" int moonep_wgrad_single_cta(int rows_per_group, int num_sms) {
-  return rows_per_group < 384 || (num_sms < 10 && (num_sms & 1) != 0) ? 1 : 0;
+  return rows_per_group <= 256 || (num_sms < 10 && (num_sms & 1) != 0) ? 1 : 0;
 }
 
 static int launch_wgrad(const CUtensorMap& tl, const CUtensorMap& tr, WgradArgs& a, int rows_per_group, int num_sms,
