@@ -38,6 +38,7 @@ from .layout import check_encoding_bounds
 
 _FIELDS = ("dst", "experts_to_copy", "zero_fill_ranges", "remote_stats", "dup_groups", "dup_loffs", "dup_counts", "src_info", "link")
 _ALIGN = 128  # words: what a tensor of its own would start on
+_MIB_WORDS = 1 << 18
 
 
 def _field_shapes(N, R, E, B, NvS) -> dict:
@@ -48,28 +49,38 @@ def _field_shapes(N, R, E, B, NvS) -> dict:
 
 
 class _PlanLayout:
-    """Where the fields of a plan lie in one int32 allocation (words), and their shapes and strides."""
+    """Where the fields of a plan lie in its int32 allocation (words), and their shapes and strides.  A plan beyond a MiB whose
+    parts are below it comes in two parts, ``dup_groups`` and the rest: larger requests come out of larger segments, and a graph
+    capture, which has a pool of its own, pays for the segment (about 1 ms)."""
 
-    __slots__ = ("fields", "index", "offsets", "words")
+    __slots__ = ("fields", "index", "places", "words")
 
     def __init__(self, N, R, E, B, NvS):
-        self.fields, self.offsets, self.words = {}, [], 0
-        self.index = {name: i for i, name in enumerate(_FIELDS)}
-        for name, shape in _field_shapes(N, R, E, B, NvS).items():
+        sizes = {}
+        shapes = _field_shapes(N, R, E, B, NvS)
+        for name, shape in shapes.items():
+            n = max(1, shape[0] * (shape[1] if len(shape) == 2 else 1))
+            sizes[name] = -(-n // _ALIGN) * _ALIGN
+        apart = "dup_groups" if sum(sizes.values()) > _MIB_WORDS >= max(sizes["dup_groups"],
+                                                                       sum(sizes.values()) - sizes["dup_groups"]) else None  # fmt: skip
+        self.fields, self.words = {}, [0] if apart is None else [0, 0]
+        for name, shape in shapes.items():
+            part = 1 if name == apart else 0
             strides = (1,) if len(shape) == 1 else (shape[1], 1)
-            self.fields[name] = (shape, strides, self.words)
-            self.offsets.append(self.words)
-            self.words += -(-max(1, shape[0] * (shape[1] if len(shape) == 2 else 1)) // _ALIGN) * _ALIGN
+            self.fields[name] = (part, shape, strides, self.words[part])
+            self.words[part] += sizes[name]
+        self.index = {name: i for i, name in enumerate(_FIELDS)}
+        self.places = [(part, 4 * offset) for part, _, _, offset in self.fields.values()]  # part and bytes, in order
 
 
 class _Packed:
     """What a plan from ``allocate_planning_outputs`` on a GPU keeps in the place of its tensors until they are asked for:
-    the allocation, its layout and the tensors made so far."""
+    the allocations, their layout and the tensors made so far."""
 
-    __slots__ = ("base", "layout", "made")
+    __slots__ = ("parts", "layout", "made")
 
-    def __init__(self, base, layout):
-        self.base, self.layout, self.made = base, layout, {}
+    def __init__(self, parts, layout):
+        self.parts, self.layout, self.made = parts, layout, {}
 
 
 class _PackSlot:
@@ -108,21 +119,21 @@ class MoonEPCommPlan(_PackSlot):
         """A field of a packed plan that nobody has used yet: a view of the plan's allocation, made once."""
         try:
             pack = object.__getattribute__(self, "_pack")
-            shape, strides, offset = pack.layout.fields[name]
+            part, shape, strides, offset = pack.layout.fields[name]
         except (AttributeError, KeyError):
             raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}") from None
-        t = pack.base.as_strided(shape, strides, offset)
+        t = pack.parts[part].as_strided(shape, strides, offset)
         object.__setattr__(self, name, t)
         pack.made[name] = t
         return t
 
     @classmethod
-    def _packed(cls, base, layout, N, R, E, B, NvS, K) -> "MoonEPCommPlan":
-        """A plan whose tensors are views of ``base``.  A round trip uses one of the nine; the others cost what they
+    def _packed(cls, parts, layout, N, R, E, B, NvS, K) -> "MoonEPCommPlan":
+        """A plan whose tensors are views of ``parts``.  A round trip uses one of the nine; the others cost what they
         cost only where they are used, and the allocation is one call instead of nine (18 us of host time)."""
         plan = object.__new__(cls)
         put = object.__setattr__
-        put(plan, "_pack", _Packed(base, layout))
+        put(plan, "_pack", _Packed(parts, layout))
         put(plan, "N", N)
         put(plan, "R", R)
         put(plan, "E", E)
@@ -137,15 +148,15 @@ class MoonEPCommPlan(_PackSlot):
         pack = getattr(self, "_pack", None)
         if pack is None:
             return [None if t is None else t.data_ptr() for t in (getattr(self, name) for name in _FIELDS)]
-        p = pack.base.data_ptr()
-        out = [p + 4 * o for o in pack.layout.offsets]
+        p = [t.data_ptr() for t in pack.parts]
+        out = [p[part] + at for part, at in pack.layout.places]
         for name, t in pack.made.items():
             out[pack.layout.index[name]] = t.data_ptr()
         return out
 
     def _dst_address(self) -> int:
         pack = getattr(self, "_pack", None)
-        return self.dst.data_ptr() if pack is None or "dst" in pack.made else pack.base.data_ptr()  # dst comes first
+        return self.dst.data_ptr() if pack is None or "dst" in pack.made else pack.parts[0].data_ptr()  # dst comes first
 
     def tensors(self):
         """The tensors a stream must keep alive while it uses this plan."""
@@ -200,9 +211,9 @@ def allocate_planning_outputs(ctx: dict) -> tuple[MoonEPCommPlan, torch.Tensor]:
         layout = ctx.get("_plan_layout")
         if layout is None:
             layout = ctx["_plan_layout"] = _PlanLayout(N, R, E, B, NvS)
-        base = torch.empty(layout.words, dtype=torch.int32, device=dev)
+        parts = [torch.empty(n, dtype=torch.int32, device=dev) for n in layout.words]
         # a tensor of its own: it may be kept long after the plan
-        return MoonEPCommPlan._packed(base, layout, N, R, E, B, NvS, K), torch.empty(E + B, dtype=torch.int32, device=dev)
+        return MoonEPCommPlan._packed(parts, layout, N, R, E, B, NvS, K), torch.empty(E + B, dtype=torch.int32, device=dev)
     plan = MoonEPCommPlan(
         dst=_i32(N, dev),
         experts_to_copy=_i32(R * B, dev).view(R, B),
@@ -242,7 +253,7 @@ def check_plan_for_ctx(ctx: dict, plan: MoonEPCommPlan, device) -> None:
     device = torch.device(device)
     pack = getattr(plan, "_pack", None)
     if pack is not None:  # fields not used so far are views yet to be made, in the layout of these sizes
-        assert pack.base.device == device, "plan is on the wrong device"
+        assert pack.parts[0].device == device, "plan is on the wrong device"
         items = list(pack.made.items())
     else:
         items = [(name, getattr(plan, name)) for name in _FIELDS]

@@ -14,22 +14,24 @@ FIELDS = ("dst", "experts_to_copy", "zero_fill_ranges", "remote_stats", "dup_gro
 
 def _packed(N=15, R=2, E=6, B=3, NvS=40, K=5):
     layout = _PlanLayout(N, R, E, B, NvS)
-    base = torch.arange(layout.words, dtype=torch.int32)
-    return MoonEPCommPlan._packed(base, layout, N, R, E, B, NvS, K), base
+    parts = [torch.zeros(n, dtype=torch.int32) for n in layout.words]
+    return MoonEPCommPlan._packed(parts, layout, N, R, E, B, NvS, K), parts
 
 
-@pytest.mark.parametrize("sizes", [dict(), dict(N=1, R=1, E=1, B=0, NvS=1, K=1), dict(N=129, E=128, NvS=300)])
+@pytest.mark.parametrize("sizes", [dict(), dict(N=1, R=1, E=1, B=0, NvS=1, K=1), dict(N=129, E=128, NvS=300),
+                                   dict(N=128, R=1, E=256, B=256, NvS=65152, K=8), dict(N=9, NvS=90000)])  # two parts; one
 def test_fields_are_disjoint_aligned_views(sizes):
-    plan, base = _packed(**sizes)
+    plan, parts = _packed(**sizes)
     addresses, dst = plan._addresses(), plan._dst_address()
-    assert dst == addresses[0] == base.data_ptr()
+    assert dst == addresses[0] == parts[0].data_ptr()
     for name, at in zip(FIELDS, addresses):
         t = getattr(plan, name)
-        assert (t.numel() == 0 or t.data_ptr() == at) and (at - base.data_ptr()) % 512 == 0 and t.is_contiguous() and t.dtype == torch.int32
+        inside = [at - p.data_ptr() for p in parts if 0 <= at - p.data_ptr() < 4 * p.numel()]
+        assert (t.numel() == 0 or t.data_ptr() == at) and len(inside) == 1 and inside[0] % 512 == 0
+        assert t.is_contiguous() and t.dtype == torch.int32
         assert getattr(plan, name) is t, "made once"
         t.view(-1).fill_(-1)
-    used = base == -1
-    assert int(used.sum()) == sum(getattr(plan, n).numel() for n in FIELDS), "fields overlap"
+    assert sum(int((p == -1).sum()) for p in parts) == sum(getattr(plan, n).numel() for n in FIELDS), "fields overlap"
     assert plan.dst.shape == (plan.N,) and plan.experts_to_copy.shape == (plan.R, plan.B)
     assert plan.zero_fill_ranges.shape == (plan.E + plan.B, 2) and plan.dup_groups.shape == (plan.NvS, 3)
     assert [a for n, a in zip(FIELDS, plan._addresses()) if getattr(plan, n).numel()] == \
@@ -39,7 +41,7 @@ def test_fields_are_disjoint_aligned_views(sizes):
 
 
 def test_copies_and_attributes():
-    plan, base = _packed()
+    plan, parts = _packed()
     twin = plan.clone()
     assert twin._addresses() == [getattr(twin, n).data_ptr() for n in FIELDS] and all(torch.equal(getattr(twin, n), getattr(plan, n)) for n in FIELDS)
     assert all(getattr(twin, n).data_ptr() != getattr(plan, n).data_ptr() for n in FIELDS)
@@ -47,7 +49,7 @@ def test_copies_and_attributes():
         assert torch.equal(other.link, plan.link) and other.NvS == plan.NvS and len(other.tensors()) == 9
     assert not hasattr(plan, "nothing")
     with pytest.raises(dataclasses.FrozenInstanceError):
-        plan.dst = base
+        plan.dst = parts[0]
 
 
 def test_checks_see_what_was_handed_out():
