@@ -39,6 +39,12 @@ constexpr int kPlanWarps = 12;     // warps 0..11 plan, then up to kCopyWarps of
 // H=4096, K=6.
 constexpr int kCopyWarps = 6;
 constexpr int kEntries = kPlanWarps * 32;  // routing entries planned at a time (whole tokens)
+// A copy warp asks for its tokens one at a time, and in the end looks through the other CTAs' counters for what is left: about
+// 4 us of latency, for which a CTA with little to move waits longer than for the slowest SM.  So up to kDealtBytes read and
+// written per CTA the tokens are dealt to its warps at once.  Dispatch of S=2048, H=2048, K=4 24.1 -> 20.5 us, S=1024, H=4096,
+// K=2 21.5 -> 18.0, S=4096, H=1024, K=8 30.2 -> 28.2; with 1 MB per CTA (S=2048, H=4096, K=8) it would be 50.5 -> 52.2.
+constexpr long long kDealtBytes = 768 << 10;
+constexpr int kDealtRounds = 6;
 constexpr int kUnits = 64;         // units remembered per copy warp: those loaded and those not flagged yet
 constexpr int kGrabs = 64;         // grabs of pad rows remembered per warp
 constexpr int kMaxGroups = 4096;   // experts, and prefetch slots: up to four words of shared memory each
@@ -83,6 +89,7 @@ struct SingleArgs {
   int stage_bytes, npieces;  // a row is moved in npieces pieces of at most stage_bytes
   int copy_warps;            // warps that stream rows, each through a ring of its own
   int tokens_per_unit;       // whole rows that share a stage (npieces == 1)
+  int rounds;                // units of its CTA that a copy warp gets without asking
   int pads_per_grab;         // at least
   int tokens_per_cta;
   int* work;
@@ -234,11 +241,12 @@ struct Units {
   const SingleArgs& a;
   const int epoch;
   int tok, piece;  // a row moved in several pieces: the piece that comes next
-  int state;  // 0: the unit that is this warp's from the start, 1: more of the own CTA's, 2: other CTAs'
+  int state;  // 0: the units that are this warp's from the start, 1: more of the own CTA's, 2: other CTAs'
+  int round;
 
   __device__ int count_of(int cta) const { return max(0, min(c.S - cta * a.tokens_per_cta, a.tokens_per_cta)); }
   // tokens of a CTA that are dealt to its warps without the counter
-  __device__ int dealt() const { return a.copy_warps * a.tokens_per_unit; }
+  __device__ int dealt() const { return a.rounds * a.copy_warps * a.tokens_per_unit; }
 
   __device__ bool take(int cta, Unit& u) {
     int g = 0;
@@ -270,8 +278,11 @@ struct Units {
       return true;
     }
     if (state == 0) {
+      if (round < a.rounds) {
+        const int g = (round++ * a.copy_warps + (int)(threadIdx.x >> 5)) * a.tokens_per_unit;
+        if (unit_at(blockIdx.x, g, u)) return true;
+      }
       state = 1;
-      if (unit_at(blockIdx.x, (int)(threadIdx.x >> 5) * a.tokens_per_unit, u)) return true;
     }
     if (a.tokens_per_cta <= dealt()) return false;  // nothing beyond what was dealt, here or elsewhere
     if (state == 1) {
@@ -318,7 +329,7 @@ __device__ bool copy_bulk(const MoonepDevCtx& c, const SingleArgs& a, SingleShar
   unsigned char* ring = stages + (size_t)warp * kRing * a.stage_bytes;
   unsigned long long* bar = s.bar + warp * kRing;
   Unit* units = s.unit[warp];
-  Units from = {c, a, epoch, 0, a.npieces, 0};
+  Units from = {c, a, epoch, 0, a.npieces, 0, 0};
   int loaded = 0, stored = 0;
   auto load = [&]() {
     Unit u;
@@ -1028,6 +1039,8 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, int exact, const int
   int grid = imax(1, imin(imin(c.local_sms, h->sm_count), kMaxCtas));
   if (n_ctas > 0) grid = imin(grid, n_ctas);
   a.tokens_per_cta = (c.S + grid - 1) / grid;
+  const int per_round = imax(1, a.copy_warps * a.tokens_per_unit), rounds = (a.tokens_per_cta + per_round - 1) / per_round;
+  a.rounds = rounds <= kDealtRounds && a.tokens_per_cta * (c.K + 1) * row_bytes <= kDealtBytes ? rounds : 1;
   if (int rc = check_cuda(launch_maybe_pdl(dispatch_single_kernel, grid, kThreads, smem, (cudaStream_t)stream,
                                            h->enable_pdl != 0, c, a),
                           "launch dispatch_single_kernel"))
