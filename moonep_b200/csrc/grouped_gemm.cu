@@ -67,12 +67,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     fence_barrier_init();
   }
+  // What the kernels before wrote is read from here on.  TMEM, which one of them may still be about to take, is taken
+  // after it.
+  griddep_wait();
+  griddep_launch();
   if (warp == 1) {
     tmem_alloc(&s_tmem_base, kTmemCols);
     tmem_relinquish();
   }
-  griddep_wait();  // what the kernels before wrote is read from here on
-  griddep_launch();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

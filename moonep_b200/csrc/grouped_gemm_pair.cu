@@ -164,12 +164,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads<kEpi>, 
     mbar_init(&s_done, 1);
     fence_barrier_init();
   }
+  // What the kernels before wrote is read from here on.  TMEM, which one of them may still be about to take, is taken
+  // after it.
+  griddep_wait();
+  if (!has_hooks(a.hooks)) griddep_launch();
   if (warp == 1) {
     tmem_alloc(&s_tmem_base, kPairTmemCols);
     tmem_relinquish();
   }
-  griddep_wait();  // what the kernels before wrote is read from here on
-  if (!has_hooks(a.hooks)) griddep_launch();
   __shared__ int s_hook_ok;
   if (threadIdx.x == 0) {
     s_hook_ok = 1;

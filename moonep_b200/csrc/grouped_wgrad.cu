@@ -155,12 +155,14 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap* tmap_l, const CUte
     mbar_init(&s_done, 1);
     fence_barrier_init();
   }
+  // What the kernels before wrote is read from here on.  TMEM, which one of them may still be about to take, is taken
+  // after it.
+  griddep_wait();
+  griddep_launch();
   if (warp == 1) {
     tmem_alloc(&s_tmem_base, kTmemCols);
     tmem_relinquish();
   }
-  griddep_wait();  // what the kernels before wrote is read from here on
-  griddep_launch();
   if (warp == 0) wgrad_list_groups(a, s_groups, lane);
   tc_fence_before();
   __syncthreads();

@@ -52,9 +52,9 @@ inline cudaError_t launch_maybe_pdl(void (*kernel)(KArgs...), int grid, int bloc
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// The kernels of the expert computation are launched the same way unless MOONEP_PDL=0: their barriers and TMEM are set up
-// while the kernel before drains (about 2 us between one and the next otherwise).  Not where they leave SMs to another stream
-// (num_sms > 0): the next kernel in line would take them.
+// The kernels of the expert computation are launched the same way unless MOONEP_PDL=0: their barriers are set up and their
+// CTAs placed while the kernel before drains (about 2 us between one and the next otherwise).  Not where they leave SMs to
+// another stream (num_sms > 0): the next kernel in line would take them.
 inline bool expert_pdl(int num_sms) {
   if (num_sms > 0) return false;
   const char* v = getenv("MOONEP_PDL");
