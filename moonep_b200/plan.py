@@ -150,7 +150,7 @@ class MoonEPCommPlan(_PackSlot):
             return [None if t is None else t.data_ptr() for t in (getattr(self, name) for name in _FIELDS)]
         p = [t.data_ptr() for t in pack.parts]
         out = [p[part] + at for part, at in pack.layout.places]
-        for name, t in pack.made.items():
+        for name, t in list(pack.made.items()):  # another thread may be making one
             out[pack.layout.index[name]] = t.data_ptr()
         return out
 
