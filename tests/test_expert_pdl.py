@@ -38,3 +38,25 @@ def test_layer_steps_with_and_without(S, K, E, monkeypatch):
 
     for a, b in zip(steps("1"), steps("0")):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("S,K,E", [(24, 2, 4), (700, 3, 5)])
+def test_captured_forward_follows_its_inputs(S, K, E):
+    """The same kernels as nodes of a graph: replays on new inputs equal the calls."""
+    buf = Buffer(S, 256, K, E, 1, num_sms=8, token_padding=128)
+    layer = ExpertParallelMoE(buf, 256, init_std=0.05, seed=3)
+    g = torch.Generator().manual_seed(1)
+    x = torch.randn(S, 256, generator=g).to(torch.bfloat16).cuda()
+    topk, tpe, gates = (t.cuda() for t in make_routing("softmax", S, K, E, 1, 0, seed=1))
+    step = buf.capture(lambda: layer.forward(x, gates, topk, tpe, save_for_backward=False)[0])
+    for i in range(3):
+        new = make_routing("softmax", S, K, E, 1, 0, seed=10 + i)
+        for dst, src in zip((topk, tpe, gates), new):
+            dst.copy_(src)
+        x.copy_(torch.randn(S, 256, generator=g))
+        got = step.replay().clone()
+        want = layer.forward(x, gates, topk, tpe, save_for_backward=False)[0]
+        assert torch.equal(got, want)
+    layer.check()
+    layer.destroy()
+    buf.destroy()
