@@ -100,6 +100,14 @@ def test_prefetch_paths_on_odd_sizes(path, stages, monkeypatch):
     _prefetch_and_reduce_grad("cuda", "fan_in", 4, Hw=128, Hp=128, epn=2, B=12, num_sms=2)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("Hw,Hp,B,num_sms", [(128, 128, 1, 148), (1024, 1152, 1, 1), (640, 896, 1, 40), (384, 640, 40, 3)])
+def test_slots_are_cut_into_even_pieces(Hw, Hp, B, num_sms):
+    """From pieces of the smallest size, fewer than there are warps, to several rounds of the largest, the last one ragged."""
+    for table in ("fan_in", "random", "empty"):
+        _prefetch_and_reduce_grad("cuda", table, 2, Hw=Hw, Hp=Hp, epn=2, B=B, num_sms=num_sms)
+
+
 @pytest.mark.parametrize("device", DEVICES)
 def test_reduce_grad_one_weight_at_a_time(device):
     """A weight whose gradient and reduce buffer are both None is left out; three calls with one weight each
