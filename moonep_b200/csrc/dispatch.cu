@@ -22,6 +22,10 @@
 //            a copy of src_info and link words in the plan), then copies each primary row to its
 //            duplicate rows as soon as the primary's row flag shows it has landed.  Ends with a wait for
 //            every peer's FLAG_SENT, so all rows of the shard are present when the kernel is.
+//   OWN      in launches of single roles only: the CTAs beside the senders clear the pad rows and write the rows of this
+//            rank's own tokens, which need nothing of a peer; the EXPAND launch is left with the rows of other ranks.
+//            Two emulated ranks, S=4096, H=7168, K=8, E=64: the 117 MB that the 32 senders move keep HBM busy to a
+//            third, and the two launches of a rank took 70 + 115 us.
 //
 // CTA order: TABLES is CTA 0, senders follow, expanders come last, so a CTA only ever waits for CTAs with a
 // lower index (which the hardware dispatches first) or for other GPUs.  Every wait is bounded.
@@ -95,7 +99,9 @@ struct DispatchArgs {
   int bulk;
   int expand_bulk;  // EXPAND copies through shared memory with bulk copies (needs (kExpandCopyWarps + 1) pieces of smem)
   int build_only;  // EXPAND: only build the duplicate map (no zero fill, no copies)
-  int local_rows;  // rows whose source is this rank are written by EXPAND from the input; SEND skips them
+  int local_rows;  // rows whose source is this rank are written by EXPAND (or OWN) from the input; SEND skips them
+  int n_own;       // CTAs with the OWN role, behind the senders
+  int own_done;    // EXPAND: the launch before had the OWN role
   int publish;     // the launch starts with the exchange plan_publish does as a kernel of its own
   const int* tpe_row;  // [E] this rank's tokens per expert, pushed to every peer by the publish step (null: a [R, E]
                        // table was given and nothing is pushed)
@@ -302,6 +308,7 @@ __device__ __forceinline__ bool flagq_push(const MoonepDevCtx& c, FlagQueue& q, 
 }
 
 // Helper warp of bulk warp w: release the row flags of every token the bulk warp hands over.
+template <bool kOwn>
 __device__ void flag_helper(const MoonepDevCtx& c, const DispatchArgs& a, int epoch, FlagQueue& q, int w) {
   const int lane = threadIdx.x & 31;
   int consumed = 0;
@@ -329,7 +336,9 @@ __device__ void flag_helper(const MoonepDevCtx& c, const DispatchArgs& a, int ep
     if (avail <= 0) break;
     // A system-scope fence waits for everything this SM has in flight, so it is paid once per batch: lane 0
     // fences, then stores the flags of all tokens that have queued up meanwhile.
-    if (lane == 0) fence_sys();
+    if (lane == 0) {
+      if (kOwn) fence_gpu(); else fence_sys();
+    }
     for (int i = 0; i < avail; ++i, ++consumed) {
       const int tok = q.tok[w][consumed % kFlagQ];
       int* f = nullptr;
@@ -337,7 +346,8 @@ __device__ void flag_helper(const MoonepDevCtx& c, const DispatchArgs& a, int ep
         const int d = a.dst[tok * c.K + lane];
         int dest, loff;
         decode_dst(d, c.NvS, dest, loff);
-        if (d >= 0 && dst_in_range(c, dest, loff) && !(a.local_rows && dest == c.rank)) f = rowflag_ptr(c, dest, loff);
+        if (dst_in_range(c, dest, loff) && (kOwn ? dest == c.rank : d >= 0 && !(a.local_rows && dest == c.rank)))
+          f = rowflag_ptr(c, dest, loff);
       }
       unsigned m = __ballot_sync(0xffffffffu, f != nullptr);
       while (m) {
@@ -419,11 +429,14 @@ __device__ void send_ldst(const MoonepDevCtx& c, const DispatchArgs& a, int epoc
 // ---- send role, bulk-copy path -----------------------------------------------------------------
 
 // Runs in warps 0..kBulkWarps-1 of a sender CTA.  s_ring: [kBulkWarps][kBulkStages][chunk_bytes],
-// s_bar: [kBulkWarps][kBulkStages] initialised mbarriers (count 1).  Returns false after a timeout.
+// s_bar: [kBulkWarps][kBulkStages] initialised mbarriers (count 1).  kOwn: the OWN role, which writes a token's rows on this
+// rank, duplicates included, instead of its primary rows on other ranks.  Returns false after a timeout.
+template <bool kOwn>
 __device__ bool send_bulk(const MoonepDevCtx& c, const DispatchArgs& a, int epoch, unsigned char* s_ring,
                           unsigned long long* s_bar, FlagQueue& fq) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int* work = c.counters + MOONEP_CTR_SEND_WORK;
+  int* work = c.counters + (kOwn ? MOONEP_CTR_OWN_WORK : MOONEP_CTR_SEND_WORK);
+  constexpr int kKernelId = kOwn ? MOONEP_K_DISPATCH_EXPAND : MOONEP_K_DISPATCH_SEND;
   const int H = c.H, K = c.K, S = c.S;
   const long long row_bytes = (long long)H * 2;
   unsigned char* ring = s_ring + (size_t)warp * kBulkStages * a.chunk_bytes;
@@ -451,7 +464,7 @@ __device__ bool send_bulk(const MoonepDevCtx& c, const DispatchArgs& a, int epoc
     for (int q = 0; q < kBulkBatch; ++q) {
       const bool in = lane < K && first + q < S;
       t.d[q] = in ? a.dst[(first + q) * K + lane] : 0;
-      t.w[q] = in && a.weights != nullptr ? a.weights[(first + q) * K + lane] : 0.f;
+      t.w[q] = !kOwn && in && a.weights != nullptr ? a.weights[(first + q) * K + lane] : 0.f;
     }
   };
   int first_batch = 0;
@@ -461,7 +474,11 @@ __device__ bool send_bulk(const MoonepDevCtx& c, const DispatchArgs& a, int epoc
   }
   load_batch(__shfl_sync(0xffffffffu, first_batch, 0), next);
   auto put_weight = [&](int dest, int loff, float w) {
-    if (a.weights != nullptr) reinterpret_cast<float*>(c.meta_peer[dest] + c.weights_off)[loff] = w;
+    if (!kOwn && a.weights != nullptr) reinterpret_cast<float*>(c.meta_peer[dest] + c.weights_off)[loff] = w;
+  };
+  // lanes whose routing entry's row this role writes
+  auto writes = [&](bool valid, int d, int dest) {
+    return valid && (kOwn ? dest == c.rank : d >= 0 && !(a.local_rows && dest == c.rank));
   };
   auto next_item = [&](int& tok, int& ch, int& d, float& w) -> bool {
     for (;;) {
@@ -478,15 +495,15 @@ __device__ bool send_bulk(const MoonepDevCtx& c, const DispatchArgs& a, int epoc
       for (int q = 0; q < kBulkBatch; ++q)
         if (q == pos) d = cur.d[q], w = cur.w[q];
       if (a.local_rows && ch == 0) {
-        // a token whose rows all stay on this rank is the EXPAND role's: only its gate weights are stored here
+        // a token whose rows all stay on this rank is the EXPAND or OWN role's: only its gate weights are stored here
         int dest = 0, loff = 0;
         bool valid = false;
         if (lane < K) {
           decode_dst(d, c.NvS, dest, loff);
           valid = dst_in_range(c, dest, loff);
         }
-        if (__ballot_sync(0xffffffffu, valid && d >= 0 && dest != c.rank) == 0) {
-          if (lane < K && !valid) record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_DISPATCH_SEND, 6, d, tok, lane);
+        if (__ballot_sync(0xffffffffu, writes(valid, d, dest)) == 0) {
+          if (lane < K && !valid) record_status(c, MOONEP_STATUS_BAD_INDEX, kKernelId, 6, d, tok, lane);
           if (valid) put_weight(dest, loff, w);
           ++pos;
           continue;
@@ -529,7 +546,7 @@ __device__ bool send_bulk(const MoonepDevCtx& c, const DispatchArgs& a, int epoc
     if (lane == 0) {
       const int ftok = fq.lagged[warp][j % (kFlagLag + 4)];
       if (ftok >= 0 && !flagq_push(c, fq, warp, pushed, ftok)) {
-        record_status(c, MOONEP_STATUS_TIMEOUT, MOONEP_K_DISPATCH_SEND, 101, warp, pushed, ftok);
+        record_status(c, MOONEP_STATUS_TIMEOUT, kKernelId, 101, warp, pushed, ftok);
         failed = true;  // lane 0 only; the loop condition below is evaluated after a warp-wide exchange
       }
     }
@@ -560,15 +577,15 @@ __device__ bool send_bulk(const MoonepDevCtx& c, const DispatchArgs& a, int epoc
     if (lane < K) {
       decode_dst(d, c.NvS, dest, loff);
       valid = dst_in_range(c, dest, loff);
-      if (!valid) record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_DISPATCH_SEND, 6, d, ctok, lane);
+      if (!valid) record_status(c, MOONEP_STATUS_BAD_INDEX, kKernelId, 6, d, ctok, lane);
     }
     if (valid && cch == 0) put_weight(dest, loff, w);
-    unsigned m = __ballot_sync(0xffffffffu, valid && d >= 0 && !(a.local_rows && dest == c.rank));
+    unsigned m = __ballot_sync(0xffffffffu, writes(valid, d, dest));
     int got = 1;
     if (lane == 0) got = mbar_wait(bar + s, (unsigned)((done / kBulkStages) & 1), c.timeout_ns) ? 1 : 0;
     got = __shfl_sync(0xffffffffu, got, 0);
     if (!got) {
-      if (lane == 0) record_status(c, MOONEP_STATUS_TIMEOUT, MOONEP_K_DISPATCH_SEND, 100, s, done, ctok);
+      if (lane == 0) record_status(c, MOONEP_STATUS_TIMEOUT, kKernelId, 100, s, done, ctok);
       failed = true;
       break;
     }
@@ -770,6 +787,7 @@ __device__ bool expand_as_rows_arrive(const MoonepDevCtx& c, const DispatchArgs&
           if (token >= c.S) token = -1;
         }
         if (e <= -2 && token < 0) primary = -1;  // a lone row of another rank's token: nothing to do here
+        if (a.own_done && token >= 0) primary = -1;
         ready = primary < 0 || token >= 0 || ld_acquire_sys(rowflag + primary) - epoch >= 0;
       }
       unsigned now = __ballot_sync(0xffffffffu, ready);
@@ -834,8 +852,8 @@ __device__ __forceinline__ int dealt_rows(int n, int xcnt) {
 // With a.expand_bulk the copies go through shared memory with bulk copies: warps 0..kExpandCopyWarps-1 own one piece
 // of chunk_bytes each in s_dyn, followed by one piece of zeros that the zero fill stores from.
 __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xidx, int xcnt, bool ok, unsigned char* s_dyn,
-                            unsigned long long* s_xbar, int* s_scratch) {
-  __shared__ int s_groups[kExpandSlice];  // group numbers found by this CTA in the current slice
+                            unsigned long long* s_xbar, int* s_groups, int* s_scratch) {
+  // s_groups: kExpandSlice words, group numbers found by this CTA in the current slice
   __shared__ int s_ngroups;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const bool bulk = a.expand_bulk != 0;
@@ -857,7 +875,7 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
     ok = wait_local_epoch(c, MOONEP_CTR_TABLES_READY, abs_epoch(c, MOONEP_FLAG_PLAN, a.epoch_plan),
                           MOONEP_K_DISPATCH_EXPAND) && ok;
   unsigned long long t0 = globaltimer_ns();
-  if (ok && a.zero_fill != nullptr && !a.build_only)
+  if (ok && a.zero_fill != nullptr && !a.build_only && !a.own_done)
     zero_fill_rows(c, a.zero_fill, a.with_weights, a.vec_ok, epoch, xidx * nwarps + warp, xcnt * nwarps, s_groups,
                    s_scratch, zeros, a.chunk_bytes);
   __syncthreads();
@@ -889,12 +907,14 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
         const int loff = dealt_row(base + threadIdx.x, xidx, xcnt);
         int dup_n = 0, first = -1;
         bool single = false;  // a primary row without duplicates whose token lives on this rank
+        bool mine = true;     // its copies are made by this launch
         if (base + (int)threadIdx.x < s1 && loff < used) {
           const int si = src_info[loff];
           const int l = si >= 0 ? link[loff] : 0;
           if (a.plan_src_info != nullptr) a.plan_src_info[loff] = si;
           if (a.plan_link != nullptr) a.plan_link[loff] = l;
-          single = a.local_rows && si >= 0 && (l & MOONEP_LINK_PRIMARY) && !(l & MOONEP_LINK_HAS_NEXT) &&
+          mine = !(a.own_done && si >= 0 && si / NvS == c.rank);
+          single = a.local_rows && mine && si >= 0 && (l & MOONEP_LINK_PRIMARY) && !(l & MOONEP_LINK_HAS_NEXT) &&
                    si / NvS == c.rank;
           if (si >= 0 && (l & MOONEP_LINK_PRIMARY) && (l & MOONEP_LINK_HAS_NEXT)) {
             first = l & MOONEP_NVS_MASK;
@@ -921,6 +941,7 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
         }
         const unsigned has = __ballot_sync(0xffffffffu, dup_n > 0);
         if (has == 0) continue;
+        const unsigned listed = __ballot_sync(0xffffffffu, dup_n > 0 && mine);
         int incl = dup_n;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -932,7 +953,7 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
         if (lane == 0) {
           gbase = atomicAdd(a.dup_counts, __popc(has));
           dbase = atomicAdd(a.dup_counts + 1, total);
-          lbase = atomicAdd(&s_ngroups, __popc(has));
+          lbase = atomicAdd(&s_ngroups, __popc(listed));
         }
         gbase = __shfl_sync(0xffffffffu, gbase, 0);
         dbase = __shfl_sync(0xffffffffu, dbase, 0);
@@ -941,6 +962,7 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
           const int before = __popc(has & ((1u << lane) - 1u));
           const int g = gbase + before;
           const int ds = dbase + incl - dup_n;
+          int entry = -1;
           if (g < NvS && ds + dup_n <= NvS) {
             a.dup_groups[3 * g] = loff;
             a.dup_groups[3 * g + 1] = ds;
@@ -950,10 +972,9 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
               a.dup_loffs[ds + q] = cur;
               cur = link[cur] & MOONEP_NVS_MASK;
             }
-            s_groups[lbase + before] = g;
-          } else {
-            s_groups[lbase + before] = -1;
+            entry = g;
           }
+          if (mine) s_groups[lbase + __popc(listed & ((1u << lane) - 1u))] = entry;
         }
       }
       __syncthreads();
@@ -974,7 +995,7 @@ __device__ bool expand_role(const MoonepDevCtx& c, const DispatchArgs& a, int xi
       ok = expand_as_rows_arrive(
           c, a, (ngroups - g0 + gstride - 1) / gstride, [&](int k) { return g0 + k * gstride; }, a.plan_src_info, epoch,
           lane, bulk, my_stage, s_xbar + warp, xphase, pend);
-    if (a.local_rows && a.plan_src_info != nullptr && a.plan_link != nullptr) {
+    if (a.local_rows && !a.own_done && a.plan_src_info != nullptr && a.plan_link != nullptr) {
       // the lone primary rows of this rank's own tokens: found in the plan's copy of the link words, a slice of rows
       // per CTA and round
       const int share = dealt_rows(NvS, xcnt);
@@ -1028,6 +1049,7 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const Moo
   __shared__ TokenScratch s_tok;
   __shared__ FlagQueue s_fq;
   __shared__ __align__(8) unsigned long long s_xbar[kExpandCopyWarps];
+  __shared__ int s_groups[kExpandSlice];
   const int roles = a.roles;
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x < kBulkWarps * kBulkStages) mbar_init(s_bar + threadIdx.x, 1);
@@ -1158,9 +1180,9 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const Moo
     if (ok) {
       if (a.bulk) {
         if (warp < kBulkWarps)
-          send_bulk(c, a, epoch, s_dyn, s_bar, s_fq);
+          send_bulk<false>(c, a, epoch, s_dyn, s_bar, s_fq);
         else if (warp < 2 * kBulkWarps)
-          flag_helper(c, a, epoch, s_fq, warp - kBulkWarps);
+          flag_helper<false>(c, a, epoch, s_fq, warp - kBulkWarps);
       } else {
         send_ldst(c, a, epoch);
       }
@@ -1176,7 +1198,38 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const Moo
 
   // the token stage's scratch (>= kZfChunk words) is free by now: the zero fill keeps its tables there
   static_assert(sizeof(TokenScratch) >= kZfChunk * sizeof(int) && kExpandSlice >= kZfChunk, "scratch too small");
-  if (is_expander) expand_role(c, a, xidx, xcnt, ok, s_dyn, s_xbar, reinterpret_cast<int*>(&s_tok));
+  int* s_scratch = reinterpret_cast<int*>(&s_tok);
+  const int oidx = (int)blockIdx.x - a.n_send;
+  if (!mixed && oidx >= 0 && oidx < a.n_own) {
+    if (a.fresh && a.wait_family < 0)
+      ok = wait_local_epoch(c, MOONEP_CTR_PLAN_DONE, plan_epoch, MOONEP_K_DISPATCH_EXPAND) && ok;
+    else
+      ok = block_wait_flags(c, a.wait_family, a.wait_epoch, MOONEP_K_DISPATCH_EXPAND) && ok;
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    const int epoch = abs_epoch(c, MOONEP_FLAG_SENT, a.epoch_sent);
+    unsigned long long t0 = globaltimer_ns();
+    if (ok) {
+      unsigned char* zeros = s_dyn + (size_t)kBulkWarps * kBulkStages * a.chunk_bytes;
+      for (int i = threadIdx.x; i < a.chunk_bytes / 16; i += blockDim.x)
+        reinterpret_cast<int4*>(zeros)[i] = make_int4(0, 0, 0, 0);
+      fence_proxy_async();
+      __syncthreads();
+      const int nwarps = blockDim.x >> 5;
+      if (a.zero_fill != nullptr)
+        zero_fill_rows(c, a.zero_fill, a.with_weights, a.vec_ok, epoch, oidx * nwarps + warp, a.n_own * nwarps, s_groups, s_scratch,
+                       zeros, a.chunk_bytes);
+      if (threadIdx.x == 0) stat_phase(c, MOONEP_PH_ZERO, t0);
+      t0 = globaltimer_ns();
+      if (warp < kBulkWarps)
+        send_bulk<true>(c, a, epoch, s_dyn, s_bar, s_fq);
+      else if (warp < 2 * kBulkWarps)
+        flag_helper<true>(c, a, epoch, s_fq, warp - kBulkWarps);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) stat_phase(c, MOONEP_PH_BUILD_EXPAND, t0);
+    if (role_tail(c, MOONEP_CTR_OWN_ARRIVE, a.n_own) && threadIdx.x == 0) c.counters[MOONEP_CTR_OWN_WORK] = 0;
+  }
+  if (is_expander) expand_role(c, a, xidx, xcnt, ok, s_dyn, s_xbar, s_groups, s_scratch);
 }
 
 }  // namespace
@@ -1220,7 +1273,8 @@ extern "C" int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk,
   // the modifier needs the input rows in the EXPAND launch and src_info of the landed rows
   a.local_rows = ((roles & MOONEP_ROLE_LOCAL_ROWS) && hidden != nullptr && !build_only &&
                   (fresh || (plan_src_info != nullptr && plan_link != nullptr))) ? 1 : 0;
-  roles &= ~MOONEP_ROLE_LOCAL_ROWS;
+  const bool own = (roles & MOONEP_ROLE_OWN) && a.local_rows;
+  roles &= ~(MOONEP_ROLE_LOCAL_ROWS | MOONEP_ROLE_OWN);
   a.publish = ((roles & MOONEP_ROLE_PUBLISH) && (roles & MOONEP_ROLE_TOKENS) && topk != nullptr) ? 1 : 0;
   roles &= ~MOONEP_ROLE_PUBLISH;
   a.tpe_row = tpe_row;
@@ -1251,6 +1305,12 @@ extern "C" int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk,
   const bool want_bulk = !(xp != nullptr && strcmp(xp, "ldst") == 0);
   a.expand_bulk = (want_bulk && (roles & MOONEP_ROLE_EXPAND) && a.vec_ok && a.chunk_bytes % 16 == 0 && expand_bytes <= limit) ? 1 : 0;
   if (a.expand_bulk && expand_bytes > smem) smem = expand_bytes;
+  // the OWN role is made of bulk copies: a ring like the senders' and a piece of zeros; what decides it is the same in both launches
+  const size_t own_bytes = ring_bytes + (size_t)a.chunk_bytes;
+  const bool own_ok = own && want_bulk && a.bulk && own_bytes <= limit;
+  const bool own_now = own_ok && (roles & MOONEP_ROLE_SEND) && !(roles & MOONEP_ROLE_EXPAND);
+  a.own_done = own_ok && !(roles & MOONEP_ROLE_SEND) ? 1 : 0;
+  if (own_now && own_bytes > smem) smem = own_bytes;
   a.tables_in_smem = 0;
   if (roles & MOONEP_ROLE_TABLES) {
     const size_t tb = (size_t)table_words(c.R, c.E) * sizeof(int);
@@ -1278,17 +1338,19 @@ extern "C" int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk,
   int grid = 1;
   a.n_send = 0;
   if (senders) {
-    a.n_send = imax(1, imin(n_send > 0 ? n_send : c.num_sms, h->sm_count - (expanders ? 2 : 0)));
+    a.n_send = imax(1, imin(n_send > 0 ? n_send : c.num_sms, h->sm_count - (expanders || own_now ? 2 : 0)));
     // a single rank whose rows are all written by the EXPAND role: the senders only store gate weights
     if (c.R == 1 && a.local_rows && expanders) a.n_send = imin(a.n_send, 4);
     grid = a.n_send;
     // planning is local work: as many CTAs as there are blocks of tokens (S=4096, K=8 on 32 CTAs: 19 us of planning each way, 10 on 64)
     if (!expanders && (roles & MOONEP_ROLE_TOKENS)) grid = imax(grid, imin(a.n_blocks, imin(c.local_sms, h->sm_count)));
   }
-  if (expanders) {
+  a.n_own = 0;
+  if (expanders || own_now) {
     const int room = imax(1, imin(c.local_sms, h->sm_count) - a.n_send);
     const int nx = n_expand > 0 ? imin(n_expand, room) : room;
-    grid = a.n_send + imax(1, nx);
+    if (own_now) a.n_own = imax(1, nx);
+    grid = imax(own_now ? grid : 0, a.n_send + imax(1, nx));
   }
   if (int rc = check_cuda(launch_maybe_pdl(dispatch_kernel, grid, kDispatchThreads, smem, (cudaStream_t)stream,
                                            h->enable_pdl != 0, c, a),

@@ -79,6 +79,8 @@
 #define MOONEP_CTR_PREFETCH_ARRIVE 26  // CTAs of the prefetch kernel that reached its end
 #define MOONEP_CTR_FOLD_WORK 27      // group hand-out of the combine fold role
 #define MOONEP_CTR_PUBLISH_ARRIVE 28 // CTAs of the dispatch kernel that finished the publish role
+#define MOONEP_CTR_OWN_WORK 29       // token hand-out of the dispatch kernel's OWN role
+#define MOONEP_CTR_OWN_ARRIVE 30     // CTAs that finished the OWN role
 // stats[MOONEP_STAT_WAIT_MAX_NS + family]: longest time CTA 0 of any kernel spun on a flag of that family (ns);
 // stats[MOONEP_STAT_WAIT_COUNT + family]: number of such waits that did not find the flag already set.
 #define MOONEP_STAT_WAIT_MAX_NS 0
@@ -121,6 +123,10 @@
 // The launch begins with what plan_publish does as a kernel of its own (push of the tokens-per-expert row, reset of
 // src_info, per-block expert counts, FLAG_TPE to every peer), spread over all CTAs of the launch.
 #define MOONEP_ROLE_PUBLISH 32
+// Modifier of MOONEP_ROLE_LOCAL_ROWS for launches of single roles (emulated ranks), given to the SEND and the EXPAND launch
+// alike: the CTAs that the senders leave free in the SEND launch clear the pad rows and write the rows of this rank's own
+// tokens, primary rows and duplicates, and the EXPAND launch leaves both out.
+#define MOONEP_ROLE_OWN 64
 // Roles of the push-combine kernel.
 #define MOONEP_ROLE_PUSH 1     // expert side: copy primary rows (folded where they have duplicates) to the tokens' home ranks
 #define MOONEP_ROLE_SUM 2      // home side: sum the rows of a token as they arrive

@@ -47,6 +47,7 @@ _KERNEL_NAMES = {
 _PHASE_NAMES = ("tables", "tokens", "send", "zero_fill", "wait_plan", "build_expand", "wait_sent", "fold", "push", "sum")
 ROLE_TABLES, ROLE_TOKENS, ROLE_SEND, ROLE_EXPAND = 1, 2, 4, 8
 ROLE_PUBLISH = 32  # modifier: the launch begins with the exchange that plan_publish does as a kernel of its own
+ROLE_OWN = 64  # modifier: in launches of single roles, the rows of this rank's own tokens and the pad rows go with SEND
 ROLE_LOCAL_ROWS = 16  # modifier: EXPAND writes the rows of this rank's own tokens from the input, SEND skips them
 ROLE_PUSH, ROLE_SUM, ROLE_FOLD = 1, 2, 4
 ROLE_LOCAL_HOME = 8  # modifier: rows of this rank's own tokens go from FOLD straight into the local staging chunk
@@ -105,7 +106,8 @@ class CudaBackend:
         # the planner's alloc[d*E+e]; only current when its tables did not fit shared memory (use global_alloc())
         c["alloc"] = self.tables[2 * E : 2 * E + R * E]
         # Emulated ranks share one GPU and one stream: a kernel of one rank must never wait for a kernel of another
-        # rank that is launched later, so they run the dispatch and combine kernels one role per phase.
+        # rank that is launched later, so they run the dispatch and combine kernels in phases: TABLES, TOKENS, SEND and OWN,
+        # then EXPAND; FOLD and PUSH, then SUM.
         self.phased = (bool(getattr(world, "emulated", False)) and world.size > 1) or config.force_phased()
         # one rank: dispatch and combine are kernels of their own (csrc/single_rank.cu)
         self.single = R == 1 and bool(self.lib.moonep_single_supported(E, B, S, K)) and not self.phased
@@ -378,6 +380,8 @@ class CudaBackend:
         with_w = route_weights_sk is not None
         self._sent_weights = with_w
         lr = ROLE_LOCAL_ROWS if config.local_rows_by_expand() else 0
+        if lr and self.phased and not config.force_phased() and (planning_args is not None or inter_rank_sync):
+            lr |= ROLE_OWN  # a peer that still reads this rank's rows has been waited for when they are written
         self.counts_checked = False
         if self.single and lr and (planning_args is None or config.planner_on_gpu()):
             self.counts_checked = self.exact_counts
