@@ -525,8 +525,11 @@ class CudaBackend:
         if not self.phased:
             self._call("moonep_combine_push", ROLE_FOLD | ROLE_PUSH | ROLE_SUM | lh, *args, tag="combine_fused")
         else:
-            self._call("moonep_combine_push", ROLE_FOLD | lh, *args, tag="combine_fold")
-            self._call("moonep_combine_push", ROLE_PUSH | lh, *args, tag="combine_push")
+            if config.force_phased():  # per-role timing
+                self._call("moonep_combine_push", ROLE_FOLD | lh, *args, tag="combine_fold")
+                self._call("moonep_combine_push", ROLE_PUSH | lh, *args, tag="combine_push")
+            else:  # neither role waits for a launch of another rank
+                self._call("moonep_combine_push", ROLE_FOLD | ROLE_PUSH | lh, *args, tag="combine_fold_push")
             self.world.step()
             self._call("moonep_combine_push", ROLE_SUM | lh, *args, tag="combine_sum")
         self.world.step()
