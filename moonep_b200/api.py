@@ -27,7 +27,7 @@ from . import config
 from .constants import FLAG_PLAN, FLAG_READY
 from .layout import check_encoding_bounds, compute_layout
 from .parallel.world import World, make_world
-from .plan import MoonEPCommPlan, allocate_planning_outputs, check_plan_for_ctx, check_planning_outputs
+from .plan import MoonEPCommPlan, allocate_planning_outputs, check_plan_for_ctx
 
 logger = logging.getLogger(__name__)
 
@@ -282,9 +282,9 @@ class Buffer:
 
     # -- dispatch ---------------------------------------------------------------------
     def _run_dispatch(self, ctx, hidden_sh, route_weights_sk, planning_args, plan, hidden_nvsh, route_weights_nvs,
-                      *, inter_rank_sync, zero_copy):  # fmt: skip
+                      inter_rank_sync, zero_copy):  # fmt: skip
         be = ctx["_backend"]
-        if hasattr(be, "dispatch_all"):  # CUDA: fused launches (one role per phase for emulated ranks)
+        if hasattr(be, "dispatch_all"):  # CUDA: fused launches (in phases for emulated ranks)
             copy_to = None if zero_copy else (hidden_nvsh, route_weights_nvs)
             if not be.dispatch_all(hidden_sh, route_weights_sk, plan, planning_args, inter_rank_sync, copy_to) and copy_to:
                 be.copy_out(*copy_to)
@@ -334,11 +334,12 @@ class Buffer:
                 "a fresh dispatch needs topk_experts_sk and tokens_per_expert"
             )
             assert topk_experts_sk.numel() == S * K, "topk_experts_sk shape mismatch"
-            topk_flat = _contiguous_i32(topk_experts_sk.reshape(-1))
+            topk_flat = _contiguous_i32(topk_experts_sk)  # kernels read it as one list of entries
+            if not topk_flat.is_cuda:
+                topk_flat = topk_flat.reshape(-1)
             tpe = _contiguous_i32(tokens_per_expert)
             assert tpe.numel() in (ctx["E"], ctx["R"] * ctx["E"]), "tokens_per_expert must be [E] or [R, E]"
             plan, cu_seqlens = allocate_planning_outputs(ctx)
-            check_planning_outputs(ctx, cu_seqlens, plan)
             planning_args = (topk_flat, tpe, cu_seqlens)
         else:
             check_plan_for_ctx(ctx, plan, dev)
@@ -352,19 +353,14 @@ class Buffer:
                 torch.empty(NvS, dtype=torch.float32, device=dev) if route_weights_sk is not None else None
             )
 
-        def run():
-            self._run_dispatch(
-                ctx, hidden_sh, route_weights_sk, planning_args, plan, hidden_nvsh, route_weights_nvs,
-                inter_rank_sync=inter_rank_sync, zero_copy=zero_copy,
-            )  # fmt: skip
-
+        args = (ctx, hidden_sh, route_weights_sk, planning_args, plan, hidden_nvsh, route_weights_nvs, inter_rank_sync, zero_copy)
         if not async_finish:
-            run()
+            self._run_dispatch(*args)
             return hidden_nvsh, route_weights_nvs, cu_seqlens, plan
         tensors = [hidden_sh, route_weights_sk, hidden_nvsh, route_weights_nvs, *plan.tensors()]
         if planning_args is not None:
             tensors.extend(planning_args)
-        done = self._on_comm_stream(tensors, run)
+        done = self._on_comm_stream(tensors, lambda: self._run_dispatch(*args))
         return hidden_nvsh, route_weights_nvs, cu_seqlens, plan, done
 
     # -- expert weights ---------------------------------------------------------------
@@ -387,7 +383,7 @@ class Buffer:
 
     # -- combine ------------------------------------------------------------------------
     def _run_combine(self, ctx, hidden_sh, plan, hidden_nvsh, route_weights_nvs, route_weights_sk,
-                     *, inter_rank_sync, zero_copy, ready=None):  # fmt: skip
+                     inter_rank_sync, zero_copy, ready=None):  # fmt: skip
         be = ctx["_backend"]
         if hasattr(be, "combine_all"):
             rdy, expect = ready if ready is not None else (None, 0)
@@ -444,16 +440,12 @@ class Buffer:
         hidden_sh = torch.empty(S, H, dtype=torch.bfloat16, device=dev)
         route_weights_sk = torch.empty(S, K, dtype=torch.float32, device=dev) if route_weights_nvs is not None else None
 
-        def run():
-            self._run_combine(
-                ctx, hidden_sh, plan, hidden_nvsh, route_weights_nvs, route_weights_sk,
-                inter_rank_sync=inter_rank_sync, zero_copy=zero_copy, ready=ready,
-            )  # fmt: skip
-
+        args = (ctx, hidden_sh, plan, hidden_nvsh, route_weights_nvs, route_weights_sk, inter_rank_sync, zero_copy, ready)
         if not async_finish:
-            run()
+            self._run_combine(*args)
             return hidden_sh, route_weights_sk, None
-        done = self._on_comm_stream((hidden_sh, *plan.tensors(), hidden_nvsh, route_weights_nvs, route_weights_sk), run)
+        done = self._on_comm_stream((hidden_sh, *plan.tensors(), hidden_nvsh, route_weights_nvs, route_weights_sk),
+                                    lambda: self._run_combine(*args))  # fmt: skip
         return hidden_sh, route_weights_sk, done
 
     # -- gradients ----------------------------------------------------------------------

@@ -984,10 +984,13 @@ extern "C" int moonep_combine_push(void* ctx, int roles, const int* src_info, co
   }
   // The attribute belongs to the kernel, not to the launch, and emulated ranks launch from several threads with
   // different sizes: always allow the same maximum, so that no thread lowers it under another one's launch.
-  if (int rc = check_cuda(cudaFuncSetAttribute(combine_push_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               h->max_smem_optin - 8192),
-                          "cudaFuncSetAttribute(combine_push_kernel)"))
-    return rc;
+  if (!h->push_smem_set) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(combine_push_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 h->max_smem_optin - 8192),
+                            "cudaFuncSetAttribute(combine_push_kernel)"))
+      return rc;
+    h->push_smem_set = 1;
+  }
   const bool local = (roles & (MOONEP_ROLE_FOLD | MOONEP_ROLE_SUM)) != 0;
   int grid = 0;
   a.n_push = 0;

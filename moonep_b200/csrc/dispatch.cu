@@ -1329,9 +1329,12 @@ extern "C" int moonep_dispatch(void* ctx, int roles, int fresh, const int* topk,
   }
   // The attribute belongs to the kernel, not to the launch, and emulated ranks launch from several threads with
   // different sizes: always allow the same maximum, so that no thread lowers it under another one's launch.
-  if (int rc = check_cuda(cudaFuncSetAttribute(dispatch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit),
-                          "cudaFuncSetAttribute(dispatch_kernel)"))
-    return rc;
+  if (!h->dispatch_smem_set) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(dispatch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit),
+                            "cudaFuncSetAttribute(dispatch_kernel)"))
+      return rc;
+    h->dispatch_smem_set = 1;
+  }
 
   const bool senders = (roles & (MOONEP_ROLE_TOKENS | MOONEP_ROLE_SEND)) != 0;
   const bool expanders = (roles & MOONEP_ROLE_EXPAND) != 0;

@@ -19,7 +19,8 @@ struct HostCtx {
   int sm_count = 0;
   int max_smem_optin = 0;
   int enable_pdl = 0;  // launch the dispatch/combine kernels with programmatic dependent launch
-  int single_smem_set = 0;  // dispatch_single_kernel may use all of max_smem_optin
+  // the kernel may use the shared memory that its launches of this context ask for at most
+  int single_smem_set = 0, dispatch_smem_set = 0, push_smem_set = 0;
   cudaEvent_t prefetch_begun = nullptr;  // the latest marked prefetch is on its SMs (moonep_prefetch), made when first used
   int expand_ldst = 0; // MOONEP_EXPAND_PATH=ldst when the context was made (single-rank dispatch)
 };

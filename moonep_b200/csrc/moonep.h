@@ -178,6 +178,9 @@ extern "C" {
 #endif
 
 int moonep_version(void);
+// One of the functions below by number (the list is in runtime.cu), its arguments as one 64-bit word each.  Converting two
+// dozen arguments one by one costs a caller that is not C more than the launch itself.  words == null: the number of arguments.
+int moonep_call(int fn, const long long* words);
 const char* moonep_last_error(void);
 int moonep_sizeof_devctx(void);
 // Number of kernels this library has launched in the calling process.

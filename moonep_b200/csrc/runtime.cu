@@ -142,6 +142,49 @@ extern "C" int moonep_ctx_set_timeout_ms(void* ctx, long long ms) {
   return 0;
 }
 
+// ---- calls by number ------------------------------------------------------------------------------
+
+namespace {
+
+template <typename T>
+T as_arg(long long word) {
+  if constexpr (std::is_pointer_v<T>) return reinterpret_cast<T>(static_cast<uintptr_t>(word));
+  else return static_cast<T>(word);
+}
+
+template <typename... A, size_t... I>
+int call_words(int (*f)(A...), const long long* words, std::index_sequence<I...>) {
+  return f(as_arg<A>(words[I])...);
+}
+
+// words == null: the number of arguments.
+template <typename... A>
+int call_words(int (*f)(A...), const long long* words) {
+  if (words == nullptr) return (int)sizeof...(A);
+  return call_words(f, words, std::index_sequence_for<A...>{});
+}
+
+}  // namespace
+
+extern "C" int moonep_call(int fn, const long long* words) {
+  switch (fn) {
+    case 0: return call_words(moonep_dispatch_single, words);
+    case 1: return call_words(moonep_combine_single, words);
+    case 2: return call_words(moonep_dispatch, words);
+    case 3: return call_words(moonep_combine_push, words);
+    case 4: return call_words(moonep_grouped_gemm, words);
+    case 5: return call_words(moonep_grouped_gemm_pair, words);
+    case 6: return call_words(moonep_grouped_gemm_pair_hooked, words);
+    case 7: return call_words(moonep_grouped_gemm_pair_kn, words);
+    case 8: return call_words(moonep_grouped_wgrad_rows, words);
+    case 9: return call_words(moonep_signal_wait, words);
+    case 10: return call_words(moonep_plan_publish, words);
+    case 11: return call_words(moonep_swiglu_bwd, words);
+  }
+  set_error("moonep_call: no such function");
+  return -1;
+}
+
 // ---- VMM ----------------------------------------------------------------------------------------
 
 namespace {

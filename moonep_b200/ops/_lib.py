@@ -13,6 +13,7 @@ import ctypes
 import hashlib
 import os
 import shutil
+import struct
 import subprocess
 import threading
 from pathlib import Path
@@ -97,8 +98,16 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 _vp, _i, _ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
 _ull = ctypes.c_ulonglong
 
+# functions that moonep_call knows by number, in its order
+_BY_NUMBER = (
+    "moonep_dispatch_single", "moonep_combine_single", "moonep_dispatch", "moonep_combine_push", "moonep_grouped_gemm",
+    "moonep_grouped_gemm_pair", "moonep_grouped_gemm_pair_hooked", "moonep_grouped_gemm_pair_kn", "moonep_grouped_wgrad_rows",
+    "moonep_signal_wait", "moonep_plan_publish", "moonep_swiglu_bwd",
+)  # fmt: skip
+
 _SIGNATURES = {
     "moonep_version": (_i, []),
+    "moonep_call": (_i, [_i, ctypes.c_char_p]),
     "moonep_last_error": (ctypes.c_char_p, []),
     "moonep_sizeof_devctx": (_i, []),
     "moonep_launch_count": (_ll, []),
@@ -168,10 +177,30 @@ def load():
     return _lib
 
 
+_callers: dict = {}
+
+
+def caller(name: str):
+    """The library's function ``name``.  Those that ``moonep_call`` knows take plain integers (0 for a null pointer), which go
+    over as one packed block: 27 arguments cost 1 us instead of 5."""
+    fn = _callers.get(name)
+    if fn is None:
+        lib = load()
+        if name in _BY_NUMBER:
+            number, call, n = _BY_NUMBER.index(name), lib.moonep_call, len(_SIGNATURES[name][1])
+            assert call(number, None) == n, f"{name}: the library takes {call(number, None)} arguments, not {n}"
+            pack = struct.Struct(f"{n}q").pack
+            fn = lambda *args: call(number, pack(*args))  # noqa: E731
+        else:
+            fn = getattr(lib, name)
+        _callers[name] = fn
+    return fn
+
+
 def current_stream() -> int:
     """Handle of the current stream of the current device (``torch.cuda.current_stream().cuda_stream`` without the
     Stream object, whose construction costs several microseconds)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 class on_device:
@@ -180,7 +209,7 @@ class on_device:
     __slots__ = ("guard",)
 
     def __init__(self, dev: torch.device):
-        self.guard = None if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+        self.guard = None if dev.index == torch._C._cuda_getDevice() else torch.cuda.device(dev)
 
     def __enter__(self):
         if self.guard is not None:

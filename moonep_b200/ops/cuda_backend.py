@@ -55,12 +55,11 @@ _FAMILY_NAMES = {0: "READY", 1: "TPE", 2: "PLAN", 3: "SENT", 4: "COMB", 5: "GRAD
 _BIAS_OFF, _CTR_TABLES_READY = 32, 18  # words of the counters block (csrc/moonep.h)
 
 
-def _ptr(t: torch.Tensor | None) -> int | None:
-    return None if t is None else t.data_ptr()
+def _ptr(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
-def _stream() -> int:
-    return _lib.current_stream()
+_stream = _lib.current_stream
 
 
 class CudaBackend:
@@ -86,6 +85,7 @@ class CudaBackend:
             else _PATHS["ldst"]
         self._profile = None
         self._nvtx = config.nvtx()
+        self._dev_index = dev.index
         self._begun = self._begun_seen = None  # whether the latest prefetch was captured, and the stream that waits for it
         self._quiesced = False  # every peer is known to be past its last pull from this rank's shard
 
@@ -112,6 +112,7 @@ class CudaBackend:
         # one rank: dispatch and combine are kernels of their own (csrc/single_rank.cu)
         self.single = R == 1 and bool(self.lib.moonep_single_supported(E, B, S, K)) and not self.phased
         self.single_work = i32(self.lib.moonep_single_work_words()) if self.single else None
+        self._single_work_ptr = _ptr(self.single_work)
         # set around a dispatch whose rows are used whether or not something landed in them (the MoE layer's products without
         # row flags): counts above what was routed are then an index error, if the dispatch that runs can tell
         self.exact_counts = False
@@ -257,20 +258,26 @@ class CudaBackend:
         self._quiesced = end["quiesced"]
 
     def _call(self, name, *args, tag=None):
+        fn = _lib.caller(name)
+        if self._profile is None and not self._nvtx and torch._C._cuda_getDevice() == self._dev_index:
+            rc = fn(self.handle, *args)
+            if rc != 0:
+                _lib.check(rc, name)
+            return
         with _lib.on_device(self.ctx["device"]):
             if self._nvtx:
                 torch.cuda.nvtx.range_push(tag or name)
                 try:
-                    _lib.check(getattr(self.lib, name)(self.handle, *args), name)
+                    _lib.check(fn(self.handle, *args), name)
                 finally:
                     torch.cuda.nvtx.range_pop()
                 return
             if self._profile is None:
-                _lib.check(getattr(self.lib, name)(self.handle, *args), name)
+                _lib.check(fn(self.handle, *args), name)
                 return
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-            _lib.check(getattr(self.lib, name)(self.handle, *args), name)
+            _lib.check(fn(self.handle, *args), name)
             e1.record()
             self._profile.append((tag or name.replace("moonep_", ""), e0, e1))
 
@@ -311,7 +318,7 @@ class CudaBackend:
     def plan_compute(self, topk_flat, tpe, cu_seqlens, plan):
         if not config.planner_on_gpu():
             return self._plan_compute_host(topk_flat, tpe, cu_seqlens, plan)
-        tpe2d = _ptr(tpe) if tpe.dim() == 2 else None
+        tpe2d = _ptr(tpe) if tpe.dim() == 2 else 0
         self._call(
             "moonep_plan_compute", _ptr(topk_flat), tpe2d, _ptr(plan.dst), _ptr(cu_seqlens),
             _ptr(plan.experts_to_copy), _ptr(plan.zero_fill_ranges), _ptr(plan.remote_stats), _ptr(plan.dup_counts),
@@ -359,13 +366,12 @@ class CudaBackend:
                          with_weights=False, wait_family=-1, wait_epoch=0, epoch_sent=0, n_send=0, build_only=False,
                          tag=None):  # fmt: skip
         """One launch of the dispatch kernel with the given roles (``csrc/dispatch.cu``)."""
-        tpe2d = _ptr(tpe) if (tpe is not None and tpe.dim() == 2) else None
-        tpe_row = _ptr(tpe) if (tpe is not None and tpe.dim() == 1 and (roles & ROLE_PUBLISH)) else None
+        tpe2d = _ptr(tpe) if (tpe is not None and tpe.dim() == 2) else 0
+        tpe_row = _ptr(tpe) if (tpe is not None and tpe.dim() == 1 and (roles & ROLE_PUBLISH)) else 0
+        dst, etc, zf, rs, dg, dl, dc, si, lk = plan._addresses()
         self._call(
-            "moonep_dispatch", int(roles), int(bool(fresh)), _ptr(topk), tpe2d, _ptr(plan.dst), _ptr(cu_seqlens),
-            _ptr(plan.experts_to_copy), _ptr(plan.zero_fill_ranges), _ptr(plan.remote_stats), _ptr(hidden),
-            _ptr(weights), int(bool(with_weights)), _ptr(plan.dup_groups), _ptr(plan.dup_loffs), _ptr(plan.dup_counts),
-            _ptr(plan.src_info), _ptr(plan.link), int(wait_family), int(wait_epoch), self._cur(FLAG_TPE),
+            "moonep_dispatch", int(roles), int(bool(fresh)), _ptr(topk), tpe2d, dst, _ptr(cu_seqlens), etc, zf, rs, _ptr(hidden),
+            _ptr(weights), int(bool(with_weights)), dg, dl, dc, si, lk, int(wait_family), int(wait_epoch), self._cur(FLAG_TPE),
             self._cur(FLAG_PLAN), int(epoch_sent), self.send_path, int(n_send), int(self.n_expand), int(bool(build_only)),
             tpe_row, _stream(),
             tag=tag,
@@ -444,16 +450,18 @@ class CudaBackend:
         """Fresh or replayed dispatch of a single rank: one launch, no READY round (there are no peers to wait for)."""
         topk, tpe, cu = planning_args if planning_args is not None else (None, None, None)
         out, out_w = copy_to if copy_to is not None else (None, None)
+        epoch, bias = self.epoch, self.bias
         if topk is not None:
             self._topk = topk
-            self._next(FLAG_TPE)
-            self._next(FLAG_PLAN)
+            epoch[FLAG_TPE] += 1
+            epoch[FLAG_PLAN] += 1
+        epoch[FLAG_SENT] += 1
         dst, etc, zf, rs, dg, dl, dc, si, lk = plan._addresses()
         self._call(
-            "moonep_dispatch_single", int(topk is not None), int(self.exact_counts), _ptr(topk), _ptr(tpe), dst, _ptr(cu),
-            etc, zf, rs, dg, dl, dc, si, lk, _ptr(hidden), _ptr(weights),
-            int(weights is not None), self._cur(FLAG_TPE), self._cur(FLAG_PLAN), self._next(FLAG_SENT), self.n_expand,
-            _ptr(self.single_work), _ptr(out), _ptr(out_w), _stream(), tag="dispatch_single",
+            "moonep_dispatch_single", topk is not None, self.exact_counts, _ptr(topk), _ptr(tpe), dst, _ptr(cu),
+            etc, zf, rs, dg, dl, dc, si, lk, hidden.data_ptr(), _ptr(weights), weights is not None,
+            epoch[FLAG_TPE] - bias[FLAG_TPE], epoch[FLAG_PLAN] - bias[FLAG_PLAN], epoch[FLAG_SENT] - bias[FLAG_SENT],
+            self.n_expand, self._single_work_ptr, _ptr(out), _ptr(out_w), _stream(), tag="dispatch_single",
         )  # fmt: skip
 
     def copy_out(self, out_hidden, out_weights):
@@ -518,10 +526,10 @@ class CudaBackend:
         comb = self._next(FLAG_COMB)
         lh = ROLE_LOCAL_HOME if config.local_home_by_fold() else 0
         fold_buf, fold_flag = self._fold_scratch()
-        args = (_ptr(plan.src_info), _ptr(plan.link), _ptr(plan.dst), _ptr(hidden_nvsh), _ptr(route_weights_nvs),
-                _ptr(out_hidden), _ptr(out_weights_sk), wf, we, comb, _ptr(ready), int(ready_expect),
-                _ptr(plan.dup_groups), _ptr(plan.dup_loffs), _ptr(plan.dup_counts), _ptr(fold_buf), _ptr(fold_flag),
-                int(fold_flag.numel()), 0, 0, _stream())  # fmt: skip
+        dst, _, _, _, dg, dl, dc, si, lk = plan._addresses()
+        args = (si, lk, dst, _ptr(hidden_nvsh), _ptr(route_weights_nvs), _ptr(out_hidden), _ptr(out_weights_sk), wf, we, comb,
+                _ptr(ready), int(ready_expect), dg, dl, dc, _ptr(fold_buf), _ptr(fold_flag), fold_flag.numel(), 0, 0,
+                _stream())  # fmt: skip
         if not self.phased:
             self._call("moonep_combine_push", ROLE_FOLD | ROLE_PUSH | ROLE_SUM | lh, *args, tag="combine_fused")
         else:
@@ -584,12 +592,14 @@ class CudaBackend:
             assert int(w.shape[1]) * int(w.shape[2]) == per, "gate, up and down must have equally sized experts"
             assert w.shape[1] % 128 == 0 and w.shape[2] % 128 == 0, f"H and H' must be multiples of 128, got {tuple(w.shape[1:])}"
         assert experts_to_copy.dtype == torch.int32 and experts_to_copy.is_contiguous()
-        row = experts_to_copy[c["rank"]]
-        self.prefetch_launch([w[:E] for w in ws], [w[E:] for w in ws], row)
+        if c["rank"] >= int(experts_to_copy.shape[0]):
+            raise IndexError(f"prefetch: rank {c['rank']} of a table for {int(experts_to_copy.shape[0])} ranks")
+        at = [w.data_ptr() for w in ws]
+        self._prefetch(at, [p + E * per * 2 for p in at], experts_to_copy.data_ptr() + 4 * c["rank"] * int(experts_to_copy.shape[1]),
+                       per, int(experts_to_copy.shape[1]), B, E)  # fmt: skip
 
     def prefetch_launch(self, remote_experts, prefetch_buffers, experts_row):
         """Launch-level form: ``remote_experts[i]`` is ``[E', H, Hp]``, ``prefetch_buffers[i]`` ``[B', H, Hp]``."""
-        n = len(remote_experts)
         nexp, H, Hp = (int(v) for v in remote_experts[0].shape)
         nslots = int(prefetch_buffers[0].shape[0])
         if nslots == 0 or experts_row.numel() == 0:
@@ -598,10 +608,16 @@ class CudaBackend:
             assert s.dtype == torch.bfloat16 and s.is_contiguous() and d.dtype == torch.bfloat16 and d.is_contiguous()
             assert s.shape[0] == nexp and d.shape[0] == nslots and s.shape[1:] == d.shape[1:]
             assert int(s.shape[1]) * int(s.shape[2]) == H * Hp, "all tensors must have equally sized experts"
-        assert experts_row.dtype == torch.int32 and experts_row.is_contiguous() and experts_row.numel() == nslots
+        assert experts_row.dtype == torch.int32 and experts_row.is_contiguous()
         assert H % 128 == 0 and Hp % 128 == 0, f"H and H' must be multiples of 128, got ({H}, {Hp})"
-        src = (ctypes.c_void_p * n)(*[t.data_ptr() for t in remote_experts])
-        dst = (ctypes.c_void_p * n)(*[t.data_ptr() for t in prefetch_buffers])
+        self._prefetch([t.data_ptr() for t in remote_experts], [t.data_ptr() for t in prefetch_buffers], experts_row.data_ptr(),
+                       H * Hp, experts_row.numel(), nslots, nexp)  # fmt: skip
+
+    def _prefetch(self, src, dst, experts_row, elems, nentries, nslots, nexp):
+        """Launch with addresses; ``experts_row`` holds ``nentries`` expert ids, which have to be one per slot."""
+        assert nentries == nslots
+        n = len(src)
+        src, dst = (ctypes.c_void_p * n)(*src), (ctypes.c_void_p * n)(*dst)
         flags = done = None
         epoch = mark = 0
         if nslots == self.ctx["B"]:  # the Buffer's own prefetch slots: per-slot flags for a GEMM that runs beside the copy
@@ -610,8 +626,8 @@ class CudaBackend:
             capturing = torch.cuda.is_current_stream_capturing()
             mark = 2 if capturing else 1
             self._begun, self._begun_seen = capturing, None
-        self._call("moonep_prefetch", src, dst, n, _ptr(experts_row), H * Hp, nslots, nexp, self.prefetch_path, _ptr(flags),
-                   _ptr(done), epoch, mark, _stream())  # fmt: skip
+        self._call("moonep_prefetch", src, dst, n, experts_row, elems, nslots, nexp, self.prefetch_path, _ptr(flags), _ptr(done),
+                   epoch, mark, _stream())  # fmt: skip
 
     def _wait_prefetch_begun(self):
         """The current stream waits until the latest prefetch is on its SMs (in a capture: has ended)."""

@@ -112,22 +112,21 @@ def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", o
         assert mode == "swiglu", "save_pre goes with mode='swiglu'"
         for t in save_pre:
             assert t.is_contiguous() and t.shape == out.shape and t.dtype == torch.bfloat16 and t.device == out.device
-    lib = _lib.load()
     use_pair = config.gemm_on_cta_pairs() if pair is None else pair
     assert hooks is None or use_pair, "hooks need the CTA-pair kernel"
     with _lib.on_device(x.device):
         args = (
-            x.data_ptr(), w.data_ptr(), None if w_up is None else w_up.data_ptr(), out.data_ptr(),
-            None if row_scale is None else row_scale.data_ptr(), cu_seqlens.data_ptr(), G, int(x.shape[0]), K, N,
-            _MODES[mode], None if status is None else status.data_ptr(), config.timeout_ms(), int(num_sms),
-            None if group_map is None else group_map.data_ptr(), W,
-            None if save_pre is None else save_pre[0].data_ptr(), None if save_pre is None else save_pre[1].data_ptr(),
+            x.data_ptr(), w.data_ptr(), 0 if w_up is None else w_up.data_ptr(), out.data_ptr(),
+            0 if row_scale is None else row_scale.data_ptr(), cu_seqlens.data_ptr(), G, int(x.shape[0]), K, N,
+            _MODES[mode], 0 if status is None else status.data_ptr(), config.timeout_ms(), int(num_sms),
+            0 if group_map is None else group_map.data_ptr(), W,
+            0 if save_pre is None else save_pre[0].data_ptr(), 0 if save_pre is None else save_pre[1].data_ptr(),
         )  # fmt: skip
         st = _lib.current_stream()
         if hooks is not None:
-            rc = lib.moonep_grouped_gemm_pair_hooked(*args, ctypes.byref(hooks), st)
+            rc = _lib.caller("moonep_grouped_gemm_pair_hooked")(*args, ctypes.addressof(hooks), st)
         else:
-            rc = (lib.moonep_grouped_gemm_pair if use_pair else lib.moonep_grouped_gemm)(*args, st)
+            rc = _lib.caller("moonep_grouped_gemm_pair" if use_pair else "moonep_grouped_gemm")(*args, st)
     _lib.check(rc, "moonep_grouped_gemm")
     return out
 
@@ -172,11 +171,10 @@ def grouped_gemm_kn(x, ws, cu_seqlens, *, out=None, status=None, num_sms=0):
     if out is None:
         out = torch.empty(x.shape[0], N, dtype=torch.bfloat16, device=x.device)
     assert out.is_contiguous() and out.shape == (x.shape[0], N) and out.dtype == torch.bfloat16
-    lib = _lib.load()
     with _lib.on_device(x.device):
-        rc = lib.moonep_grouped_gemm_pair_kn(
-            x.data_ptr(), ws[0].data_ptr(), Ks[0], ws[1].data_ptr() if len(ws) == 2 else None, Ks[1] if len(ws) == 2 else 0,
-            out.data_ptr(), cu_seqlens.data_ptr(), G, int(x.shape[0]), N, G, None if status is None else status.data_ptr(),
+        rc = _lib.caller("moonep_grouped_gemm_pair_kn")(
+            x.data_ptr(), ws[0].data_ptr(), Ks[0], ws[1].data_ptr() if len(ws) == 2 else 0, Ks[1] if len(ws) == 2 else 0,
+            out.data_ptr(), cu_seqlens.data_ptr(), G, int(x.shape[0]), N, G, 0 if status is None else status.data_ptr(),
             config.timeout_ms(), int(num_sms), _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_grouped_gemm_pair_kn")
@@ -258,11 +256,10 @@ def grouped_wgrad_rows(left, right, cu_seqlens, out_ptrs, flags, *, status=None,
     assert out_ptrs.dtype == torch.int64 and out_ptrs.numel() == G and out_ptrs.is_cuda and out_ptrs.is_contiguous()
     assert flags.dtype == torch.int32 and flags.numel() == G and flags.is_cuda and flags.is_contiguous()
     assert cu_seqlens.dtype == torch.int32 and cu_seqlens.is_contiguous() and cu_seqlens.is_cuda
-    lib = _lib.load()
     with _lib.on_device(left.device):
-        rc = lib.moonep_grouped_wgrad_rows(
+        rc = _lib.caller("moonep_grouped_wgrad_rows")(
             left.data_ptr(), ldl, right.data_ptr(), ldr, rows, P, Q, cu_seqlens.data_ptr(), G, out_ptrs.data_ptr(),
-            flags.data_ptr(), None if status is None else status.data_ptr(), config.timeout_ms(), int(rows_per_group),
+            flags.data_ptr(), 0 if status is None else status.data_ptr(), config.timeout_ms(), int(rows_per_group),
             int(adds), int(num_sms), _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_grouped_wgrad_rows")

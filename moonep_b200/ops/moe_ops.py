@@ -52,8 +52,8 @@ def swiglu_bwd(a, u, g, w, total_rows, dadu, hsw, dgate) -> None:
         assert t.is_contiguous() and t.dtype == torch.bfloat16
     assert w.dtype == torch.float32 and dgate.dtype == torch.float32 and w.is_contiguous() and dgate.is_contiguous()
     with _lib.on_device(a.device):
-        rc = _lib.load().moonep_swiglu_bwd(
-            a.data_ptr(), u.data_ptr(), g.data_ptr(), w.data_ptr(), None if total_rows is None else total_rows.data_ptr(),
+        rc = _lib.caller("moonep_swiglu_bwd")(
+            a.data_ptr(), u.data_ptr(), g.data_ptr(), w.data_ptr(), 0 if total_rows is None else total_rows.data_ptr(),
             rows, I, dadu.data_ptr(), hsw.data_ptr(), dgate.data_ptr(), _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_swiglu_bwd")

@@ -146,11 +146,11 @@ class MoonEPCommPlan(_PackSlot):
         return plan
 
     def _addresses(self):
-        """Addresses of the fields in the order of ``_FIELDS`` (None for an absent one), without making a packed plan's
+        """Addresses of the fields in the order of ``_FIELDS`` (0 for an absent one), without making a packed plan's
         tensors."""
         pack = getattr(self, "_pack", None)
         if pack is None:
-            return [None if t is None else t.data_ptr() for t in (getattr(self, name) for name in _FIELDS)]
+            return [0 if t is None else t.data_ptr() for t in (getattr(self, name) for name in _FIELDS)]
         p = [t.data_ptr() for t in pack.parts]
         out = [p[part] + at for part, at in pack.layout.places]
         for name, t in list(pack.made.items()):  # another thread may be making one
@@ -270,14 +270,16 @@ def check_plan_for_ctx(ctx: dict, plan: MoonEPCommPlan, device) -> None:
     assert isinstance(plan, MoonEPCommPlan), "plan must be a MoonEPCommPlan"
     assert plan.N == ctx["N"] and plan.R == ctx["R"] and plan.K == ctx["K"] and plan.NvS == ctx["NvS"]
     assert plan.E == ctx["E"] and plan.B == ctx["B"]
-    shapes = _field_shapes(plan.N, plan.R, plan.E, plan.B, plan.NvS)
     device = torch.device(device)
     pack = getattr(plan, "_pack", None)
     if pack is not None:  # fields not used so far are views yet to be made, in the layout of these sizes
         assert pack.parts[0].device == device, "plan is on the wrong device"
         items = list(pack.made.items())
+        if not items:
+            return
     else:
         items = [(name, getattr(plan, name)) for name in _FIELDS]
+    shapes = _field_shapes(plan.N, plan.R, plan.E, plan.B, plan.NvS)
     for name, t in items:
         if t is None:  # the two optional trailing fields
             continue

@@ -108,6 +108,21 @@ def test_slots_are_cut_into_even_pieces(Hw, Hp, B, num_sms):
         _prefetch_and_reduce_grad("cuda", table, 2, Hw=Hw, Hp=Hp, epn=2, B=B, num_sms=num_sms)
 
 
+@pytest.mark.gpu
+def test_prefetch_refuses_a_table_without_this_rank():
+    lw, bufs = _world(2, "cuda")
+    plans = _plans(lw, bufs, 2, 32, 64, 2, 8, "cuda")
+
+    def body(r):
+        plan = dataclasses.replace(plans[r], R=1, experts_to_copy=plans[r].experts_to_copy[:1].contiguous())
+        w = torch.zeros(8 + 3, 128, 128, dtype=torch.bfloat16, device="cuda")
+        if r == 1:
+            with pytest.raises(IndexError):
+                bufs[r].prefetch_weight(plan, full_gate_weight=w, full_up_weight=w, full_down_weight=w)
+
+    lw.run(body)
+
+
 @pytest.mark.parametrize("device", DEVICES)
 def test_reduce_grad_one_weight_at_a_time(device):
     """A weight whose gradient and reduce buffer are both None is left out; three calls with one weight each
