@@ -16,6 +16,7 @@ namespace moonep {
 struct HostCtx {
   MoonepDevCtx dev;
   void* peer_tables = nullptr;
+  void *hidden_own = nullptr, *meta_own = nullptr;  // this rank's chunks, as in the peer tables
   int sm_count = 0;
   int max_smem_optin = 0;
   int enable_pdl = 0;  // launch the dispatch/combine kernels with programmatic dependent launch

@@ -110,6 +110,8 @@ extern "C" void* moonep_ctx_create(const long long* p, int nparams, const unsign
     }
     d.stage_peer = (unsigned char* const*)((char*)tab + 2 * tbytes);
   }
+  h->hidden_own = (void*)(uintptr_t)hidden_peers[d.rank];
+  h->meta_own = (void*)(uintptr_t)meta_peers[d.rank];
   const char* xp = getenv("MOONEP_EXPAND_PATH");
   h->expand_ldst = xp != nullptr && strcmp(xp, "ldst") == 0 ? 1 : 0;
   cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, 0);

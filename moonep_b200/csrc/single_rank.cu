@@ -92,6 +92,8 @@ struct SingleArgs {
   int rounds;                // units of its CTA that a copy warp gets without asking
   int pads_per_grab;         // at least
   int tokens_per_cta;
+  uint16_t* shard;
+  int* meta;
   int* work;
   int epoch_tpe, epoch_plan, epoch_sent;
 };
@@ -105,7 +107,7 @@ struct Unit {
 struct SingleShared {
   unsigned long long bar[kCopyWarps * kRing];
   Unit unit[kCopyWarps][kUnits];
-  int warp_sum[kWarps];
+  int2 warp_sum[kWarps];
   int grab[kWarps - kPlanWarps][kGrabs];
   int loff[kEntries];  // destination row of every entry in hand, -1: none
   int bad;             // entries in hand without a row
@@ -114,26 +116,26 @@ struct SingleShared {
 
 __device__ __forceinline__ void plan_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kPlanWarps * 32) : "memory"); }
 
-// Inclusive prefix sum over the threads of the CTA; all threads call it.
-__device__ __forceinline__ int block_scan(int v, int* warp_sum, int& total) {
+// Inclusive prefix sums of two values over the threads of the CTA; all threads call it.
+__device__ __forceinline__ int2 block_scan(int2 v, int2* warp_sum, int2& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += u;
+    const int x = __shfl_up_sync(0xffffffffu, v.x, o), y = __shfl_up_sync(0xffffffffu, v.y, o);
+    if (lane >= o) v.x += x, v.y += y;
   }
   if (lane == 31) warp_sum[warp] = v;
   __syncthreads();
-  int before = 0;
-  total = 0;
+  int2 before = make_int2(0, 0);
+  total = make_int2(0, 0);
 #pragma unroll
   for (int w = 0; w < kWarps; ++w) {
-    const int x = warp_sum[w];
-    if (w < warp) before += x;
-    total += x;
+    const int2 x = warp_sum[w];
+    if (w < warp) before.x += x.x, before.y += x.y;
+    total.x += x.x, total.y += x.y;
   }
   __syncthreads();
-  return v + before;
+  return make_int2(v.x + before.x, v.y + before.y);
 }
 
 __device__ __forceinline__ int padded_rows(int cnt, int P) { return cnt > 0 ? ((cnt + P - 1) / P) * P : 0; }
@@ -267,8 +269,8 @@ struct Units {
     return true;
   }
 
-  __device__ bool next(Unit& u) {
-    const int lane = threadIdx.x & 31;
+  // The units that need no counter: the next piece of a row, and those that are this warp's from the start.
+  __device__ bool next_dealt(Unit& u) {
     if (piece < a.npieces) {
       u.tok = tok;
       u.ntok = 1;
@@ -277,13 +279,17 @@ struct Units {
       ++piece;
       return true;
     }
-    if (state == 0) {
-      if (round < a.rounds) {
-        const int g = (round++ * a.copy_warps + (int)(threadIdx.x >> 5)) * a.tokens_per_unit;
-        if (unit_at(blockIdx.x, g, u)) return true;
-      }
-      state = 1;
+    if (state == 0 && round < a.rounds) {
+      const int g = (round++ * a.copy_warps + (int)(threadIdx.x >> 5)) * a.tokens_per_unit;
+      if (unit_at(blockIdx.x, g, u)) return true;
     }
+    if (state == 0) state = 1;
+    return false;
+  }
+
+  __device__ bool next(Unit& u) {
+    const int lane = threadIdx.x & 31;
+    if (next_dealt(u)) return true;
     if (a.tokens_per_cta <= dealt()) return false;  // nothing beyond what was dealt, here or elsewhere
     if (state == 1) {
       if (take(blockIdx.x, u)) return true;
@@ -320,32 +326,59 @@ struct Units {
 };
 
 // A copy warp: units go global -> shared -> their K destination rows; a lane per (row, destination) issues the store.
-// Row flags are released at the end, or when the list of units is full, behind one wait and one fence.
-__device__ bool copy_bulk(const MoonepDevCtx& c, const SingleArgs& a, SingleShared& s, unsigned char* stages,
-                          unsigned char* shard, int* meta, int epoch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long row_bytes = (long long)c.H * 2;
-  const int K = c.K, NvS = c.NvS;
-  unsigned char* ring = stages + (size_t)warp * kRing * a.stage_bytes;
-  unsigned long long* bar = s.bar + warp * kRing;
-  Unit* units = s.unit[warp];
-  Units from = {c, a, epoch, 0, a.npieces, 0, 0};
-  int loaded = 0, stored = 0;
-  auto load = [&]() {
-    Unit u;
-    if (!from.next(u)) return false;
-    if (lane == 0) {
-      units[loaded % kUnits] = u;
+// Row flags are released at the end, or when the list of units is full, behind one wait and one fence.  The units that are the
+// warp's from the start are asked for before their tokens are planned (start).
+struct CopyWarp {
+  const MoonepDevCtx& c;
+  const SingleArgs& a;
+  SingleShared& s;
+  unsigned char* ring;
+  Units from;
+  int loaded, more;
+
+  __device__ CopyWarp(const MoonepDevCtx& c_, const SingleArgs& a_, SingleShared& s_, unsigned char* stages, int epoch)
+      : c(c_), a(a_), s(s_), ring(stages + (size_t)(threadIdx.x >> 5) * kRing * a_.stage_bytes),
+        from{c_, a_, epoch, 0, a_.npieces, 0, 0}, loaded(0), more(1) {}
+
+  __device__ void issue(const Unit& u) {
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+      s.unit[warp][loaded % kUnits] = u;
       const int q = loaded % kRing;
-      mbar_expect_tx(bar + q, u.len);
-      bulk_g2s(ring + (size_t)q * a.stage_bytes, reinterpret_cast<const unsigned char*>(a.hidden) + u.tok * row_bytes + u.off,
-               u.len, bar + q);
+      unsigned long long* bar = s.bar + warp * kRing + q;
+      mbar_expect_tx(bar, u.len);
+      bulk_g2s(ring + (size_t)q * a.stage_bytes,
+               reinterpret_cast<const unsigned char*>(a.hidden) + u.tok * (c.H * 2ll) + u.off, u.len, bar);
     }
     __syncwarp();
     ++loaded;
+  }
+
+  __device__ void start() {
+    Unit u;
+    while (loaded < kRing - 1 && from.next_dealt(u)) issue(u);
+  }
+
+  __device__ bool load() {
+    Unit u;
+    if (!from.next(u)) return false;
+    issue(u);
     return true;
-  };
+  }
+
+  __device__ bool run(unsigned char* shard, int* meta, int epoch, int t_lo, int t_hi);
+};
+
+// [t_lo, t_hi): tokens whose rows are listed in s.loff.
+__device__ bool CopyWarp::run(unsigned char* shard, int* meta, int epoch, int t_lo, int t_hi) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long row_bytes = (long long)c.H * 2;
+  const int K = c.K, NvS = c.NvS;
+  unsigned long long* bar = s.bar + warp * kRing;
+  const Unit* units = s.unit[warp];
+  int stored = 0;
   auto row_of = [&](const Unit& u, int e) {
+    if (u.tok >= t_lo && u.tok < t_hi) return s.loff[(u.tok - t_lo) * K + e];
     const int d = a.dst[u.tok * K + e];
     const int loff = d < 0 ? -d - 1 : d;
     return loff >= 0 && loff < NvS ? loff : -1;
@@ -364,8 +397,7 @@ __device__ bool copy_bulk(const MoonepDevCtx& c, const SingleArgs& a, SingleShar
     }
     __syncwarp();
   };
-  bool more = true;
-  for (int q = 0; q < kRing - 1 && more; ++q) more = load();
+  while (loaded < kRing - 1 && more) more = load();
   while (stored < loaded) {
     const Unit u = units[stored % kUnits];
     const int q = stored % kRing;
@@ -479,30 +511,57 @@ __device__ void copy_tail(const MoonepDevCtx& c, const SingleArgs& a, const int*
     for (int i = lo + t; i < hi; i += n) a.out_w[i] = reinterpret_cast<const float*>(meta + c.weights_off)[i];
 }
 
+// What a thread of the planning warps asks for before the group layout is known: the entries before the CTA's tokens that it
+// counts first, and the first entry that it plans, with its weight.  Beside other CTAs' rows and pads each of these round trips
+// takes microseconds.  With them, and the first rows of the copy warps, asked for where they were used: last CTA planned 21 us
+// after the layout where it takes 12 (S=4096, K=8, E=256) and 4.5 (3.5; S=2048, K=4, E=16), kernel 39.5 (37.5; S=2048, H=4096,
+// K=8) and 15.0 (12.4; S=2048, H=2048, K=4).  Counting in bytes per thread instead of atomics gained nothing beyond that.
+constexpr int kCountLoads = 8;
+struct Early {
+  int4 v[kCountLoads];
+  int e;
+  float w;
+};
+
+__device__ __forceinline__ Early load_early(const SingleArgs& a, int K, int before, int t_lo, int t_hi) {
+  Early p;
+  const int tid = threadIdx.x, nv = a.topk_vec ? before / 4 : 0;
+  const bool mine = tid < kEntries / K * K && t_lo * K + tid < t_hi * K;
+  p.e = mine ? a.topk[t_lo * K + tid] : -1;
+  p.w = mine && a.weights != nullptr ? a.weights[t_lo * K + tid] : 0.f;
+#pragma unroll
+  for (int u = 0; u < kCountLoads; ++u)
+    p.v[u] = tid + u * kEntries < nv ? __ldg(reinterpret_cast<const int4*>(a.topk) + tid + u * kEntries) : make_int4(-1, -1, -1, -1);
+  return p;
+}
+
 // Threads of the planning warps: rows for the entries of tokens [t_lo, t_hi), and everything the plan says about them.
-__device__ void plan_tokens(const MoonepDevCtx& c, const SingleArgs& a, SingleShared& s, const int* cnt, const int* off,
-                            int* cur, int* meta, int t_lo, int t_hi) {
+__device__ void plan_tokens(const MoonepDevCtx& c, const SingleArgs& a, SingleShared& s, const Early& early, const int* cnt,
+                            const int* off, int* cur, int* meta, int before, int t_lo, int t_hi) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int E = c.E, K = c.K, NvS = c.NvS;
   float* wbuf = reinterpret_cast<float*>(meta + c.weights_off);
   // routing entries before this CTA's tokens
-  const int before = t_lo * K;
   const int nv = a.topk_vec ? before / 4 : 0;
   auto count = [&](int e) {
     if ((unsigned)e < (unsigned)E) atomicAdd(cur + e, 1);
   };
-  for (int i0 = tid; i0 < nv; i0 += 8 * kEntries) {
-    int4 v[8];
+  // half of a thread's loads are on their way while it counts the other half
+  int4 v[kCountLoads];
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      v[u] = i0 + u * kEntries < nv ? __ldg(reinterpret_cast<const int4*>(a.topk) + i0 + u * kEntries)
-                                    : make_int4(-1, -1, -1, -1);
+  for (int u = 0; u < kCountLoads; ++u) v[u] = early.v[u];
+  for (int i0 = tid; i0 < nv; i0 += kCountLoads * kEntries) {
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      count(v[u].x);
-      count(v[u].y);
-      count(v[u].z);
-      count(v[u].w);
+    for (int u0 = 0; u0 < kCountLoads; u0 += kCountLoads / 2) {
+#pragma unroll
+      for (int u = u0; u < u0 + kCountLoads / 2; ++u) {
+        count(v[u].x);
+        count(v[u].y);
+        count(v[u].z);
+        count(v[u].w);
+        const int i = i0 + (kCountLoads + u) * kEntries;
+        v[u] = i < nv ? __ldg(reinterpret_cast<const int4*>(a.topk) + i) : make_int4(-1, -1, -1, -1);
+      }
     }
   }
   for (int i = nv * 4 + tid; i < before; i += kEntries) count(a.topk[i]);
@@ -510,7 +569,8 @@ __device__ void plan_tokens(const MoonepDevCtx& c, const SingleArgs& a, SingleSh
   for (int t0 = t_lo; t0 < t_hi; t0 += tokens_per_step) {
     const int nent = min(tokens_per_step, t_hi - t0) * K, slot = t0 * K + tid;
     const bool in = tid < nent;
-    int e = in ? a.topk[slot] : -1;
+    int e = !in ? -1 : t0 == t_lo ? early.e : a.topk[slot];
+    const float weight = t0 == t_lo ? early.w : in && a.weights != nullptr ? a.weights[slot] : 0.f;
     if (in && (unsigned)e >= (unsigned)E) {
       record_status(c, MOONEP_STATUS_BAD_INDEX, MOONEP_K_PLAN_TOKENS, 2, e, E, slot);
       e = -1;
@@ -581,9 +641,8 @@ __device__ void plan_tokens(const MoonepDevCtx& c, const SingleArgs& a, SingleSh
     if (a.plan_src_info != nullptr) a.plan_src_info[loff] = slot;
     if (a.plan_link != nullptr) a.plan_link[loff] = link;
     if (a.weights != nullptr) {
-      const float w = a.weights[slot];
-      wbuf[loff] = w;
-      if (a.out_w != nullptr) a.out_w[loff] = w;
+      wbuf[loff] = weight;
+      if (a.out_w != nullptr) a.out_w[loff] = weight;
     }
   }
   if (t_hi == c.S) {
@@ -616,14 +675,21 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
   griddep_wait();
   griddep_launch();
   const unsigned long long t_begin = globaltimer_ns();
+  // what the kernel begins with, in one round trip to memory
+  const int epoch = abs_epoch(c, MOONEP_FLAG_SENT, a.epoch_sent);
+  const int first_count = a.fresh && tid < E ? a.tpe[tid] : 0;
+  const int t_lo = min(c.S, (int)blockIdx.x * a.tokens_per_cta), t_hi = min(c.S, t_lo + a.tokens_per_cta);
+  const int before = t_lo * K;  // routing entries before this CTA's tokens
+  Early early;
+  if (a.fresh && warp < kPlanWarps) early = load_early(a, K, before, t_lo, t_hi);
   // one answer for the CTA: the code below contains barriers
   const bool run = __syncthreads_and(poisoned(c) ? 0 : 1) != 0;
   bool ok = run;
   if (run) {
-    int* meta = c.meta_peer[0];
-    uint16_t* shard = c.hidden_peer[0];
-    const int epoch = abs_epoch(c, MOONEP_FLAG_SENT, a.epoch_sent);
-    const int t_lo = min(c.S, (int)blockIdx.x * a.tokens_per_cta), t_hi = min(c.S, t_lo + a.tokens_per_cta);
+    int* meta = a.meta;
+    uint16_t* shard = a.shard;
+    CopyWarp copier(c, a, s, s_dyn, epoch);
+    if (a.bulk && warp < a.copy_warps && t_lo < t_hi) copier.start();
     Layout lay = {nullptr, nullptr, nullptr, nullptr, 0};
     int *cnt = tables, *off = tables + E, *cur = tables + 2 * E;
     int used = NvS;
@@ -632,19 +698,18 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
       int carry = 0, pads = 0;
       for (int e0 = 0; e0 < E; e0 += kThreads) {
         const int e = e0 + tid;
-        const int n = e < E ? a.tpe[e] : 0;
+        const int n = e0 == 0 ? first_count : e < E ? a.tpe[e] : 0;
         const int rows = padded_rows(n, c.token_padding);
-        int total, total_pads;
-        const int end = carry + block_scan(rows, s.warp_sum, total);
-        const int pend = pads + block_scan(rows > 0 ? rows - n : 0, s.warp_sum, total_pads);
+        int2 total;
+        const int2 sum = block_scan(make_int2(rows, rows > 0 ? rows - n : 0), s.warp_sum, total);
         if (e < E) {
           cnt[e] = n;
-          off[e] = end - rows;
+          off[e] = carry + sum.x - rows;
           cur[e] = 0;
-          cum[e] = pend;
+          cum[e] = pads + sum.y;
         }
-        carry += total;
-        pads += total_pads;
+        carry += total.x;
+        pads += total.y;
       }
       used = min(max(carry, 0), NvS);
       lay = {nullptr, cnt, off, cum, E};
@@ -686,13 +751,14 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
       int pads = 0;
       for (int g0 = 0; g0 < groups; g0 += kThreads) {
         const int g = g0 + tid;
-        int total;
-        const int pend = pads + block_scan(g < groups ? min(max(0, a.zero_fill[2 * g + 1]), NvS) : 0, s.warp_sum, total);
+        const int2 range = g < groups ? make_int2(a.zero_fill[2 * g], a.zero_fill[2 * g + 1]) : make_int2(0, 0);
+        int2 total;
+        const int2 sum = block_scan(make_int2(min(max(0, range.y), NvS), 0), s.warp_sum, total);
         if (g < groups) {
-          first[g] = a.zero_fill[2 * g];
-          cum[g] = pend;
+          first[g] = range.x;
+          cum[g] = pads + sum.x;
         }
-        pads += total;
+        pads += total.x;
       }
       lay = {first, nullptr, nullptr, cum, groups};
       __syncthreads();
@@ -715,10 +781,10 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
     } else {
       if (t_lo < t_hi) {
         if (a.fresh) {
-          plan_tokens(c, a, s, cnt, off, cur, meta, t_lo, t_hi);
-          fence_gpu();
+          plan_tokens(c, a, s, early, cnt, off, cur, meta, before, t_lo, t_hi);
           plan_sync();
-          if (tid == 0) st_release_gpu(a.work + kWorkReady + blockIdx.x, epoch);
+          // the release covers what the barrier has ordered before it
+          if (tid == kEntries - 32) st_release_gpu(a.work + kWorkReady + blockIdx.x, epoch);
           if (times_plan) stat_phase(c, MOONEP_PH_TOKENS, t_laid);
         } else {
           for (int i = t_lo * K + tid; i < t_hi * K; i += kEntries) {
@@ -734,8 +800,10 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
       if (tid == 0) t_planned = globaltimer_ns();
       if (!a.bulk)
         copy_plain(c, a, t_lo, t_hi, shard, meta, epoch);
-      else if (warp < a.copy_warps)
-        ok = copy_bulk(c, a, s, s_dyn, reinterpret_cast<unsigned char*>(shard), meta, epoch);
+      else if (warp < a.copy_warps) {
+        const bool listed = a.fresh && (t_hi - t_lo) * K <= kEntries;  // planned in one step: s.loff still holds them all
+        ok = copier.run(reinterpret_cast<unsigned char*>(shard), meta, epoch, t_lo, listed ? t_hi : t_lo);
+      }
       // rows behind the last group go into the copy as they are; the warps that do not stream rows see to it
       const int w0 = a.bulk ? a.copy_warps : 0;
       if (a.out != nullptr && a.fresh && warp >= w0)
@@ -749,8 +817,8 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_single_kernel(const Moon
       stat_phase(c, MOONEP_PH_BUILD_EXPAND, t_begin, t_end);
     }
   }
-  // the last CTA resets the counters and publishes what the general kernels' stages publish
-  fence_gpu();
+  // the last CTA resets the counters and publishes what the general kernels' stages publish; the fence covers what the barrier
+  // has ordered before it
   ok = __syncthreads_and(ok ? 1 : 0) != 0;
   if (tid == 0) {
     fence_gpu();
@@ -826,7 +894,7 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(cons
   constexpr int kRows = kCombineLoads / kItems;  // rows of an item whose loads are in flight together
   griddep_wait();
   griddep_launch();
-  if (poisoned(c)) return;
+  const int failed = ld_volatile(c.status + MOONEP_ST_CODE);  // looked at when the first entries are on their way
   const int lane = threadIdx.x & 31;
   const int K = c.K, H = c.H, NvS = c.NvS;
   const int npieces = (H + 255) / 256;
@@ -840,6 +908,7 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_single_kernel(cons
   int it = first + (threadIdx.x >> 5);
   auto lookup = [&](int i) { return looks && i < end ? a.dst[i / npieces * K + k_of] : 0; };
   int d_next = lookup(it + j_of * step);
+  if (failed != 0) return;
   for (; it < end; it += kItems * step) {
     const int mine = it + j_of * step;
     const int my_tok = mine / npieces, my_piece = mine - my_tok * npieces;
@@ -989,6 +1058,8 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, int exact, const int
   a.plan_src_info = plan_src_info;
   a.plan_link = plan_link;
   a.hidden = (const uint16_t*)hidden;
+  a.shard = (uint16_t*)h->hidden_own;
+  a.meta = (int*)h->meta_own;
   a.work = work;
   a.out = fresh ? (uint16_t*)out : nullptr;
   a.out_w = fresh ? out_w : nullptr;
@@ -1040,7 +1111,8 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, int exact, const int
   if (n_ctas > 0) grid = imin(grid, n_ctas);
   a.tokens_per_cta = (c.S + grid - 1) / grid;
   const int per_round = imax(1, a.copy_warps * a.tokens_per_unit), rounds = (a.tokens_per_cta + per_round - 1) / per_round;
-  a.rounds = rounds <= kDealtRounds && a.tokens_per_cta * (c.K + 1) * row_bytes <= kDealtBytes ? rounds : 1;
+  // elsewhere as many as are asked for before the tokens are planned
+  a.rounds = rounds <= kDealtRounds && a.tokens_per_cta * (c.K + 1) * row_bytes <= kDealtBytes ? rounds : imin(rounds, kRing - 1);
   if (int rc = check_cuda(launch_maybe_pdl(dispatch_single_kernel, grid, kThreads, smem, (cudaStream_t)stream,
                                            h->enable_pdl != 0, c, a),
                           "launch dispatch_single_kernel"))
