@@ -45,6 +45,12 @@ constexpr int kEntries = kPlanWarps * 32;  // routing entries planned at a time 
 // K=2 21.5 -> 18.0, S=4096, H=1024, K=8 30.2 -> 28.2; with 1 MB per CTA (S=2048, H=4096, K=8) it would be 50.5 -> 52.2.
 constexpr long long kDealtBytes = 768 << 10;
 constexpr int kDealtRounds = 6;
+// Rows that share a stage at most, as far as the rings of six warps have room and the CTA's tokens make equal shares for them.  A
+// unit costs a copy warp a chain of round trips, and an SM has more on its way with more in a stage.  Against rows that fill
+// 4 KB, dispatch and combine, us: S=16384, K=4, H=1000 79.3 -> 74.9, H=2048 135.2 -> 127.9; S=4096, K=8, H=2048 64.2 -> 61.4.
+// Stages of 16 KB for four warps make the dispatch alone another 2 to 5 % shorter, but the combine behind it longer by more
+// (S=16384, K=4: H=2048 132.9 together, H=4096 249.6 instead of 237.7).
+constexpr int kUnitTokens = 8;
 constexpr int kUnits = 64;         // units remembered per copy warp: those loaded and those not flagged yet
 constexpr int kGrabs = 64;         // grabs of pad rows remembered per warp
 constexpr int kMaxGroups = 4096;   // experts, and prefetch slots: up to four words of shared memory each
@@ -1098,6 +1104,9 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, int exact, const int
   const size_t limit = (size_t)imax(0, h->max_smem_optin - (int)static_bytes);
   const size_t tables = (fresh ? (size_t)4 * c.E : (size_t)2 * (c.E + c.B)) * sizeof(int);
   const long long row_bytes = (long long)c.H * 2;
+  int grid = imax(1, imin(imin(c.local_sms, h->sm_count), kMaxCtas));
+  if (n_ctas > 0) grid = imin(grid, n_ctas);
+  a.tokens_per_cta = (c.S + grid - 1) / grid;
   a.stage_bytes = 0;
   a.npieces = a.tokens_per_unit = 1;
   a.copy_warps = 0;
@@ -1107,8 +1116,10 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, int exact, const int
     a.npieces = (int)((row_bytes + most - 1) / most);
     if (a.npieces > 1) {
       a.stage_bytes = (int)(((row_bytes + a.npieces - 1) / a.npieces + 15) / 16 * 16);
-    } else {  // rows below 4 KB share a stage of about that size
-      a.tokens_per_unit = imax(1, imin(16, (int)(4096 / row_bytes)));
+    } else {
+      const int share = imax(1, imin(kUnitTokens, (int)(room / (kCopyWarps * kRing) / row_bytes)));
+      const int units = kCopyWarps * ((a.tokens_per_cta + kCopyWarps * share - 1) / (kCopyWarps * share));  // as many for each warp
+      a.tokens_per_unit = (a.tokens_per_cta + units - 1) / units;
       a.stage_bytes = (int)(a.tokens_per_unit * row_bytes);
     }
     a.copy_warps = imin(kCopyWarps, (int)(room / ((long long)kRing * a.stage_bytes)));
@@ -1121,9 +1132,6 @@ extern "C" int moonep_dispatch_single(void* ctx, int fresh, int exact, const int
       return rc;
     h->single_smem_set = 1;
   }
-  int grid = imax(1, imin(imin(c.local_sms, h->sm_count), kMaxCtas));
-  if (n_ctas > 0) grid = imin(grid, n_ctas);
-  a.tokens_per_cta = (c.S + grid - 1) / grid;
   const int per_round = imax(1, a.copy_warps * a.tokens_per_unit), rounds = (a.tokens_per_cta + per_round - 1) / per_round;
   // elsewhere as many as are asked for before the tokens are planned
   a.rounds = rounds <= kDealtRounds && a.tokens_per_cta * (c.K + 1) * row_bytes <= kDealtBytes ? rounds : imin(rounds, kRing - 1);
