@@ -50,6 +50,7 @@ struct WgradArgs {
   float* const* out_ptrs;  // [G] device array
   const int* flags;        // [G]
   const int* cu_seqlens;   // [G] inclusive padded ends
+  const int* pads;         // [G, 2] or null: first of the group's last rows that hold zeros, and how many, or 0
   int* status;
   unsigned long long timeout_ns;
   int G, P, Q, p_tiles, q_tiles, rows_cap;
@@ -83,6 +84,10 @@ __device__ __forceinline__ void wgrad_list_groups(const WgradArgs& a, WgradGroup
       // the K coordinate of a TMA copy must be a multiple of 8 elements and the MMAs take 16 rows at a time:
       // a group that does not start and end on a multiple of 16 is refused (reported as rows without a target)
       if (((start | end) & 15) != 0) out = nullptr;
+      if (a.pads != nullptr && krows > 0) {  // rows of zeros add nothing: up to the next multiple of 16
+        const int n = a.pads[2 * g + 1], used = (a.pads[2 * g] - start + 15) & ~15;
+        if (n > 0 && used > 0 && used < krows && a.pads[2 * g] + n == end) krows = used;
+      }
       listed = krows > 0 || (out != nullptr && flag == 0);
     }
     const unsigned mask = __ballot_sync(0xffffffffu, listed);
@@ -465,6 +470,7 @@ extern "C" int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld
   a.out_ptrs = (float* const*)out_ptrs;
   a.flags = flags;
   a.cu_seqlens = cu_seqlens;
+  a.pads = nullptr;
   a.status = status;
   a.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 10000) * 1000000ull;
   a.G = G;
@@ -477,11 +483,11 @@ extern "C" int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld
 
 // The same with the operands as they are: l = L [rows, P] and r = R [rows, Q] bf16, rows ldl / ldr elements apart
 // (multiples of 8), so that column slices of wider tensors can be passed.  No transposed copies are needed: the
-// tiles are staged MN-major (see make_smem_desc_mn).
+// tiles are staged MN-major (see make_smem_desc_mn).  pads (optional): a plan's zero_fill_ranges, whose rows hold zeros.
 extern "C" int moonep_grouped_wgrad_rows(const void* l, long long ldl, const void* r, long long ldr, int rows, int P,
                                          int Q, const int* cu_seqlens, int G, void* const* out_ptrs, const int* flags,
                                          int* status, long long timeout_ms, int rows_per_group, int adds,
-                                         int num_sms, void* stream) {
+                                         int num_sms, const int* pads, void* stream) {
   if (P <= 0 || Q <= 0 || P % BM != 0 || Q % BN != 0) {
     set_error("moonep_grouped_wgrad_rows: P must be a multiple of 128 and Q a multiple of 256");
     return 1;
@@ -501,6 +507,7 @@ extern "C" int moonep_grouped_wgrad_rows(const void* l, long long ldl, const voi
   a.out_ptrs = (float* const*)out_ptrs;
   a.flags = flags;
   a.cu_seqlens = cu_seqlens;
+  a.pads = nullptr;
   a.status = status;
   a.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 10000) * 1000000ull;
   a.G = G;
@@ -508,5 +515,6 @@ extern "C" int moonep_grouped_wgrad_rows(const void* l, long long ldl, const voi
   a.Q = Q;
   a.rows_cap = rows;
   a.row_major = 1;
+  a.pads = pads;
   return launch_wgrad(tl, tr, a, rows_per_group, adds, num_sms, stream);
 }

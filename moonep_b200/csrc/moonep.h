@@ -338,10 +338,11 @@ int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld, int P, in
 int moonep_wgrad_single_cta(int rows_per_group, int num_sms);
 int moonep_wgrad_single_cta_adding(int rows_per_group, int num_sms);
 // The same from the operands as they are, l = L [rows, P], r = R [rows, Q] (rows ldl / ldr elements apart): no
-// transposed copies, the tiles are staged MN-major.
+// transposed copies, the tiles are staged MN-major.  pads (optional): [G, 2] (first, number) of a group's last rows that hold
+// zeros, which are left out.
 int moonep_grouped_wgrad_rows(const void* l, long long ldl, const void* r, long long ldr, int rows, int P, int Q,
                               const int* cu_seqlens, int G, void* const* out_ptrs, const int* flags, int* status,
-                              long long timeout_ms, int rows_per_group, int adds, int num_sms, void* stream);
+                              long long timeout_ms, int rows_per_group, int adds, int num_sms, const int* pads, void* stream);
 // Helpers of the MoE layer's backward pass and optimiser step, see moe_kernels.cu.
 int moonep_transpose_experts(const void* src, void* dst, int n, int d0, int d1, long long dst_ld,
                              long long dst_expert_stride, int col0, const int* active, void* stream);

@@ -285,7 +285,7 @@ class ExpertParallelMoE:
         if overlap:
             total = torch.cuda.get_device_properties(dev).multi_processor_count
             sms = max(2, (total - int(self.buffer._require_ctx()["num_sms"])) // 2 * 2)
-        if not self._weight_grads_on_kernel(x_nvs, dy_nvs, dadu, hsw, cu, after=reduce_one if overlap else None, num_sms=sms):
+        if not self._weight_grads_on_kernel(x_nvs, dy_nvs, dadu, hsw, cu, plan, after=reduce_one if overlap else None, num_sms=sms):
             self._weight_grads_per_group(x_nvs, dy_nvs, dadu, hsw, cu)
         self._times_weights(dadu, [self.w_gate, self.w_up], cu, plan, out=dy_nvs,
                             num_sms=sms if reduced else 0)  # dx rows = da Wg + du Wu
@@ -306,7 +306,7 @@ class ExpertParallelMoE:
         return grouped_gemm(x, self._local_transposed(ws, plan), cu, group_map=self.group_map, out=out,
                             status=self.buffer._require_ctx()["_backend"].status if x.is_cuda else None)
 
-    def _weight_grads_on_kernel(self, x_nvs, dy_nvs, dadu, hsw, cu, after=None, num_sms=0) -> bool:
+    def _weight_grads_on_kernel(self, x_nvs, dy_nvs, dadu, hsw, cu, plan, after=None, num_sms=0) -> bool:
         """All weight gradients with three launches of the grouped tcgen05 kernel (no host synchronisation); every
         group's result goes straight to the owner's gradient or to the reduce-buffer slot of a prefetched copy.
         Returns False (nothing done) when the shapes do not fit the kernel.  ``after(i)`` is called once the
@@ -330,6 +330,7 @@ class ExpertParallelMoE:
         # rows of an owned expert, on average; the prefetch slots of a step are mostly empty
         kw = {"status": status, "rows_per_group": max(1, self.S * self.K // self.epn), "adds": not self._fresh}
         if config.wgrad_layout() == "rows":  # the kernel stages MN-major tiles: the activations as they are
+            kw["pads"] = plan.zero_fill_ranges  # rows of zeros in all of them
             grouped_wgrad_rows(dy_nvs, hsw, cu, ptrs[2], flags, **kw)  # dW_down = dy^T (h * gate weight)
             done(2)
             grouped_wgrad_rows(dadu[:, :I], x_nvs, cu, ptrs[0], flags, num_sms=later, **kw)  # dW_gate = da^T x

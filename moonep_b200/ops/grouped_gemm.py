@@ -241,9 +241,12 @@ def grouped_wgrad(left_t, right_t, cu_seqlens, out_ptrs, flags, *, status=None, 
     _lib.check(rc, "moonep_grouped_wgrad")
 
 
-def grouped_wgrad_rows(left, right, cu_seqlens, out_ptrs, flags, *, status=None, num_sms=0, rows_per_group=0, adds=False):
+def grouped_wgrad_rows(left, right, cu_seqlens, out_ptrs, flags, *, status=None, num_sms=0, rows_per_group=0, adds=False,
+                       pads=None):  # fmt: skip
     """``grouped_wgrad`` from the operands as they are: ``left`` ``[rows, P]`` and ``right`` ``[rows, Q]`` bf16 with unit
-    column stride (column slices of wider tensors are fine), no transposed copies.  Same targets, flags and bounds."""
+    column stride (column slices of wider tensors are fine), no transposed copies.  Same targets, flags and bounds.
+    ``pads`` (int32 ``[G, 2]``, e.g. a plan's ``zero_fill_ranges``): the first and the number of each group's last rows that
+    hold zeros in both operands; they are left out, which changes nothing but the time."""
     rows, P = (int(v) for v in left.shape)
     Q = int(right.shape[1])
     G = int(cu_seqlens.numel())
@@ -256,11 +259,13 @@ def grouped_wgrad_rows(left, right, cu_seqlens, out_ptrs, flags, *, status=None,
     assert out_ptrs.dtype == torch.int64 and out_ptrs.numel() == G and out_ptrs.is_cuda and out_ptrs.is_contiguous()
     assert flags.dtype == torch.int32 and flags.numel() == G and flags.is_cuda and flags.is_contiguous()
     assert cu_seqlens.dtype == torch.int32 and cu_seqlens.is_contiguous() and cu_seqlens.is_cuda
+    if pads is not None:
+        assert pads.dtype == torch.int32 and tuple(pads.shape) == (G, 2) and pads.is_contiguous() and pads.device == left.device
     with _lib.on_device(left.device):
         rc = _lib.caller("moonep_grouped_wgrad_rows")(
             left.data_ptr(), ldl, right.data_ptr(), ldr, rows, P, Q, cu_seqlens.data_ptr(), G, out_ptrs.data_ptr(),
             flags.data_ptr(), 0 if status is None else status.data_ptr(), config.timeout_ms(), int(rows_per_group),
-            int(adds), int(num_sms), _lib.current_stream(),
+            int(adds), int(num_sms), 0 if pads is None else pads.data_ptr(), _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_grouped_wgrad_rows")
 
