@@ -24,8 +24,8 @@ MOONEP_EXPAND_PATH    ``bulk`` (default) or ``ldst``: how the destination side o
                       when the Buffer is made).
 MOONEP_COMBINE        ``push`` (default: the expert side folds duplicates and pushes rows to the tokens' home ranks,
                       which sum them as they arrive) or ``pull`` (fold pass, then the home ranks pull).
-MOONEP_PHASED         ``1``: launch the dispatch and combine kernels one role at a time even on real multi-GPU worlds
-                      (what emulated ranks always do); for per-role timing and debugging.
+MOONEP_PHASED         ``1``: launch the dispatch and combine kernels one role at a time, on real multi-GPU worlds too
+                      (emulated ranks otherwise launch roles that need not wait together); for per-role timing and debugging.
 MOONEP_PDL            ``0`` turns programmatic dependent launch off even for Buffers created with ``enable_pdl=True``, and for the
                       expert kernels (GEMMs, weight gradients, SwiGLU backward), which no Buffer launches.
 MOONEP_LOCAL_SMS      CTAs of the kernels that only touch local memory (default: all SMs); ``num_sms`` of
