@@ -306,9 +306,9 @@ typedef struct MoonepGemmHooks {
 int moonep_grouped_gemm(const void* x, const void* w0, const void* w1, void* out, const float* row_scale,
                         const int* cu_seqlens, int G, int rows_cap, int K, int n_per_group, int mode, int* status,
                         long long timeout_ms, int num_sms, const int* group_map, int w_slots, void* pre_gate,
-                        void* pre_up, void* stream);
+                        void* pre_up, int weights_early, void* stream);
 // The same operation on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles per cluster of two CTAs), see
-// grouped_gemm_pair.cu.  Same arguments.
+// grouped_gemm_pair.cu.  Same arguments, without weights_early.
 int moonep_grouped_gemm_pair(const void* x, const void* w0, const void* w1, void* out, const float* row_scale,
                              const int* cu_seqlens, int G, int rows_cap, int K, int n_per_group, int mode, int* status,
                              long long timeout_ms, int num_sms, const int* group_map, int w_slots, void* pre_gate,

@@ -188,6 +188,7 @@ struct GemmArgs {
   uint16_t* pre_gate;    // SwiGLU only, optional: the pre-activations x Wg^T and x Wu^T, [rows, ldo] bf16 each,
   uint16_t* pre_up;      // kept for the backward pass so that it need not recompute them
   int early;             // launched with expert_pdl: the next kernel's CTAs may come while this one runs
+  int weights_early;     // single CTAs only: W and the group tables may be read before the kernel before has ended
   MoonepGemmHooks hooks; // CTA-pair kernel only: hand-off with the communication kernels (all null = none)
 };
 

@@ -179,7 +179,7 @@ class ExpertParallelMoE:
             # counted from zero every time: blocks without rows are not counted, and which those are changes with the routing
             self._done.zero_()
             ready = (self._done, 4 * (self.H // 256))
-        grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=self._y, status=status, pair=pair,
+        grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=self._y, status=status, pair=pair, weights_early=alone,
                      hooks=buf.gemm_hooks(slots=not alone, done_counter=self._done) if hooked else None)  # fmt: skip
         out, _, _ = buf.combine(plan, self._y, None, ready=ready)
         if hooked and fetched is not None:

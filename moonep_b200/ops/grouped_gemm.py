@@ -66,7 +66,7 @@ def kernel_supports(x, w, mode: str) -> bool:
 
 
 def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", out=None, status=None, num_sms=0,
-                 group_map=None, save_pre=None, pair=None, hooks=None):
+                 group_map=None, save_pre=None, pair=None, hooks=None, weights_early=False):
     """See module docstring.  ``x``: ``[rows, K]`` bf16, ``w``: ``[G, N, K]`` bf16, returns ``[rows, N]`` bf16.
 
     Rows beyond ``cu_seqlens[-1]`` are not written.  Group ends must be multiples of 128 (the kernels record an index
@@ -78,6 +78,8 @@ def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", o
     ``pair`` selects the kernel: True = CTA pairs (``cta_group::2``), False = one CTA per tile, None = ``MOONEP_GEMM_PAIR``.
     ``hooks`` (a ``GemmHooks``, CTA-pair kernel only) lets the kernel run beside the communication kernels: it waits
     per row block / weight slot for their flags and counts finished output tiles per row block.
+    ``weights_early``: the kernel launched just before on this stream is another of these GEMMs, which writes neither the
+    weights nor the group tables: one CTA per tile then asks for weights while that kernel still runs.
     """
     assert mode in _MODES
     W, N, K = (int(v) for v in w.shape)
@@ -126,7 +128,8 @@ def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", o
         if hooks is not None:
             rc = _lib.caller("moonep_grouped_gemm_pair_hooked")(*args, ctypes.addressof(hooks), st)
         else:
-            rc = _lib.caller("moonep_grouped_gemm_pair" if use_pair else "moonep_grouped_gemm")(*args, st)
+            rc = _lib.caller("moonep_grouped_gemm_pair")(*args, st) if use_pair else _lib.caller("moonep_grouped_gemm")(
+                *args, int(weights_early), st)
     _lib.check(rc, "moonep_grouped_gemm")
     return out
 
