@@ -10,7 +10,7 @@
 //                       projection's weight gradient) and dgate.
 //
 //   sgd_update          w (bf16) -= lr * g (fp32), vectorised.
-//   adamw_update        one AdamW step of up to kAdamTensors weights in one pass: fp32 master, moments and gradient in,
+//   adamw_update        one AdamW step of up to kUpdateTensors weights in one pass: fp32 master, moments and gradient in,
 //                       master, moments and the rounded bf16 weight out.
 //
 // The reference has no expert computation; these serve the MoE training-step configuration.
@@ -24,7 +24,7 @@ namespace moonep {
 namespace {
 
 constexpr int kTile = 64;
-constexpr int kAdamTensors = 3;
+constexpr int kUpdateTensors = 3;  // weights per launch of the weight updates
 constexpr int kUpdateSteps = 4;  // vectors per thread of the weight updates, at most
 
 __global__ void __launch_bounds__(256)
@@ -107,11 +107,27 @@ __global__ void __launch_bounds__(256)
 }
 
 // w (bf16) -= lr * g (fp32), 8 elements per thread and step.  Short CTAs as in adamw_kernel: 117 M elements 160 -> 145 us.
-__global__ void __launch_bounds__(256)
-    sgd_update_kernel(uint16_t* __restrict__ w, const float* __restrict__ g, long long n8, float lr, int steps) {
-  const long long first = (long long)blockIdx.x * (256 * steps) + threadIdx.x;
+// The weights of a layer share a launch: a training step of S=64, H=1024, I=256, 6 experts 98.7 -> 92.7 us, S=1500, H=4096,
+// I=1024, 8 experts 469 -> 460.  Placed while the kernel before still ran (PDL), the latter took 499.
+struct SgdTensor {
+  uint16_t* w;
+  const float* g;
+  long long n8;  // groups of eight elements
+};
+struct SgdArgs {
+  SgdTensor t[kUpdateTensors];
+  float lr;
+  int steps;  // vectors per thread
+};
+
+__global__ void __launch_bounds__(256) sgd_update_kernel(const __grid_constant__ SgdArgs a) {
+  uint16_t* __restrict__ w = a.t[blockIdx.y].w;
+  const float* __restrict__ g = a.t[blockIdx.y].g;
+  const long long n8 = a.t[blockIdx.y].n8;
+  const float lr = a.lr;
+  const long long first = (long long)blockIdx.x * (256 * a.steps) + threadIdx.x;
 #pragma unroll 1
-  for (int s = 0; s < steps; ++s) {
+  for (int s = 0; s < a.steps; ++s) {
     const long long v = first + s * 256;
     if (v >= n8) break;
     int4 wv = ld16(w + v * 8);
@@ -138,7 +154,7 @@ struct AdamTensor {
   long long n4;    // groups of four elements
 };
 struct AdamArgs {
-  AdamTensor t[kAdamTensors];
+  AdamTensor t[kUpdateTensors];
   int steps;              // vectors per thread
   float decay;            // 1 - lr * weight_decay
   float b1, b2;           // decay rates of the moments
@@ -191,8 +207,8 @@ static int update_steps(long long vectors) {
 extern "C" int moonep_adamw_update(int count, void* const* master, void* const* m, void* const* v, void* const* g,
                                    void* const* w, const long long* n, double step, double b1, double b2, double eps,
                                    double decay, double c2, void* stream) {
-  if (count < 1 || count > kAdamTensors) {
-    set_error("moonep_adamw_update: 1 to " + std::to_string(kAdamTensors) + " weights per call");
+  if (count < 1 || count > kUpdateTensors) {
+    set_error("moonep_adamw_update: 1 to " + std::to_string(kUpdateTensors) + " weights per call");
     return 1;
   }
   AdamArgs a;
@@ -222,16 +238,28 @@ extern "C" int moonep_adamw_update(int count, void* const* master, void* const* 
   return check_launch("adamw_kernel");
 }
 
-// w: [n] bf16, g: [n] fp32, n a multiple of 8: w -= lr * g.
-extern "C" int moonep_sgd_update(void* w, const float* g, long long n, float lr, void* stream) {
-  if (n % 8 != 0) {
-    set_error("moonep_sgd_update: element count must be a multiple of 8");
+// count weights, w: [n[i]] bf16, g: [n[i]] fp32, n[i] a multiple of 8: w -= lr * g.
+extern "C" int moonep_sgd_update(int count, void* const* w, void* const* g, const long long* n, float lr, void* stream) {
+  if (count < 1 || count > kUpdateTensors) {
+    set_error("moonep_sgd_update: 1 to " + std::to_string(kUpdateTensors) + " weights per call");
     return 1;
   }
-  if (n == 0) return 0;
-  const int steps = update_steps(n / 8);
-  const long long per_cta = 256 * 8 * steps;
-  sgd_update_kernel<<<(unsigned)((n + per_cta - 1) / per_cta), 256, 0, (cudaStream_t)stream>>>((uint16_t*)w, g, n / 8, lr, steps);
+  SgdArgs a;
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    if (n[i] % 8 != 0) {
+      set_error("moonep_sgd_update: element counts must be multiples of 8");
+      return 1;
+    }
+    a.t[i] = {(uint16_t*)w[i], (const float*)g[i], n[i] / 8};
+    most = n[i] > most ? n[i] : most;
+  }
+  if (most == 0) return 0;
+  a.lr = lr;
+  a.steps = update_steps(most / 8 * count);
+  const long long per_cta = 256 * 8 * a.steps;
+  const dim3 grid((unsigned)((most + per_cta - 1) / per_cta), (unsigned)count);
+  sgd_update_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
   return check_launch("sgd_update_kernel");
 }
 

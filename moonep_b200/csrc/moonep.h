@@ -353,7 +353,7 @@ int moonep_swiglu_bwd(const void* a, const void* u, const void* g, const float* 
 int moonep_adamw_update(int count, void* const* master, void* const* m, void* const* v, void* const* g, void* const* w,
                         const long long* n, double step, double b1, double b2, double eps, double decay, double c2,
                         void* stream);
-int moonep_sgd_update(void* w, const float* g, long long n, float lr, void* stream);
+int moonep_sgd_update(int count, void* const* w, void* const* g, const long long* n, float lr, void* stream);
 
 // CUDA VMM symmetric allocator (driver API through cudaGetDriverEntryPoint).
 int moonep_vmm_granularity(int device, unsigned long long* gran);

@@ -44,7 +44,7 @@ from ..ops.grouped_gemm import (
     grouped_wgrad_rows,
     wgrad_kernel_supports,
 )
-from ..ops.moe_ops import sgd_update, swiglu_bwd, transpose_experts
+from ..ops.moe_ops import sgd_updates, swiglu_bwd, transpose_experts
 from ..parallel.symm import create_full_expert_weight, create_nvl_dist_tensor, view_nvl_dist_rows
 
 
@@ -400,8 +400,7 @@ class ExpertParallelMoE:
     def sgd_step(self, lr: float):
         """Plain SGD on the owned experts (enough for a benchmark step)."""
         s = slice(self.rank * self.epn, (self.rank + 1) * self.epn)
-        for w, g in ((self.w_gate, self.g_gate), (self.w_up, self.g_up), (self.w_down, self.g_down)):
-            sgd_update(w[s], g, lr)
+        sgd_updates([self.w_gate[s], self.w_up[s], self.w_down[s]], self.owner_grads(), lr)
         self.publish_owned()
 
     def publish_owned(self):

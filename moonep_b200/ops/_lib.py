@@ -144,7 +144,7 @@ _SIGNATURES = {
     "moonep_grouped_wgrad_rows": (_i, [_vp, _ll, _vp, _ll, _i, _i, _i, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _vp, _vp]),
     "moonep_transpose_experts": (_i, [_vp, _vp, _i, _i, _i, _ll, _ll, _i, _vp, _vp]),
     "moonep_adamw_update": (_i, [_i] + [ctypes.POINTER(_vp)] * 5 + [ctypes.POINTER(_ll)] + [ctypes.c_double] * 6 + [_vp]),
-    "moonep_sgd_update": (_i, [_vp, _vp, _ll, ctypes.c_float, _vp]),
+    "moonep_sgd_update": (_i, [_i] + [ctypes.POINTER(_vp)] * 2 + [ctypes.POINTER(_ll), ctypes.c_float, _vp]),
     "moonep_swiglu_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp]),
     "moonep_router_fwd": (_i, [_vp, _vp, _i, _i, _i, _i] + [_vp] * 7),
     "moonep_router_bwd": (_i, [_vp] * 5 + [_i] * 4 + [_vp, _vp, _vp]),

@@ -59,20 +59,33 @@ def swiglu_bwd(a, u, g, w, total_rows, dadu, hsw, dgate) -> None:
     _lib.check(rc, "moonep_swiglu_bwd")
 
 
+_UPDATE_TENSORS = 3  # weights per launch of the update kernels
+
+
 def sgd_update(w: torch.Tensor, g: torch.Tensor, lr: float) -> None:
     """``w -= lr * g`` for a bf16 weight tensor and its fp32 gradient (same shape, contiguous)."""
-    assert w.shape == g.shape
-    if not w.is_cuda or w.numel() % 8 != 0:
-        w.add_(g, alpha=-lr)
-        return
-    assert w.is_contiguous() and g.is_contiguous() and w.dtype == torch.bfloat16 and g.dtype == torch.float32
-    with _lib.on_device(w.device):
-        rc = _lib.load().moonep_sgd_update(w.data_ptr(), g.data_ptr(), w.numel(), float(lr),
-                                           _lib.current_stream())  # fmt: skip
-    _lib.check(rc, "moonep_sgd_update")
+    sgd_updates([w], [g], lr)
 
 
-_ADAM_TENSORS = 3  # weights per launch of the AdamW kernel
+def sgd_updates(weights, grads, lr: float) -> None:
+    """``w -= lr * g`` for any number of bf16 weights and their fp32 gradients, the kernel's share in one launch."""
+    todo = []
+    for w, g in zip(weights, grads):
+        assert w.shape == g.shape
+        if not w.is_cuda or w.numel() % 8 != 0 or (w.data_ptr() | g.data_ptr()) % 16 != 0:
+            w.add_(g, alpha=-lr)
+            continue
+        assert w.is_contiguous() and g.is_contiguous() and w.dtype == torch.bfloat16 and g.dtype == torch.float32
+        todo.append((w, g))
+    while todo:
+        some = [t for t in todo if t[0].device == todo[0][0].device][:_UPDATE_TENSORS]
+        todo = [t for t in todo if all(t is not s for s in some)]
+        n = len(some)
+        ws, gs = ((ctypes.c_void_p * n)(*[t[i].data_ptr() for t in some]) for i in (0, 1))
+        sizes = (ctypes.c_longlong * n)(*[w.numel() for w, _ in some])
+        with _lib.on_device(some[0][0].device):
+            rc = _lib.load().moonep_sgd_update(n, ws, gs, sizes, float(lr), _lib.current_stream())
+        _lib.check(rc, "moonep_sgd_update")
 
 
 def adamw_update(masters, exp_avgs, exp_avg_sqs, grads, weights, *, lr, b1, b2, eps, weight_decay, c1, c2) -> None:
@@ -81,8 +94,8 @@ def adamw_update(masters, exp_avgs, exp_avg_sqs, grads, weights, *, lr, b1, b2, 
     tensors = [list(ts) for ts in (masters, exp_avgs, exp_avg_sqs, grads, weights)]
     if len({len(ts) for ts in tensors}) != 1:
         raise ValueError(f"adamw_update: lists of {[len(ts) for ts in tensors]} tensors")
-    for i in range(0, len(tensors[4]), _ADAM_TENSORS):
-        _adamw_step([ts[i : i + _ADAM_TENSORS] for ts in tensors], lr, b1, b2, eps, weight_decay, c1, c2)
+    for i in range(0, len(tensors[4]), _UPDATE_TENSORS):
+        _adamw_step([ts[i : i + _UPDATE_TENSORS] for ts in tensors], lr, b1, b2, eps, weight_decay, c1, c2)
 
 
 def _adamw_step(tensors, lr, b1, b2, eps, weight_decay, c1, c2) -> None:
