@@ -343,6 +343,12 @@ int moonep_wgrad_single_cta_adding(int rows_per_group, int num_sms);
 int moonep_grouped_wgrad_rows(const void* l, long long ldl, const void* r, long long ldr, int rows, int P, int Q,
                               const int* cu_seqlens, int G, void* const* out_ptrs, const int* flags, int* status,
                               long long timeout_ms, int rows_per_group, int adds, int num_sms, const int* pads, void* stream);
+// Up to three weights (a null l ends them) of the same groups of rows in one launch.
+int moonep_grouped_wgrad_layer(const void* l0, long long ldl0, const void* r0, long long ldr0, int P0, int Q0, void* const* out0,
+                               const void* l1, long long ldl1, const void* r1, long long ldr1, int P1, int Q1, void* const* out1,
+                               const void* l2, long long ldl2, const void* r2, long long ldr2, int P2, int Q2, void* const* out2,
+                               int rows, const int* cu_seqlens, int G, const int* flags, int* status, long long timeout_ms,
+                               int rows_per_group, int adds, int num_sms, const int* pads, void* stream);
 // Helpers of the MoE layer's backward pass and optimiser step, see moe_kernels.cu.
 int moonep_transpose_experts(const void* src, void* dst, int n, int d0, int d1, long long dst_ld,
                              long long dst_expert_stride, int col0, const int* active, void* stream);

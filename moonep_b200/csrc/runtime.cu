@@ -178,7 +178,7 @@ extern "C" int moonep_call(int fn, const long long* words) {
     case 5: return call_words(moonep_grouped_gemm_pair, words);
     case 6: return call_words(moonep_grouped_gemm_pair_hooked, words);
     case 7: return call_words(moonep_grouped_gemm_pair_kn, words);
-    case 8: return call_words(moonep_grouped_wgrad_rows, words);
+    case 8: return call_words(moonep_grouped_wgrad_layer, words);
     case 9: return call_words(moonep_signal_wait, words);
     case 10: return call_words(moonep_plan_publish, words);
     case 11: return call_words(moonep_swiglu_bwd, words);

@@ -20,7 +20,7 @@ remote expert that did not get a prefetch slot is read in place over NVLink.
 
 Usage pattern of the reference's Buffer API: reference ``README.md:46-48`` and ``tests/test_e2e.py:201-431``.
 Every GEMM of the layer is a tcgen05 kernel of this package: forward and activation gradients on CTA pairs
-(``grouped_gemm``, ``grouped_gemm_kn``), weight gradients on ``grouped_wgrad_rows``; the backward takes the weights
+(``grouped_gemm``, ``grouped_gemm_kn``), weight gradients on ``grouped_wgrad_layer``; the backward takes the weights
 and activations as they are stored (MN-major tiles), the forward keeps both SwiGLU pre-activations for it.
 Per-group torch matmuls remain for CPU tensors and for shapes outside the kernels' tiling.
 """
@@ -41,6 +41,7 @@ from ..ops.grouped_gemm import (
     grouped_wgrad,
     kn_kernel_supports,
     WGRAD_MAX_GROUPS,
+    grouped_wgrad_layer,
     grouped_wgrad_rows,
     wgrad_kernel_supports,
 )
@@ -331,12 +332,15 @@ class ExpertParallelMoE:
         kw = {"status": status, "rows_per_group": max(1, self.S * self.K // self.epn), "adds": not self._fresh}
         if config.wgrad_layout() == "rows":  # the kernel stages MN-major tiles: the activations as they are
             kw["pads"] = plan.zero_fill_ranges  # rows of zeros in all of them
-            grouped_wgrad_rows(dy_nvs, hsw, cu, ptrs[2], flags, **kw)  # dW_down = dy^T (h * gate weight)
+            batch = [] if after is None else None  # in one launch, or each as soon as it can be sent on
+            grouped_wgrad_rows(dy_nvs, hsw, cu, ptrs[2], flags, batch=batch, **kw)  # dW_down = dy^T (h * gate weight)
             done(2)
-            grouped_wgrad_rows(dadu[:, :I], x_nvs, cu, ptrs[0], flags, num_sms=later, **kw)  # dW_gate = da^T x
+            grouped_wgrad_rows(dadu[:, :I], x_nvs, cu, ptrs[0], flags, num_sms=later, batch=batch, **kw)  # dW_gate = da^T x
             done(0)
-            grouped_wgrad_rows(dadu[:, I:], x_nvs, cu, ptrs[1], flags, num_sms=later, **kw)  # dW_up   = du^T x
+            grouped_wgrad_rows(dadu[:, I:], x_nvs, cu, ptrs[1], flags, num_sms=later, batch=batch, **kw)  # dW_up   = du^T x
             done(1)
+            if batch:
+                grouped_wgrad_layer(batch, cu, flags, **kw)
         else:  # K-major tiles from transposed copies
 
             def transposed(t):

@@ -101,7 +101,7 @@ _ull = ctypes.c_ulonglong
 # functions that moonep_call knows by number, in its order
 _BY_NUMBER = (
     "moonep_dispatch_single", "moonep_combine_single", "moonep_dispatch", "moonep_combine_push", "moonep_grouped_gemm",
-    "moonep_grouped_gemm_pair", "moonep_grouped_gemm_pair_hooked", "moonep_grouped_gemm_pair_kn", "moonep_grouped_wgrad_rows",
+    "moonep_grouped_gemm_pair", "moonep_grouped_gemm_pair_hooked", "moonep_grouped_gemm_pair_kn", "moonep_grouped_wgrad_layer",
     "moonep_signal_wait", "moonep_plan_publish", "moonep_swiglu_bwd",
 )  # fmt: skip
 
@@ -141,6 +141,7 @@ _SIGNATURES = {
     "moonep_grouped_wgrad": (_i, [_vp, _vp, _ll, _i, _i, _vp, _i, _vp, _vp, _i, _vp, _ll, _i, _i, _i, _vp]),
     "moonep_wgrad_single_cta": (_i, [_i, _i]),
     "moonep_wgrad_single_cta_adding": (_i, [_i, _i]),
+    "moonep_grouped_wgrad_layer": (_i, [_vp, _ll, _vp, _ll, _i, _i, _vp] * 3 + [_i, _vp, _i, _vp, _vp, _ll, _i, _i, _i, _vp, _vp]),
     "moonep_grouped_wgrad_rows": (_i, [_vp, _ll, _vp, _ll, _i, _i, _i, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _vp, _vp]),
     "moonep_transpose_experts": (_i, [_vp, _vp, _i, _i, _i, _ll, _ll, _i, _vp, _vp]),
     "moonep_adamw_update": (_i, [_i] + [ctypes.POINTER(_vp)] * 5 + [ctypes.POINTER(_ll)] + [ctypes.c_double] * 6 + [_vp]),

@@ -245,30 +245,42 @@ def grouped_wgrad(left_t, right_t, cu_seqlens, out_ptrs, flags, *, status=None, 
 
 
 def grouped_wgrad_rows(left, right, cu_seqlens, out_ptrs, flags, *, status=None, num_sms=0, rows_per_group=0, adds=False,
-                       pads=None):  # fmt: skip
+                       pads=None, batch=None):  # fmt: skip
     """``grouped_wgrad`` from the operands as they are: ``left`` ``[rows, P]`` and ``right`` ``[rows, Q]`` bf16 with unit
     column stride (column slices of wider tensors are fine), no transposed copies.  Same targets, flags and bounds.
     ``pads`` (int32 ``[G, 2]``, e.g. a plan's ``zero_fill_ranges``): the first and the number of each group's last rows that
-    hold zeros in both operands; they are left out, which changes nothing but the time."""
-    rows, P = (int(v) for v in left.shape)
-    Q = int(right.shape[1])
-    G = int(cu_seqlens.numel())
-    assert right.shape[0] == rows and left.dtype == torch.bfloat16 and right.dtype == torch.bfloat16
-    assert left.stride(1) == 1 and right.stride(1) == 1 and left.is_cuda
-    ldl, ldr = int(left.stride(0)), int(right.stride(0))
-    assert P % 128 == 0 and Q % 256 == 0 and ldl % 8 == 0 and ldr % 8 == 0, f"P={P}, Q={Q}, strides {ldl}, {ldr}"
-    assert G <= WGRAD_MAX_GROUPS, f"grouped_wgrad_rows: at most {WGRAD_MAX_GROUPS} groups per launch"
-    assert left.data_ptr() % 16 == 0 and right.data_ptr() % 16 == 0
-    assert out_ptrs.dtype == torch.int64 and out_ptrs.numel() == G and out_ptrs.is_cuda and out_ptrs.is_contiguous()
+    hold zeros in both operands; they are left out, which changes nothing but the time.
+    With ``batch`` (a list) nothing is launched: the weight joins it, for one ``grouped_wgrad_layer`` with the same groups."""
+    if batch is not None:
+        batch.append((left, right, out_ptrs))
+        return
+    grouped_wgrad_layer([(left, right, out_ptrs)], cu_seqlens, flags, status=status, num_sms=num_sms, rows_per_group=rows_per_group,
+                        adds=adds, pads=pads)  # fmt: skip
+
+
+def grouped_wgrad_layer(weights, cu_seqlens, flags, *, status=None, num_sms=0, rows_per_group=0, adds=False, pads=None):
+    """``grouped_wgrad_rows`` of one to three weights, ``(left, right, out_ptrs)`` each, in one launch."""
+    rows, G = int(weights[0][0].shape[0]), int(cu_seqlens.numel())
+    assert 1 <= len(weights) <= 3 and G <= WGRAD_MAX_GROUPS, f"grouped_wgrad_rows: at most {WGRAD_MAX_GROUPS} groups per launch"
+    words = []
+    for left, right, out_ptrs in weights:
+        P, Q = int(left.shape[1]), int(right.shape[1])
+        assert left.shape[0] == right.shape[0] == rows and left.dtype == torch.bfloat16 and right.dtype == torch.bfloat16
+        assert left.stride(1) == 1 and right.stride(1) == 1 and left.is_cuda
+        ldl, ldr = int(left.stride(0)), int(right.stride(0))
+        assert P % 128 == 0 and Q % 256 == 0 and ldl % 8 == 0 and ldr % 8 == 0, f"P={P}, Q={Q}, strides {ldl}, {ldr}"
+        assert left.data_ptr() % 16 == 0 and right.data_ptr() % 16 == 0
+        assert out_ptrs.dtype == torch.int64 and out_ptrs.numel() == G and out_ptrs.is_cuda and out_ptrs.is_contiguous()
+        words += (left.data_ptr(), ldl, right.data_ptr(), ldr, P, Q, out_ptrs.data_ptr())
+    words += (0,) * 7 * (3 - len(weights))
     assert flags.dtype == torch.int32 and flags.numel() == G and flags.is_cuda and flags.is_contiguous()
     assert cu_seqlens.dtype == torch.int32 and cu_seqlens.is_contiguous() and cu_seqlens.is_cuda
     if pads is not None:
         assert pads.dtype == torch.int32 and tuple(pads.shape) == (G, 2) and pads.is_contiguous() and pads.device == left.device
     with _lib.on_device(left.device):
-        rc = _lib.caller("moonep_grouped_wgrad_rows")(
-            left.data_ptr(), ldl, right.data_ptr(), ldr, rows, P, Q, cu_seqlens.data_ptr(), G, out_ptrs.data_ptr(),
-            flags.data_ptr(), 0 if status is None else status.data_ptr(), config.timeout_ms(), int(rows_per_group),
-            int(adds), int(num_sms), 0 if pads is None else pads.data_ptr(), _lib.current_stream(),
+        rc = _lib.caller("moonep_grouped_wgrad_layer")(
+            *words, rows, cu_seqlens.data_ptr(), G, flags.data_ptr(), 0 if status is None else status.data_ptr(), config.timeout_ms(),
+            int(rows_per_group), int(adds), int(num_sms), 0 if pads is None else pads.data_ptr(), _lib.current_stream(),
         )  # fmt: skip
     _lib.check(rc, "moonep_grouped_wgrad_rows")
 
