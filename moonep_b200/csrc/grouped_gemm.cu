@@ -23,6 +23,8 @@
 //                                                              128 output columns per tile)
 //            SCALE  y = acc * row_scale[row]                   (down projection times the gate
 //                                                              weight carried with the row)
+// W may also be given as [G, K, N] (N contiguous, MN-major tiles; PLAIN only): the activation gradients, see
+// moonep_grouped_gemm_kn.
 // Every mbarrier wait is bounded; on expiry the role records a status word and leaves its loop, the
 // CTA still frees its TMEM before it returns.
 //
@@ -60,7 +62,7 @@ struct Ring {  // barriers: of the stages, and of the two accumulators
   unsigned long long full[kMaxStages], empty[kMaxStages], tfull[2], tempty[2];
 };
 
-template <int kSplit>
+template <int kSplit, bool kKn>
 __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& maps, unsigned char* s_tiles, Ring& ring, unsigned tmem_base,
                                           int row_blocks) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -76,7 +78,17 @@ __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& map
       int stage = 0;
       unsigned phase = 0;
       bool failed = false;
-      auto load_weights = [&](unsigned char* st, int kb, int wrow0) {
+      auto load_weights = [&](unsigned char* st, int kb, int wslot, int nb) {
+        if constexpr (kKn) {  // W is [slots, K, N], of one tensor or two
+          const bool second = kb >= a.k_split;
+          const int kdim = (second ? a.k_blocks - a.k_split : a.k_split) * BK;  // K rows per expert in that tensor
+          const int y = wslot * kdim + (second ? kb - a.k_split : kb) * BK;
+#pragma unroll
+          for (int c = 0; c < 2 * half_rows / 64; ++c)
+            tma_load_mn(st + c * 64 * BK * 2, second ? maps.b1 : maps.b0, nb * (2 * half_rows / 64) + c, y, ring.full + stage);
+          return;
+        }
+        const int wrow0 = wslot * a.n_per_group + nb * b_rows_per_tile;
 #pragma unroll
         for (int r = 0; r < half_rows; r += kBoxRows) {
           tma_load_2d(st + r * BK * 2, maps.b0, kb * BK, wrow0 + r, ring.full + stage);
@@ -98,7 +110,6 @@ __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& map
           if (lane == 0) gemm_bad_index(a.status, 13, 13, lo, wslot);
           wslot = 0;
         }
-        const int wrow0 = wslot * a.n_per_group + nb * b_rows_per_tile;
         // A first tile's weights need not wait for the kernel that makes its rows, whose last CTAs leave memory and SMs idle: a
         // layer's pass, S=64, I=1024, 16 groups, H=2048 66.9 -> 64.8 us, H=4096 103.2 -> 100.3.
         int asked = 0;  // K blocks whose weights are on their way
@@ -107,7 +118,7 @@ __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& map
           for (; stage < asked; ++stage) {
             if (elect_one()) {
               mbar_expect_tx(ring.full + stage, stage_bytes);
-              load_weights(s_tiles + (size_t)stage * stage_bytes + kATileBytes, stage, wrow0);
+              load_weights(s_tiles + (size_t)stage * stage_bytes + kATileBytes, stage, wslot, nb);
             }
             __syncwarp();
           }
@@ -124,7 +135,7 @@ __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& map
             unsigned char* st = s_tiles + (size_t)stage * stage_bytes;
             if (kb >= asked) mbar_expect_tx(ring.full + stage, stage_bytes);
             tma_load_2d(st, maps.a, kb * BK, row0, ring.full + stage);
-            if (kb >= asked) load_weights(st + kATileBytes, kb, wrow0);
+            if (kb >= asked) load_weights(st + kATileBytes, kb, wslot, nb);
           }
           __syncwarp();
           if (++stage == stages) {
@@ -138,9 +149,11 @@ __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& map
   } else if (warp == 1) {
     // ---------------- MMA issuer: the whole warp waits, one lane issues ----------------
     {
-      constexpr unsigned idesc = make_idesc(BM, BN / kSplit);
+      constexpr unsigned idesc = make_idesc(BM, BN / kSplit, false, kKn);
+      constexpr unsigned bstep = kKn ? kDescStepMn : kDescStepK;
       // descriptors of stage 0; those of another lie a stage's bytes further, in 16-byte units
-      const unsigned long long adesc0 = make_smem_desc(s_tiles), bdesc0 = make_smem_desc(s_tiles + kATileBytes);
+      const unsigned long long adesc0 = make_smem_desc(s_tiles);
+      const unsigned long long bdesc0 = kKn ? make_smem_desc_mn(s_tiles + kATileBytes) : make_smem_desc(s_tiles + kATileBytes);
       int stage = 0;
       unsigned phase = 0;
       unsigned tphase[2] = {0, 0};
@@ -166,7 +179,7 @@ __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& map
 #pragma unroll
             for (int kk = 0; kk < BK / UMMA_K; ++kk) {
               // 16 bf16 = 32 bytes further along K inside the swizzled 128-byte rows
-              umma_bf16(d_tmem, adesc0 + off + (unsigned long long)(kk * kDescStepK), bdesc0 + off + (unsigned long long)(kk * kDescStepK),
+              umma_bf16(d_tmem, adesc0 + off + (unsigned long long)(kk * kDescStepK), bdesc0 + off + (unsigned long long)(kk * bstep),
                         idesc, (kb | kk) != 0 ? 1u : 0u);
             }
             umma_commit(ring.empty + stage);
@@ -204,7 +217,7 @@ __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& map
       tc_fence_after();
       const int row = mb * BM + q * 32 + lane;
       const unsigned taddr = tmem_base + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN);
-      if (a.mode == kSwiglu) {
+      if (!kKn && a.mode == kSwiglu) {
         uint16_t* orow = a.out + (long long)row * a.ldo + (long long)nb * half_rows;
         // columns of a warp; of a quarter of a tile the second warps have none
         constexpr int mine = half_rows / 2 > 32 ? half_rows / 2 : 32;
@@ -262,7 +275,7 @@ __device__ __forceinline__ void run_tiles(const GemmArgs& a, const GemmMaps& map
   }
 }
 
-template <bool kMaySplit>
+template <bool kMaySplit, bool kKn>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                         const __grid_constant__ CUtensorMap tmap_b1, const GemmArgs a) {
@@ -309,11 +322,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   int split = 1;
   while (kMaySplit && split < kMaxSplit && (long long)row_blocks * a.n_tiles * split * 2 <= gridDim.x) split *= 2;
   if (split == 1)
-    run_tiles<1>(a, maps, s_tiles, ring, tmem_base, row_blocks);
+    run_tiles<1, kKn>(a, maps, s_tiles, ring, tmem_base, row_blocks);
   else if (split == 2)
-    run_tiles<2>(a, maps, s_tiles, ring, tmem_base, row_blocks);
+    run_tiles<2, kKn>(a, maps, s_tiles, ring, tmem_base, row_blocks);
   else
-    run_tiles<kMaxSplit>(a, maps, s_tiles, ring, tmem_base, row_blocks);
+    run_tiles<kMaxSplit, kKn>(a, maps, s_tiles, ring, tmem_base, row_blocks);
 
   tc_fence_before();
   __syncthreads();
@@ -327,20 +340,37 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
 // ---- host side --------------------------------------------------------------------------------------
 
-template <bool kMaySplit>
+template <bool kMaySplit, bool kKn>
 static int launch_of(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const GemmArgs& a, int grid,
                      cudaStream_t stream) {
   const size_t smem = (size_t)kStages * kStageBytes + 1024;
   static bool attr_set = false;
   if (!attr_set) {
-    if (int rc = check_cuda(cudaFuncSetAttribute(grouped_gemm_kernel<kMaySplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (int rc = check_cuda(cudaFuncSetAttribute(grouped_gemm_kernel<kMaySplit, kKn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem),
                             "cudaFuncSetAttribute(grouped_gemm_kernel)"))
       return rc;
     attr_set = true;
   }
-  return check_cuda(launch_maybe_pdl(grouped_gemm_kernel<kMaySplit>, grid, kGemmThreads, smem, stream, a.early != 0, ta, tb0, tb1, a),
+  return check_cuda(launch_maybe_pdl(grouped_gemm_kernel<kMaySplit, kKn>, grid, kGemmThreads, smem, stream, a.early != 0, ta, tb0, tb1, a),
                     "launch grouped_gemm_kernel");
+}
+
+template <bool kKn>
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, GemmArgs& a, int num_sms, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int grid = imax(1, num_sms > 0 ? imin(num_sms, sms) : sms);
+  a.early = expert_pdl(num_sms) ? 1 : 0;
+  // The rows are known on the device only.  Half the capacity stands for them here: a dispatched shard has room for almost two
+  // blocks of padding per group.  The kernel that may cut tiles costs 0.4 us per launch where it does not (S=64, H=2048, I=1024,
+  // 16 groups: a layer's pass 66.9 without and 67.9 with it).
+  const bool may_split = (long long)a.rows_cap / BM * a.n_tiles <= grid;
+  if (int rc = may_split ? launch_of<true, kKn>(ta, tb0, tb1, a, grid, stream)
+                         : launch_of<false, kKn>(ta, tb0, tb1, a, grid, stream))
+    return rc;
+  return check_launch("grouped_gemm_kernel");
 }
 
 }  // namespace moonep
@@ -402,18 +432,43 @@ extern "C" int moonep_grouped_gemm(const void* x, const void* w0, const void* w1
   a.b_kn = 0;
   a.k_split = a.k_blocks;
   memset(&a.hooks, 0, sizeof(a.hooks));
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = imax(1, num_sms > 0 ? imin(num_sms, sms) : sms);
-  a.early = expert_pdl(num_sms) ? 1 : 0;
   a.weights_early = weights_early;
-  // The rows are known on the device only.  Half the capacity stands for them here: a dispatched shard has room for almost two
-  // blocks of padding per group.  The kernel that may cut tiles costs 0.4 us per launch where it does not (S=64, H=2048, I=1024,
-  // 16 groups: a layer's pass 66.9 without and 67.9 with it).
-  const bool may_split = (long long)rows_cap / BM * a.n_tiles <= grid;
-  if (int rc = may_split ? launch_of<true>(ta, tb0, tb1, a, grid, (cudaStream_t)stream)
-                         : launch_of<false>(ta, tb0, tb1, a, grid, (cudaStream_t)stream))
-    return rc;
-  return check_launch("grouped_gemm_kernel");
+  return launch<false>(ta, tb0, tb1, a, num_sms, (cudaStream_t)stream);
+}
+
+// The same with W given as [slots, K, N] (N contiguous), see moonep_grouped_gemm_pair_kn.  For groups of one row block, which
+// leave the second CTA of a pair without rows: training step, us, on pairs and here: S=64, H=1024, I=256, 6 experts 80.7 and 71.0;
+// S=500, I=512, 12 experts 129.6 and 117.2; S=200, H=2048, I=1024, 16 experts 339 and 323; S=1000 378 and 375.5.
+extern "C" int moonep_grouped_gemm_kn(const void* x, const void* w0, int K0, const void* w1, int K1, void* out, const int* cu_seqlens,
+                                      int G, int rows_cap, int N, int w_slots, int* status, long long timeout_ms, int num_sms,
+                                      int weights_early, void* stream) {
+  if (w1 == nullptr) K1 = 0;
+  if (K0 <= 0 || K0 % BK != 0 || K1 < 0 || K1 % BK != 0 || N <= 0 || N % BN != 0 || w_slots <= 0) {
+    set_error("moonep_grouped_gemm_kn: K0, K1 must be multiples of 64 and N a multiple of 256");
+    return 1;
+  }
+  CUtensorMap ta, tb0, tb1;
+  if (int rc = make_tmap(&ta, x, (unsigned long long)rows_cap, (unsigned long long)(K0 + K1), BM)) return rc;
+  if (int rc = make_tmap_mn(&tb0, w0, (unsigned long long)w_slots * K0, (unsigned long long)N, 0, 1)) return rc;
+  tb1 = tb0;
+  if (K1)
+    if (int rc = make_tmap_mn(&tb1, w1, (unsigned long long)w_slots * K1, (unsigned long long)N, 0, 1)) return rc;
+  GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  a.out = (uint16_t*)out;
+  a.cu_seqlens = cu_seqlens;
+  a.status = status;
+  a.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 10000) * 1000000ull;
+  a.G = G;
+  a.n_per_group = N;
+  a.n_tiles = N / BN;
+  a.k_blocks = (K0 + K1) / BK;
+  a.ldo = N;
+  a.mode = kPlain;
+  a.rows_cap = rows_cap;
+  a.w_slots = w_slots;
+  a.b_kn = 1;
+  a.k_split = K0 / BK;
+  a.weights_early = weights_early;
+  return launch<true>(ta, tb0, tb1, a, num_sms, (cudaStream_t)stream);
 }

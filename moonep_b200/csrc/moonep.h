@@ -324,6 +324,10 @@ int moonep_grouped_gemm_pair_hooked(const void* x, const void* w0, const void* w
 int moonep_grouped_gemm_pair_kn(const void* x, const void* w0, int K0, const void* w1, int K1, void* out,
                                 const int* cu_seqlens, int G, int rows_cap, int N, int w_slots, int* status,
                                 long long timeout_ms, int num_sms, void* stream);
+// With one CTA per tile, see grouped_gemm.cu; weights_early as there.
+int moonep_grouped_gemm_kn(const void* x, const void* w0, int K0, const void* w1, int K1, void* out, const int* cu_seqlens, int G,
+                           int rows_cap, int N, int w_slots, int* status, long long timeout_ms, int num_sms, int weights_early,
+                           void* stream);
 // Host-side walk of the CTA-pair kernel's tile schedule, for tests (grouped_gemm_pair.cu).
 int moonep_pair_schedule(const int* cu_seqlens, int G, int rows_cap, int n_tiles, int pair, int npairs, int* out,
                          int max_tiles);

@@ -182,6 +182,7 @@ extern "C" int moonep_call(int fn, const long long* words) {
     case 9: return call_words(moonep_signal_wait, words);
     case 10: return call_words(moonep_plan_publish, words);
     case 11: return call_words(moonep_swiglu_bwd, words);
+    case 12: return call_words(moonep_grouped_gemm_kn, words);
   }
   set_error("moonep_call: no such function");
   return -1;

@@ -183,7 +183,7 @@ struct GemmArgs {
   int rows_cap;      // rows of X
   const int* group_map;  // [G] weight slot of every group, or null for the identity
   int w_slots;           // number of weight slots (rows of W = w_slots * n_per_group)
-  int b_kn;              // CTA-pair kernel only: W is [slots, K, N] (N contiguous), staged as MN-major tiles
+  int b_kn;              // W is [slots, K, N] (N contiguous), staged as MN-major tiles
   int k_split;           // with b_kn: K blocks served by the first W tensor, the rest come from the second
   uint16_t* pre_gate;    // SwiGLU only, optional: the pre-activations x Wg^T and x Wu^T, [rows, ldo] bf16 each,
   uint16_t* pre_up;      // kept for the backward pass so that it need not recompute them
@@ -351,7 +351,7 @@ inline int make_tmap(CUtensorMap* m, const void* base, unsigned long long rows, 
 // under `lane == 0` against one issued by an elected lane: [K, N] products of 1 x 16384 rows, K=N=4096, 425 and 338 us; 8 x 1024,
 // K=7168, N=2048, 182 and 155; weight gradients 8 x 1024 rows, 2048 x 7168, 197 and 183.
 inline int make_tmap_mn(CUtensorMap* m, const void* base, unsigned long long rows, unsigned long long cols,
-                        unsigned long long ld = 0) {
+                        unsigned long long ld = 0, unsigned box_blocks = 2) {
   EncodeTiledFn fn = encode_tiled();
   if (fn == nullptr) {
     set_error("cuTensorMapEncodeTiled is not available (no CUDA driver?)");
@@ -359,7 +359,7 @@ inline int make_tmap_mn(CUtensorMap* m, const void* base, unsigned long long row
   }
   cuuint64_t dims[3] = {64, rows, cols / 64};
   cuuint64_t strides[2] = {(ld ? ld : cols) * 2, 128};
-  cuuint32_t box[3] = {64, 64, 2};
+  cuuint32_t box[3] = {64, 64, box_blocks};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -134,7 +134,8 @@ class ExpertParallelMoE:
         CTA per tile takes 0.86 to 0.92 of the pairs' time on average over 4 to 32 experts, H 1024 to 7168, I 512 to 2048
         with even and Zipf routing (0.73 to 1.19, the worst with Zipf routing, whose hot experts have several blocks: 8
         experts of 128 rows, H=7168).  At 192 rows that is 0.93 to 0.96, but 1.19 for the largest experts, at 256 rows 0.99
-        to 1.03, at 512 rows 1.04 to 1.08.  The counts are not known on the host, so their mean decides.  With several ranks
+        to 1.03, at 512 rows 1.04 to 1.08.  The activation gradients follow the same line (a training step 0.88 to 0.95 up to 64
+        rows per expert, 0.99 at 125).  The counts are not known on the host, so their mean decides.  With several ranks
         the hand-off hooks need the pairs, and ``MOONEP_GEMM_PAIR=1``, where it is set, means pairs."""
         switch = config.gemm_pair_switch()
         if switch is None:
@@ -286,10 +287,11 @@ class ExpertParallelMoE:
         if overlap:
             total = torch.cuda.get_device_properties(dev).multi_processor_count
             sms = max(2, (total - int(self.buffer._require_ctx()["num_sms"])) // 2 * 2)
-        if not self._weight_grads_on_kernel(x_nvs, dy_nvs, dadu, hsw, cu, plan, after=reduce_one if overlap else None, num_sms=sms):
+        launched = self._weight_grads_on_kernel(x_nvs, dy_nvs, dadu, hsw, cu, plan, after=reduce_one if overlap else None, num_sms=sms)
+        if not launched:
             self._weight_grads_per_group(x_nvs, dy_nvs, dadu, hsw, cu)
         self._times_weights(dadu, [self.w_gate, self.w_up], cu, plan, out=dy_nvs,
-                            num_sms=sms if reduced else 0)  # dx rows = da Wg + du Wu
+                            num_sms=sms if reduced else 0, weights_early=launched and self.R == 1)  # dx rows = da Wg + du Wu
         dx, dgates, _ = buf.combine(plan, dy_nvs, dgate_nvs, zero_copy=True)
         if reduced:
             for ev in reduced:  # the gradients are complete, and the reduce slots cleared, for whatever comes next
@@ -298,12 +300,13 @@ class ExpertParallelMoE:
             self.buffer.reduce_grad(plan, False, *grads, self.red[0], self.red[1], self.red[2], owner_local=True)
         return dx, dgates
 
-    def _times_weights(self, x, ws, cu, plan, out=None, num_sms=0):
+    def _times_weights(self, x, ws, cu, plan, out=None, num_sms=0, weights_early=False):
         """``x[rows of g] @ cat(ws, dim=1)[g]`` per group: what an activation gradient needs from forward weights
-        stored ``[E+B, out, in]`` (which is ``[G, K, N]`` for this product).  The CTA-pair kernel stages them as
+        stored ``[E+B, out, in]`` (which is ``[G, K, N]`` for this product).  The kernels stage them as
         MN-major tiles; elsewhere K-major copies of the local experts feed the ordinary grouped GEMM."""
         if kn_kernel_supports(x, ws):
-            return grouped_gemm_kn(x, ws, cu, out=out, num_sms=num_sms)
+            return grouped_gemm_kn(x, ws, cu, out=out, num_sms=num_sms, pair=self.forward_gemm_pair() is not False,
+                                   weights_early=weights_early)  # fmt: skip
         return grouped_gemm(x, self._local_transposed(ws, plan), cu, group_map=self.group_map, out=out,
                             status=self.buffer._require_ctx()["_backend"].status if x.is_cuda else None)
 

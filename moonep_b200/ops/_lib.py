@@ -102,7 +102,7 @@ _ull = ctypes.c_ulonglong
 _BY_NUMBER = (
     "moonep_dispatch_single", "moonep_combine_single", "moonep_dispatch", "moonep_combine_push", "moonep_grouped_gemm",
     "moonep_grouped_gemm_pair", "moonep_grouped_gemm_pair_hooked", "moonep_grouped_gemm_pair_kn", "moonep_grouped_wgrad_layer",
-    "moonep_signal_wait", "moonep_plan_publish", "moonep_swiglu_bwd",
+    "moonep_signal_wait", "moonep_plan_publish", "moonep_swiglu_bwd", "moonep_grouped_gemm_kn",
 )  # fmt: skip
 
 _SIGNATURES = {
@@ -136,6 +136,7 @@ _SIGNATURES = {
     "moonep_grouped_gemm": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _ll, _i, _vp, _i, _vp, _vp, _i, _vp]),
     "moonep_grouped_gemm_pair": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _ll, _i, _vp, _i, _vp, _vp, _vp]),
     "moonep_grouped_gemm_pair_hooked": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _ll, _i, _vp, _i, _vp, _vp, _vp, _vp]),
+    "moonep_grouped_gemm_kn": (_i, [_vp, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _ll, _i, _i, _vp]),
     "moonep_grouped_gemm_pair_kn": (_i, [_vp, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _ll, _i, _vp]),
     "moonep_pair_schedule": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _i]),
     "moonep_grouped_wgrad": (_i, [_vp, _vp, _ll, _i, _i, _vp, _i, _vp, _vp, _i, _vp, _ll, _i, _i, _i, _vp]),

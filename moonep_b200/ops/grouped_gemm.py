@@ -153,11 +153,12 @@ def kn_kernel_supports(x, ws) -> bool:
             and x.shape[0] >= 128 and len(ws) in (1, 2) and config.gemm_on_cta_pairs())  # fmt: skip
 
 
-def grouped_gemm_kn(x, ws, cu_seqlens, *, out=None, status=None, num_sms=0):
+def grouped_gemm_kn(x, ws, cu_seqlens, *, out=None, status=None, num_sms=0, pair=True, weights_early=False):
     """``y[rows of g] = x[rows of g] @ W[g]`` with the weights given as ``[G, K, N]`` (N contiguous): the product an
     activation gradient needs from forward weights stored ``[G, out, in]``, without transposed copies.  ``ws`` is one
-    tensor or two that continue the contraction (``x = [a | b]``, ``W = [ws[0]; ws[1]]``).  Runs on the CTA-pair kernel
-    (MN-major W tiles); a per-group fp32 reference elsewhere."""
+    tensor or two that continue the contraction (``x = [a | b]``, ``W = [ws[0]; ws[1]]``).  Runs on CTA pairs or, with
+    ``pair=False``, one CTA per tile (MN-major W tiles); a per-group fp32 reference elsewhere.  ``weights_early`` (one CTA per
+    tile): the kernel launched just before on this stream writes neither the weights nor ``cu_seqlens``."""
     ws = list(ws)
     G, _, N = (int(v) for v in ws[0].shape)
     Ks = [int(w.shape[1]) for w in ws]
@@ -175,12 +176,15 @@ def grouped_gemm_kn(x, ws, cu_seqlens, *, out=None, status=None, num_sms=0):
         out = torch.empty(x.shape[0], N, dtype=torch.bfloat16, device=x.device)
     assert out.is_contiguous() and out.shape == (x.shape[0], N) and out.dtype == torch.bfloat16
     with _lib.on_device(x.device):
-        rc = _lib.caller("moonep_grouped_gemm_pair_kn")(
+        args = (
             x.data_ptr(), ws[0].data_ptr(), Ks[0], ws[1].data_ptr() if len(ws) == 2 else 0, Ks[1] if len(ws) == 2 else 0,
             out.data_ptr(), cu_seqlens.data_ptr(), G, int(x.shape[0]), N, G, 0 if status is None else status.data_ptr(),
-            config.timeout_ms(), int(num_sms), _lib.current_stream(),
+            config.timeout_ms(), int(num_sms),
         )  # fmt: skip
-    _lib.check(rc, "moonep_grouped_gemm_pair_kn")
+        st = _lib.current_stream()
+        rc = _lib.caller("moonep_grouped_gemm_pair_kn")(*args, st) if pair else _lib.caller("moonep_grouped_gemm_kn")(
+            *args, int(weights_early), st)
+    _lib.check(rc, "moonep_grouped_gemm_kn")
     return out
 
 
