@@ -266,7 +266,8 @@ class ExpertParallelMoE:
         plan, cu, x_nvs, w_nvs = saved["plan"], saved["cu"], saved["x_nvs"], saved["w_nvs"]
         dy_nvs, _, _, _ = buf.dispatch(grad_out.contiguous(), None, plan=plan, zero_copy=True)
         rows, dev = int(x_nvs.shape[0]), x_nvs.device
-        g = self._times_weights(dy_nvs, [self.w_down], cu, plan)  # dL/dh before the gate weight: dy @ W_down
+        # dL/dh before the gate weight: dy @ W_down.  A replay on one rank writes rows only, not what the weights are found by.
+        g = self._times_weights(dy_nvs, [self.w_down], cu, plan, weights_early=self.R == 1)
         dadu = torch.empty(rows, 2 * I, dtype=torch.bfloat16, device=dev)
         hsw = torch.empty(rows, I, dtype=torch.bfloat16, device=dev)
         dgate_nvs = ctx["weights_buf_local"].view(torch.float32)  # gate gradients ride the weights channel home
