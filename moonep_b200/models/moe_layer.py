@@ -57,6 +57,7 @@ class ExpertParallelMoE:
         ctx = buffer._require_ctx()
         self.buffer = buffer
         self.world = ctx["world"]
+        self._sms = torch.cuda.get_device_properties(self.world.device).multi_processor_count if self.world.is_cuda else 0
         # the copy-free path: push combine reads the expert output where it is, the backward has its own Buffer
         self.fast = bool(ctx["world"].is_cuda and ctx["_backend"].combine_mode == "push")
         self.bwd_buffer = None
@@ -126,8 +127,8 @@ class ExpertParallelMoE:
             self.bwd_buffer = None
 
     # -- forward -------------------------------------------------------------------------------
-    def forward_gemm_pair(self):
-        """``pair`` of the forward GEMMs on the kernels: True for CTA pairs, False for one CTA per tile; None where
+    def forward_gemm_pair(self, col_tiles=0, depth=0):
+        """``pair`` of the GEMMs on the kernels: True for CTA pairs, False for one CTA per tile; None where
         ``MOONEP_GEMM_PAIR=0`` asks for the forward pass without hand-offs.
 
         Up to 128 rows per expert most groups are one row block, which leaves the second CTA of a pair without work: one
@@ -135,11 +136,21 @@ class ExpertParallelMoE:
         with even and Zipf routing (0.73 to 1.19, the worst with Zipf routing, whose hot experts have several blocks: 8
         experts of 128 rows, H=7168).  At 192 rows that is 0.93 to 0.96, but 1.19 for the largest experts, at 256 rows 0.99
         to 1.03, at 512 rows 1.04 to 1.08.  The activation gradients follow the same line (a training step 0.88 to 0.95 up to 64
-        rows per expert, 0.99 at 125).  The counts are not known on the host, so their mean decides.  With several ranks
-        the hand-off hooks need the pairs, and ``MOONEP_GEMM_PAIR=1``, where it is set, means pairs."""
+        rows per expert, 0.99 at 125).  Above 128 rows a product of ``col_tiles`` columns of
+        tiles takes pairs unless one wave of them would hold all its tiles: then single tiles, cut where they are few, use more
+        SMs (a forward pass, pairs and single: 8 experts, H=2048, I=1024, 250 rows 76.8 and 63.0 us, 300 rows, where it is two
+        waves, 76.7 and 75.0; H=1024, I=512, 500 rows 53.8 and 43.6; 2 experts, 1000 rows 44.7 and 36.1; 8 experts, H=7168,
+        I=2048, 150 rows, three waves, 187 and 210).  Pairs load less per product, which tells where the contraction (``depth``)
+        is long and the wave more than half full (8 experts, H=4096, I=512, 300 rows 83.8 and 84.8; half full, 2 experts, 500
+        rows 64.8 and 50.0).  The counts are not known on the host, so their mean decides.  With several
+        ranks the hand-off hooks need the pairs, and ``MOONEP_GEMM_PAIR=1``, where it is set, means pairs."""
         switch = config.gemm_pair_switch()
         if switch is None:
-            return self.R > 1 or self.S * self.K > 128 * self.E
+            if self.R > 1 or self.S * self.K <= 128 * self.E:
+                return self.R > 1
+            row_tiles = -(-self.S * self.K // (256 * self.E))
+            most = self._sms // (2 if depth <= 2048 or depth <= 4096 and row_tiles == 1 else 4)
+            return not 0 < self.E * row_tiles * col_tiles <= most
         return True if switch else None
 
     def _forward_fast(self, x, gates, topk, tokens_per_expert, save_for_backward, pair):
@@ -170,18 +181,18 @@ class ExpertParallelMoE:
         # The hand-off hooks need the CTA-pair kernel's tiling; other shapes run after the prefetch, in stream order.  Alone
         # there is nothing to wait for, as long as the dispatch has seen that every row of a group is one that lands.
         hooked = not (alone and be.counts_checked) and rows >= 128 and self.H % 256 == 0 and self.I % 128 == 0
-        pair = pair or hooked
         if fetched is not None and not hooked:
             torch.cuda.current_stream().wait_event(fetched)
-        h = grouped_gemm(x_nvs, self.w_gate, cu, w_up=self.w_up, mode="swiglu", status=status, pair=pair,
-                         save_pre=None if a is None else (a, u),
+        h = grouped_gemm(x_nvs, self.w_gate, cu, w_up=self.w_up, mode="swiglu", status=status,
+                         pair=hooked or pair and self.forward_gemm_pair(self.I // 128, self.H), save_pre=None if a is None else (a, u),
                          hooks=buf.gemm_hooks(rows=True, slots=not alone) if hooked else None)  # fmt: skip
         ready = None
         if hooked:
             # counted from zero every time: blocks without rows are not counted, and which those are changes with the routing
             self._done.zero_()
             ready = (self._done, 4 * (self.H // 256))
-        grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=self._y, status=status, pair=pair, weights_early=alone,
+        grouped_gemm(h, self.w_down, cu, row_scale=w_nvs, mode="scale", out=self._y, status=status, weights_early=alone,
+                     pair=hooked or pair and self.forward_gemm_pair(self.H // 256, self.I),
                      hooks=buf.gemm_hooks(slots=not alone, done_counter=self._done) if hooked else None)  # fmt: skip
         out, _, _ = buf.combine(plan, self._y, None, ready=ready)
         if hooked and fetched is not None:
@@ -306,8 +317,8 @@ class ExpertParallelMoE:
         stored ``[E+B, out, in]`` (which is ``[G, K, N]`` for this product).  The kernels stage them as
         MN-major tiles; elsewhere K-major copies of the local experts feed the ordinary grouped GEMM."""
         if kn_kernel_supports(x, ws):
-            return grouped_gemm_kn(x, ws, cu, out=out, num_sms=num_sms, pair=self.forward_gemm_pair() is not False,
-                                   weights_early=weights_early)  # fmt: skip
+            pair = self.forward_gemm_pair(int(ws[0].shape[2]) // 256, int(x.shape[1])) is not False
+            return grouped_gemm_kn(x, ws, cu, out=out, num_sms=num_sms, pair=pair, weights_early=weights_early)
         return grouped_gemm(x, self._local_transposed(ws, plan), cu, group_map=self.group_map, out=out,
                             status=self.buffer._require_ctx()["_backend"].status if x.is_cuda else None)
 
