@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kCaThreads, 1)
   extern __shared__ __align__(16) unsigned char s_ca_ring[];
   __shared__ short s_slot[kListedSlots];
   __shared__ int s_used;
-  if (poisoned(c)) return;
+  if (!__syncthreads_and(poisoned(c) ? 0 : 1)) return;  // one answer for the CTA, whose warps share the list
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long nvec = elems / 8;  // bf16: 8 elements per 16 bytes
   if (warp == 0) {  // the slots that receive an expert, in ascending order
