@@ -65,13 +65,28 @@ __global__ void epoch_bias_kernel(const MoonepDevCtx c, const BiasValues b, int 
   if (f < MOONEP_NUM_FLAG_FAMILIES) c.counters[MOONEP_BIAS_OFF + f] = (mode ? c.counters[MOONEP_BIAS_OFF + f] : 0) + b.v[f];
 }
 
+// One of a slot's `pieces` is done with: copied, or left out because the Buffer has failed.  After the last one the count is zero
+// again, and the slot is announced if every piece was copied.  One thread per piece, behind a fence.
+constexpr int kPieceLeftOut = 1 << 30;
+__device__ __forceinline__ void count_piece(int* done, int* flag, int pieces, bool copied, int epoch) {
+  if (!copied) atomicOr(done, kPieceLeftOut);
+  const int before = atomicAdd(done, 1);
+  if ((before & ~kPieceLeftOut) != pieces - 1) return;
+  *done = 0;
+  fence_gpu();
+  if (!(before & kPieceLeftOut)) st_relaxed_gpu(flag, epoch);
+}
+
 // Work items are ordered slot-major, so that the slots fill one after the other; when the last piece of a slot
 // (over all tensors) has been copied, the slot's flag is released with the prefetch epoch and a grouped GEMM that
 // runs beside this kernel may load that slot's weights (moonep_grouped_gemm_pair_hooked: slot_flags).
+// CTAs that find the Buffer failed copy nothing, but count the pieces: the counts have to be back at zero for the launches after
+// the failure has been seen, which would otherwise announce slots too early.
 __global__ void __launch_bounds__(512)
     prefetch_kernel(const MoonepDevCtx c, const TensorSet w, const int* __restrict__ experts, long long elems,
                     int nslots, int nexperts, int* slot_flags, int* slot_done, int epoch) {
-  if (poisoned(c)) return;
+  const bool live = __all_sync(0xffffffffu, !poisoned(c));
+  if (!live && slot_flags == nullptr) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const long long nvec = elems / 8;  // bf16: 8 elements per 16 bytes
   const long long pieces = (nvec + kPieceVec - 1) / kPieceVec;
@@ -80,7 +95,7 @@ __global__ void __launch_bounds__(512)
   if (slot_flags != nullptr) {
     epoch = abs_epoch(c, MOONEP_FLAG_PREFETCH, epoch);
     // slots that receive nothing are ready at once
-    if (blockIdx.x == 0)
+    if (live && blockIdx.x == 0)
       for (int b = threadIdx.x; b < nslots; b += blockDim.x)
         if (experts[b] < 0 || experts[b] >= nexperts) st_release_gpu(slot_flags + b, epoch);
   }
@@ -98,7 +113,7 @@ __global__ void __launch_bounds__(512)
     const int4* src = reinterpret_cast<const int4*>(w.p[t]) + (long long)e * nvec;
     int4* dstp = reinterpret_cast<int4*>(w.q[t]) + (long long)b * nvec;
     const long long v0 = piece * kPieceVec;
-    const long long v1 = v0 + kPieceVec < nvec ? v0 + kPieceVec : nvec;
+    const long long v1 = !live ? v0 : v0 + kPieceVec < nvec ? v0 + kPieceVec : nvec;
     for (long long i0 = v0; i0 < v1; i0 += 32 * 8) {
       int4 v[8];
 #pragma unroll
@@ -116,11 +131,7 @@ __global__ void __launch_bounds__(512)
       __syncwarp();
       if (lane == 0) {
         fence_gpu();
-        if (atomicAdd(slot_done + b, 1) == (int)per_slot - 1) {
-          slot_done[b] = 0;
-          fence_gpu();
-          st_relaxed_gpu(slot_flags + b, epoch);
-        }
+        count_piece(slot_done + b, slot_flags + b, (int)per_slot, live, epoch);
       }
     }
   }
@@ -265,7 +276,8 @@ __global__ void __launch_bounds__(kCaThreads, 1)
   extern __shared__ __align__(16) unsigned char s_ca_ring[];
   __shared__ short s_slot[kListedSlots];
   __shared__ int s_used;
-  if (!__syncthreads_and(poisoned(c) ? 0 : 1)) return;  // one answer for the CTA, whose warps share the list
+  const bool live = __syncthreads_and(poisoned(c) ? 0 : 1) != 0;  // one answer for the CTA, whose warps share the list
+  if (!live && slot_flags == nullptr) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long nvec = elems / 8;  // bf16: 8 elements per 16 bytes
   if (warp == 0) {  // the slots that receive an expert, in ascending order
@@ -291,7 +303,7 @@ __global__ void __launch_bounds__(kCaThreads, 1)
   const long long total = (long long)(listed ? used : nslots) * per_slot;
   if (slot_flags != nullptr) {
     epoch = abs_epoch(c, MOONEP_FLAG_PREFETCH, epoch);
-    if (blockIdx.x == 0)
+    if (live && blockIdx.x == 0)
       for (int b = threadIdx.x; b < nslots; b += blockDim.x)
         if (experts[b] < 0 || experts[b] >= nexperts) st_release_gpu(slot_flags + b, epoch);
   }
@@ -308,7 +320,7 @@ __global__ void __launch_bounds__(kCaThreads, 1)
     int4* dstp = reinterpret_cast<int4*>(w.q[t]) + (long long)b * nvec;
     const long long v0 = piece * piece_vec;
     const long long v1 = v0 + piece_vec < nvec ? v0 + piece_vec : nvec;
-    const int steps = (int)((v1 - v0 + kCaChunkVec - 1) / kCaChunkVec);
+    const int steps = live ? (int)((v1 - v0 + kCaChunkVec - 1) / kCaChunkVec) : 0;
     auto issue = [&](int q) {
       int4* dst = ring + (size_t)(q % kStages) * kCaChunkVec;
       const long long base = v0 + (long long)q * kCaChunkVec;
@@ -339,11 +351,7 @@ __global__ void __launch_bounds__(kCaThreads, 1)
       __syncwarp();
       if (lane == 0) {
         fence_gpu();
-        if (atomicAdd(slot_done + b, 1) == (int)per_slot - 1) {
-          slot_done[b] = 0;
-          fence_gpu();
-          st_relaxed_gpu(slot_flags + b, epoch);
-        }
+        count_piece(slot_done + b, slot_flags + b, (int)per_slot, live, epoch);
       }
     }
   }

@@ -3,6 +3,7 @@ else is written, and after ``check_status`` the Buffer prefetches as before."""
 
 import dataclasses
 import re
+import time
 
 import pytest
 import torch
@@ -12,6 +13,7 @@ from moonep_b200.constants import STATUS_BAD_INDEX
 from moonep_b200.errors import MoonEPIndexError
 from moonep_b200.models.routing import make_routing
 from moonep_b200.ops._lib import CSRC
+from moonep_b200.ops.grouped_gemm import grouped_gemm
 from moonep_b200.parallel.world import LocalWorld
 
 
@@ -39,6 +41,9 @@ def test_prefetch_on_a_failed_buffer(B, num_sms):
     table = (torch.arange(R * B, dtype=torch.int32).view(R, B) * 3 % (E + 1) - 1).cuda()  # slots without an expert among them
     empty = torch.full((B, Hw, Hp), -123.0, dtype=torch.bfloat16, device="cuda")
     experts = [torch.randn(E, Hw, Hp, generator=torch.Generator(device="cuda").manual_seed(t), device="cuda").bfloat16() for t in range(3)]
+    sms, side = torch.cuda.get_device_properties(0).multi_processor_count, torch.cuda.Stream()
+    rows, weights = torch.zeros(128 * sms, 4096, device="cuda").bfloat16(), torch.zeros(1, 16384, 4096, device="cuda").bfloat16()
+    ends = torch.tensor([128 * sms], dtype=torch.int32, device="cuda")
     wants = [[torch.where(row[:, None, None] >= 0, e[row.long().clamp(min=0)], empty) for e in experts] for row in table]
 
     def body(r):
@@ -47,8 +52,13 @@ def test_prefetch_on_a_failed_buffer(B, num_sms):
         topk, tpe, gates = make_routing("biased", S, K, E, R, r, bias=1.5, seed=5, device="cuda")
         plan = buf.dispatch(torch.ones(S, H, device="cuda").bfloat16(), gates, topk, tpe)[3]
 
-        def fetch(etc):
+        def fetch(etc, late=False):
             full = [torch.cat([e, empty]).contiguous() for e in experts]
+            if late:  # most CTAs of the prefetch have to wait for an SM, and start when the first one has seen the table
+                side.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(side):
+                    grouped_gemm(rows, weights, ends, num_sms=sms - 8, pair=False)
+                time.sleep(0.0003)
             buf.prefetch_weight(dataclasses.replace(plan, experts_to_copy=etc), full_gate_weight=full[0], full_up_weight=full[1],
                                 full_down_weight=full[2])  # fmt: skip
             torch.cuda.synchronize()
@@ -60,20 +70,22 @@ def test_prefetch_on_a_failed_buffer(B, num_sms):
             buf.check_status()
             return all(torch.equal(g, w) for g, w in zip(got, wants[r]))
 
-        def failed(etc):
-            got = fetch(etc)
+        def failed(etc, late=False):
+            got = fetch(etc, late)
             with pytest.raises(MoonEPIndexError):
                 buf.check_status()
+            # pieces counted towards slots that were not finished would announce the next prefetch's slots too early
+            assert not bool(be._slot_scratch()[1].any())
             return got
 
         assert whole()
         be.status[0] = STATUS_BAD_INDEX  # before the kernel starts: no slot is written
         assert all(torch.equal(g, empty) for g in failed(table))
         assert whole()
-        for _ in range(5):  # while it starts: the first CTA meets an expert that is none
+        for late in (False, True, True):  # while it starts: the first CTA meets an expert that is none
             bad = table.clone()
             bad[r, B - 1] = E
-            for g, w in zip(failed(bad), wants[r]):
+            for g, w in zip(failed(bad, late), wants[r]):
                 assert torch.equal(g[B - 1], empty[0])
                 assert bool(((g[:-1] == w[:-1]) | (g[:-1] == empty[:-1])).all())
             assert whole()
