@@ -102,6 +102,8 @@ __device__ __forceinline__ void stat_phase(const MoonepDevCtx& c, int phase, uns
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets a kernel launched with programmatic stream serialisation behind this one start its CTAs as soon as SMs have room
 // (it still waits in griddepcontrol.wait until this grid has completed and its writes are visible).
+// Comes after griddep_wait in every kernel that is launched programmatically: a GEMM behind it may read weights at once
+// (weights_early), which a kernel further ahead may have written.
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Absolute epoch of a launch argument: argument + this family's bias (see the header comment).

@@ -519,23 +519,15 @@ extern "C" int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld
 
 // The same with the operands as they are: l = L [rows, P] and r = R [rows, Q] bf16, rows ldl / ldr elements apart
 // (multiples of 8), so that column slices of wider tensors can be passed.  No transposed copies are needed: the
-// tiles are staged MN-major (see make_smem_desc_mn).  pads (optional): a plan's zero_fill_ranges, whose rows hold zeros.
-extern "C" int moonep_grouped_wgrad_rows(const void* l, long long ldl, const void* r, long long ldr, int rows, int P,
-                                         int Q, const int* cu_seqlens, int G, void* const* out_ptrs, const int* flags,
-                                         int* status, long long timeout_ms, int rows_per_group, int adds,
-                                         int num_sms, const int* pads, void* stream) {
-  return moonep_grouped_wgrad_layer(l, ldl, r, ldr, P, Q, out_ptrs, nullptr, 0, nullptr, 0, 0, 0, nullptr, nullptr, 0, nullptr, 0, 0, 0,
-                                    nullptr, rows, cu_seqlens, G, flags, status, timeout_ms, rows_per_group, adds, num_sms, pads, stream);
-}
-
-// Up to three weights (those after the first may be absent: l null) of the same groups of rows in one launch.
+// tiles are staged MN-major (see make_smem_desc_mn).  Up to three weights of the same groups of rows in one launch (those after
+// the first may be absent: l null).  pads (optional): a plan's zero_fill_ranges, whose rows hold zeros.
 extern "C" int moonep_grouped_wgrad_layer(const void* l0, long long ldl0, const void* r0, long long ldr0, int P0, int Q0, void* const* out0,
                                           const void* l1, long long ldl1, const void* r1, long long ldr1, int P1, int Q1, void* const* out1,
                                           const void* l2, long long ldl2, const void* r2, long long ldr2, int P2, int Q2, void* const* out2,
                                           int rows, const int* cu_seqlens, int G, const int* flags, int* status, long long timeout_ms,
                                           int rows_per_group, int adds, int num_sms, const int* pads, void* stream) {
   if (G < 1 || G > kWgradMaxGroups) {
-    set_error("moonep_grouped_wgrad_rows: at most " + std::to_string(kWgradMaxGroups) + " groups per launch");
+    set_error("moonep_grouped_wgrad_layer: at most " + std::to_string(kWgradMaxGroups) + " groups per launch");
     return 1;
   }
   const struct {
@@ -550,11 +542,11 @@ extern "C" int moonep_grouped_wgrad_layer(const void* l0, long long ldl0, const 
   for (const auto& w : ws) {
     if (w.l == nullptr && a.n_weights > 0) break;
     if (w.P <= 0 || w.Q <= 0 || w.P % BM != 0 || w.Q % BN != 0) {
-      set_error("moonep_grouped_wgrad_rows: P must be a multiple of 128 and Q a multiple of 256");
+      set_error("moonep_grouped_wgrad_layer: P must be a multiple of 128 and Q a multiple of 256");
       return 1;
     }
     if (w.ldl < w.P || w.ldr < w.Q || w.ldl % 8 != 0 || w.ldr % 8 != 0 || rows <= 0) {
-      set_error("moonep_grouped_wgrad_rows: row strides must be multiples of 8 and at least the matrix width");
+      set_error("moonep_grouped_wgrad_layer: row strides must be multiples of 8 and at least the matrix width");
       return 1;
     }
     const int i = a.n_weights++;

@@ -14,7 +14,7 @@
 
 #include <cstdint>
 
-#define MOONEP_VERSION 1
+#define MOONEP_VERSION 2
 
 // Packed encodings (must match moonep_b200/constants.py).
 #define MOONEP_KIDX_BITS 7
@@ -342,12 +342,8 @@ int moonep_grouped_wgrad(const void* lt, const void* rt, long long ld, int P, in
 int moonep_wgrad_single_cta(int rows_per_group, int num_sms);
 int moonep_wgrad_single_cta_adding(int rows_per_group, int num_sms);
 // The same from the operands as they are, l = L [rows, P], r = R [rows, Q] (rows ldl / ldr elements apart): no
-// transposed copies, the tiles are staged MN-major.  pads (optional): [G, 2] (first, number) of a group's last rows that hold
-// zeros, which are left out.
-int moonep_grouped_wgrad_rows(const void* l, long long ldl, const void* r, long long ldr, int rows, int P, int Q,
-                              const int* cu_seqlens, int G, void* const* out_ptrs, const int* flags, int* status,
-                              long long timeout_ms, int rows_per_group, int adds, int num_sms, const int* pads, void* stream);
-// Up to three weights (a null l ends them) of the same groups of rows in one launch.
+// transposed copies, the tiles are staged MN-major.  One to three weights (a null l ends them) of the same groups of rows in one
+// launch.  pads (optional): [G, 2] (first, number) of a group's last rows that hold zeros, which are left out.
 int moonep_grouped_wgrad_layer(const void* l0, long long ldl0, const void* r0, long long ldr0, int P0, int Q0, void* const* out0,
                                const void* l1, long long ldl1, const void* r1, long long ldr1, int P1, int Q1, void* const* out1,
                                const void* l2, long long ldl2, const void* r2, long long ldr2, int P2, int Q2, void* const* out2,

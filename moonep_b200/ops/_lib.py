@@ -143,7 +143,6 @@ _SIGNATURES = {
     "moonep_wgrad_single_cta": (_i, [_i, _i]),
     "moonep_wgrad_single_cta_adding": (_i, [_i, _i]),
     "moonep_grouped_wgrad_layer": (_i, [_vp, _ll, _vp, _ll, _i, _i, _vp] * 3 + [_i, _vp, _i, _vp, _vp, _ll, _i, _i, _i, _vp, _vp]),
-    "moonep_grouped_wgrad_rows": (_i, [_vp, _ll, _vp, _ll, _i, _i, _i, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _vp, _vp]),
     "moonep_transpose_experts": (_i, [_vp, _vp, _i, _i, _i, _ll, _ll, _i, _vp, _vp]),
     "moonep_adamw_update": (_i, [_i] + [ctypes.POINTER(_vp)] * 5 + [ctypes.POINTER(_ll)] + [ctypes.c_double] * 6 + [_vp]),
     "moonep_sgd_update": (_i, [_i] + [ctypes.POINTER(_vp)] * 2 + [ctypes.POINTER(_ll), ctypes.c_float, _vp]),

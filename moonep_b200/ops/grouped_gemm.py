@@ -78,8 +78,10 @@ def grouped_gemm(x, w, cu_seqlens, *, w_up=None, row_scale=None, mode="plain", o
     ``pair`` selects the kernel: True = CTA pairs (``cta_group::2``), False = one CTA per tile, None = ``MOONEP_GEMM_PAIR``.
     ``hooks`` (a ``GemmHooks``, CTA-pair kernel only) lets the kernel run beside the communication kernels: it waits
     per row block / weight slot for their flags and counts finished output tiles per row block.
-    ``weights_early``: the kernel launched just before on this stream is another of these GEMMs, which writes neither the
-    weights nor the group tables: one CTA per tile then asks for weights while that kernel still runs.
+    ``weights_early``: one CTA per tile asks for weights while the kernel launched just before on this stream still runs.  That
+    kernel must write neither the weights nor ``cu_seqlens`` and ``group_map``, and must not let its successor start before it
+    has itself waited for what runs ahead of it: true of every kernel of this package, which begins with that wait, and of
+    kernels launched without programmatic dependent launch.
     """
     assert mode in _MODES
     W, N, K = (int(v) for v in w.shape)
@@ -158,7 +160,7 @@ def grouped_gemm_kn(x, ws, cu_seqlens, *, out=None, status=None, num_sms=0, pair
     activation gradient needs from forward weights stored ``[G, out, in]``, without transposed copies.  ``ws`` is one
     tensor or two that continue the contraction (``x = [a | b]``, ``W = [ws[0]; ws[1]]``).  Runs on CTA pairs or, with
     ``pair=False``, one CTA per tile (MN-major W tiles); a per-group fp32 reference elsewhere.  ``weights_early`` (one CTA per
-    tile): the kernel launched just before on this stream writes neither the weights nor ``cu_seqlens``."""
+    tile): as in ``grouped_gemm``."""
     ws = list(ws)
     G, _, N = (int(v) for v in ws[0].shape)
     Ks = [int(w.shape[1]) for w in ws]
@@ -265,7 +267,7 @@ def grouped_wgrad_rows(left, right, cu_seqlens, out_ptrs, flags, *, status=None,
 def grouped_wgrad_layer(weights, cu_seqlens, flags, *, status=None, num_sms=0, rows_per_group=0, adds=False, pads=None):
     """``grouped_wgrad_rows`` of one to three weights, ``(left, right, out_ptrs)`` each, in one launch."""
     rows, G = int(weights[0][0].shape[0]), int(cu_seqlens.numel())
-    assert 1 <= len(weights) <= 3 and G <= WGRAD_MAX_GROUPS, f"grouped_wgrad_rows: at most {WGRAD_MAX_GROUPS} groups per launch"
+    assert 1 <= len(weights) <= 3 and G <= WGRAD_MAX_GROUPS, f"grouped_wgrad_layer: at most {WGRAD_MAX_GROUPS} groups per launch"
     words = []
     for left, right, out_ptrs in weights:
         P, Q = int(left.shape[1]), int(right.shape[1])
@@ -286,7 +288,7 @@ def grouped_wgrad_layer(weights, cu_seqlens, flags, *, status=None, num_sms=0, r
             *words, rows, cu_seqlens.data_ptr(), G, flags.data_ptr(), 0 if status is None else status.data_ptr(), config.timeout_ms(),
             int(rows_per_group), int(adds), int(num_sms), 0 if pads is None else pads.data_ptr(), _lib.current_stream(),
         )  # fmt: skip
-    _lib.check(rc, "moonep_grouped_wgrad_rows")
+    _lib.check(rc, "moonep_grouped_wgrad_layer")
 
 
 def _fallback_allowed() -> bool:
