@@ -35,7 +35,8 @@ MOONEP_NUM_SMS_DEDUP  CTAs of the dispatch kernel's destination-side role (zero 
                       senders leave free.
 MOONEP_NVTX           ``1`` wraps every native call in an NVTX range.
 MOONEP_GEMM_PAIR      ``1``: grouped GEMMs on CTA pairs (tcgen05 cta_group::2); ``0``: one CTA per tile.  Unset: pairs, except
-                      that the MoE layer's forward GEMMs on one rank take one CTA per tile up to 128 rows per expert.
+                      that the MoE layer's GEMMs on one rank, forward and activation gradients, take one CTA per tile up to 128
+                      rows per expert and for products that one wave of pairs would hold.
 MOONEP_WGRAD          ``kernel`` (default) or ``torch``: weight gradients of the MoE layer.
 MOONEP_WGRAD_LAYOUT   ``rows`` (default: activations as stored, MN-major tiles) or ``transposed``.
 

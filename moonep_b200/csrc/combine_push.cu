@@ -24,7 +24,7 @@
 // for lower-numbered CTAs (which the hardware dispatches first) and the SUM role only for PUSH CTAs of this or
 // other GPUs; the grid never exceeds the number of SMs.  Emulated ranks that share one GPU launch FOLD and PUSH, which
 // wait for nothing of another rank, and when every rank's have been launched SUM (two ranks, S=4096, H=7168, K=8, E=64,
-// 32 pushers: FOLD 118 and PUSH 65 to 86 us one behind the other, together 150).  A single rank has nothing to push:
+// 32 pushers, between events: FOLD 123 and PUSH 89 us one behind the other, together 170).  A single rank has nothing to push:
 // single_rank.cu.
 //
 // Parity: reference moonep_td/combine_prologue.py:19-40 and moonep_td/combine.py:22-68.

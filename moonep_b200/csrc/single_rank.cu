@@ -49,7 +49,9 @@ constexpr int kDealtRounds = 6;
 // unit costs a copy warp a chain of round trips, and an SM has more on its way with more in a stage.  Against rows that fill
 // 4 KB, dispatch and combine, us: S=16384, K=4, H=1000 79.3 -> 74.9, H=2048 135.2 -> 127.9; S=4096, K=8, H=2048 64.2 -> 61.4.
 // Stages of 16 KB for four warps make the dispatch alone another 2 to 5 % shorter, but the combine behind it longer by more
-// (S=16384, K=4: H=2048 132.9 together, H=4096 249.6 instead of 237.7).
+// (S=16384, K=4: H=2048 132.9 together, H=4096 249.6 instead of 237.7).  Equal shares lose where they are smaller than a stage's
+// worth: a replay of S=4096, H=256, K=8 (units of five rows, not eight) takes 16.3 us where it took 15.9, S=2048 14.8 (15.8), S=8192
+// 22.8 (24.9).
 constexpr int kUnitTokens = 8;
 constexpr int kUnits = 64;         // units remembered per copy warp: those loaded and those not flagged yet
 constexpr int kGrabs = 64;         // grabs of pad rows remembered per warp
@@ -521,7 +523,9 @@ __device__ void copy_tail(const MoonepDevCtx& c, const SingleArgs& a, const int*
 // counts first, and the first entry that it plans, with its weight.  Beside other CTAs' rows and pads each of these round trips
 // takes microseconds.  With them, and the first rows of the copy warps, asked for where they were used: last CTA planned 21 us
 // after the layout where it takes 12 (S=4096, K=8, E=256) and 4.5 (3.5; S=2048, K=4, E=16), kernel 39.5 (37.5; S=2048, H=4096,
-// K=8) and 15.0 (12.4; S=2048, H=2048, K=4).  Counting in bytes per thread instead of atomics gained nothing beyond that.
+// K=8) and 15.0 (12.4; S=2048, H=2048, K=4).  Among many large pad rows (H=8192, K=8, E=64) neither kernel is slower by itself, but
+// the round trips of two sizes are: S=200 41.8 -> 41.3, S=300 44.4 -> 45.2, S=450 48.8 -> 49.9, S=600 51.2 -> 49.8.  Counting in
+// bytes per thread instead of atomics gained nothing beyond that.
 constexpr int kCountLoads = 8;
 struct Early {
   int4 v[kCountLoads];

@@ -3,8 +3,8 @@
 //
 //   prefetch     for every slot b of this rank with experts_to_copy[rank][b] = e >= 0, copy expert e
 //                (physically on its owner, reached through the peer-mapped part of the weight
-//                tensor) into local slot b of the prefetch buffers (slot E+b of the full weight).  Gate, up and down go in one launch; persistent CTAs
-//                stride over 16 KB pieces with eight 16-byte loads in flight per lane.
+//                tensor) into local slot b of the prefetch buffers (slot E+b of the full weight).  Gate, up and down go in one launch; the warps
+//                of persistent CTAs stride over pieces of the slots in use (even shares, 256 KB at most).
 //   grad_accum   the owner of expert e adds every slot (src, b) with experts_to_copy[src][b] == e
 //                to its local gradient, in ascending src*B+b order starting from the local value,
 //                so results are bitwise reproducible.  Waits for FLAG_GRAD_READY, signals
@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(kAccumThreads, 1)
 // most a few KB per warp in flight, which over NVLink (several microseconds per round trip) bounds a pull below the
 // link rate.  Here every warp owns a ring of 2 KB shared-memory stages and fills them with 16-byte cp.async copies
 // (the same load path as register loads, but the data waits in shared memory, not in registers); every lane stores
-// what it copied itself, so the warps need no barrier.  Work items are 256 KB pieces in slot-major order, so the
-// first slots complete (and are flagged) first.  Measured on 2 B200 (2.8 GB per rank): 668 GB/s against 629 GB/s of
+// what it copied itself, so the warps need no barrier.  Work items are pieces of at most 256 KB, even shares of
+// the slots in use (even_piece), in slot-major order, so the first slots complete (and are flagged) first.  Measured on 2 B200 (2.8 GB per rank): 668 GB/s against 629 GB/s of
 // the register kernel, the same with 3, 4, 5 or 6 stages.  The same ring under grad_accum measured half the rate of
 // its register kernel (244 against 489 GB/s), whatever the ring depth, the piece size, the completion mechanism
 // (cp.async groups or an mbarrier per stage) and whether the data was consumed at all; that variant was dropped.

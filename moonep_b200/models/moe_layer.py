@@ -19,8 +19,8 @@ prefetch slot ``b``.  On multi-GPU worlds ``[:E]`` is peer mapped (``create_full
 remote expert that did not get a prefetch slot is read in place over NVLink.
 
 Usage pattern of the reference's Buffer API: reference ``README.md:46-48`` and ``tests/test_e2e.py:201-431``.
-Every GEMM of the layer is a tcgen05 kernel of this package: forward and activation gradients on CTA pairs
-(``grouped_gemm``, ``grouped_gemm_kn``), weight gradients on ``grouped_wgrad_layer``; the backward takes the weights
+Every GEMM of the layer is a tcgen05 kernel of this package: forward and activation gradients on CTA pairs or, on one rank,
+one CTA per tile (``grouped_gemm``, ``grouped_gemm_kn``), weight gradients on ``grouped_wgrad_layer``; the backward takes the weights
 and activations as they are stored (MN-major tiles), the forward keeps both SwiGLU pre-activations for it.
 Per-group torch matmuls remain for CPU tensors and for shapes outside the kernels' tiling.
 """
@@ -135,8 +135,10 @@ class ExpertParallelMoE:
         CTA per tile takes 0.86 to 0.92 of the pairs' time on average over 4 to 32 experts, H 1024 to 7168, I 512 to 2048
         with even and Zipf routing (0.73 to 1.19, the worst with Zipf routing, whose hot experts have several blocks: 8
         experts of 128 rows, H=7168).  At 192 rows that is 0.93 to 0.96, but 1.19 for the largest experts, at 256 rows 0.99
-        to 1.03, at 512 rows 1.04 to 1.08.  The activation gradients follow the same line (a training step 0.88 to 0.95 up to 64
-        rows per expert, 0.99 at 125).  Above 128 rows a product of ``col_tiles`` columns of
+        to 1.03, at 512 rows 1.04 to 1.08.  The activation gradients follow the same line: a training step takes 0.88 to 0.95 of
+        what it takes with pairs for them up to 64 rows per expert, and at 128 rows, with even and with Zipf routing, 0.97 and
+        0.98 (32 experts, H=2048, I=768), 0.99 and 0.99 (16, H=4096, I=1024), 1.00 and 1.00 (8, H=7168, I=2048; 16, H=7168,
+        I=1024), 1.01 and 1.01 (8, H=4096, I=2048).  Above 128 rows a product of ``col_tiles`` columns of
         tiles takes pairs unless one wave of them would hold all its tiles: then single tiles, cut where they are few, use more
         SMs (a forward pass, pairs and single: 8 experts, H=2048, I=1024, 250 rows 76.8 and 63.0 us, 300 rows, where it is two
         waves, 76.7 and 75.0; H=1024, I=512, 500 rows 53.8 and 43.6; 2 experts, 1000 rows 44.7 and 36.1; 8 experts, H=7168,
@@ -323,7 +325,8 @@ class ExpertParallelMoE:
                             status=self.buffer._require_ctx()["_backend"].status if x.is_cuda else None)
 
     def _weight_grads_on_kernel(self, x_nvs, dy_nvs, dadu, hsw, cu, plan, after=None, num_sms=0) -> bool:
-        """All weight gradients with three launches of the grouped tcgen05 kernel (no host synchronisation); every
+        """All weight gradients with one launch of the grouped tcgen05 kernel, or three where each is sent on by itself or the
+        operands are transposed first (no host synchronisation); every
         group's result goes straight to the owner's gradient or to the reduce-buffer slot of a prefetched copy.
         Returns False (nothing done) when the shapes do not fit the kernel.  ``after(i)`` is called once the
         gradients of weight ``i`` (0 gate, 1 up, 2 down) are enqueued; launches after the first such call use

@@ -380,7 +380,8 @@ class CudaBackend:
     def dispatch_all(self, hidden_sh, route_weights_sk, plan, planning_args, inter_rank_sync, copy_to=None):
         """The whole dispatch.  Fresh plan: ``plan_publish`` plus one fused launch (planner tables, token planning, row
         push, and on the destination side zero fill, duplicate map and duplicate expansion as rows arrive).  Replayed
-        plan: an optional READY round plus one launch (push and expansion).  Emulated ranks run one role per phase.
+        plan: an optional READY round plus one launch (push and expansion).  Emulated ranks launch the
+        roles in phases: planning, send and their own rows, then the expansion of what peers sent (``MOONEP_PHASED=1``: a role each).
         ``copy_to``: tensors that receive the shard and (or None) its weights; True is returned when this call has seen
         to it, otherwise ``copy_out`` is left to the caller."""
         with_w = route_weights_sk is not None
