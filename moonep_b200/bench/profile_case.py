@@ -6,9 +6,9 @@ L2, a handful of launches), used as the targets of the ``ncu`` captures summaris
     python -m moonep_b200.bench.profile_case --what moe --ranks 1 --S 2048 --steps 2
 
 ``roundtrip``: R emulated ranks on one GPU run dispatch + combine, two launches each (planning, send and own rows, then
-expansion; fold and push, then sum); with ``MOONEP_PHASED=1`` every role shows up as a launch of its own, with ``--ranks 1`` too.  ``weights``: ``prefetch_weight`` and ``reduce_grad`` with every slot in use.  ``moe``: forward
-and backward of the SwiGLU MoE layer (grouped GEMMs with their hand-off hooks, weight-gradient kernel, SwiGLU
-backward).
+expansion; fold and push, then sum); with ``MOONEP_PHASED=1`` every role shows up as a launch of its own, with ``--ranks 1``
+too.  ``weights``: ``prefetch_weight`` and ``reduce_grad`` with every slot in use.  ``moe``: forward and backward of the SwiGLU
+MoE layer (grouped GEMMs with their hand-off hooks, weight-gradient kernel, SwiGLU backward).
 """
 
 from __future__ import annotations
