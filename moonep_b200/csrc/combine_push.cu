@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(kPushThreads, 1) combine_push_kernel(const Moo
       }
       if ((threadIdx.x & 31) == 0 && warp < kMoveWarps) stat_phase(c, MOONEP_PH_PUSH, t0);
     }
-  } else if (has_local && !poisoned(c)) {
+  } else if (has_local && __syncthreads_and(poisoned(c) ? 0 : 1)) {
     unsigned long long t0 = globaltimer_ns();
     if (a.roles & MOONEP_ROLE_FOLD) {
       fold_role(c, a);

@@ -1062,15 +1062,13 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const Moo
   fence_barrier_init();
   griddep_wait();  // the set-up above may overlap the previous kernel's tail; its results are needed from here on
   griddep_launch();  // the next kernel of the stream may set itself up on SMs as the CTAs of this one leave them
-  __syncthreads();
-  bool ok = !poisoned(c);
+  bool ok = __syncthreads_and(poisoned(c) ? 0 : 1) != 0;  // one answer per CTA: the roles below share tables and barriers
 
   if (a.publish) {
     // What plan_publish does as a kernel of its own, on all CTAs of this launch: reset this rank's src_info, push
     // the tokens-per-expert row into every peer's meta chunk, count the experts of every planner block; the last
     // CTA to finish signals FLAG_TPE to every peer (which also tells them that this rank is done with every
     // earlier use of the buffers).
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;  // one answer per CTA: the loops below contain barriers
     if (ok) {
       const int tid = blockIdx.x * blockDim.x + threadIdx.x;
       const int nth = gridDim.x * blockDim.x;

@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(kTokensThreads)
                         int tokens_per_block, int epoch_tpe) {
   extern __shared__ int s_hist[];  // [E]
   griddep_launch();  // the dispatch kernel behind this one may set itself up meanwhile
-  const bool live = !poisoned(c);
+  const bool live = __syncthreads_and(poisoned(c) ? 0 : 1) != 0;  // one answer per CTA, which shares the counts
   if (live) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nth = gridDim.x * blockDim.x;

@@ -35,7 +35,7 @@ struct TensorSet {
 
 __global__ void __launch_bounds__(256)
     signal_wait_kernel(const MoonepDevCtx c, int signal_family, int signal_epoch, int wait_family, int wait_epoch) {
-  if (signal_family >= 0 && !poisoned(c)) {
+  if (signal_family >= 0 && __syncthreads_and(poisoned(c) ? 0 : 1)) {
     if (threadIdx.x == 0) fence_sys();
     __syncthreads();
     for (int r = threadIdx.x; r < c.R; r += blockDim.x)

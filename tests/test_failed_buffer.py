@@ -1,5 +1,5 @@
-"""Prefetch on a Buffer that has failed, or fails while the kernel starts: slots keep what they held or get their expert, nothing
-else is written, and after ``check_status`` the Buffer prefetches as before."""
+"""Kernels of a Buffer that has failed, or fails while they start.  Of a prefetch, slots keep what they held or get their
+expert, nothing else is written, and after ``check_status`` the Buffer prefetches as before."""
 
 import dataclasses
 import re
@@ -17,18 +17,29 @@ from moonep_b200.ops.grouped_gemm import grouped_gemm
 from moonep_b200.parallel.world import LocalWorld
 
 
-def test_threads_that_share_something_leave_a_failed_kernel_together():
-    """The status word can change between two threads' looks at it.  A kernel in which every thread leaves by its own look must
-    not have threads that wait for others, or for what others write to shared memory."""
-    alone = re.compile(r"if \((?:poisoned\(c\)|failed != 0)\) return;")
-    shared = re.compile(r"__syncthreads|__shared__|bar\.sync|\bs_[a-z]")
+def _block(text, start):
+    """From ``start`` to the end of the braces that are open there."""
+    depth = 1
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start:i]
+    raise AssertionError("braces")
+
+
+def test_threads_that_share_something_look_at_the_status_together():
+    """The status word can change between two threads' looks at it.  Where every thread goes by its own look, none may wait for
+    another in a barrier, or for what others write to shared memory."""
+    leaves = re.compile(r"if \((?:poisoned\(c\)|failed != 0)\) return;|= !poisoned\(c\);")  # what follows in the function counts
+    enters = re.compile(r"\bif \(.*!poisoned\(c\)\) \{")  # what is in the block counts
+    shared = re.compile(r"__syncthreads|__shared__|bar\.sync")
     seen = 0
     for path in sorted(CSRC.glob("*.cu")):
         text = path.read_text()
-        for m in alone.finditer(text):
-            seen += 1
-            rest = text[m.end() : text.index("\n}\n", m.end())]
-            assert not shared.search(rest), f"{path.name}: threads leave one by one before they share something"
+        parts = [text[m.end() : text.index("\n}\n", m.end())] for m in leaves.finditer(text)]
+        parts += [_block(text, m.end()) for m in enters.finditer(text)]
+        seen += len(parts)
+        assert not any(shared.search(part) for part in parts), f"{path.name}: threads share something, but each by its own look"
     assert seen
 
 
